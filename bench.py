@@ -1267,6 +1267,8 @@ def run_ours(args, ws, rank, local):
     name_a = "k_cg_a_fresh (q = A p_new, p.q)" if (prec == H.PREC_MIXED and pc != H.PRECOND_AMG) else \
         "k_cg_a (q = A z + beta q, p update, p.q)"
     name_b = ("k_cg_b_mg + multigrid V-cycle + k_cg_c" if pc == H.PRECOND_AMG else "k_cg_b (x, r, z update, r.z, r.r)")
+    if avg("cg_a_ms") > 0 and avg("cg_b_ms") == 0:  # both phases of an iteration in one resident launch
+        name_a = "k_cg_resident (one iteration of a launch that makes many)"
     kern = {
         name_a: (avg("cg_a_ms"), lib_a if lib_a > 0 else bytes_a, it_mean),
         name_b: (avg("cg_b_ms"), lib_b if lib_b > 0 else bytes_b, it_mean),

@@ -59,6 +59,7 @@ hdg_system::~hdg_system() {
   if (amg) destroy_amg(amg);
   for (auto* e : ev_cg_a) delete e;
   for (auto* e : ev_cg_b) delete e;
+  for (auto* e : ev_res) delete e;
   for (auto* e : ev_cheb0) delete e;
   for (auto* e : ev_l1) delete e;
 }
@@ -909,6 +910,15 @@ int hdg_system_timings(hdg_system* s, hdg_timings* out) {
       out->cg_b_ms = tb / out->cg_samples;
       out->cg_a_bytes = s->prof_a_bytes / out->cg_samples;
       out->cg_b_bytes = s->prof_b_bytes / out->cg_samples;
+    }
+    if (s->prof_res_iters > 0) {  // resident iteration: one launch makes many, both phases in it
+      double tr = 0;
+      for (auto* e : s->ev_res) tr += e->ms();
+      out->cg_samples = (int)s->prof_res_iters;
+      out->cg_a_ms = tr / (double)s->prof_res_iters;
+      out->cg_b_ms = 0;
+      out->cg_a_bytes = s->prof_all_bytes / (double)s->prof_res_iters;
+      out->cg_b_bytes = 0;
     }
     out->cg_iterations = s->cg_iterations;
     out->cg_bytes = s->prof_all_bytes;

@@ -6,7 +6,9 @@
 //   A: q = A p_new, p_new = z + beta p, pq = p_new.q
 //   B: alpha = rz/pq;  x += alpha p_new;  r -= alpha q;  z = D^-1 r;  rz, rr
 // In FP64, A uses q_{k+1} = A z_{k+1} + beta q_k so that p and q update in place in the same pass.
-// Reductions are deterministic per problem (seg_finish in hdg_device.cuh).  Every CUDA block
+// A system that holds one problem, preconditioned by Jacobi, runs many iterations per launch instead, with its state
+// resident on the chip (cg_resident.cu); what follows is then the initialisation, the true residuals and the host
+// loop.  Reductions are deterministic per problem (seg_finish in hdg_device.cuh).  Every CUDA block
 // belongs to one problem, so many problems share one launch and a converged problem's blocks
 // return at once.  CHUNK iterations are captured in a CUDA graph and replayed; the host reads the
 // per-problem status between replays, and drives several systems (degree bins of a batch) in one
@@ -26,6 +28,7 @@
 #include <cstring>
 #include <thread>
 
+#include "cg_resident.cuh"
 #include "hdg_device.cuh"
 
 namespace {
@@ -34,11 +37,13 @@ constexpr int CG_BLOCK = 256;
 // rows per SM that a large problem gets): 6 in FP32 (40 registers), 4 in FP64 (64 registers)
 template <typename T> constexpr int cg_min_blocks() { return sizeof(T) == sizeof(float) ? 6 : 4; }
 constexpr int SAMPLE_EVERY = 8;  // with profiling on, every 8th chunk runs un-graphed and timed
-constexpr int SC = 10;           // per problem: rz, rz_old, pq, rr, bb, tol2, alpha, beta, rr_true, -
+constexpr int SC = HDG_CG_SC;
 constexpr int ST = HDG_CG_ST;    // per problem: status, iterations, maxit, refine flag
+constexpr int RESIDENT_CHUNK = 512;  // iterations of one launch of the resident iteration
 constexpr double DELTA = 0.1;    // refine once the recursive residual fell by this factor
 // status: 0 running, 1 converged (recursive, FP64), 2 iteration cap, 3 breakdown (p'Ap <= 0),
-//         4 converged (true residual, mixed), 5 stopped (mixed: cap or stagnation)
+//         4 converged (true residual, mixed), 5 stopped (mixed: cap or stagnation),
+//         6 a barrier of the resident iteration gave up (CG_LOST)
 }  // namespace
 
 struct CgState {
@@ -48,6 +53,8 @@ struct CgState {
   DevBuf<double> r, z, p, q, dinv;
   DevBuf<float> rf, zf, pf, pf2, qf, dinvf, xh, xl;
   DevBuf<float> r32, z32;  // multigrid preconditioner input / output
+  DevBuf<float2> pairs;    // resident FP32 iteration: (z, p) of every row, two buffers
+  DevBuf<unsigned char> sync;  // resident iteration: barrier counter and partials
   cudaGraphExec_t graph64 = nullptr, graph32 = nullptr;
   int chunk64 = 0, chunk32 = 0;
   bool graph_mg = false;  // graph64 holds the multigrid iteration
@@ -67,25 +74,6 @@ struct CgState {
 void destroy_cg(CgState* c) { delete c; }
 
 namespace {
-
-template <typename T> struct CgArgs {
-  SegArgs g;
-  const int32_t* bcol5;
-  int nf;
-  const T* val;
-  const double* b;
-  const T* dinv;
-  double* x;
-  T* r;
-  T* z;
-  T* p;
-  T* q;
-  T* p2;
-  double* sc;
-  int32_t* st;
-  float* xh;  // FP32 iteration: steps since the last refinement as a float-float pair (hi, lo)
-  float* xl;
-};
 
 // (A v)_row over the block-ELL layout: 5 block slots, values slot-major and row-contiguous.
 template <int NT, typename T, typename V>
@@ -498,6 +486,7 @@ template <int NT> struct SolverNT : CgSolver {
   int nrow, nprob, chunk = 32;
   bool mixed = false;
   bool mg = false;  // multigrid preconditioner (FP64 iteration)
+  CgResident res;   // one problem with Jacobi whose state fits on the chip: chunks are single launches
   CgArgs<double> a64;
   CgArgs<float> a32;
   // Segment compaction: once most problems have finished, the launch grid is rebuilt from the
@@ -590,6 +579,9 @@ template <int NT> struct SolverNT : CgSolver {
     for (auto* e : s->ev_cg_b) delete e;
     s->ev_cg_a.clear();
     s->ev_cg_b.clear();
+    for (auto* e : s->ev_res) delete e;
+    s->ev_res.clear();
+    s->prof_res_iters = 0;
     s->prof_a_bytes = s->prof_b_bytes = s->prof_all_bytes = 0.0;
     for (auto* e : s->ev_cheb0) delete e;
     s->ev_cheb0.clear();
@@ -611,6 +603,14 @@ template <int NT> struct SolverNT : CgSolver {
     }
     HDG_CUDA(cudaMemcpyAsync(c->sc.p, c->h_sc, sizeof(double) * SC * nprob, cudaMemcpyHostToDevice, st));
     HDG_CUDA(cudaMemcpyAsync(c->st.p, c->h_st, sizeof(int32_t) * ST * nprob, cudaMemcpyHostToDevice, st));
+    res = CgResident{};
+    if (!mg && nprob == 1)
+      res = mixed ? cg_resident_plan<float>(NT, s->nf, s->ctx->device)
+                  : cg_resident_plan<double>(NT, s->nf, s->ctx->device);
+    if (res.kind != CgResident::NONE) {
+      c->sync.alloc(CG_SYNC_BYTES);
+      if (mixed) c->pairs.alloc(2 * (size_t)nrow);
+    }
     if (mg) {
       c->r.alloc(nrow); c->z.alloc(nrow); c->p.alloc(nrow); c->q.alloc(nrow); c->dinv.alloc(nrow);
       c->r32.alloc(nrow); c->z32.alloc(nrow);
@@ -637,7 +637,7 @@ template <int NT> struct SolverNT : CgSolver {
       k_cg_init<NT, double><<<s->nseg, CG_BLOCK, 0, st>>>(a64);
       if (c->graph_mg && c->graph64) { cudaGraphExecDestroy(c->graph64); c->graph64 = nullptr; }
       c->graph_mg = false;
-      build_graph<double>(a64, &c->graph64, &c->chunk64);
+      if (res.kind == CgResident::NONE) build_graph<double>(a64, &c->graph64, &c->chunk64);
     } else {
       const int64_t nval = (int64_t)hdg_system::SLOTS * NT * nrow;
       s->d_valf.alloc((size_t)nval);
@@ -649,7 +649,7 @@ template <int NT> struct SolverNT : CgSolver {
       a32 = CgArgs<float>{seg(), s->d_bcol5.p, s->nf, s->d_valf.p, s->d_b.p, c->dinvf.p, s->d_x.p, c->rf.p, c->zf.p,
                           c->pf.p, c->qf.p, c->pf2.p, c->sc.p, c->st.p, c->xh.p, c->xl.p};
       k_cg_init<NT, float><<<s->nseg, CG_BLOCK, 0, st>>>(a32);
-      build_graph<float>(a32, &c->graph32, &c->chunk32);
+      if (res.kind == CgResident::NONE) build_graph<float>(a32, &c->graph32, &c->chunk32);
       s->ctx->launches++;
     }
     HDG_CUDA(cudaGetLastError());
@@ -660,6 +660,18 @@ template <int NT> struct SolverNT : CgSolver {
   }
 
   template <typename T> void chunk_t(const CgArgs<T>& a, cudaGraphExec_t graph, int rep) {
+    if (res.kind != CgResident::NONE) {
+      // one launch per chunk; a chunk's end costs a host round trip (about 20 us), so it is long
+      EventPair* ep = s->ctx->profiling ? new EventPair() : nullptr;
+      if (ep) ep->start(st);
+      cg_resident_launch<T>(res, NT, a, c->pairs.p, c->sync.p, std::max(chunk, RESIDENT_CHUNK), s->ctx->device, st);
+      s->ctx->launches++;
+      if (ep) {
+        ep->stop(st);
+        s->ev_res.push_back(ep);
+      }
+      return;
+    }
     if (s->ctx->profiling && rep % SAMPLE_EVERY == SAMPLE_EVERY - 1) {
       sample_it0.resize(nprob);
       for (int P = 0; P < nprob; ++P) sample_it0[P] = c->h_st[ST * P + 1];
@@ -782,6 +794,7 @@ template <int NT> struct SolverNT : CgSolver {
     double rows_all = 0.0;
     for (int P = 0; P < nprob; ++P) {
       const int32_t now = c->h_st[ST * P + 1];
+      if (!s->ev_res.empty()) s->prof_res_iters += now - it_prev[P];
       rows_all += (double)(now - it_prev[P]) * (double)(s->h_prob_row0[P + 1] - s->h_prob_row0[P]);
       it_prev[P] = now;
     }
@@ -820,6 +833,7 @@ template <int NT> struct SolverNT : CgSolver {
     for (int P = 0; P < nprob; ++P) {
       int32_t* stp = c->h_st + ST * P;
       const double* scp = c->h_sc + SC * P;
+      if (stp[0] == CG_LOST) throw HdgError{HDG_ERR_CUDA, "a barrier of the resident CG iteration gave up"};
       if (c->rr_best[P] == 0.0) c->rr_best[P] = scp[4];
       stp[3] = 0;
       if (stp[0] == 3) {

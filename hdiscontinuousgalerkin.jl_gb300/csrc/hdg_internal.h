@@ -305,6 +305,8 @@ struct hdg_system {
   // profiling
   EventPair ev_element, ev_gather, ev_apply, ev_cg, ev_recover;
   std::vector<EventPair*> ev_cg_a, ev_cg_b;
+  std::vector<EventPair*> ev_res;  // each launch of the resident CG iteration, and the iterations they made
+  int64_t prof_res_iters = 0;
   // level-0 multigrid smoother sweeps of the sampled chunks, each timed on its own
   bool prof_cheb0 = false;
   // The multigrid V-cycle autotuner may time candidates when it has no cached choice for this

@@ -237,7 +237,8 @@ typedef struct {
   double gather_ms;    /* matrix + rhs gather of the last (re)assembly */
   double apply_ms;     /* apply! (meandiag, lift, zeroing) */
   double cg_ms;        /* whole CG loop of the last solve */
-  double cg_a_ms;      /* mean duration of the CG product kernel (q = A z + beta q), sampled */
+  double cg_a_ms;      /* mean duration of the CG product kernel (q = A z + beta q), sampled; where one launch makes
+                        * many iterations (one problem, Jacobi): a whole iteration, and cg_b_ms is 0 */
   double cg_b_ms;      /* mean duration of the CG update kernel (x, r, z), sampled */
   int cg_samples;      /* number of sampled iterations */
   int cg_iterations;   /* iterations of the last solve */
