@@ -33,7 +33,7 @@ struct ElemArgs {
   double* AB;
   double* KB;
   int* err;
-  int schur;  // 1: the Schur-complement path (invertible reference mass, kappa constant per cell)
+  int schur;  // 1: the Schur path (invertible reference mass, kappa constant per cell), 2: with one null function
   int he_tau; // 1: He carries tau
   RefLayout L;  // offsets of the packed reference tables (tables.cpp: ref_layout)
 };
@@ -241,213 +241,281 @@ __global__ void __launch_bounds__(EWARPS * 32) k_element_condense(ElemArgs a) {
   }
 }
 
-// Schur path with an LDL' factorisation: invertible reference mass and kappa constant on each
-// cell (p = 1, and p = 3, 4 with exact-enough rules).  Then Ae = (det J / kappa) diag(M, M) is
-// inverted in closed form, and with kf = kappa / det J the condensation needs only the nw x nw
-// Schur complement
+// Schur path with an LDL' factorisation: a reference mass matrix M that is invertible, or has one null function z (p = 2
+// with the default rule), and kappa constant on each cell.  Then Ae = (det J / kappa) diag(M, M) is inverted in closed form,
+// and with kf = kappa / det J the condensation needs only the nw x nw Schur complement
 //   S  = C + kf sum_c B_c' M^-1 B_c = C + kf (a00 Q00 + a01 (Q01 + Q01') + a11 Q11)    (SPD)
 //   R' = [R'_f] with R'_f = tau |e_f| F_{f,o} + kf (b0_f DMF0_{f,o} + b1_f DMF1_{f,o}), and be,
-// where B_c = adl0_c D0 + adl1_c D1, b_l f = adj(J) row l . wn_f.  Writing S = U' D U (U unit
+// where B_c = adl0_c D0 + adl1_c D1, b_l f = adj(J) row l . wn_f.  A null function adds an unknown a_c per component of q,
+// q_c = kf M^+ (B_c u - Ee_c u_hat) + z a_c, and the rows z' (B_c u - Ee_c u_hat) = 0: S becomes [S Z; Z' 0] with
+// Z_c = B_c' z and R' gets the rows G_c = wn_f,c z' F_{f,o}; its last two pivots are negative.  Writing S = U' D U (U unit
 // upper triangular) and R~ = U'^-1 [R' | be], the condensed blocks are
 //   Ate_{fi,gj} = (R~' D^-1 R~)_{fi,gj} - kf (wn_f . wn_g) (F_{f,o}' M^-1 F_{g,o'})_{ij} - [f = g] |e_f| He_ij
 //   bte_{fi}    = -(R~' D^-1 R~)_{fi,be}
 // (the same Ate = [Ee;Fe]' Me^-1 [-Ee;Fe] - He and bte = -[Ee;Fe]' Me^-1 [0;be] that the full
 // elimination of examples/poisson2D_HDG.jl:155-174 forms, reordered), symmetric by construction, so
-// only the upper triangle is computed.  The u rows of [K_e | b_e], X_u = U^-1 D^-1 R~, are stored;
+// every pair of columns is formed once.  The u rows of [K_e | b_e], X_u = U^-1 D^-1 R~ (and a_c), are stored;
 // the q rows follow linearly from them, q = kf (adl0 M^-1 D0 u + adl1 M^-1 D1 u - sum_f wn_f M^-1
-// F_f u_hat_f), and are formed at recovery (k_recover_u) or when the blocks are exported
-// (k_expand_ke).  Per cell at p = 4 this is about 8k FP64 FMAs instead of the 20k of the pivoted
-// elimination of S with the q rows, and 3.8 KB written instead of 7.7 KB.  The kernel is bound by
-// the FP64 pipe, which counts warp instructions: the pivots need no square root, their
-// reciprocals come from recip_newton, and the bump source's -1/(2 s^2) is formed on the host.
+// F_f u_hat_f) + z a, and are formed at recovery (k_recover_u) or when the blocks are exported (k_expand_ke).
+//
+// The kernel is bound by the FP64 pipe, which issues a warp instruction in 16 clocks however few of its lanes are
+// active.  So a warp takes CPW = 32 / (m + 1) cells at once, a lane per right-hand-side column: 2 cells of 16 columns at
+// p = 4, 2 of 13, 3 of 10, 4 of 7 at p = 3, 2, 1.  The lane keeps its column, and the column of S of the same number, in
+// registers; a row of S is broadcast through shared memory when it is final.  The pairs of columns are taken
+// cyclically (a lane its own column against the one d further on, d = 0..(m+1)/2), the source's terms are spread over
+// (point, part) pairs, and the entries of S over all lanes.  Measured on 65522 cells with eight bumps as the source, one
+// cell per warp before / here: p = 4 4.31 / 2.27 ms, p = 3 2.30 / 1.05, p = 2 (then by the pivoted elimination of the
+// 18 x 18 system) 2.70 / 0.59, p = 1 1.16 / 0.22.
 // v[f] for a face index f known only at run time, without indexing a local array (which would
 // place the array in local memory)
 __device__ __forceinline__ double sel3(int f, double v0, double v1, double v2) {
   return f == 0 ? v0 : (f == 1 ? v1 : v2);
 }
 
-template <int P, int EWARPS>
-__global__ void __launch_bounds__(EWARPS * 32) k_element_chol(ElemArgs a) {
+template <int P, int NZ> struct SchurDims {
   using D = Dims<P>;
-  constexpr int NW = D::NW, NT = D::NT, M = D::M;
-  constexpr int RC = NW + M + 1;  // columns of [S | R' | be]
-  constexpr int LDW = RC | 1;     // odd row stride: conflict-free FP64 column reads
+  static constexpr int NW = D::NW, NT = D::NT, M = D::M;
+  static constexpr int NA = NW + 2 * NZ;          // rows of [S Z; Z' 0]
+  static constexpr int COLS = M + 1;              // right-hand sides: R' and be
+  static constexpr int CPW = 32 / COLS;           // cells per warp
+  static constexpr int TRI = NW * (NW + 1) / 2;   // S, upper triangle by columns
+  static constexpr int PARTS = P == 2 || P == 3 ? 4 : 2;  // lanes per point in the source (the fuller last round)
+  static constexpr int GEO = 16;                  // per cell: tau |e_f|, kf a_lm; kf wn_f . wn_g
+  static constexpr int W = NA * NA, Y = NA * COLS > TRI ? NA * COLS : TRI;
+  static_assert(CPW >= 1 && NA <= COLS, "a lane per column of S");
+  __host__ __device__ static constexpr int tables(int nq) {  // doubles staged per CTA
+    return 6 * TRI + 18 * NW * NT + NT * NT + NW * nq + 2 * nq + 36 * NT * NT + NZ * (2 * NW + 6 * NT);
+  }
+  __host__ __device__ static constexpr int per_warp(int nq) { return CPW * (W + Y + GEO + NW + nq); }
+};
+
+template <int P, int NZ>
+__global__ void __launch_bounds__(256) k_element_schur(ElemArgs a) {
+  using SD = SchurDims<P, NZ>;
+  constexpr int NW = SD::NW, NT = SD::NT, M = SD::M, NA = SD::NA, COLS = SD::COLS, CPW = SD::CPW, TRI = SD::TRI;
+  constexpr int PARTS = SD::PARTS, GEO = SD::GEO;
   extern __shared__ double smem[];
   const int nq = a.nq;
   const RefLayout G = a.L;
-  // staged tables: [C .. Q] (C, F, H, N w, points), [Q00 Q01 Q11], [DMF .. PFF]
-  const int n1 = G.Q + 2 * nq - G.C, n2 = 3 * NW * NW, n3 = G.PFF + 36 * NT * NT - G.SDMF;
-  for (int i = threadIdx.x; i < n1; i += blockDim.x) smem[i] = a.ref[G.C + i];
-  for (int i = threadIdx.x; i < n2; i += blockDim.x) smem[n1 + i] = a.ref[G.SQ00 + i];
-  for (int i = threadIdx.x; i < n3; i += blockDim.x) smem[n1 + n2 + i] = a.ref[G.SDMF + i];
-  const double* Cf = smem;                       // [3][NW][NW]
-  const double* Ff = smem + (G.F - G.C);         // [6][NW][NT]   (f, o)
-  const double* Hh = smem + (G.H - G.C);         // [NT][NT]
-  const double* Nw = smem + (G.NW - G.C);        // [NW][nq]      N times the weights
-  const double* Qp = smem + (G.Q - G.C);         // [nq][2]
-  const double* SQ = smem + n1;                  // [3][NW][NW]   Q00, Q01, Q11
-  const double* DMF = smem + n1 + n2;            // [2][6][NW][NT]
-  const double* PFF = DMF + 12 * NW * NT;        // [6][6][NT][NT]
+  // ---- tables ------------------------------------------------------------------------------------------------
+  double* tS = smem;                    // [6][TRI]: C_f, Q00, Q01 + Q01', Q11
+  double* tF = tS + 6 * TRI;            // [6][NW][NT]  (f, o)
+  double* tD = tF + 6 * NW * NT;        // [2][6][NW][NT]  DMF
+  double* tH = tD + 12 * NW * NT;       // [NT][NT]
+  double* tN = tH + NT * NT;            // [NW][nq]  N times the weights
+  double* tQ = tN + NW * nq;            // [nq][2]
+  double* tP = tQ + 2 * nq;             // [6][6][NT][NT]  PFF
+  double* tZ = tP + 36 * NT * NT;       // [2][NW] D_l' z, [6][NT] F' z
+  for (int t = threadIdx.x; t < 6 * TRI; t += blockDim.x) {
+    const int k = t / TRI, e = t - k * TRI;
+    int j = 0;
+    while ((j + 1) * (j + 2) / 2 <= e) ++j;
+    const int i = e - j * (j + 1) / 2;  // i <= j
+    double v;
+    if (k < 3) v = a.ref[G.C + (k * NW + i) * NW + j];
+    else if (k == 3) v = a.ref[G.SQ00 + i * NW + j];
+    else if (k == 4) v = a.ref[G.SQ01 + i * NW + j] + a.ref[G.SQ01 + j * NW + i];
+    else v = a.ref[G.SQ11 + i * NW + j];
+    tS[t] = v;
+  }
+  for (int t = threadIdx.x; t < 6 * NW * NT; t += blockDim.x) tF[t] = a.ref[G.F + t];
+  for (int t = threadIdx.x; t < 12 * NW * NT; t += blockDim.x) tD[t] = a.ref[G.SDMF + t];
+  for (int t = threadIdx.x; t < NT * NT; t += blockDim.x) tH[t] = a.ref[G.H + t];
+  for (int t = threadIdx.x; t < NW * nq; t += blockDim.x) tN[t] = a.ref[G.NW + t];
+  for (int t = threadIdx.x; t < 2 * nq; t += blockDim.x) tQ[t] = a.ref[G.Q + t];
+  for (int t = threadIdx.x; t < 36 * NT * NT; t += blockDim.x) tP[t] = a.ref[G.PFF + t];
+  if constexpr (NZ > 0) {
+    for (int t = threadIdx.x; t < 2 * NW; t += blockDim.x) tZ[t] = a.ref[G.ZD + t];
+    for (int t = threadIdx.x; t < 6 * NT; t += blockDim.x) tZ[2 * NW + t] = a.ref[G.ZF + t];
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wstride = ((NW * LDW + NW * (M + 1) + nq + 2 * NW) + 1) & ~1;
-  double* W = smem + ((n1 + n2 + n3 + 1) & ~1) + warp * wstride;
-  double* Y = W + NW * LDW;   // D^-1 R~ (NW x (M+1))
-  double* sq = Y + NW * (M + 1);  // f at the quadrature points
-  double* be = sq + nq;
-  double* rinv = be + NW;     // 1 / d_k
+  double* base = smem + SD::tables(nq) + warp * SD::per_warp(nq);
+  const bool on_lane = lane < CPW * COLS;
+  const int cl = on_lane ? lane / COLS : CPW - 1;       // cell of the warp's tile
+  const int col = on_lane ? lane - cl * COLS : COLS - 1; // the idle lanes repeat the last column
+  double* Wc = base + cl * SD::W;                        // final rows of [S Z; Z' 0]
+  double* Yc = base + CPW * SD::W + cl * SD::Y;          // D^-1 R~ (NA x COLS); before it, S by columns
+  double* geo0 = base + CPW * (SD::W + SD::Y);
+  double* geo = geo0 + cl * GEO;
+  double* be0 = geo0 + CPW * GEO;
+  double* be = be0 + cl * NW;
+  double* sq0 = be0 + CPW * NW;
+  const int f = col < M ? col / NT : 0, fj = col < M ? col - f * NT : 0;
+  const int nwarps = blockDim.x >> 5;
   __syncthreads();
 
-  for (int e = blockIdx.x * EWARPS + warp; e < a.nc; e += gridDim.x * EWARPS) {
+  for (int e0 = (blockIdx.x * nwarps + warp) * CPW; e0 < a.nc; e0 += gridDim.x * nwarps * CPW) {
+    const bool mine = on_lane && e0 + cl < a.nc;
+    const int e = min(e0 + cl, a.nc - 1);
     // ---- geometry (reinit!, src/ScalarFunctionSpaces.jl:101-132) -------------------------
-    int nid = (lane < 3) ? a.cells[3 * e + lane] : 0;
-    double px = 0.0, py = 0.0;
-    if (lane < 3) {
-      px = a.xy[2 * nid];
-      py = a.xy[2 * nid + 1];
-    }
-    const double x1 = __shfl_sync(0xffffffffu, px, 0), y1 = __shfl_sync(0xffffffffu, py, 0);
-    const double x2 = __shfl_sync(0xffffffffu, px, 1), y2 = __shfl_sync(0xffffffffu, py, 1);
-    const double x3 = __shfl_sync(0xffffffffu, px, 2), y3 = __shfl_sync(0xffffffffu, py, 2);
-    const double J00 = x2 - x1, J01 = x3 - x1, J10 = y2 - y1, J11 = y3 - y1;
+    const int n0 = a.cells[3 * e], n1 = a.cells[3 * e + 1], n2 = a.cells[3 * e + 2];
+    const double x1 = a.xy[2 * n0], y1 = a.xy[2 * n0 + 1];
+    const double J00 = a.xy[2 * n1] - x1, J01 = a.xy[2 * n2] - x1;
+    const double J10 = a.xy[2 * n1 + 1] - y1, J11 = a.xy[2 * n2 + 1] - y1;
     const double detJ = J00 * J11 - J01 * J10;
-    if (!(detJ > 0.0) && lane == 0) atomicOr(a.err, 1);
+    if (!(detJ > 0.0) && mine && col == 0) atomicOr(a.err, 1);
     const double ad00 = J11, ad01 = -J01, ad10 = -J10, ad11 = J00;  // adj(J) = det J J^-1
-    const double wn[3][2] = {{-(J10 - J11), J00 - J01}, {-J11, J01}, {J10, -J00}};  // src/shapes.jl:80-87
-    double el[3];
-#pragma unroll
-    for (int f = 0; f < 3; ++f) el[f] = sqrt(wn[f][0] * wn[f][0] + wn[f][1] * wn[f][1]);
+    const double wx0 = J11 - J10, wy0 = J00 - J01;                  // weighted normals, src/shapes.jl:80-87
+    const double wx = sel3(f, wx0, -J11, J10), wy = sel3(f, wy0, J01, -J00);  // of this lane's face
+    const double el = sqrt(wx * wx + wy * wy);
     const unsigned ob = a.orient[e];
+    const int fo = 2 * f + ((ob >> f) & 1);
     const int prob = a.co.cell_prob[e];
     const double tau = a.co.tau[prob];
-    const double hs = a.he_tau ? tau : 1.0;
-    const int fkind = a.co.fkind[prob];
-    const double* fprm = a.co.fprep + a.co.foff[prob];
-    const double kinv = (a.kappa_mode == 1) ? 1.0 / a.kcell[e] : 1.0;
-    const double kf = 1.0 / (kinv * detJ);
+    const double kf = (a.kappa_mode == 1) ? a.kcell[e] / detJ : 1.0 / detJ;
+    if (on_lane) {  // the cell's coefficients: the columns of a face know its edge length
+      if (col < M && fj == 0) geo[f] = tau * el;
+      if (col == COLS - 1) {
+        geo[3] = kf * (ad00 * ad00 + ad01 * ad01);
+        geo[4] = kf * (ad00 * ad10 + ad01 * ad11);
+        geo[5] = kf * (ad10 * ad10 + ad11 * ad11);
+      }
+      if (col < 6) {  // kf wn_g . wn_h for (g, h) = (0,0), (0,1), (0,2), (1,1), (1,2), (2,2)
+        const int g = col < 3 ? 0 : (col < 5 ? 1 : 2), h = col < 3 ? col : (col < 5 ? col - 2 : 2);
+        geo[6 + col] = kf * (sel3(g, wx0, -J11, J10) * sel3(h, wx0, -J11, J10) +
+                             sel3(g, wy0, J01, -J00) * sel3(h, wy0, J01, -J00));
+      }
+      if (col == 6) {
+        geo[12] = x1;
+        geo[13] = y1;
+      }
+    }
     // ---- source at the volume points, be ----------------------------------------------------
-    for (int q = lane; q < nq; q += 32) {
-      const double xi = Qp[2 * q], eta = Qp[2 * q + 1];
-      const double xq = (1.0 - xi - eta) * x1 + xi * x2 + eta * x3;
-      const double yq = (1.0 - xi - eta) * y1 + xi * y2 + eta * y3;
-      sq[q] = eval_source_prepared(fkind, fprm, xq, yq);
+    for (int t0 = 0; t0 < CPW * nq * PARTS; t0 += 32) {
+      const int t = t0 + lane;
+      const int pt = t / PARTS, part = t - pt * PARTS;
+      const int c = min(pt / nq, CPW - 1), q = pt < CPW * nq ? pt - c * nq : 0;
+      // this point's cell, from the lanes that hold its columns
+      const int src = c * COLS;
+      const double X = __shfl_sync(0xffffffffu, x1, src), Yv = __shfl_sync(0xffffffffu, y1, src);
+      const double A00 = __shfl_sync(0xffffffffu, J00, src), A01 = __shfl_sync(0xffffffffu, J01, src);
+      const double A10 = __shfl_sync(0xffffffffu, J10, src), A11 = __shfl_sync(0xffffffffu, J11, src);
+      const int pr = __shfl_sync(0xffffffffu, prob, src);
+      const double xi = tQ[2 * q], eta = tQ[2 * q + 1];
+      double v = 0.0;
+      if (pt < CPW * nq)
+        v = eval_source_part(a.co.fkind[pr], a.co.fprep + a.co.foff[pr], fma(A01, eta, fma(A00, xi, X)),
+                             fma(A11, eta, fma(A10, xi, Yv)), part, PARTS);
+#pragma unroll
+      for (int o = PARTS / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (part == 0 && pt < CPW * nq) sq0[pt] = v;
     }
     __syncwarp();
-    for (int i = lane; i < NW; i += 32) {
+    if (col < NW && on_lane) {
       double t = 0.0;
-      for (int q = 0; q < nq; ++q) t += Nw[i * nq + q] * sq[q];
-      be[i] = t * detJ;
+      for (int q = 0; q < nq; ++q) t += tN[col * nq + q] * sq0[cl * nq + q];
+      be[col] = t * detJ;
+    }
+    // ---- S (upper triangle, by columns) over all lanes; the columns into registers ---------------
+    for (int t = lane; t < CPW * TRI; t += 32) {
+      const int c = t / TRI, k = t - c * TRI;
+      const double* g = geo0 + c * GEO;
+      base[CPW * SD::W + c * SD::Y + k] = g[0] * tS[k] + g[1] * tS[TRI + k] + g[2] * tS[2 * TRI + k] +
+                                          g[3] * tS[3 * TRI + k] + g[4] * tS[4 * TRI + k] + g[5] * tS[5 * TRI + k];
     }
     __syncwarp();
-    // ---- [S (upper triangle) | R' | be] ------------------------------------------------------
-    const double a00 = ad00 * ad00 + ad01 * ad01, a11 = ad10 * ad10 + ad11 * ad11, a01 = ad00 * ad10 + ad01 * ad11;
-    double b0f[3], b1f[3];
+    double s[NA], r[NA], ri[NA];
 #pragma unroll
-    for (int f = 0; f < 3; ++f) {
-      b0f[f] = ad00 * wn[f][0] + ad01 * wn[f][1];
-      b1f[f] = ad10 * wn[f][0] + ad11 * wn[f][1];
+    for (int i = 0; i < NA; ++i) s[i] = 0.0;
+    if (col < NW) {
+#pragma unroll
+      for (int i = 0; i < NW; ++i)
+        if (i <= col) s[i] = Yc[col * (col + 1) / 2 + i];
     }
-    for (int idx = lane; idx < NW * RC; idx += 32) {
-      const int ia = idx / RC, col = idx - ia * RC;
-      double v;
-      if (col < NW) {
-        if (col < ia) continue;  // lower triangle of S: never read
-        const int ib = col;
-        v = tau * (el[0] * Cf[(0 * NW + ia) * NW + ib] + el[1] * Cf[(1 * NW + ia) * NW + ib] +
-                   el[2] * Cf[(2 * NW + ia) * NW + ib]) +
-            kf * (a00 * SQ[ia * NW + ib] + a01 * (SQ[NW * NW + ia * NW + ib] + SQ[NW * NW + ib * NW + ia]) +
-                  a11 * SQ[2 * NW * NW + ia * NW + ib]);
-      } else if (col < NW + M) {
-        const int f = (col - NW) / NT, j = (col - NW) - f * NT;
-        const int fo = f * 2 + ((ob >> f) & 1);
-        v = tau * sel3(f, el[0], el[1], el[2]) * Ff[(fo * NW + ia) * NT + j] +
-            kf * (sel3(f, b0f[0], b0f[1], b0f[2]) * DMF[((0 * 6 + fo) * NW + ia) * NT + j] +
-                  sel3(f, b1f[0], b1f[1], b1f[2]) * DMF[((1 * 6 + fo) * NW + ia) * NT + j]);
-      } else {
-        v = be[ia];
+    if constexpr (NZ > 0) {  // Z_c = B_c' z
+      if (col >= NW && col < NA) {
+        const double z0 = col == NW ? ad00 : ad01, z1 = col == NW ? ad10 : ad11;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) s[i] = z0 * tZ[i] + z1 * tZ[NW + i];
       }
-      W[ia * LDW + col] = v;
     }
-    __syncwarp();
+    if (col < M) {
+      const double te = tau * el, b0 = kf * (ad00 * wx + ad01 * wy), b1 = kf * (ad10 * wx + ad11 * wy);
+      const double *pF = tF + fo * NW * NT + fj, *p0 = tD + fo * NW * NT + fj, *p1 = p0 + 6 * NW * NT;
+#pragma unroll
+      for (int i = 0; i < NW; ++i) r[i] = te * pF[i * NT] + b0 * p0[i * NT] + b1 * p1[i * NT];
+      if constexpr (NZ > 0) {
+        r[NW] = wx * tZ[2 * NW + fo * NT + fj];
+        r[NW + 1] = wy * tZ[2 * NW + fo * NT + fj];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NA; ++i) r[i] = i < NW ? be[i] : 0.0;
+    }
+    __syncwarp();  // S has been read: its place becomes Y
     // ---- S = U' D U (LDL', no square roots), carrying the right-hand sides ---------------------
-    // Elimination without pivoting (S is SPD): after step k, row k holds d_k and d_k U_k., and the
-    // right-hand sides R~ = (D U)'^-1 ... = L^-1 [R' | be]; Y = D^-1 R~ (row k scaled when it is
-    // final).  Lane l owns column j = k+1+l (RC - k - 1 <= 31 columns: one pass).
-    static_assert(RC <= 32, "one lane per column of [S | R' | be]");
-    for (int k = 0; k < NW; ++k) {
-      const double d = W[k * LDW + k];
-      if (!(d > 0.0) && lane == 0) atomicOr(a.err, 2);  // not positive definite (LAPACK PosDefException)
-      const double r = recip_newton(d);
-      const int j = k + 1 + lane;
-      if (lane == 0) rinv[k] = r;
-      if (j < RC) {
-        const double t = W[k * LDW + j] * r;
-        if (j >= NW) Y[k * (M + 1) + (j - NW)] = t;
-#pragma unroll 4
-        for (int i = k + 1; i < NW; ++i)
-          if (j >= i) W[i * LDW + j] -= W[k * LDW + i] * t;
-      }
-      __syncwarp();
-    }
-    // ---- [Ate | bte] from Z'Z (upper triangle and the be column), then the face-face term and He
-    double* AB = a.AB + (size_t)e * M * (M + 1);
-    constexpr int NPAIR = M * (M + 1) / 2 + M;
-    for (int t = lane; t < NPAIR; t += 32) {
-      int r = 0, rem = t;
-      while (rem >= M - r + 1) {  // row r holds columns r..M-1 and the be column
-        rem -= M - r + 1;
-        ++r;
-      }
-      const int c = (rem == M - r) ? M : r + rem;
-      double dot = 0.0;  // (R~' D^-1 R~)_rc = (R' S^-1 R')_rc
 #pragma unroll
-      for (int ia = 0; ia < NW; ++ia) dot += Y[ia * (M + 1) + r] * W[ia * LDW + NW + c];
-      if (c == M) {
-        AB[r * (M + 1) + M] = -dot;
-      } else {
-        const int f = r / NT, i = r - f * NT, g = c / NT, j = c - g * NT;
-        const int fo = f * 2 + ((ob >> f) & 1), go = g * 2 + ((ob >> g) & 1);
-        const double wfx = sel3(f, wn[0][0], wn[1][0], wn[2][0]), wfy = sel3(f, wn[0][1], wn[1][1], wn[2][1]);
-        const double wgx = sel3(g, wn[0][0], wn[1][0], wn[2][0]), wgy = sel3(g, wn[0][1], wn[1][1], wn[2][1]);
-        double v = dot - kf * (wfx * wgx + wfy * wgy) * PFF[((fo * 6 + go) * NT + i) * NT + j];
-        if (f == g) v -= hs * sel3(f, el[0], el[1], el[2]) * Hh[i * NT + j];
-        AB[r * (M + 1) + c] = v;
-        if (c != r) AB[c * (M + 1) + r] = v;
+    for (int k = 0; k < NA; ++k) {
+      if (on_lane && col >= k && col < NA) Wc[k * NA + col] = s[k];
+      __syncwarp();
+      const double d = Wc[k * NA + k];
+      const bool fits = k < NW ? d > 0.0 : d < 0.0;
+      if (!fits && mine && col == 0) atomicOr(a.err, 2);  // not definite as it must be (LAPACK PosDefException)
+      const double rk = recip_cubic(d);
+      ri[k] = rk;
+      const double ts = s[k] * rk, tr = r[k] * rk;
+      if (on_lane) Yc[k * COLS + col] = tr;
+#pragma unroll
+      for (int i = k + 1; i < NA; ++i) {
+        const double w = Wc[k * NA + i];
+        s[i] -= w * ts;
+        r[i] -= w * tr;
       }
     }
     __syncwarp();
-    // ---- X_u = U^-1 Y: lane j <= m owns column j; the back substitution runs in its registers,
-    // and each row of X_u goes out as one coalesced store of m+1 values --------------------------
-    if (lane <= M) {
-      double x[NW];
+    // ---- [Ate | bte]: R~' D^-1 R~ by pairs of columns, then the face-face term and He -------------
+    double* AB = a.AB + (size_t)e * M * COLS;
+    const double* Hh = tH + fj * NT;
+    const double he = (a.he_tau ? tau : 1.0) * el;
+#pragma unroll 1
+    for (int d = 0; d <= COLS / 2; ++d) {
+      int o = col + d;
+      if (o >= COLS) o -= COLS;
+      double dot = 0.0;
 #pragma unroll
-      for (int k = NW - 1; k >= 0; --k) {
-        double t = 0.0;
-#pragma unroll
-        for (int i = k + 1; i < NW; ++i) t += W[k * LDW + i] * x[i];
-        x[k] = Y[k * (M + 1) + lane] - rinv[k] * t;
+      for (int k = 0; k < NA; ++k) dot += r[k] * Yc[k * COLS + o];
+      const bool twice = 2 * d == COLS && col >= COLS / 2;  // that pair is the other lane's
+      if (mine && !twice && !(col == M && o == M)) {
+        if (col == M || o == M) {
+          AB[(col == M ? o : col) * COLS + M] = -dot;
+        } else {
+          const int g = o / NT, gj = o - g * NT, go = 2 * g + ((ob >> g) & 1);
+          const int lo = min(f, g), hi = max(f, g);
+          double v = dot - geo[6 + lo + hi + (lo > 0 ? 1 : 0)] * tP[((fo * 6 + go) * NT + fj) * NT + gj];
+          if (f == g) v -= he * Hh[gj];
+          AB[col * COLS + o] = v;
+          if (d) AB[o * COLS + col] = v;
+        }
       }
-      double* KB = a.KB + (size_t)e * NW * (M + 1);
+    }
+    // ---- X_u = U^-1 Y in the lane's registers; a row goes out as m+1 consecutive values -----------
+    double* KB = a.KB + (size_t)e * NA * COLS + col;
 #pragma unroll
-      for (int ia = 0; ia < NW; ++ia) KB[ia * (M + 1) + lane] = x[ia];
+    for (int k = NA - 1; k >= 0; --k) {
+      double t = 0.0;
+#pragma unroll
+      for (int i = k + 1; i < NA; ++i) t += Wc[k * NA + i] * r[i];
+      r[k] = Yc[k * COLS + col] - ri[k] * t;  // R~ is not needed below row k + 1 any more
+      if (mine) KB[k * COLS] = r[k];
     }
     __syncwarp();
   }
 }
 
-// The q rows of [K_e | b_e] from the stored u rows (the Cholesky-Schur path stores X_u only):
+// The q rows of [K_e | b_e] from the stored u rows (the Schur path stores X_u only, and a_c below it):
 // X_q,c = kf (adl0_c M^-1 D0 X_u + adl1_c M^-1 D1 X_u - [j < m] wn_f,c M^-1 F_{f,o}), one thread per
 // entry of the full n x (m+1) block.  Used when the blocks are exported, not on the solve path.
-template <int P>
+template <int P, int NZ>
 __global__ void k_expand_ke(ElemArgs a, const double* __restrict__ KBu, double* __restrict__ KB) {
   using D = Dims<P>;
-  constexpr int NW = D::NW, NT = D::NT, NV = D::NV, N = D::N, M = D::M;
+  constexpr int NW = D::NW, NT = D::NT, NV = D::NV, N = D::N, M = D::M, NA = NW + 2 * NZ;
   const RefLayout G = a.L;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= (int64_t)a.nc * N * (M + 1)) return;
   const int e = (int)(t / (N * (M + 1)));
   const int rj = (int)(t - (int64_t)e * N * (M + 1));
   const int r = rj / (M + 1), j = rj - r * (M + 1);
-  const double* Xu = KBu + (size_t)e * NW * (M + 1);
+  const double* Xu = KBu + (size_t)e * NA * (M + 1);
   if (r >= NV) {
     KB[t] = Xu[(r - NV) * (M + 1) + j];
     return;
@@ -473,16 +541,7 @@ __global__ void k_expand_ke(ElemArgs a, const double* __restrict__ KBu, double* 
     const int fo = f * 2 + ((a.orient[e] >> f) & 1);
     v -= wn[f][c] * a.ref[G.SMF + (fo * NW + ia) * NT + jj];
   }
-  KB[t] = kf * v;
-}
-
-template <int P, int EWARPS> size_t smem_bytes_chol(const ElemArgs& a) {
-  using D = Dims<P>;
-  constexpr int LDW = (D::NW + D::M + 1) | 1;
-  const RefLayout& G = a.L;
-  const int tab = (G.Q + 2 * a.nq - G.C) + 3 * D::NW * D::NW + (G.PFF + 36 * D::NT * D::NT - G.SDMF);
-  const int wstride = ((D::NW * LDW + D::NW * (D::M + 1) + a.nq + 2 * D::NW) + 1) & ~1;
-  return (size_t)(((tab + 1) & ~1) + EWARPS * wstride) * sizeof(double);
+  KB[t] = kf * v + (NZ ? a.ref[G.ZV + ia] * Xu[(NW + c) * (M + 1) + j] : 0.0);
 }
 
 template <int P, int EWARPS> size_t smem_bytes_lu(const ElemArgs& a) {
@@ -493,58 +552,55 @@ template <int P, int EWARPS> size_t smem_bytes_lu(const ElemArgs& a) {
 
 constexpr size_t ELEM_SMEM_MAX = 200 * 1024;
 
-// Launches one path's kernel with EWARPS warps per CTA and a grid of `oversub` x the resident CTAs
+int sm_count(int device) {
+  int n = 152;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+  return n;
+}
+
+// Launches one path's kernel with `warps` warps per CTA and a grid of `oversub` x the resident CTAs
 // (a grid-stride loop covers the rest).  Returns false when the configuration does not fit.
-template <int P, int EWARPS, bool CHOL>
-bool launch_pw(hdg_system* s, cudaStream_t st, const ElemArgs& a, int oversub) {
-  void (*kern)(ElemArgs);
-  size_t smem;
-  if constexpr (CHOL) {
-    kern = k_element_chol<P, EWARPS>;
-    smem = smem_bytes_chol<P, EWARPS>(a);
-  } else {
-    kern = k_element_condense<P, EWARPS>;
-    smem = smem_bytes_lu<P, EWARPS>(a);
-  }
+template <class K>
+bool launch_kernel(hdg_system* s, cudaStream_t st, const ElemArgs& a, K kern, int warps, int cells_per_warp, size_t smem,
+                   int oversub) {
   if (smem > ELEM_SMEM_MAX) return false;
-  static bool attr_set = false;
-  if (!attr_set) {
-    HDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ELEM_SMEM_MAX));
-    attr_set = true;
-  }
-  int dev_sms = 152;
-  cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, s->ctx->device);
+  HDG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ELEM_SMEM_MAX));
   int blocks_per_sm = 0;
-  HDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, EWARPS * 32, smem));
+  HDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, kern, warps * 32, smem));
   if (blocks_per_sm < 1) return false;
-  const long need = (a.nc + EWARPS - 1) / EWARPS;
-  long grid = std::min<long>(need, (long)dev_sms * blocks_per_sm * oversub);
+  const long per = (long)warps * cells_per_warp, need = (a.nc + per - 1) / per;
+  long grid = std::min<long>(need, (long)sm_count(s->ctx->device) * blocks_per_sm * oversub);
   if (grid < 1) grid = 1;
-  kern<<<(unsigned)grid, EWARPS * 32, smem, st>>>(a);
+  kern<<<(unsigned)grid, warps * 32, smem, st>>>(a);
   HDG_CUDA(cudaGetLastError());
   s->ctx->launches++;
   return true;
 }
 
-template <int P, bool CHOL>
-bool launch_cfg_path(hdg_system* s, cudaStream_t st, const ElemArgs& a, int warps, int oversub) {
-  switch (warps) {
-    case 1: return launch_pw<P, 1, CHOL>(s, st, a, oversub);
-    case 2: return launch_pw<P, 2, CHOL>(s, st, a, oversub);
-    case 4: return launch_pw<P, 4, CHOL>(s, st, a, oversub);
-    case 8: return launch_pw<P, 8, CHOL>(s, st, a, oversub);
-    case 16: return launch_pw<P, 16, CHOL>(s, st, a, oversub);
-  }
-  return false;
+template <int P, int EWARPS> bool launch_lu(hdg_system* s, cudaStream_t st, const ElemArgs& a, int oversub) {
+  return launch_kernel(s, st, a, k_element_condense<P, EWARPS>, EWARPS, 1, smem_bytes_lu<P, EWARPS>(a), oversub);
 }
 
-// P = 2 never takes the Schur path with the default rule (Strang(3) leaves M^ of rank 5), so its
-// Cholesky-Schur kernels are not built; launch_element_condense keeps it on the full LU.
+template <int P, int NZ> bool launch_schur(hdg_system* s, cudaStream_t st, const ElemArgs& a, int warps, int oversub) {
+  using SD = SchurDims<P, NZ>;
+  if (warps > 8) return false;  // the kernel's launch bound
+  const size_t smem = sizeof(double) * ((size_t)SD::tables(a.nq) + (size_t)warps * SD::per_warp(a.nq));
+  return launch_kernel(s, st, a, k_element_schur<P, NZ>, warps, SD::CPW, smem, oversub);
+}
+
 template <int P> bool launch_cfg(hdg_system* s, cudaStream_t st, const ElemArgs& a, int warps, int oversub) {
-  if constexpr (P != 2) {
-    if (a.schur) return launch_cfg_path<P, true>(s, st, a, warps, oversub);
+  if (a.schur == 1) return launch_schur<P, 0>(s, st, a, warps, oversub);
+  if constexpr (P == 2) {
+    if (a.schur == 2) return launch_schur<P, 1>(s, st, a, warps, oversub);
   }
-  return launch_cfg_path<P, false>(s, st, a, warps, oversub);
+  switch (warps) {
+    case 1: return launch_lu<P, 1>(s, st, a, oversub);
+    case 2: return launch_lu<P, 2>(s, st, a, oversub);
+    case 4: return launch_lu<P, 4>(s, st, a, oversub);
+    case 8: return launch_lu<P, 8>(s, st, a, oversub);
+    case 16: return launch_lu<P, 16>(s, st, a, oversub);
+  }
+  return false;
 }
 
 // Autotuner: the first launch for a (device, degree, quadrature size, log2 of the cell count, path)
@@ -560,7 +616,8 @@ template <int P> void launch_p(hdg_system* s, cudaStream_t st, const ElemArgs& a
   static std::mutex mu;
   static std::map<std::tuple<int, int, int, int>, std::pair<int, int>> best;
   if (const char* env = std::getenv("HDG_ELEMENT_WARPS")) {
-    if (!launch_cfg<P>(s, st, a, std::atoi(env), 4)) throw HdgError{HDG_ERR_ARG, "HDG_ELEMENT_WARPS does not fit"};
+    const int w = std::atoi(env);
+    if (!launch_cfg<P>(s, st, a, a.schur ? std::min(w, 8) : w, 4)) throw HdgError{HDG_ERR_ARG, "HDG_ELEMENT_WARPS does not fit"};
     return;
   }
   int lg = 0;
@@ -637,12 +694,11 @@ ElemArgs element_args(hdg_system* s) {
   a.AB = s->d_AB.p;
   a.KB = s->d_KB.p;
   a.err = reinterpret_cast<int*>(s->d_scal.p + 1);
-  // Cholesky-Schur path: invertible reference mass and kappa constant on each cell (a kappa field
+  // Schur path: its tables are valid (2: with a null function) and kappa is constant on each cell (a kappa field
   // makes Ae a weighted mass matrix that is no multiple of the reference one)
-  a.schur = (sp->t.schur && a.kappa_mode != 2 && sp->t.p != 2 && std::getenv("HDG_ELEMENT_FULL_LU") == nullptr) ? 1
-                                                                                                                 : 0;
+  a.schur = (sp->t.schur && a.kappa_mode != 2 && std::getenv("HDG_ELEMENT_FULL_LU") == nullptr) ? 1 + sp->t.nullity : 0;
   a.L = ref_layout(sp->t.nw, sp->t.nt, sp->t.nq);
-  a.ref_len = a.L.SMD0;  // the full path stages [M .. Q]; the Cholesky path stages its own ranges
+  a.ref_len = a.L.SMD0;  // the full path stages [M .. Q]; the Schur path stages its own ranges
   return a;
 }
 }  // namespace
@@ -664,10 +720,14 @@ void launch_expand_ke(hdg_system* s, double* out, cudaStream_t st) {
   const int64_t tot = (int64_t)a.nc * s->n * (s->m + 1);
   const unsigned grid = (unsigned)((tot + 255) / 256);
   switch (s->space->t.p) {
-    case 1: k_expand_ke<1><<<grid, 256, 0, st>>>(a, s->d_KB.p, out); break;
-    case 3: k_expand_ke<3><<<grid, 256, 0, st>>>(a, s->d_KB.p, out); break;
-    case 4: k_expand_ke<4><<<grid, 256, 0, st>>>(a, s->d_KB.p, out); break;
-    default: throw HdgError{HDG_ERR_ARG, "the stored element blocks are complete for this degree"};
+    case 1: k_expand_ke<1, 0><<<grid, 256, 0, st>>>(a, s->d_KB.p, out); break;
+    case 2:
+      if (s->space->t.nullity) k_expand_ke<2, 1><<<grid, 256, 0, st>>>(a, s->d_KB.p, out);
+      else k_expand_ke<2, 0><<<grid, 256, 0, st>>>(a, s->d_KB.p, out);
+      break;
+    case 3: k_expand_ke<3, 0><<<grid, 256, 0, st>>>(a, s->d_KB.p, out); break;
+    case 4: k_expand_ke<4, 0><<<grid, 256, 0, st>>>(a, s->d_KB.p, out); break;
+    default: throw HdgError{HDG_ERR_ARG, "degree not supported"};
   }
   HDG_CUDA(cudaGetLastError());
   s->ctx->launches++;

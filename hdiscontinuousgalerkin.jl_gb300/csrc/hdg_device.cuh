@@ -57,6 +57,44 @@ __device__ __forceinline__ double eval_source_prepared(int kind, const double* _
   return s;
 }
 
+// The terms part, part + parts, ... of a source that is a sum (Gaussian bumps, Fourier modes), so that several lanes can
+// share a point; a source that is no sum is evaluated whole by part 0.  The parts add up to the source.
+__device__ __forceinline__ double eval_source_part(int kind, const double* __restrict__ p, double x, double y, int part,
+                                                   int parts) {
+  if (kind == HDG_FIELD_BUMPS) {
+    const int K = (int)p[0];
+    double s = 0.0;
+    for (int k = part; k < K; k += parts) {
+      const double* b = p + 1 + 4 * k;
+      const double dx = x - b[0], dy = y - b[1];
+      s += b[3] * exp((dx * dx + dy * dy) * b[2]);
+    }
+    return s;
+  }
+  if (kind == HDG_FIELD_FOURIER) {
+    const int K = (int)p[0];
+    double g = part == 0 ? p[1] : 0.0;
+    for (int k = part; k < K; k += parts) {
+      const double* b = p + 2 + 4 * k;
+      g += b[3] * cos(6.283185307179586 * (b[0] * x + b[1] * y) + b[2]);
+    }
+    return g;
+  }
+  return part == 0 ? eval_field_kind(kind, p, x, y) : 0.0;
+}
+
+// 1/d to an ulp from the hardware's FP64 estimate (some 20 bits, not on the FP64 pipe) by one step of third order,
+// r <- r (1 + e + e^2) with e = 1 - d r, which cubes the error: three FP64 instructions.  Where the estimate or the step
+// under- or overflows: the division.
+__device__ __forceinline__ double recip_cubic(double d) {
+  const unsigned e = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+  if (e < 24u || e > 2022u) return 1.0 / d;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double x = fma(-d, r, 1.0);
+  return fma(r, fma(x, x, x), r);
+}
+
 // 1/d by Newton-Raphson iteration from the FP32 approximate reciprocal: each step r <- r + r (1 - d r)
 // squares the relative error (about 2^-22 -> 2^-44 -> below 2^-53), so two steps give the FP64
 // reciprocal to within an ulp at a fraction of the cost of a correctly rounded FP64 division.

@@ -198,7 +198,8 @@ struct RefTables {
   std::vector<double> E;           // [nw][nfq][3]
   std::vector<double> T;           // [nt][nfq]
   std::vector<double> Nv;          // [nw][3] basis at the reference vertices (0,0), (1,0), (0,1)
-  bool schur = false;              // the reference mass matrix is invertible (see tables.cpp)
+  bool schur = false;              // the Schur tables are valid (see tables.cpp)
+  int nullity = 0;                 // dimension of the reference mass matrix's null space (0 or 1 with schur)
   // packed device tables (see tables.cpp: ref_layout)
   std::vector<double> packed;
 };
@@ -216,9 +217,10 @@ bool build_lagrange_tables(int order, int qd, LagrangeTables* t);
 // Offsets of the packed table, in doubles.
 struct RefLayout {
   int M, D0, D1, C, F, H, NW, N, Q;
-  // Schur-complement tables (valid when RefTables::schur): M^-1 D_l, Q_lm = D_l' M^-1 D_m,
-  // MF_{f,o} = M^-1 F_{f,o}, DMF_{l,f,o} = D_l' M^-1 F_{f,o}, PFF_{g,o';f,o} = F_{g,o'}' M^-1 F_{f,o}
-  int SMD0, SMD1, SQ00, SQ01, SQ11, SMF, SDMF, PFF, total;
+  // Schur-complement tables (valid when RefTables::schur; M^-1 is the pseudo-inverse where the rule leaves M a
+  // null function): M^-1 D_l, Q_lm = D_l' M^-1 D_m, MF_{f,o} = M^-1 F_{f,o}, DMF_{l,f,o} = D_l' M^-1 F_{f,o},
+  // PFF_{g,o';f,o} = F_{g,o'}' M^-1 F_{f,o}; the null function z, D_l' z and F_{f,o}' z (zero when M is invertible)
+  int SMD0, SMD1, SQ00, SQ01, SQ11, SMF, SDMF, PFF, ZV, ZD, ZF, total;
 };
 RefLayout ref_layout(int nw, int nt, int nq);
 
@@ -265,7 +267,8 @@ struct hdg_system {
                    d_tau.p, d_fprep.p};
   }
   // per-cell condensed blocks: AB = [Ate | bte] (m x (m+1)), KB = [K_e | b_e] (n x (m+1)), or,
-  // after the Cholesky-Schur element path (kb_u_only), only its u rows [X_u | b_u] (nw x (m+1))
+  // after the Schur element path (kb_u_only), only its u rows [X_u | b_u] (nw x (m+1)), with the rows of the two
+  // null-function coefficients of q below them where the rule leaves the mass matrix a null function
   DevBuf<double> d_AB, d_KB;
   bool kb_u_only = false;
   DevBuf<float> d_ABf, d_KBf;

@@ -26,18 +26,19 @@ __global__ void k_recover(const int nc, const int32_t* __restrict__ cfaces, cons
   qu[t] = s;
 }
 
-// Recovery for the Cholesky-Schur element path, which stores only the u rows [X_u | b_u] of
+// Recovery for the Schur element path, which stores only the u rows [X_u | b_u] of
 // [K_e | b_e]: u = X_u u_hat_e + b_u, then q from u, q_c = kf (adl0_c M^-1 D0 u + adl1_c M^-1 D1 u
 // - sum_f wn_f,c M^-1 F_{f,o} u_hat_f) (the q rows of K_e applied to the same u_hat_e, in closed form:
-// Ae = (det J / kappa) diag(M, M) on this path).  One thread per cell; tables read through L1.
-template <int P>
+// Ae = (det J / kappa) diag(M, M) on this path; NZ: plus z a_c, whose rows lie below X_u's).  One thread per cell;
+// tables read through L1.
+template <int P, int NZ>
 __global__ void k_recover_u(const int nc, const int32_t* __restrict__ cells, const int32_t* __restrict__ cfaces,
                             const uint8_t* __restrict__ orient, const double* __restrict__ xy,
                             const double* __restrict__ kcell, const double* __restrict__ SMD0,
                             const double* __restrict__ SMD1, const double* __restrict__ SMF,
-                            const double* __restrict__ KBu, const double* __restrict__ x, double* __restrict__ qu) {
+                            const double* __restrict__ ZV, const double* __restrict__ KBu, const double* __restrict__ x, double* __restrict__ qu) {
   using D = Dims<P>;
-  constexpr int NW = D::NW, NT = D::NT, NV = D::NV, N = D::N, M = D::M;
+  constexpr int NW = D::NW, NT = D::NT, NV = D::NV, N = D::N, M = D::M, NA = NW + 2 * NZ;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= nc) return;
   double uh[M];
@@ -47,8 +48,17 @@ __global__ void k_recover_u(const int nc, const int32_t* __restrict__ cells, con
 #pragma unroll
     for (int j = 0; j < NT; ++j) uh[f * NT + j] = x[g * NT + j];
   }
-  const double* Xu = KBu + (size_t)e * NW * (M + 1);
-  double u[NW];
+  const double* Xu = KBu + (size_t)e * NA * (M + 1);
+  double u[NW], z0 = 0.0, z1 = 0.0;
+  if constexpr (NZ > 0) {
+    z0 = Xu[NW * (M + 1) + M];
+    z1 = Xu[(NW + 1) * (M + 1) + M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+      z0 += Xu[NW * (M + 1) + j] * uh[j];
+      z1 += Xu[(NW + 1) * (M + 1) + j] * uh[j];
+    }
+  }
 #pragma unroll
   for (int ia = 0; ia < NW; ++ia) {
     double t = Xu[ia * (M + 1) + M];
@@ -84,8 +94,9 @@ __global__ void k_recover_u(const int nc, const int32_t* __restrict__ cells, con
       q0 -= wn[f][0] * mf;
       q1 -= wn[f][1] * mf;
     }
-    qu[(size_t)e * N + ia] = kf * q0;
-    qu[(size_t)e * N + NW + ia] = kf * q1;
+    const double zv = NZ ? __ldg(ZV + ia) : 0.0;
+    qu[(size_t)e * N + ia] = kf * q0 + zv * z0;
+    qu[(size_t)e * N + NW + ia] = kf * q1 + zv * z1;
   }
 }
 
@@ -141,17 +152,19 @@ template <int P> void recover_p(hdg_system* s, cudaStream_t st) {
   hdg_mesh* m = s->space->mesh;
   const int64_t tot = (int64_t)m->nc * D::N;
   s->d_qu.alloc((size_t)tot);
-  if constexpr (P != 2) {
-    if (s->kb_u_only) {
-      const RefLayout L = ref_layout(s->space->t.nw, s->space->t.nt, s->space->t.nq);
-      const double* ref = s->space->d_ref.p;
-      k_recover_u<P><<<(unsigned)((m->nc + 127) / 128), 128, 0, st>>>(
-          m->nc, m->d_cells.p, m->d_cfaces.p, m->d_orient.p, m->d_xy.p, s->kappa_cells ? s->d_kappa.p : nullptr,
-          ref + L.SMD0, ref + L.SMD1, ref + L.SMF, s->d_KB.p, s->d_x.p, s->d_qu.p);
-      HDG_CUDA(cudaGetLastError());
-      s->ctx->launches++;
-      return;
+  if (s->kb_u_only) {
+    const RefLayout L = ref_layout(s->space->t.nw, s->space->t.nt, s->space->t.nq);
+    const double* ref = s->space->d_ref.p;
+    auto* kern = k_recover_u<P, 0>;
+    if constexpr (P == 2) {
+      if (s->space->t.nullity) kern = k_recover_u<P, 1>;
     }
+    kern<<<(unsigned)((m->nc + 127) / 128), 128, 0, st>>>(
+        m->nc, m->d_cells.p, m->d_cfaces.p, m->d_orient.p, m->d_xy.p, s->kappa_cells ? s->d_kappa.p : nullptr,
+        ref + L.SMD0, ref + L.SMD1, ref + L.SMF, ref + L.ZV, s->d_KB.p, s->d_x.p, s->d_qu.p);
+    HDG_CUDA(cudaGetLastError());
+    s->ctx->launches++;
+    return;
   }
   k_recover<P><<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(m->nc, m->d_cfaces.p, s->d_KB.p, s->d_x.p, s->d_qu.p);
   HDG_CUDA(cudaGetLastError());

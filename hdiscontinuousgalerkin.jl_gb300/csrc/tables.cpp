@@ -188,6 +188,44 @@ void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w) {
 // reference edges of the triangle (src/shapes.jl:19-23): 1: (1,0)->(0,1), 2: (0,1)->(0,0), 3: (0,0)->(1,0)
 const double EDGE[3][4] = {{1, 0, 0, 1}, {0, 1, 0, 0}, {0, 0, 1, 0}};
 
+// Eigenvalues and eigenvectors (columns) of a small symmetric matrix, cyclic Jacobi rotations in long double.
+void symmetric_eigen(int n, const double* m, std::vector<long double>* lam, std::vector<long double>* vec) {
+  std::vector<long double> a(m, m + (size_t)n * n);
+  vec->assign((size_t)n * n, 0.0L);
+  for (int i = 0; i < n; ++i) (*vec)[(size_t)i * n + i] = 1.0L;
+  for (int sweep = 0; sweep < 60; ++sweep) {
+    long double off = 0.0L, all = 0.0L;
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < n; ++j) (i == j ? all : off) += a[(size_t)i * n + j] * a[(size_t)i * n + j];
+    if (off <= 1e-40L * all) break;
+    for (int p = 0; p < n; ++p)
+      for (int q = p + 1; q < n; ++q) {
+        const long double apq = a[(size_t)p * n + q];
+        if (apq == 0.0L) continue;
+        const long double th = (a[(size_t)q * n + q] - a[(size_t)p * n + p]) / (2.0L * apq);
+        const long double t = (th >= 0 ? 1.0L : -1.0L) / (std::fabs(th) + std::sqrt(th * th + 1.0L));
+        const long double c = 1.0L / std::sqrt(t * t + 1.0L), s = t * c;
+        for (int k = 0; k < n; ++k) {
+          const long double x = a[(size_t)k * n + p], y = a[(size_t)k * n + q];
+          a[(size_t)k * n + p] = c * x - s * y;
+          a[(size_t)k * n + q] = s * x + c * y;
+        }
+        for (int k = 0; k < n; ++k) {
+          const long double x = a[(size_t)p * n + k], y = a[(size_t)q * n + k];
+          a[(size_t)p * n + k] = c * x - s * y;
+          a[(size_t)q * n + k] = s * x + c * y;
+        }
+        for (int k = 0; k < n; ++k) {
+          const long double x = (*vec)[(size_t)k * n + p], y = (*vec)[(size_t)k * n + q];
+          (*vec)[(size_t)k * n + p] = c * x - s * y;
+          (*vec)[(size_t)k * n + q] = s * x + c * y;
+        }
+      }
+  }
+  lam->resize(n);
+  for (int i = 0; i < n; ++i) (*lam)[i] = a[(size_t)i * n + i];
+}
+
 }  // namespace
 
 RefLayout ref_layout(int nw, int nt, int nq) {
@@ -211,6 +249,9 @@ RefLayout ref_layout(int nw, int nt, int nq) {
   L.SMF = o; o += 6 * nw * nt;
   L.SDMF = o; o += 12 * nw * nt;
   L.PFF = o; o += 36 * nt * nt;
+  L.ZV = o; o += nw;
+  L.ZD = o; o += 2 * nw;
+  L.ZF = o; o += 6 * nt;
   L.total = o;
   return L;
 }
@@ -322,8 +363,11 @@ bool build_ref_tables(int p, int qd, RefTables* t) {
   // Schur-complement tables.  With the mass block Ae = (det J / kappa) diag(M, M) of an affine
   // cell and constant kappa, Me^-1 follows from M^-1 and the Schur complement
   // S = Ce + Be' Ae^-1 Be (nw x nw); every product of reference matrices it needs is tabulated
-  // here once.  They are used only when the volume rule makes M invertible (for p = 2 the
-  // default Strang(3) rule leaves M of rank 5, and the element kernel keeps its full LU).
+  // here once.  They are used when the volume rule makes M invertible, and for p = 2 also with the
+  // default Strang(3) rule, whose six points lie on a conic and leave M one null function z: then q = M^+ (...) + z a
+  // with the pseudo-inverse M^+ and one unknown a per component, which the element kernel carries as two more rows of
+  // S, [S Z; Z' 0] with Z = [D_l' z] (the rows z' (Be u - Ee u_hat) = 0 of the local system).  Other rank-deficient
+  // rules keep the full LU.
   {
     std::vector<long double> a((size_t)nw * 2 * nw, 0.0L);
     for (int i = 0; i < nw; ++i) {
@@ -350,8 +394,49 @@ bool build_ref_tables(int p, int qd, RefTables* t) {
       }
     }
     t->schur = ok && minpiv > 1e-10L * maxpiv;
+    std::vector<long double> inv((size_t)nw * nw, 0.0L);
     if (t->schur) {
-      auto Mi = [&](int i, int j) { return a[(size_t)i * 2 * nw + nw + j]; };
+      for (int i = 0; i < nw; ++i)
+        for (int j = 0; j < nw; ++j) inv[(size_t)i * nw + j] = a[(size_t)i * 2 * nw + nw + j];
+    } else if (p == 2) {
+      std::vector<long double> lam, vec;
+      symmetric_eigen(nw, &P[L.M], &lam, &vec);
+      int nul = 0, iz = 0;
+      long double top = 0.0L, low = 1e300L;
+      for (long double v : lam) top = std::max(top, std::fabs(v));
+      for (int k = 0; k < nw; ++k) {
+        if (std::fabs(lam[k]) <= 1e-12L * top) {
+          ++nul;
+          iz = k;
+        } else {
+          low = std::min(low, lam[k]);
+        }
+      }
+      if (nul == 1 && low > 1e-6L * top) {
+        t->schur = true;
+        t->nullity = 1;
+        for (int k = 0; k < nw; ++k)
+          if (k != iz)
+            for (int i = 0; i < nw; ++i)
+              for (int j = 0; j < nw; ++j)
+                inv[(size_t)i * nw + j] += vec[(size_t)i * nw + k] * vec[(size_t)j * nw + k] / lam[k];
+        for (int i = 0; i < nw; ++i) P[L.ZV + i] = (double)vec[(size_t)i * nw + iz];
+        for (int l = 0; l < 2; ++l)
+          for (int j = 0; j < nw; ++j) {
+            long double s = 0;
+            for (int i = 0; i < nw; ++i) s += vec[(size_t)i * nw + iz] * P[(l ? L.D1 : L.D0) + i * nw + j];
+            P[L.ZD + l * nw + j] = (double)s;
+          }
+        for (int fo = 0; fo < 6; ++fo)
+          for (int j = 0; j < nt; ++j) {
+            long double s = 0;
+            for (int i = 0; i < nw; ++i) s += vec[(size_t)i * nw + iz] * P[L.F + (fo * nw + i) * nt + j];
+            P[L.ZF + fo * nt + j] = (double)s;
+          }
+      }
+    }
+    if (t->schur) {
+      auto Mi = [&](int i, int j) { return inv[(size_t)i * nw + j]; };
       const double* D[2] = {&P[L.D0], &P[L.D1]};
       std::vector<long double> MD[2];
       for (int l = 0; l < 2; ++l) {

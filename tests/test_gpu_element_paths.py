@@ -1,0 +1,58 @@
+"""The element kernels that condense through the Schur complement, several cells per warp, against the pivoted
+elimination of the whole local system (HDG_ELEMENT_FULL_LU), on the same cells.
+
+Both are held to 1e-12 of the largest entry of a cell's block against the exact blocks elsewhere, so here they may
+differ by 2e-12 of it."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+BOUND = 2e-12
+
+
+@pytest.fixture(scope="module")
+def H():
+    import __graft_entry__ as g
+    g.build()
+    return g.import_package()
+
+
+def blocks(H, mesh, p, qd, f, tau=1.3, he_tau=False, **kappa):
+    fe = H.GenericFiniteElement(H.Dubiner(2, H.RefTetrahedron, p))
+    Wh, Vh = H.ScalarFunctionSpace(mesh, fe, quad_degree=qd), H.VectorFunctionSpace(mesh, fe, quad_degree=qd)
+    Mh = H.ScalarTraceFunctionSpace(Wh, H.GenericFiniteElement(H.Legendre(1, H.RefTetrahedron, p)))
+    K, _, _, _ = H.doassemble(Vh, Wh, Mh, tau, f, he_tau=he_tau, **kappa)
+    return K.element_blocks()
+
+
+def source(H, kind, rng):
+    if kind == "sinsin":
+        return H.Field.sinsin(2.0, 1.7, 0.6)
+    if kind == "bumps":
+        k = int(rng.integers(1, 10))  # fewer and more terms than lanes share a point
+        return H.Field.bumps(rng.random((k, 2)), 0.05 + 0.2 * rng.random(k), rng.standard_normal(k))
+    k = int(rng.integers(1, 40))
+    return H.Field.fourier(0.3, rng.uniform(-2, 2, (k, 4)), exponential=kind == "exp_fourier")
+
+
+def check(a, b):
+    for x, y in zip(a, b):
+        axes = tuple(range(1, y.ndim))
+        scale = np.abs(y).max(axis=axes, keepdims=True)
+        assert np.isfinite(x).all()
+        assert (np.abs(x - y) <= BOUND * np.maximum(scale, 1e-300)).all()
+
+
+# 2 cells (less than one warp takes), 8, 18 and 50 (remainders of the cells per warp), 578
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 17])
+@pytest.mark.parametrize("p,qd", [(1, 2), (2, 3), (2, 4), (3, 6), (4, 9)])
+@pytest.mark.parametrize("kind", ["sinsin", "bumps", "fourier", "exp_fourier"])
+def test_schur_blocks_match_full_elimination(H, monkeypatch, n, p, qd, kind):
+    rng = np.random.default_rng(100 * n + 10 * p + qd)
+    mesh = H.rectangle_mesh(H.TriangleCell, (n, n), (0.0, 0.0), (1.0, 1.0))
+    mesh.jitter(0.2, 3)
+    f, kappa = source(H, kind, rng), np.exp(rng.uniform(-2.3, 2.3, 2 * n * n))
+    kw = dict(kappa_cell=kappa if kind != "sinsin" else None, he_tau=kind == "bumps")
+    got = blocks(H, mesh, p, qd, f, **kw)
+    monkeypatch.setenv("HDG_ELEMENT_FULL_LU", "1")
+    check(got, blocks(H, mesh, p, qd, f, **kw))
