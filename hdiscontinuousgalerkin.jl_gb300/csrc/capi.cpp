@@ -354,16 +354,20 @@ static void set_coefficients_many(hdg_system* s, const double* taus, const hdg_f
   s->d_fprm.upload(fp.data(), fp.size(), st);
   // the element kernels evaluate a Gaussian bump as a exp(|x - c|^2 k) with k = -1/(2 s^2) formed
   // here once, instead of dividing by 2 s^2 at every quadrature point
-  std::vector<double> fpp(fp);
-  for (int P = 0; P < np; ++P)
-    if (fk[P] == HDG_FIELD_BUMPS) {
-      const int K = (int)fpp[fo[P]];
-      for (int b = 0; b < K; ++b) {
-        double& sw = fpp[fo[P] + 1 + 4 * b + 2];
-        sw = -1.0 / (2.0 * sw * sw);
+  auto prepared = [&](std::vector<double> prm, const std::vector<int32_t>& kind, const std::vector<int32_t>& off) {
+    for (int P = 0; P < np; ++P)
+      if (kind[P] == HDG_FIELD_BUMPS) {
+        const int K = (int)prm[off[P]];
+        for (int b = 0; b < K; ++b) {
+          double& sw = prm[off[P] + 1 + 4 * b + 2];
+          sw = -1.0 / (2.0 * sw * sw);
+        }
       }
-    }
+    return prm;
+  };
+  const std::vector<double> fpp = prepared(fp, fk, fo), kpp = prepared(kp, kk, ko);
   s->d_fprep.upload(fpp.data(), fpp.size(), st);
+  s->d_kprep.upload(kpp.data(), kpp.size(), st);
   s->d_kkind.upload(kk.data(), np, st);
   s->d_koff.upload(ko.data(), np, st);
   s->d_kprm.upload(kp.data(), kp.size(), st);

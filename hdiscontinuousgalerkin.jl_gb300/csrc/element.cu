@@ -33,7 +33,9 @@ struct ElemArgs {
   double* AB;
   double* KB;
   int* err;
-  int schur;  // 1: the Schur path (invertible reference mass, kappa constant per cell), 2: with one null function
+  int32_t* list;  // kappa field: the cells left to the general kernel (their number, their ids); NULL: all cells
+  int schur;  // 1: the Schur path (invertible reference mass, kappa constant per cell), 2: with one null function,
+              // 3: kappa a field, 4: with one null function
   int he_tau; // 1: He carries tau
   RefLayout L;  // offsets of the packed reference tables (tables.cpp: ref_layout)
 };
@@ -62,7 +64,9 @@ __global__ void __launch_bounds__(EWARPS * 32) k_element_condense(ElemArgs a) {
   double* sq = W + N * LDW;  // per-warp scratch: f (or kappa^-1) at the quadrature points, be
   __syncthreads();
 
-  for (int e = blockIdx.x * EWARPS + warp; e < a.nc; e += gridDim.x * EWARPS) {
+  const int ntodo = a.list ? a.list[0] : a.nc;
+  for (int todo = blockIdx.x * EWARPS + warp; todo < ntodo; todo += gridDim.x * EWARPS) {
+    const int e = a.list ? a.list[1 + todo] : todo;
     // ---- geometry (reinit!, src/ScalarFunctionSpaces.jl:101-132) -------------------------
     int nid = (lane < 3) ? a.cells[3 * e + lane] : 0;
     double px = 0.0, py = 0.0;
@@ -398,7 +402,7 @@ __global__ void __launch_bounds__(256) k_element_schur(ElemArgs a) {
                              fma(A11, eta, fma(A10, xi, Yv)), part, PARTS);
 #pragma unroll
       for (int o = PARTS / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (part == 0 && pt < CPW * nq) sq0[pt] = v;
+      if (part == 0 && pt < CPW * nq) sq0[pt] = finish_parts(a.co.fkind[pr], v);
     }
     __syncwarp();
     if (col < NW && on_lane) {
@@ -502,6 +506,363 @@ __global__ void __launch_bounds__(256) k_element_schur(ElemArgs a) {
   }
 }
 
+// The Schur path for a kappa that varies within the cell (a field), with positive volume weights.  Ae = diag(Aw, Aw) with
+// Aw = int kappa^-1 phi phi' differs from cell to cell, so the products that the tables hold for a constant kappa are formed
+// here: Aw = U' D U on the range of the reference mass matrix (NR functions), the 2 NW + M columns [V'D0 | V'D1 | V'F_{f,o}]
+// carried along, and the products of all their pairs in the D^-1 metric, which are D_l' Aw^-1 D_m, D_l' Aw^-1 F and
+// F' Aw^-1 F.  From there the condensation is that of k_element_schur.  The q rows are stored here (they need Aw).
+//
+// One cell per warp at p = 2 and 3 (21 and 32 columns, a lane each), two at p = 1.  The fields' modes are spread over
+// (point, part) pairs: at p = 3 and 64 modes each for f and kappa, a lane per point kept 12 of 32 lanes busy for more than
+// half of the 43 us a cell took an SM.  A cell with kappa <= 0 (or not finite) at a point may have an indefinite Aw; it goes
+// on the list for the pivoted kernel.  Measured on 65522 cells with 64 modes each, pivoted elimination / here: p = 3
+// 18.6 / 8.2 ms, p = 2 13.6 / 4.6, p = 1 11.9 / 1.7.
+template <int P, int NZ> struct FieldDims {
+  using D = Dims<P>;
+  static constexpr int NW = D::NW, NT = D::NT, M = D::M, N = D::N;
+  static constexpr int NR = NW - NZ, NA = NW + 2 * NZ, COLS = M + 1;
+  static constexpr int NC = 2 * NW + M;           // columns of the first elimination
+  static constexpr int CPW = 32 / NC;
+  static constexpr int TRI = NW * (NW + 1) / 2, TRR = NR * (NR + 1) / 2, PAIRS = NC * (NC + 1) / 2;
+  static constexpr int PARTS = P == 3 ? 8 : 16;   // lanes per point
+  static constexpr int GEO = 8;
+  static constexpr int YA = NR * NC, WA = NR * NR, W = NA * NA, Y = NA * COLS;
+  static constexpr int PR = PAIRS > 2 * NR * NW ? PAIRS : 2 * NR * NW;  // products; afterwards B_c in the D^-1 metric
+  static_assert(CPW >= 1, "a lane per column");
+  __host__ __device__ static constexpr int tables(int nq) {
+    return 3 * TRI + 6 * NW * NT + NT * NT + NW * nq + 2 * nq + TRR * nq + 2 * NR * NW + 6 * NR * NT + NW * NR +
+           NZ * (3 * NW + 6 * NT);
+  }
+  __host__ __device__ static constexpr int per_warp(int nq) {
+    return CPW * (YA + WA + PR + W + Y + GEO + NW + 2 * nq);
+  }
+};
+
+template <int P, int NZ>
+__global__ void __launch_bounds__(256) k_element_field(ElemArgs a) {
+  using FD = FieldDims<P, NZ>;
+  constexpr int NW = FD::NW, NT = FD::NT, M = FD::M, N = FD::N, NR = FD::NR, NA = FD::NA, COLS = FD::COLS, NC = FD::NC;
+  constexpr int CPW = FD::CPW, TRI = FD::TRI, TRR = FD::TRR, PARTS = FD::PARTS, GEO = FD::GEO;
+  extern __shared__ double smem[];
+  const int nq = a.nq;
+  const RefLayout G = a.L;
+  double* tC = smem;                   // [3][TRI]
+  double* tF = tC + 3 * TRI;           // [6][NW][NT]
+  double* tH = tF + 6 * NW * NT;       // [NT][NT]
+  double* tN = tH + NT * NT;           // [NW][nq]
+  double* tQ = tN + NW * nq;           // [nq][2]
+  double* tW = tQ + 2 * nq;            // [TRR][nq]  w N_i N_j in the range basis
+  double* tD = tW + TRR * nq;          // [2][NR][NW]
+  double* tG = tD + 2 * NR * NW;       // [6][NR][NT]
+  double* tV = tG + 6 * NR * NT;       // [NW][NR]
+  double* tZ = tV + NW * NR;           // [2][NW] D_l' z, [6][NT] F' z, [NW] z
+  for (int t = threadIdx.x; t < 3 * TRI; t += blockDim.x) {
+    const int k = t / TRI, e = t - k * TRI;
+    int j = 0;
+    while ((j + 1) * (j + 2) / 2 <= e) ++j;
+    tC[t] = a.ref[G.C + (k * NW + (e - j * (j + 1) / 2)) * NW + j];
+  }
+  auto stage = [&](double* to, int from, int n) {
+    for (int t = threadIdx.x; t < n; t += blockDim.x) to[t] = a.ref[from + t];
+  };
+  stage(tF, G.F, 6 * NW * NT);
+  stage(tH, G.H, NT * NT);
+  stage(tN, G.NW, NW * nq);
+  stage(tQ, G.Q, 2 * nq);
+  stage(tW, G.RW, TRR * nq);
+  stage(tD, G.RD, 2 * NR * NW);
+  stage(tG, G.RF, 6 * NR * NT);
+  stage(tV, G.RV, NW * NR);
+  if constexpr (NZ > 0) {
+    stage(tZ, G.ZD, 2 * NW);
+    stage(tZ + 2 * NW, G.ZF, 6 * NT);
+    stage(tZ + 2 * NW + 6 * NT, G.ZV, NW);
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  double* base = smem + FD::tables(nq) + warp * FD::per_warp(nq);
+  // first elimination: lane = (cell, column of [D0 | D1 | F])
+  const bool on1 = lane < CPW * NC;
+  const int cl = on1 ? lane / NC : CPW - 1, c1 = on1 ? lane - cl * NC : NC - 1;
+  double* Ya = base + cl * FD::YA;                          // D^-1 R~ of the first elimination (NR x NC)
+  double* Wa = base + CPW * FD::YA + cl * FD::WA;           // its rows
+  double* pr = base + CPW * (FD::YA + FD::WA) + cl * FD::PR;
+  double* Wc = base + CPW * (FD::YA + FD::WA + FD::PR) + cl * FD::W;
+  double* Yc = base + CPW * (FD::YA + FD::WA + FD::PR + FD::W) + cl * FD::Y;
+  double* geo0 = base + CPW * (FD::YA + FD::WA + FD::PR + FD::W + FD::Y);
+  double* geo = geo0 + cl * GEO;
+  double* be = geo0 + CPW * GEO + cl * NW;
+  double* sq0 = geo0 + CPW * (GEO + NW);                    // f at the points, then kappa^-1
+  double* sk0 = sq0 + CPW * nq;
+  // second elimination: the first COLS lanes of a cell, a right-hand side each
+  const bool on2 = on1 && c1 < COLS;
+  const int col = min(c1, COLS - 1);
+  const int f = col < M ? col / NT : 0, fj = col < M ? col - f * NT : 0;
+  auto pair_at = [](int i, int j) { return i <= j ? j * (j + 1) / 2 + i : i * (i + 1) / 2 + j; };
+  __syncthreads();
+
+  for (int e0 = (blockIdx.x * nwarps + warp) * CPW; e0 < a.nc; e0 += gridDim.x * nwarps * CPW) {
+    const bool mine = on1 && e0 + cl < a.nc;
+    const int e = min(e0 + cl, a.nc - 1);
+    const int n0 = a.cells[3 * e], n1 = a.cells[3 * e + 1], n2 = a.cells[3 * e + 2];
+    const double x1 = a.xy[2 * n0], y1 = a.xy[2 * n0 + 1];
+    const double J00 = a.xy[2 * n1] - x1, J01 = a.xy[2 * n2] - x1;
+    const double J10 = a.xy[2 * n1 + 1] - y1, J11 = a.xy[2 * n2 + 1] - y1;
+    const double detJ = J00 * J11 - J01 * J10;
+    if (!(detJ > 0.0) && mine && c1 == 0) atomicOr(a.err, 1);
+    const double ad00 = J11, ad01 = -J01, ad10 = -J10, ad11 = J00;
+    const double wx0 = J11 - J10, wy0 = J00 - J01;
+    const double wx = sel3(f, wx0, -J11, J10), wy = sel3(f, wy0, J01, -J00);
+    const double el = sqrt(wx * wx + wy * wy);
+    const unsigned ob = a.orient[e];
+    const int fo = 2 * f + ((ob >> f) & 1);
+    const int prob = a.co.cell_prob[e];
+    const double tau = a.co.tau[prob];
+    if (on2) {
+      if (col < M && fj == 0) geo[f] = tau * el;
+      if (col == COLS - 1) {
+        geo[3] = ad00 * ad00 + ad01 * ad01;
+        geo[4] = ad00 * ad10 + ad01 * ad11;
+        geo[5] = ad10 * ad10 + ad11 * ad11;
+      }
+    }
+    // ---- f and kappa^-1 at the points; be -------------------------------------------------------
+    bool good = true;
+    for (int t0 = 0; t0 < CPW * nq * PARTS; t0 += 32) {
+      const int t = t0 + lane;
+      const int pt = t / PARTS, part = t - pt * PARTS;
+      const bool in = pt < CPW * nq;
+      const int c = min(pt / nq, CPW - 1), q = in ? pt - c * nq : 0, src = c * NC;
+      const double X = __shfl_sync(0xffffffffu, x1, src), Yv = __shfl_sync(0xffffffffu, y1, src);
+      const double A00 = __shfl_sync(0xffffffffu, J00, src), A01 = __shfl_sync(0xffffffffu, J01, src);
+      const double A10 = __shfl_sync(0xffffffffu, J10, src), A11 = __shfl_sync(0xffffffffu, J11, src);
+      const int po = __shfl_sync(0xffffffffu, prob, src);
+      const double xi = tQ[2 * q], eta = tQ[2 * q + 1];
+      const double xq = fma(A01, eta, fma(A00, xi, X)), yq = fma(A11, eta, fma(A10, xi, Yv));
+      double v = 0.0, w = 0.0;
+      if (in) {
+        v = eval_source_part(a.co.fkind[po], a.co.fprep + a.co.foff[po], xq, yq, part, PARTS);
+        w = eval_source_part(a.co.kkind[po], a.co.kprep + a.co.koff[po], xq, yq, part, PARTS);
+      }
+#pragma unroll
+      for (int o = PARTS / 2; o > 0; o >>= 1) {
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+        w += __shfl_xor_sync(0xffffffffu, w, o);
+      }
+      if (part == 0 && in) {
+        sq0[pt] = finish_parts(a.co.fkind[po], v);
+        w = finish_parts(a.co.kkind[po], w);
+        sk0[pt] = 1.0 / w;
+        good = good && w > 0.0 && w < 1e300;
+      }
+    }
+    const bool all_good = __all_sync(0xffffffffu, good);
+    __syncwarp();
+    if (!all_good) {  // the tile's cells go to the pivoted kernel
+      if (mine && c1 == 0) a.list[1 + atomicAdd(a.list, 1)] = e;
+      continue;
+    }
+    if (c1 < NW && on1) {
+      double t = 0.0;
+      for (int q = 0; q < nq; ++q) t += tN[c1 * nq + q] * sq0[cl * nq + q];
+      be[c1] = t * detJ;
+    }
+    // ---- Aw / det J (upper triangle, by columns) over all lanes, into the place of the products ---
+    for (int t = lane; t < CPW * TRR; t += 32) {
+      const int c = t / TRR, k = t - c * TRR;
+      double v = 0.0;
+      for (int q = 0; q < nq; ++q) v += tW[k * nq + q] * sk0[c * nq + q];
+      base[CPW * (FD::YA + FD::WA) + c * FD::PR + k] = v;
+    }
+    __syncwarp();
+    double ra[NR];
+    {
+      double s[NR], g[NR];
+#pragma unroll
+      for (int i = 0; i < NR; ++i) s[i] = 0.0;
+      if (c1 < NR) {
+#pragma unroll
+        for (int i = 0; i < NR; ++i)
+          if (i <= c1) s[i] = pr[c1 * (c1 + 1) / 2 + i] * detJ;
+      }
+      {
+        const int fc = c1 < 2 * NW ? 0 : c1 - 2 * NW, ff = fc / NT;
+        const double* from = c1 < 2 * NW ? tD + (c1 / NW) * NR * NW + c1 % NW
+                                         : tG + (2 * ff + ((ob >> ff) & 1)) * NR * NT + (fc - ff * NT);
+        const int ld = c1 < 2 * NW ? NW : NT;
+#pragma unroll
+        for (int i = 0; i < NR; ++i) g[i] = from[i * ld];
+      }
+      __syncwarp();
+      // ---- Aw = U' D U, carrying the columns ------------------------------------------------------
+#pragma unroll
+      for (int k = 0; k < NR; ++k) {
+        if (on1 && c1 >= k && c1 < NR) Wa[k * NR + c1] = s[k];
+        __syncwarp();
+        const double d = Wa[k * NR + k];
+        if (!(d > 0.0) && mine && c1 == 0) atomicOr(a.err, 2);
+        const double rk = recip_cubic(d);
+        ra[k] = rk;
+        const double ts = s[k] * rk, tg = g[k] * rk;
+        if (on1) Ya[k * NC + c1] = tg;
+#pragma unroll
+        for (int i = k + 1; i < NR; ++i) {
+          const double w = Wa[k * NR + i];
+          s[i] -= w * ts;
+          g[i] -= w * tg;
+        }
+      }
+      __syncwarp();
+      // ---- products of all pairs of columns -------------------------------------------------------
+#pragma unroll 1
+      for (int d = 0; d <= NC / 2; ++d) {
+        int o = c1 + d;
+        if (o >= NC) o -= NC;
+        double dot = 0.0;
+#pragma unroll
+        for (int k = 0; k < NR; ++k) dot += g[k] * Ya[k * NC + o];
+        if (on1 && !(2 * d == NC && c1 >= NC / 2)) pr[pair_at(c1, o)] = dot;  // at 2 d = NC: the other lane's pair
+      }
+    }
+    __syncwarp();
+    // ---- S and R' --------------------------------------------------------------------------------
+    double s[NA], r[NA], ri[NA];
+#pragma unroll
+    for (int i = 0; i < NA; ++i) s[i] = 0.0;
+    if (col < NW) {
+#pragma unroll
+      for (int i = 0; i < NW; ++i)
+        if (i <= col) {
+          const int k = col * (col + 1) / 2 + i;
+          s[i] = geo[0] * tC[k] + geo[1] * tC[TRI + k] + geo[2] * tC[2 * TRI + k] + geo[3] * pr[pair_at(i, col)] +
+                 geo[4] * (pr[pair_at(i, NW + col)] + pr[pair_at(col, NW + i)]) + geo[5] * pr[pair_at(NW + i, NW + col)];
+        }
+    }
+    if constexpr (NZ > 0) {
+      if (col >= NW && col < NA) {
+        const double z0 = col == NW ? ad00 : ad01, z1 = col == NW ? ad10 : ad11;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) s[i] = z0 * tZ[i] + z1 * tZ[NW + i];
+      }
+    }
+    if (col < M) {
+      const double te = tau * el, b0 = ad00 * wx + ad01 * wy, b1 = ad10 * wx + ad11 * wy;
+#pragma unroll
+      for (int i = 0; i < NW; ++i)
+        r[i] = te * tF[(fo * NW + i) * NT + fj] + b0 * pr[pair_at(i, 2 * NW + col)] + b1 * pr[pair_at(NW + i, 2 * NW + col)];
+      if constexpr (NZ > 0) {
+        r[NW] = wx * tZ[2 * NW + fo * NT + fj];
+        r[NW + 1] = wy * tZ[2 * NW + fo * NT + fj];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NA; ++i) r[i] = i < NW ? be[i] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < NA; ++k) {
+      if (on2 && col >= k && col < NA) Wc[k * NA + col] = s[k];
+      __syncwarp();
+      const double d = Wc[k * NA + k];
+      const bool fits = k < NW ? d > 0.0 : d < 0.0;
+      if (!fits && mine && c1 == 0) atomicOr(a.err, 2);
+      const double rk = recip_cubic(d);
+      ri[k] = rk;
+      const double ts = s[k] * rk, tr = r[k] * rk;
+      if (on2) Yc[k * COLS + col] = tr;
+#pragma unroll
+      for (int i = k + 1; i < NA; ++i) {
+        const double w = Wc[k * NA + i];
+        s[i] -= w * ts;
+        r[i] -= w * tr;
+      }
+    }
+    __syncwarp();
+    // ---- [Ate | bte] -------------------------------------------------------------------------------
+    double* AB = a.AB + (size_t)e * M * COLS;
+    const double* Hh = tH + fj * NT;
+    const double he = (a.he_tau ? tau : 1.0) * el;
+#pragma unroll 1
+    for (int d = 0; d <= COLS / 2; ++d) {
+      int o = col + d;
+      if (o >= COLS) o -= COLS;
+      double dot = 0.0;
+#pragma unroll
+      for (int k = 0; k < NA; ++k) dot += r[k] * Yc[k * COLS + o];
+      const bool twice = 2 * d == COLS && col >= COLS / 2;
+      if (mine && on2 && !twice && !(col == M && o == M)) {
+        if (col == M || o == M) {
+          AB[(col == M ? o : col) * COLS + M] = -dot;
+        } else {
+          const int g = o / NT, gj = o - g * NT;
+          const double gx = sel3(g, wx0, -J11, J10), gy = sel3(g, wy0, J01, -J00);
+          double v = dot - (wx * gx + wy * gy) * pr[pair_at(2 * NW + col, 2 * NW + o)];
+          if (f == g) v -= he * Hh[gj];
+          AB[col * COLS + o] = v;
+          if (d) AB[o * COLS + col] = v;
+        }
+      }
+    }
+    // ---- X_u (and a_c), kept for the q rows in the place of Y -----------------------------------------
+    double* KB = a.KB + (size_t)e * N * COLS;
+#pragma unroll
+    for (int k = NA - 1; k >= 0; --k) {
+      double t = 0.0;
+#pragma unroll
+      for (int i = k + 1; i < NA; ++i) t += Wc[k * NA + i] * r[i];
+      r[k] = Yc[k * COLS + col] - ri[k] * t;
+      if (mine && on2 && k < NW) KB[(2 * NW + k) * COLS + col] = r[k];
+    }
+    __syncwarp();
+    if (on2) {
+#pragma unroll
+      for (int k = 0; k < NA; ++k) Yc[k * COLS + col] = r[k];
+    }
+    // B_c = adl0_c D0 + adl1_c D1 in the D^-1 metric, [2][NR][NW], in the place of the products
+    for (int t = c1; t < 2 * NR * NW; t += NC)
+      if (on1) {
+        const int c = t / (NR * NW), ki = t - c * NR * NW, k = ki / NW, i = ki - k * NW;
+        pr[t] = (c ? ad01 : ad00) * Ya[k * NC + i] + (c ? ad11 : ad10) * Ya[k * NC + NW + i];
+      }
+    __syncwarp();
+    // ---- q rows: Aw q_c = B_c u - wn_f,c F u_hat, a lane per (component, column) -----------------------
+    for (int t = c1; t < 2 * COLS; t += NC) {
+      const int c = t / COLS, j = t - c * COLS;
+      double x[NW], v[NR];
+#pragma unroll
+      for (int i = 0; i < NW; ++i) x[i] = Yc[i * COLS + j];
+      double wc = 0.0;
+      if (j < M) {
+        const int g = j / NT;
+        wc = c ? sel3(g, wy0, J01, -J00) : sel3(g, wx0, -J11, J10);
+      }
+#pragma unroll
+      for (int k = NR - 1; k >= 0; --k) {
+        double u = j < M ? -wc * Ya[k * NC + 2 * NW + j] : 0.0;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) u += pr[(c * NR + k) * NW + i] * x[i];
+        double w = 0.0;
+#pragma unroll
+        for (int i = k + 1; i < NR; ++i) w += Wa[k * NR + i] * v[i];
+        v[k] = u - ra[k] * w;
+      }
+      if (mine) {
+#pragma unroll
+        for (int ia = 0; ia < NW; ++ia) {
+          double qv;
+          if constexpr (NZ > 0) {
+            qv = tZ[2 * NW + 6 * NT + ia] * Yc[(NW + c) * COLS + j];
+#pragma unroll
+            for (int k = 0; k < NR; ++k) qv += tV[ia * NR + k] * v[k];
+          } else {
+            qv = v[ia];
+          }
+          KB[(c * NW + ia) * COLS + j] = qv;
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // The q rows of [K_e | b_e] from the stored u rows (the Schur path stores X_u only, and a_c below it):
 // X_q,c = kf (adl0_c M^-1 D0 X_u + adl1_c M^-1 D1 X_u - [j < m] wn_f,c M^-1 F_{f,o}), one thread per
 // entry of the full n x (m+1) block.  Used when the blocks are exported, not on the solve path.
@@ -588,7 +949,25 @@ template <int P, int NZ> bool launch_schur(hdg_system* s, cudaStream_t st, const
   return launch_kernel(s, st, a, k_element_schur<P, NZ>, warps, SD::CPW, smem, oversub);
 }
 
+// The kappa-field kernel, then the pivoted one over the cells that it listed (mostly none).
+template <int P, int NZ> bool launch_field(hdg_system* s, cudaStream_t st, const ElemArgs& a, int warps, int oversub) {
+  using FD = FieldDims<P, NZ>;
+  if (warps > 8) return false;  // the kernel's launch bound
+  const size_t smem = sizeof(double) * ((size_t)FD::tables(a.nq) + (size_t)warps * FD::per_warp(a.nq));
+  if (smem > ELEM_SMEM_MAX) return false;
+  HDG_CUDA(cudaMemsetAsync(a.list, 0, sizeof(int32_t), st));
+  ElemArgs all = a;
+  if (!launch_kernel(s, st, all, k_element_field<P, NZ>, warps, FD::CPW, smem, oversub)) return false;
+  return launch_lu<P, 2>(s, st, a, 1);
+}
+
 template <int P> bool launch_cfg(hdg_system* s, cudaStream_t st, const ElemArgs& a, int warps, int oversub) {
+  if constexpr (P <= 3) {
+    if (a.schur == 3) return launch_field<P, 0>(s, st, a, warps, oversub);
+  }
+  if constexpr (P == 2) {
+    if (a.schur == 4) return launch_field<P, 1>(s, st, a, warps, oversub);
+  }
   if (a.schur == 1) return launch_schur<P, 0>(s, st, a, warps, oversub);
   if constexpr (P == 2) {
     if (a.schur == 2) return launch_schur<P, 1>(s, st, a, warps, oversub);
@@ -696,7 +1075,15 @@ ElemArgs element_args(hdg_system* s) {
   a.err = reinterpret_cast<int*>(s->d_scal.p + 1);
   // Schur path: its tables are valid (2: with a null function) and kappa is constant on each cell (a kappa field
   // makes Ae a weighted mass matrix that is no multiple of the reference one)
-  a.schur = (sp->t.schur && a.kappa_mode != 2 && std::getenv("HDG_ELEMENT_FULL_LU") == nullptr) ? 1 + sp->t.nullity : 0;
+  a.schur = (sp->t.schur && a.kappa_mode != 2) ? 1 + sp->t.nullity : 0;
+  // ... or a field: the same with Aw formed per cell, where the weights are positive (the rules of p = 4 are not)
+  if (sp->t.schur && a.kappa_mode == 2 && sp->t.positive && sp->t.p <= 3) a.schur = 3 + sp->t.nullity;
+  if (std::getenv("HDG_ELEMENT_FULL_LU") != nullptr) a.schur = 0;
+  a.list = nullptr;
+  if (a.schur >= 3) {
+    s->d_elem_list.alloc((size_t)m->nc + 1);
+    a.list = s->d_elem_list.p;
+  }
   a.L = ref_layout(sp->t.nw, sp->t.nt, sp->t.nq);
   a.ref_len = a.L.SMD0;  // the full path stages [M .. Q]; the Schur path stages its own ranges
   return a;
@@ -705,7 +1092,7 @@ ElemArgs element_args(hdg_system* s) {
 
 void launch_element_condense(hdg_system* s, cudaStream_t st) {
   const ElemArgs a = element_args(s);
-  s->kb_u_only = a.schur != 0;
+  s->kb_u_only = a.schur == 1 || a.schur == 2;
   switch (s->space->t.p) {
     case 1: launch_p<1>(s, st, a); break;
     case 2: launch_p<2>(s, st, a); break;

@@ -58,7 +58,8 @@ __device__ __forceinline__ double eval_source_prepared(int kind, const double* _
 }
 
 // The terms part, part + parts, ... of a source that is a sum (Gaussian bumps, Fourier modes), so that several lanes can
-// share a point; a source that is no sum is evaluated whole by part 0.  The parts add up to the source.
+// share a point; a source that is no sum is evaluated whole by part 0.  The parts add up to the source (or to what
+// finish_parts makes it from).
 __device__ __forceinline__ double eval_source_part(int kind, const double* __restrict__ p, double x, double y, int part,
                                                    int parts) {
   if (kind == HDG_FIELD_BUMPS) {
@@ -71,7 +72,7 @@ __device__ __forceinline__ double eval_source_part(int kind, const double* __res
     }
     return s;
   }
-  if (kind == HDG_FIELD_FOURIER) {
+  if (kind == HDG_FIELD_FOURIER || kind == HDG_FIELD_EXP_FOURIER) {
     const int K = (int)p[0];
     double g = part == 0 ? p[1] : 0.0;
     for (int k = part; k < K; k += parts) {
@@ -81,6 +82,10 @@ __device__ __forceinline__ double eval_source_part(int kind, const double* __res
     return g;
   }
   return part == 0 ? eval_field_kind(kind, p, x, y) : 0.0;
+}
+// The field from the sum of its parts.
+__device__ __forceinline__ double finish_parts(int kind, double v) {
+  return kind == HDG_FIELD_EXP_FOURIER ? exp(v) : v;
 }
 
 // 1/d to an ulp from the hardware's FP64 estimate (some 20 bits, not on the FP64 pipe) by one step of third order,

@@ -116,6 +116,7 @@ struct CoefDev {
   const double* tau;         // [nprob]
   // fprm with each Gaussian bump's width s replaced by -1/(2 s^2) (element kernels' source)
   const double* fprep;
+  const double* kprep;  // kprm likewise
 };
 
 // ------------------------------------------------------------------ objects
@@ -199,6 +200,7 @@ struct RefTables {
   std::vector<double> T;           // [nt][nfq]
   std::vector<double> Nv;          // [nw][3] basis at the reference vertices (0,0), (1,0), (0,1)
   bool schur = false;              // the Schur tables are valid (see tables.cpp)
+  bool positive = false;           // every volume weight is positive
   int nullity = 0;                 // dimension of the reference mass matrix's null space (0 or 1 with schur)
   // packed device tables (see tables.cpp: ref_layout)
   std::vector<double> packed;
@@ -220,7 +222,10 @@ struct RefLayout {
   // Schur-complement tables (valid when RefTables::schur; M^-1 is the pseudo-inverse where the rule leaves M a
   // null function): M^-1 D_l, Q_lm = D_l' M^-1 D_m, MF_{f,o} = M^-1 F_{f,o}, DMF_{l,f,o} = D_l' M^-1 F_{f,o},
   // PFF_{g,o';f,o} = F_{g,o'}' M^-1 F_{f,o}; the null function z, D_l' z and F_{f,o}' z (zero when M is invertible)
-  int SMD0, SMD1, SQ00, SQ01, SQ11, SMF, SDMF, PFF, ZV, ZD, ZF, total;
+  int SMD0, SMD1, SQ00, SQ01, SQ11, SMF, SDMF, PFF, ZV, ZD, ZF;
+  // for a kappa that varies within the cell: an orthonormal basis V of the range of M (the identity when M is
+  // invertible; nr columns), w N_i N_j in it (upper triangle by columns, per point), V' D_l and V' F_{f,o}
+  int RV, RW, RD, RF, total;
 };
 RefLayout ref_layout(int nw, int nt, int nq);
 
@@ -264,7 +269,7 @@ struct hdg_system {
   std::vector<int32_t> h_seg_prob, h_seg_row0, h_seg_row1, h_prob_blk0, h_prob_nblk;  // host copies
   CoefDev coef_dev() const {
     return CoefDev{space->mesh->d_cell_prob.p, d_fkind.p, d_foff.p, d_fprm.p, d_kkind.p, d_koff.p, d_kprm.p,
-                   d_tau.p, d_fprep.p};
+                   d_tau.p, d_fprep.p, d_kprep.p};
   }
   // per-cell condensed blocks: AB = [Ate | bte] (m x (m+1)), KB = [K_e | b_e] (n x (m+1)), or,
   // after the Schur element path (kb_u_only), only its u rows [X_u | b_u] (nw x (m+1)), with the rows of the two
@@ -274,7 +279,7 @@ struct hdg_system {
   DevBuf<float> d_ABf, d_KBf;
   DevBuf<double> d_kappa;  // per-cell kappa (optional)
   DevBuf<double> d_fprm, d_kprm;
-  DevBuf<double> d_fprep;  // d_fprm prepared for the element kernels (CoefDev::fprep)
+  DevBuf<double> d_fprep, d_kprep;  // d_fprm, d_kprm prepared for the element kernels (CoefDev::fprep)
   FieldSpec f, kappa;
   bool kappa_field = false, kappa_cells = false;
   // Trace matrix.  Host: block rows sorted by face id (h_browptr/h_bcol, the export pattern).
@@ -333,6 +338,7 @@ struct hdg_system {
   AmgHierarchy* amg = nullptr;      // multigrid preconditioner (symbolic part kept across reassembly)
   int amg_gen = 0;                  // count of symbolic setups (captured CG graphs hold their buffers)
   int last_max_iters = 0;           // most CG iterations of any problem in the last solve (scheduling hint)
+  DevBuf<int32_t> d_elem_list;      // cells the kappa-field element kernel leaves to the general one: count, ids
   std::vector<char> h_dir_face;     // faces whose dofs apply! prescribed (set by hdg_apply_dirichlet)
   ~hdg_system();
   // partials: 2 per segment; tickets: 4 per problem (CG product, CG update, residual, meandiag)

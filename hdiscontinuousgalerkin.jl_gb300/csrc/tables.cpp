@@ -252,6 +252,10 @@ RefLayout ref_layout(int nw, int nt, int nq) {
   L.ZV = o; o += nw;
   L.ZD = o; o += 2 * nw;
   L.ZF = o; o += 6 * nt;
+  L.RV = o; o += nw * nw;
+  L.RW = o; o += nw * (nw + 1) / 2 * nq;
+  L.RD = o; o += 2 * nw * nw;
+  L.RF = o; o += 6 * nw * nt;
   L.total = o;
   return L;
 }
@@ -394,7 +398,10 @@ bool build_ref_tables(int p, int qd, RefTables* t) {
       }
     }
     t->schur = ok && minpiv > 1e-10L * maxpiv;
-    std::vector<long double> inv((size_t)nw * nw, 0.0L);
+    t->positive = std::all_of(t->qw.begin(), t->qw.end(), [](double w) { return w > 0.0; });
+    std::vector<long double> inv((size_t)nw * nw, 0.0L), range((size_t)nw * nw, 0.0L);  // range: V, nr columns
+    int nr = nw;
+    for (int i = 0; i < nw; ++i) range[(size_t)i * nw + i] = 1.0L;
     if (t->schur) {
       for (int i = 0; i < nw; ++i)
         for (int j = 0; j < nw; ++j) inv[(size_t)i * nw + j] = a[(size_t)i * 2 * nw + nw + j];
@@ -415,6 +422,12 @@ bool build_ref_tables(int p, int qd, RefTables* t) {
       if (nul == 1 && low > 1e-6L * top) {
         t->schur = true;
         t->nullity = 1;
+        nr = 0;
+        for (int k = 0; k < nw; ++k) {
+          if (k == iz) continue;
+          for (int i = 0; i < nw; ++i) range[(size_t)i * (nw - 1) + nr] = vec[(size_t)i * nw + k];
+          ++nr;
+        }
         for (int k = 0; k < nw; ++k)
           if (k != iz)
             for (int i = 0; i < nw; ++i)
@@ -436,6 +449,30 @@ bool build_ref_tables(int p, int qd, RefTables* t) {
       }
     }
     if (t->schur) {
+      auto V = [&](int i, int k) { return range[(size_t)i * nr + k]; };
+      for (int i = 0; i < nw; ++i)
+        for (int k = 0; k < nr; ++k) P[L.RV + i * nr + k] = (double)V(i, k);
+      for (int q = 0; q < nq; ++q) {
+        std::vector<long double> v(nr, 0.0L);
+        for (int k = 0; k < nr; ++k)
+          for (int i = 0; i < nw; ++i) v[k] += V(i, k) * t->N[(size_t)i * nq + q];
+        for (int j = 0; j < nr; ++j)
+          for (int i = 0; i <= j; ++i) P[L.RW + (j * (j + 1) / 2 + i) * nq + q] = (double)(t->qw[q] * v[i] * v[j]);
+      }
+      for (int l = 0; l < 2; ++l)
+        for (int k = 0; k < nr; ++k)
+          for (int j = 0; j < nw; ++j) {
+            long double s = 0;
+            for (int i = 0; i < nw; ++i) s += V(i, k) * P[(l ? L.D1 : L.D0) + i * nw + j];
+            P[L.RD + (l * nr + k) * nw + j] = (double)s;
+          }
+      for (int fo = 0; fo < 6; ++fo)
+        for (int k = 0; k < nr; ++k)
+          for (int j = 0; j < nt; ++j) {
+            long double s = 0;
+            for (int i = 0; i < nw; ++i) s += V(i, k) * P[L.F + (fo * nw + i) * nt + j];
+            P[L.RF + (fo * nr + k) * nt + j] = (double)s;
+          }
       auto Mi = [&](int i, int j) { return inv[(size_t)i * nw + j]; };
       const double* D[2] = {&P[L.D0], &P[L.D1]};
       std::vector<long double> MD[2];

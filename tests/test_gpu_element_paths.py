@@ -56,3 +56,36 @@ def test_schur_blocks_match_full_elimination(H, monkeypatch, n, p, qd, kind):
     got = blocks(H, mesh, p, qd, f, **kw)
     monkeypatch.setenv("HDG_ELEMENT_FULL_LU", "1")
     check(got, blocks(H, mesh, p, qd, f, **kw))
+
+
+# kappa a field: an exponential of modes, one that changes its sign (those cells go to the pivoted kernel), bumps, a
+# constant
+@pytest.mark.parametrize("n", [1, 3, 5, 17])
+@pytest.mark.parametrize("p,qd", [(1, 2), (2, 3), (2, 4), (3, 6)])
+@pytest.mark.parametrize("kind", ["exp_fourier", "sign", "bumps", "const"])
+def test_field_blocks_match_full_elimination(H, monkeypatch, n, p, qd, kind):
+    rng = np.random.default_rng(1000 * n + 10 * p + qd)
+    mesh = H.rectangle_mesh(H.TriangleCell, (n, n), (0.0, 0.0), (1.0, 1.0))
+    mesh.jitter(0.2, 5)
+    modes = np.stack([rng.uniform(-1, 1, 17), rng.uniform(-1, 1, 17), rng.uniform(0, 6, 17), 0.2 * rng.standard_normal(17)], 1)
+    kappa = {"exp_fourier": H.Field.fourier(0.1, modes, exponential=True),
+             "sign": H.Field.fourier(0.0, [[0.5, 0.0, 0.0, 1.0]]),  # cos(pi x): negative for x > 1/2
+             "bumps": H.Field.bumps([[0.4, 0.6], [0.5, 0.5]], [0.3, 3.0], [2.0, 1.0]),
+             "const": H.Field.const(0.7)}[kind]
+    f = source(H, "fourier", rng)
+    got = blocks(H, mesh, p, qd, f, kappa=kappa)
+    monkeypatch.setenv("HDG_ELEMENT_FULL_LU", "1")
+    want = blocks(H, mesh, p, qd, f, kappa=kappa)
+    if kind != "sign":
+        check(got, want)
+        return
+    # a cell whose kappa changes its sign may be close to singular: only the definite ones are held to the bound
+    # (x < 0.3: no cell that reaches there touches x = 1/2 from n = 5 on); the others took the same kernel
+    xy, cells = H.get_vertices_matrix(mesh), H.getcells_matrix(mesh) - 1
+    right = xy[cells][:, :, 0].max(axis=1)
+    left = right < 0.45
+    check([x[left] for x in got], [x[left] for x in want])
+    far = xy[cells][:, :, 0].min(axis=1) > 0.55
+    if p != 1:  # one cell per warp there: exactly the cells with a negative value are left to it
+        for x, y in zip(got, want):
+            assert np.array_equal(x[far], y[far])
