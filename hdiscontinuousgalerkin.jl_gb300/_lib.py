@@ -95,6 +95,7 @@ SIGNATURES = {
     "hdg_system_kernel_sample": ([vp, ip, dp, dp, intp], ip),
     "hdg_refine": ([vp, C.POINTER(hdg_solver), ip, C.c_double, dp, C.POINTER(hdg_stats)], ip),
     "hdg_recover": ([vp, dp, dp, dp], ip),
+    "hdg_recover_into": ([vp, dp, dp, dp, ip], ip),
     "hdg_errornorm_l2sq": ([vp, C.POINTER(hdg_field), dp], ip),
     "hdg_nodal_avg": ([vp, dp], ip),
     "hdg_system_destroy": ([vp], ip),

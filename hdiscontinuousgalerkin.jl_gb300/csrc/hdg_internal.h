@@ -396,6 +396,9 @@ struct CgSolver {
 CgSolver* make_cg_solver(hdg_system* s);
 void mesh_concat(hdg_mesh* out, const std::vector<const hdg_mesh*>& parts);
 void launch_recover(hdg_system* s, cudaStream_t st);
+// The recovered q (ncells x nv) and u (ncells x nw) and the cells' trace values (ncells x 3 x nt, or ncells x nt x 3
+// by_function) as arrays of their own on the device; a NULL one is left out.
+void launch_recover_split(hdg_system* s, double* q, double* u, double* uhat_cell, bool by_function, cudaStream_t st);
 // The full [K_e | b_e] (ncells x n x (m+1), device) from the stored u rows (kb_u_only systems).
 void launch_expand_ke(hdg_system* s, double* out, cudaStream_t st);
 double run_errornorm(hdg_system* s, const FieldSpec& uex, cudaStream_t st);

@@ -100,6 +100,31 @@ __global__ void k_recover_u(const int nc, const int32_t* __restrict__ cells, con
   }
 }
 
+// q, u and the cells' trace values out of [q; u] and u_hat, a thread per value (grid-stride); bound by HBM, and small
+// beside the copies to the host that follow.
+__global__ void k_recover_split(const int64_t nc, const int nw, const int nt, const int32_t* __restrict__ cfaces,
+                                const double* __restrict__ qu, const double* __restrict__ x, double* __restrict__ q,
+                                double* __restrict__ u, double* __restrict__ uc, const bool by_function) {
+  const int nv = 2 * nw, n = nv + nw, m = 3 * nt;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x, t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (q)
+    for (int64_t t = t0; t < nc * nv; t += step) {
+      const int64_t c = t / nv;
+      q[t] = qu[c * n + (t - c * nv)];
+    }
+  if (u)
+    for (int64_t t = t0; t < nc * nw; t += step) {
+      const int64_t c = t / nw;
+      u[t] = qu[c * n + nv + (t - c * nw)];
+    }
+  if (uc)
+    for (int64_t t = t0; t < nc * m; t += step) {
+      const int64_t c = t / m;
+      const int k = (int)(t - c * m), f = by_function ? k % 3 : k / nt, j = by_function ? k / 3 : k % nt;
+      uc[t] = x[(int64_t)cfaces[3 * c + f] * nt + j];
+    }
+}
+
 template <int P>
 __global__ void k_errornorm(const int nc, const int32_t* __restrict__ cells, const double* __restrict__ xy,
                             const double* __restrict__ ref, int nq, int offN, int offQ, const double* __restrict__ qw,
@@ -266,6 +291,14 @@ void launch_recover(hdg_system* s, cudaStream_t st) {
     case 3: recover_p<3>(s, st); break;
     case 4: recover_p<4>(s, st); break;
   }
+}
+
+void launch_recover_split(hdg_system* s, double* q, double* u, double* uhat_cell, bool by_function, cudaStream_t st) {
+  const int64_t tot = (int64_t)s->nc * s->n;
+  k_recover_split<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 152 * 16), 256, 0, st>>>(
+      s->nc, s->nw, s->nt, s->space->mesh->d_cfaces.p, s->d_qu.p, s->d_x.p, q, u, uhat_cell, by_function);
+  HDG_CUDA(cudaGetLastError());
+  s->ctx->launches++;
 }
 
 double run_errornorm(hdg_system* s, const FieldSpec& uex, cudaStream_t st) {

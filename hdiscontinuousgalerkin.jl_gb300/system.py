@@ -134,7 +134,7 @@ class TraceSystem:
         o = L.hdg_solver(float(tol), int(maxit), int(self.precision if precision is None else precision), int(chunk),
                          float(inner_tol), int(preconditioner))
         st = L.hdg_stats()
-        out = np.zeros(self.ndofs) if to_host else None
+        out = np.empty(self.ndofs) if to_host else None
         L.check(L.load().hdg_solve(self._h, C.byref(o), None if refine else L.dptr(out), C.byref(st)), self.ctx)
         self.stats = SolveStats(st)
         if refine:
@@ -149,11 +149,20 @@ class TraceSystem:
             L.check(L.load().hdg_recover(self._h, None, None, None), self.ctx)
             return None
         nw = self.sp.nw
-        q = np.zeros((self.ncells, 2 * nw))
-        u = np.zeros((self.ncells, nw))
-        uc = np.zeros((self.ncells, 3, self.sp.nt))
+        q = np.empty((self.ncells, 2 * nw))
+        u = np.empty((self.ncells, nw))
+        uc = np.empty((self.ncells, 3, self.sp.nt))
         L.check(L.load().hdg_recover(self._h, L.dptr(q), L.dptr(u), L.dptr(uc)), self.ctx)
         return q, u, uc
+
+    def recover_into(self, q, u, uhat):
+        """Recovery straight into the caller's arrays: q (cells, nv), u (cells, nw) and the trace values (cells, nt, 3),
+        as the TrialFunctions hold them."""
+        nc, nw, nt = self.ncells, self.sp.nw, self.sp.nt
+        for a, shape in ((q, (nc, 2 * nw)), (u, (nc, nw)), (uhat, (nc, nt, 3))):
+            if a.shape != shape or a.dtype != np.float64 or not (a.flags.c_contiguous and a.flags.writeable):
+                raise ValueError(f"recover_into needs a contiguous float64 array of shape {shape}")
+        L.check(L.load().hdg_recover_into(self._h, L.dptr(q), L.dptr(u), L.dptr(uhat), 1), self.ctx)
 
     def timings(self) -> dict:
         """Per-phase device times recorded while the context's profiling was on (ms)."""
@@ -266,10 +275,16 @@ class TrialFunction:
 def get_usigma_(sigma_h: TrialFunction, u_h: TrialFunction, uhat_h: TrialFunction, uhat, K_e, b_e, mesh):
     """get_uσ! (examples/poisson2D_HDG.jl:197-212): recover q and u cell by cell on the device."""
     K = K_e.system if isinstance(K_e, _LocalView) else K_e
-    q, u, uc = K.recover()
-    sigma_h.m_values[:] = q
-    u_h.m_values[:] = u
-    uhat_h.m_values[:] = np.transpose(uc, (0, 2, 1))
+    out = (sigma_h.m_values, u_h.m_values, uhat_h.m_values)
+    shapes = ((K.ncells, 2 * K.sp.nw), (K.ncells, K.sp.nw), (K.ncells, K.sp.nt, 3))
+    if all(type(a) is np.ndarray and a.shape == s and a.dtype == np.float64 and a.flags.c_contiguous
+           and a.flags.writeable for a, s in zip(out, shapes)):
+        K.recover_into(*out)
+    else:  # values of another type, order or shape (broadcast as numpy does)
+        q, u, uc = K.recover()
+        out[0][:] = q
+        out[1][:] = u
+        out[2][:] = np.transpose(uc, (0, 2, 1))
     u_h.system = sigma_h.system = uhat_h.system = K
 
 
@@ -330,7 +345,7 @@ def solve_poisson(mesh, p: int, f, tau: float = 1.0, kappa=None, kappa_cell=None
     o = L.hdg_solver(float(tol), int(maxit), int(precision), 32, 1e-5, int(preconditioner))
     st = L.hdg_stats()
     nd = mesh.nfaces * sp.nt
-    uhat, q, u = np.zeros(nd), np.zeros((mesh.ncells, sp.nv)), np.zeros((mesh.ncells, sp.nw))
+    uhat, q, u = np.empty(nd), np.empty((mesh.ncells, sp.nv)), np.empty((mesh.ncells, sp.nw))
     L.check(L.load().hdg_solve_poisson(sp.h, float(tau), C.byref(fc), C.byref(kc) if kc is not None else None,
                                        L.dptr(kk), faceset.encode(), C.byref(gc), C.byref(o), L.dptr(uhat), L.dptr(q),
                                        L.dptr(u), C.byref(st)), mesh.ctx)

@@ -207,6 +207,9 @@ int hdg_refine(hdg_system* sys, const hdg_solver* opts, int steps, double correc
 /* get_uσ!, examples/poisson2D_HDG.jl:197-212 (trace slice for any nt): q (ncells x nv),
  * u (ncells x nw), uhat per cell (ncells x 3 x nt).  Host outputs; NULL skips a copy. */
 int hdg_recover(hdg_system* sys, double* q, double* u, double* uhat_cell);
+/* The same into arrays that the caller keeps; by_function != 0 lays the trace values out as ncells x nt x 3 (the
+ * m_values[cell, i, face] of a trace TrialFunction, src/DiscreteFunctions.jl:27-54). */
+int hdg_recover_into(hdg_system* sys, double* q, double* u, double* uhat_cell, int by_function);
 /* errornorm(u_h, u_ex), src/DiscreteFunctions.jl:97-120: the SQUARED L2 error of the last
  * recovery. */
 int hdg_errornorm_l2sq(hdg_system* sys, const hdg_field* u_exact, double* out);
