@@ -29,14 +29,10 @@
 #include <mutex>
 
 #include "cg_resident.cuh"
+#include "cg_sync.cuh"
 
 namespace {
 
-constexpr int RB = 512;                 // threads per CTA
-constexpr int MAX_CLUSTER = 16;
-constexpr int MAX_GRID = 256;           // CTAs whose partials fit the synchronisation buffer
-constexpr int SPIN_LIMIT = 1 << 22;
-constexpr size_t SMEM_MAX = 216 * 1024; // dynamic; the static part (reduction staging) is below 12 KB
 
 template <typename T> struct ResArgs {
   CgArgs<T> a;
@@ -61,165 +57,11 @@ template <int NT> __device__ __forceinline__ void load_z(const double* __restric
   }
 }
 
-struct Shared {
-  double stage[2][RB];
-  double part[2][RB / 4];
-  float2 ff[2][RB / 32];
-  double slot[2][MAX_CLUSTER][2];  // cluster: every CTA's partials, written by their owners
-  double bc;                       // broadcast within the CTA: alpha, beta
-  double rz, rz_inv;               // r.z and, formed off the critical path, its reciprocal
-  float bch, bcl;                  // alpha as a float-float pair
-  int status;
-};
-
-// The CTA's sums of NV values per thread, in lanes 0..NV-1 of warp 0.  FP64: four warps (one per scheduler) add four
-// values per lane, then one warp adds the rest, its lower lanes the first value's and its upper lanes the second's: as
-// few FP64 instructions as the depth of the tree allows.
-template <int NV> __device__ __forceinline__ double cta_sum(Shared& sh, const double (&v)[NV]) {
-  const int t = threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) sh.stage[i][t] = v[i];
-  __syncthreads();
-  if (t < RB / 4) {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const double* s = sh.stage[i] + t;
-      sh.part[i][t] = (s[0] + s[RB / 4]) + (s[RB / 2] + s[3 * RB / 4]);
-    }
-  }
-  __syncthreads();
-  if (t >= 32) return 0.0;
-  if constexpr (NV == 1) {
-    const double* s = sh.part[0] + t;
-    return warp_sum((s[0] + s[32]) + (s[64] + s[96]));
-  } else {
-    const double* s = sh.part[t >> 4] + (t & 15);
-    double x = ((s[0] + s[16]) + (s[32] + s[48])) + ((s[64] + s[80]) + (s[96] + s[112]));
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    return __shfl_sync(0xffffffffu, x, (t & 1) << 4);  // lane i: value i
-  }
-}
-template <int NV> __device__ __forceinline__ double cta_sum(Shared& sh, const FF (&v)[NV]) {
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const FF t = warp_sum(v[i]);
-    if (l == 0) sh.ff[i][w] = make_float2(t.hi, t.lo);
-  }
-  __syncthreads();
-  double out = 0.0;
-  if (w == 0) {
-#pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      FF t;
-      if (l < RB / 32) {
-        t.hi = sh.ff[i][l].x;
-        t.lo = sh.ff[i][l].y;
-      }
-      t = warp_sum(t);
-      if (l == i) out = t.to_double();
-    }
-  }
-  return out;
-}
-
-// 1/d to an ulp: the hardware's approximation (some 20 bits) and two Newton steps, each squaring the error; a third of
-// a division's latency.  Outside the range where neither the estimate nor the steps under- or overflow: the division.
-__device__ __forceinline__ double recip(double d) {
-  if (!(fabs(d) > 1e-290 && fabs(d) < 1e290)) return 1.0 / d;
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  r = fma(r, fma(-d, r, 1.0), r);
-  return fma(r, fma(-d, r, 1.0), r);
-}
-
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// The sums over all CTAs of the CTA sums `mine` (lanes 0..NV-1 of warp 0), valid in every lane of warp 0; what any
-// thread wrote to global memory before is visible to every CTA after its next __syncthreads.  Returns false (in warp 0)
-// when the barrier gave up.  Contains barriers: every thread calls it.
-template <bool GRID, int NV>
-__device__ __forceinline__ bool all_sum(Shared& sh, unsigned* count, double* part, int epoch, double mine,
-                                        double (&out)[NV]) {
-  const int par = epoch & 1, l = threadIdx.x & 31;
-  bool ok = true;
-  if constexpr (GRID) {
-    __syncthreads();  // the CTA's writes before this point are ordered before lane 0's release
-    if (threadIdx.x < 32) {
-      double* slot = part + (size_t)par * MAX_GRID * 2;
-      if (l < NV) __stcg(slot + 2 * blockIdx.x + l, mine);
-      __syncwarp();
-      if (l == 0) {  // release: the CTA's writes; acquire: every other CTA's
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
-        const unsigned want = (unsigned)(epoch + 1) * gridDim.x;
-        unsigned seen;
-        int n = 0;
-        do {
-          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
-          if (++n > SPIN_LIMIT) {
-            ok = false;
-            break;
-          }
-        } while (seen < want);
-      }
-      ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-      // all partials are loaded before the first is added (one L2 latency)
-      constexpr int PER = MAX_GRID / 32;
-      double2 v[PER];
-#pragma unroll
-      for (int k = 0; k < PER; ++k)
-        v[k] = (l + 32 * k < (int)gridDim.x) ? __ldcg(reinterpret_cast<const double2*>(slot) + l + 32 * k)
-                                             : make_double2(0.0, 0.0);
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        double t[PER];
-#pragma unroll
-        for (int k = 0; k < PER; ++k) t[k] = i ? v[k].y : v[k].x;
-#pragma unroll
-        for (int o = PER / 2; o > 0; o >>= 1)
-#pragma unroll
-          for (int k = 0; k < o; ++k)
-            if (32 * (k + o) < (int)gridDim.x) t[k] += t[k + o];
-        out[i] = warp_sum(t[0]);
-      }
-    }
-  } else {
-    uint32_t me;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(me));
-    if (threadIdx.x < 32) {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const double v = __shfl_sync(0xffffffffu, mine, i);
-        if (l < MAX_CLUSTER) {
-          uint32_t to;
-          const uint32_t at = (uint32_t)__cvta_generic_to_shared(&sh.slot[par][me][i]);
-          asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(l));
-          asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(v) : "memory");
-        }
-      }
-    }
-    cluster_sync_all();
-    if (threadIdx.x < 32) {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        double t = sh.slot[par][l & (MAX_CLUSTER - 1)][i];
-#pragma unroll
-        for (int o = MAX_CLUSTER / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        out[i] = t;
-      }
-    }
-  }
-  return ok;
-}
-
 template <int NT, typename T, bool GRID, bool MAT>
 __global__ void __launch_bounds__(RB, 1) k_cg_resident(ResArgs<T> q) {
   constexpr bool F64 = sizeof(T) == sizeof(double);
   const CgArgs<T>& a = q.a;
-  __shared__ Shared sh;
+  __shared__ ResShared sh;
   extern __shared__ __align__(16) unsigned char dyn[];
   const int fpc = q.faces_per_cta, cap = fpc * NT;
   const int f0 = blockIdx.x * fpc, nfl = max(0, min(fpc, a.nf - f0)), nr = nfl * NT, row0 = f0 * NT;
@@ -446,22 +288,7 @@ template <int NT, typename T, bool GRID, bool MAT> void set_attributes() {
 
 template <int NT, typename T, bool MAT> int max_clusters(int ctas, size_t smem) {
   set_attributes<NT, T, false, MAT>();
-  cudaLaunchConfig_t cf = {};
-  cf.gridDim = dim3((unsigned)ctas);
-  cf.blockDim = dim3(RB);
-  cf.dynamicSmemBytes = smem;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = (unsigned)ctas;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cf.attrs = &at;
-  cf.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_cg_resident<NT, T, false, MAT>, &cf) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return n;
+  return res_max_clusters(k_cg_resident<NT, T, false, MAT>, ctas, smem);
 }
 
 // Rows up to which one cluster is the faster form: beyond, the rows' arithmetic on 16 SMs costs more than the
@@ -470,18 +297,9 @@ template <int NT, typename T, bool MAT> int max_clusters(int ctas, size_t smem) 
 // 30.8k rows 18.0 / 15.8 ms.
 template <typename T> constexpr int cluster_rows() { return sizeof(T) == sizeof(double) ? 11000 : 20000; }
 
-int forced_kind() {  // HDG_CG_RESIDENT=none|cluster|grid (where it fits)
-  const char* e = std::getenv("HDG_CG_RESIDENT");
-  if (!e) return -1;
-  if (std::strcmp(e, "none") == 0) return (int)CgResident::NONE;
-  if (std::strcmp(e, "cluster") == 0) return (int)CgResident::CLUSTER;
-  if (std::strcmp(e, "grid") == 0) return (int)CgResident::GRID;
-  return -1;
-}
-
 template <int NT, typename T> CgResident plan_nt(int nf, int device) {
   CgResident pl;
-  const int forced = forced_kind();
+  const int forced = res_forced_kind();
   if (forced == CgResident::NONE) return pl;
   const int64_t rows = (int64_t)nf * NT;
   if (forced != CgResident::GRID && (rows <= cluster_rows<T>() || forced == CgResident::CLUSTER)) {
@@ -493,10 +311,8 @@ template <int NT, typename T> CgResident plan_nt(int nf, int device) {
       return CgResident{CgResident::CLUSTER, c, fpc, mat != 0, sm};
     }
   }
-  int sms = 0, coop = 0;
-  HDG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  HDG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
-  if (!coop || sms > MAX_GRID) return pl;
+  int sms = 0;
+  if ((sms = res_grid_ctas(device)) == 0) return pl;
   const int fpc = (nf + sms - 1) / sms;
   for (int mat = 1; mat >= 0; --mat) {
     const size_t sm = res_smem<NT, T>(fpc, mat);
@@ -505,44 +321,11 @@ template <int NT, typename T> CgResident plan_nt(int nf, int device) {
   return pl;  // the vectors do not fit on the chip
 }
 
-// Cooperative launches of this process on one device follow one another: two grids that each hold a part of the
-// SMs would wait for the rest of them.
-struct GridTurn {
-  std::mutex mu;
-  cudaEvent_t last = nullptr;
-};
-GridTurn& grid_turn(int device) {
-  static GridTurn t[64];
-  return t[device & 63];
-}
-
 template <int NT, typename T, bool GRID, bool MAT>
 void launch_one(const CgResident& pl, ResArgs<T> q, int device, cudaStream_t st) {
   set_attributes<NT, T, GRID, MAT>();
-  auto* k = k_cg_resident<NT, T, GRID, MAT>;
-  if constexpr (GRID) {
-    HDG_CUDA(cudaMemsetAsync(q.count, 0, sizeof(unsigned), st));
-    GridTurn& turn = grid_turn(device);
-    std::lock_guard<std::mutex> lk(turn.mu);
-    if (!turn.last) HDG_CUDA(cudaEventCreateWithFlags(&turn.last, cudaEventDisableTiming));
-    HDG_CUDA(cudaStreamWaitEvent(st, turn.last, 0));
-    void* args[] = {&q};
-    HDG_CUDA(cudaLaunchCooperativeKernel((const void*)k, dim3(pl.ctas), dim3(RB), args, pl.smem, st));
-    HDG_CUDA(cudaEventRecord(turn.last, st));
-  } else {
-    cudaLaunchConfig_t cf = {};
-    cf.gridDim = dim3((unsigned)pl.ctas);
-    cf.blockDim = dim3(RB);
-    cf.dynamicSmemBytes = pl.smem;
-    cf.stream = st;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)pl.ctas;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cf.attrs = &at;
-    cf.numAttrs = 1;
-    HDG_CUDA(cudaLaunchKernelEx(&cf, k, q));
-  }
+  if (GRID) HDG_CUDA(cudaMemsetAsync(q.count, 0, sizeof(unsigned), st));
+  res_launch<GRID>(k_cg_resident<NT, T, GRID, MAT>, pl.ctas, pl.smem, q, device, st);
 }
 
 template <int NT, typename T>

@@ -12,10 +12,11 @@
 //  * apply! (src/boundary.jl:121-158, APPLY_TRANSPOSE): b -= v K[:, d] for the prescribed dofs
 //    in increasing order, prescribed rows and columns zeroed, K[d, d] = mean |diag K|,
 //    b[d] = v mean |diag K|.
-//  * K \ b (poisson2D_CG.jl:126) by Jacobi-preconditioned CG in FP64.  Two kernels per
-//    iteration; the dot products are per-block partial sums that every block of the next kernel
-//    adds in the same fixed order, so all blocks take the same decisions and the result is
-//    reproducible.
+//  * K \ b (poisson2D_CG.jl:126) by Jacobi-preconditioned CG in FP64, many iterations per launch with
+//    the vectors resident on the chip (k_lag_resident; the reductions are those of cg_sync.cuh).  Above
+//    the rows that fit, two kernels per iteration; the dot products are per-block partial sums that
+//    every block of the next kernel adds in the same fixed order.  Either way all blocks take the
+//    same decisions and the result is reproducible.
 //  * errornorm (src/DiscreteFunctions.jl:97-120): sum over cells and points of
 //    (u_h(x_q) - u(x_q))^2 detJ w_q.
 #include <algorithm>
@@ -23,6 +24,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cg_sync.cuh"
 #include "hdg_device.cuh"
 
 struct hdg_lagrange {
@@ -44,6 +46,15 @@ struct hdg_lagrange {
   DevBuf<int32_t> d_err;
   bool assembled = false, applied = false, solved = false;
   std::vector<int32_t> h_colptr, h_rowval;
+  // resident CG: every CTA's rows in slots of 32 of similar length, their entries 32-row slices apart
+  CgResident res;
+  int slots = 0;                          // per CTA (a multiple of 32)
+  DevBuf<int32_t> d_srow;                 // [ctas * slots] row of a slot, -1: none
+  DevBuf<int32_t> d_sdiag;                // its diagonal entry's place in the CSC values (-1: none)
+  DevBuf<int64_t> d_sptr;                 // [ctas * slots / 32 + 1] first entry of a slice
+  DevBuf<int32_t> d_scol, d_ssrc;         // entries: column, place in the CSC values (-1: padding)
+  DevBuf<double> d_sval;
+  DevBuf<unsigned char> d_sync;
 };
 
 namespace {
@@ -351,6 +362,338 @@ __global__ void k_lag_errornorm(int nc, int nl, int nq, const double* __restrict
 
 unsigned nblk(int64_t n, int t = 256) { return (unsigned)std::max<int64_t>(1, (n + t - 1) / t); }
 
+// ---- resident Jacobi-PCG --------------------------------------------------------------------------
+// The iteration of k_lag_cg_a/b with the q recurrence of cg.cu (q = K z + beta q needs one product term per entry where
+// K (z + beta p) formed on the fly needs two), many iterations per launch.  A CTA owns a range of rows; its slots of x, r, p,
+// q, D^-1 and z stay in shared memory, z travels through L2, the matrix is read from L2 slice by slice (a warp a slice of 32
+// rows, entry k of its rows in consecutive addresses; the rows of a CTA are sorted by length, since P2 rows have 9 or 19
+// entries) or kept in shared memory where it fits.  Measured at P2 on 2*256^2 cells (263169 rows, 3.0 M entries):
+// two kernels per iteration 47 us (thread-per-column walks of the CSC arrays, 2 x 592 partials added by every block), here
+// 19 us; 10 x 10 cells P1, assembly and solve together, 0.92 ms before, 0.37 ms here.
+struct LagRes {
+  int n, slots, iters, maxit, fresh;
+  double tol2;
+  const int32_t *srow, *sdiag, *scol;
+  const int64_t* sptr;
+  const double *sval, *val, *b;
+  double *x, *r, *z, *p, *q, *sc;  // sc: [1] b.b, [2] r.z, [3] beta, [4] status, [5] iterations, [6] r.r
+  unsigned* count;
+  double* part;
+};
+
+template <bool GRID, bool MAT> __global__ void __launch_bounds__(RB, 1) k_lag_resident(LagRes a) {
+  __shared__ ResShared sh;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  const int S = a.slots;
+  double* sx = reinterpret_cast<double*>(dyn);
+  double *sr = sx + S, *sp = sr + S, *sq = sp + S, *sd = sq + S, *sz = sd + S;
+  int32_t* row = reinterpret_cast<int32_t*>(sz + S);
+  const int64_t slice0 = (int64_t)blockIdx.x * (S / 32), e0 = a.sptr[slice0], ne = a.sptr[slice0 + S / 32] - e0;
+  int32_t* first = row + S;  // [S / 32 + 1] first entry of a slice, from e0
+  double* mv = reinterpret_cast<double*>(first + ((S / 32 + 2) & ~1));
+  int32_t* mc = reinterpret_cast<int32_t*>(mv + (MAT ? ne : 0));
+  double rz = 0.0, rr = 0.0, bb = 0.0, beta0 = 0.0;
+  int status = 0, it = 0;
+  if (!a.fresh) {
+    bb = a.sc[1];
+    rz = a.sc[2];
+    beta0 = a.sc[3];
+    status = (int)a.sc[4];
+    it = (int)a.sc[5];
+    rr = a.sc[6];
+    if (status != 0) return;  // uniform over the grid
+  }
+  for (int l = threadIdx.x; l <= S / 32; l += RB) first[l] = (int32_t)(a.sptr[slice0 + l] - e0);
+  if constexpr (MAT)
+    for (int64_t k = threadIdx.x; k < ne; k += RB) {
+      mv[k] = a.sval[e0 + k];
+      mc[k] = a.scol[e0 + k];
+    }
+  double rz0 = 0.0, rr0 = 0.0;
+  for (int l = threadIdx.x; l < S; l += RB) {
+    const int64_t g = (int64_t)blockIdx.x * S + l;
+    const int i = a.srow[g];
+    row[l] = i;
+    double x = 0.0, r = 0.0, p = 0.0, q = 0.0, d = 0.0, z = 0.0;
+    if (i >= 0) {
+      const int at = a.sdiag[g];
+      const double dv = at >= 0 ? a.val[at] : 0.0;
+      d = dv != 0.0 ? 1.0 / dv : 1.0;
+      if (a.fresh) {
+        r = a.b[i];
+        z = d * r;
+        a.z[i] = z;
+        rz0 += r * z;
+        rr0 += r * r;
+      } else {
+        x = a.x[i];
+        r = a.r[i];
+        p = a.p[i];
+        q = a.q[i];
+        z = a.z[i];
+      }
+    }
+    sx[l] = x;
+    sr[l] = r;
+    sp[l] = p;
+    sq[l] = q;
+    sd[l] = d;
+    sz[l] = z;
+  }
+  int epoch = 0;
+  if constexpr (!GRID) cluster_sync_all();  // every CTA of the cluster runs before its shared memory is written
+  if (a.fresh) {
+    double s0[2];
+    const double mine = cta_sum<2>(sh, {rz0, rr0});
+    const bool ok = all_sum<GRID, 2>(sh, a.count, a.part, epoch++, mine, s0);
+    if (threadIdx.x == 0) {
+      rz = s0[0];
+      rr = bb = s0[1];
+      sh.status = !ok ? CG_LOST : ((rr <= a.tol2 * bb) ? 1 : ((rr == rr) ? (a.maxit <= 0 ? 2 : 0) : 3));
+    }
+    __syncthreads();
+    status = sh.status;
+  }
+  const double stop_rr = a.tol2 * bb;  // of thread 0, as rz, rr and bb
+  double pq = 0.0, alpha = 0.0, beta = beta0;
+  if (threadIdx.x == 0) sh.rz = rz;
+  __syncthreads();
+  for (int n = 0; n < a.iters && status == 0; ++n) {
+    const double bt = n == 0 ? beta0 : sh.bc;
+    if (threadIdx.x == RB - 1) sh.rz_inv = recip(sh.rz);
+    double dpq = 0.0;
+    for (int l = threadIdx.x; l < S; l += RB) {
+      const int k0 = first[l >> 5] + (l & 31), k1 = first[(l >> 5) + 1];
+      double w = 0.0;
+#pragma unroll 8
+      for (int k = k0; k < k1; k += 32) {
+        const int c = MAT ? mc[k] : __ldg(a.scol + e0 + k);
+        w += (MAT ? mv[k] : __ldg(a.sval + e0 + k)) * __ldcg(a.z + c);
+      }
+      const double pn = sz[l] + bt * sp[l], qn = w + bt * sq[l];
+      sp[l] = pn;
+      sq[l] = qn;
+      dpq += pn * qn;
+    }
+    {
+      double s1[1];
+      const double mine = cta_sum<1>(sh, {dpq});
+      const bool ok = all_sum<GRID, 1>(sh, a.count, a.part, epoch++, mine, s1);
+      if (threadIdx.x == 0) {
+        pq = s1[0];
+        alpha = (pq > 0.0) ? rz * recip(pq) : 0.0;
+        sh.bc = alpha;
+        sh.status = ok ? 0 : CG_LOST;
+      }
+    }
+    __syncthreads();
+    if (sh.status != 0) {
+      status = CG_LOST;
+      break;
+    }
+    const double at = sh.bc;
+    double drz = 0.0, drr = 0.0;
+    for (int l = threadIdx.x; l < S; l += RB) {
+      sx[l] += at * sp[l];
+      const double rn = sr[l] - at * sq[l], zn = sd[l] * rn;
+      sr[l] = rn;
+      sz[l] = zn;
+      if (row[l] >= 0) a.z[row[l]] = zn;
+      drz += rn * zn;
+      drr += rn * rn;
+    }
+    {
+      double s2[2];
+      const double mine = cta_sum<2>(sh, {drz, drr});
+      const bool ok = all_sum<GRID, 2>(sh, a.count, a.part, epoch++, mine, s2);
+      if (threadIdx.x == 0) {
+        rz = s2[0];
+        rr = s2[1];
+        beta = rz * sh.rz_inv;
+        sh.bc = beta;
+        sh.rz = rz;
+        // converged, non-finite, or at the cap (the order of k_lag_cg_a)
+        sh.status = !ok ? CG_LOST : (rr <= stop_rr ? 1 : (!(rr == rr) ? 3 : (it + 1 >= a.maxit ? 2 : 0)));
+      }
+    }
+    __syncthreads();
+    status = sh.status;
+    if (status == CG_LOST) break;
+    ++it;
+  }
+  for (int l = threadIdx.x; l < S; l += RB)
+    if (row[l] >= 0) {
+      const int i = row[l];
+      a.x[i] = sx[l];
+      a.r[i] = sr[l];
+      a.p[i] = sp[l];
+      a.q[i] = sq[l];
+    }
+  if (threadIdx.x == 0 && blockIdx.x == 0) {
+    a.sc[1] = bb;
+    a.sc[2] = rz;
+    a.sc[3] = beta;
+    a.sc[5] = it;
+    a.sc[6] = rr;
+  }
+  if (threadIdx.x == 0 && (blockIdx.x == 0 || status == CG_LOST)) a.sc[4] = status;
+}
+
+__global__ void k_lag_slices(int64_t n, const int32_t* __restrict__ src, const double* __restrict__ val,
+                             double* __restrict__ out) {
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
+    out[k] = src[k] >= 0 ? val[src[k]] : 0.0;
+}
+
+constexpr int LAG_CLUSTER_ROWS = 11000;  // up to here one cluster (as the FP64 iteration of cg_resident.cu)
+
+size_t lag_smem(int slots, int64_t entries) {
+  return sizeof(double) * 6 * (size_t)slots + sizeof(int32_t) * ((size_t)slots + ((slots / 32 + 2) & ~1)) +
+         (sizeof(double) + sizeof(int32_t)) * (size_t)entries;
+}
+
+template <bool GRID, bool MAT> void lag_attributes() {
+  HDG_CUDA(cudaFuncSetAttribute(k_lag_resident<GRID, MAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+  if (!GRID) HDG_CUDA(cudaFuncSetAttribute(k_lag_resident<GRID, MAT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+}
+
+// The slots and slices of the resident iteration; L->res stays NONE where the vectors do not fit on the chip.
+void lag_plan(hdg_lagrange* L) {
+  const int n = L->ndofs, forced = res_forced_kind();
+  L->res = CgResident{};
+  if (forced == CgResident::NONE) return;
+  const int grid = res_grid_ctas(L->ctx->device);
+  CgResident::Kind kind = CgResident::GRID;
+  if (forced != CgResident::GRID && (n <= LAG_CLUSTER_ROWS || forced == CgResident::CLUSTER)) kind = CgResident::CLUSTER;
+  for (;; kind = CgResident::GRID) {
+    const int ctas = kind == CgResident::CLUSTER ? MAX_CLUSTER : grid;
+    if (ctas > 0) {
+      const int per = (n + ctas - 1) / ctas, slots = (per + 31) / 32 * 32;
+      // rows of every CTA by length (longest first, rows of one length in order), slices as long as their longest row
+      std::vector<int32_t> srow((size_t)ctas * slots, -1), order;
+      std::vector<int64_t> sptr(1, 0);
+      int64_t most = 0;
+      auto len = [&](int i) { return L->h_colptr[i + 1] - L->h_colptr[i]; };
+      for (int c = 0; c < ctas; ++c) {
+        const int r0 = std::min(n, c * per), r1 = std::min(n, r0 + per);
+        order.resize(r1 - r0);
+        for (int i = r0; i < r1; ++i) order[i - r0] = i;
+        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return len(x) > len(y); });
+        std::copy(order.begin(), order.end(), srow.begin() + (size_t)c * slots);
+        const int64_t at = sptr.back();
+        for (int s = 0; s < slots; s += 32)
+          sptr.push_back(sptr.back() + 32 * (int64_t)(s < r1 - r0 ? len(order[s]) : 0));
+        most = std::max(most, sptr.back() - at);
+      }
+      const bool small = lag_smem(slots, 0) <= SMEM_MAX, mat = lag_smem(slots, most) <= SMEM_MAX;
+      const size_t smem = lag_smem(slots, mat ? most : 0);
+      bool fits = small;
+      if (fits && kind == CgResident::CLUSTER) {
+        lag_attributes<false, true>();
+        lag_attributes<false, false>();
+        fits = (mat ? res_max_clusters(k_lag_resident<false, true>, ctas, smem)
+                    : res_max_clusters(k_lag_resident<false, false>, ctas, smem)) >= 1;
+      }
+      if (fits) {
+        std::vector<int32_t> scol((size_t)sptr.back(), 0), ssrc((size_t)sptr.back(), -1), sdiag(srow.size(), -1);
+        for (size_t g = 0; g < srow.size(); ++g) {
+          const int64_t base = sptr[g / 32] + (int64_t)(g % 32), end = sptr[g / 32 + 1];
+          const int i = srow[g];
+          int64_t k = base;
+          if (i >= 0)
+            for (int e = L->h_colptr[i]; e < L->h_colptr[i + 1]; ++e, k += 32) {
+              scol[k] = L->h_rowval[e];
+              ssrc[k] = e;
+              if (L->h_rowval[e] == i) sdiag[g] = e;
+            }
+          for (; k < end; k += 32) scol[k] = i >= 0 ? i : 0;  // padding: zero times a value that is there
+        }
+        cudaStream_t st = L->ctx->stream;
+        L->d_srow.upload(srow.data(), srow.size(), st);
+        L->d_sdiag.upload(sdiag.data(), sdiag.size(), st);
+        L->d_sptr.upload(sptr.data(), sptr.size(), st);
+        L->d_scol.upload(scol.data(), scol.size(), st);
+        L->d_ssrc.upload(ssrc.data(), ssrc.size(), st);
+        L->d_sval.alloc(scol.size());
+        L->d_sync.alloc(CG_SYNC_BYTES);
+        HDG_CUDA(cudaStreamSynchronize(st));
+        L->slots = slots;
+        L->res = CgResident{kind, ctas, 0, mat, smem};
+        return;
+      }
+    }
+    if (kind == CgResident::GRID) return;
+  }
+}
+
+int lag_solve_resident(hdg_lagrange* L, double tol, int maxit, double* sc) {
+  cudaStream_t st = L->ctx->stream;
+  const int n = L->ndofs;
+  L->d_x.alloc(n); L->d_r.alloc(n); L->d_z.alloc(n); L->d_p.alloc(n); L->d_q.alloc(n);
+  k_lag_slices<<<(unsigned)std::min<int64_t>(((int64_t)L->d_scol.n + 255) / 256, 152 * 16), 256, 0, st>>>(
+      (int64_t)L->d_scol.n, L->d_ssrc.p, L->d_val.p, L->d_sval.p);
+  HDG_CUDA(cudaGetLastError());
+  L->ctx->launches++;
+  constexpr int ITERS = 512;  // per launch; a launch's end costs a host round trip
+  for (int first = 1;; first = 0) {
+    const bool grid = L->res.kind == CgResident::GRID, mat = L->res.mat_smem;
+    LagRes a{n, L->slots, ITERS, maxit, first, tol * tol, L->d_srow.p, L->d_sdiag.p, L->d_scol.p, L->d_sptr.p, L->d_sval.p,
+             L->d_val.p, L->d_b.p, L->d_x.p, L->d_r.p, L->d_z.p, L->d_p.p, L->d_q.p, L->d_sc.p,
+             (unsigned*)L->d_sync.p, (double*)(L->d_sync.p + 256)};
+    if (grid) HDG_CUDA(cudaMemsetAsync(L->d_sync.p, 0, sizeof(unsigned), st));
+    const int dev = L->ctx->device, ct = L->res.ctas;
+    const size_t sm = L->res.smem;
+    if (grid && mat) {
+      lag_attributes<true, true>();
+      res_launch<true>(k_lag_resident<true, true>, ct, sm, a, dev, st);
+    } else if (grid) {
+      lag_attributes<true, false>();
+      res_launch<true>(k_lag_resident<true, false>, ct, sm, a, dev, st);
+    } else if (mat) {
+      lag_attributes<false, true>();
+      res_launch<false>(k_lag_resident<false, true>, ct, sm, a, dev, st);
+    } else {
+      lag_attributes<false, false>();
+      res_launch<false>(k_lag_resident<false, false>, ct, sm, a, dev, st);
+    }
+    L->ctx->launches++;
+    HDG_CUDA(cudaMemcpyAsync(sc, L->d_sc.p, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    HDG_CUDA(cudaStreamSynchronize(st));
+    if (sc[4] != 0.0) return (int)sc[4];
+  }
+}
+
+// The iteration as two kernels, for systems whose vectors do not fit on the chip.
+void lag_solve_launched(hdg_lagrange* L, double tol, int maxit, double* sc) {
+  cudaStream_t st = L->ctx->stream;
+  const int n = L->ndofs;
+  const int nb = (int)std::min<int64_t>(nblk(n, LB), LMAX_BLOCKS);
+  L->d_x.alloc(n); L->d_r.alloc(n); L->d_z.alloc(n); L->d_p.alloc(n); L->d_p2.alloc(n); L->d_q.alloc(n);
+  L->d_dinv.alloc(n);
+  L->d_part.alloc((size_t)3 * nb);
+  HDG_CUDA(cudaMemsetAsync(L->d_sc.p + 1, 0, sizeof(double) * 7, st));
+  k_lag_cg_init<<<nb, LB, 0, st>>>(n, L->d_colptr.p, L->d_rowval.p, L->d_val.p, L->d_b.p, L->d_x.p, L->d_r.p,
+                                   L->d_z.p, L->d_p.p, L->d_dinv.p, L->d_part.p, nb);
+  L->ctx->launches++;
+  constexpr int CHUNK = 32;
+  int it = 0;
+  for (;;) {
+    for (int k = 0; k < CHUNK; ++k, ++it) {
+      double* pold = (it & 1) ? L->d_p2.p : L->d_p.p;
+      double* pnew = (it & 1) ? L->d_p.p : L->d_p2.p;
+      k_lag_cg_a<<<nb, LB, 0, st>>>(n, L->d_colptr.p, L->d_rowval.p, L->d_val.p, L->d_z.p, pold, pnew, L->d_q.p,
+                                    L->d_part.p, L->d_sc.p, nb, it, maxit, tol * tol);
+      k_lag_cg_b<<<nb, LB, 0, st>>>(n, pnew, L->d_q.p, L->d_dinv.p, L->d_x.p, L->d_r.p, L->d_z.p, L->d_part.p,
+                                    L->d_sc.p, nb, it);
+    }
+    HDG_CUDA(cudaGetLastError());
+    L->ctx->launches += 2 * CHUNK;
+    HDG_CUDA(cudaMemcpyAsync(sc, L->d_sc.p, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    HDG_CUDA(cudaStreamSynchronize(st));
+    if (sc[4] != 0.0) break;
+  }
+}
+
 // contributions of (cell, i[, j]) to the stored entries / dofs, in cell order
 void build_contributions(hdg_lagrange* L, const std::vector<int32_t>& cd) {
   const int nc = L->nc, nl = L->nl;
@@ -456,6 +799,7 @@ int hdg_lagrange_create(hdg_ctx* ctx, const hdg_mesh* mesh, int order, int quad_
     L->d_b.alloc(ndofs);
     L->d_err.alloc(1);
     L->d_sc.alloc(8);
+    lag_plan(L);
     return HDG_OK;
   });
   if (rc != HDG_OK) {
@@ -556,31 +900,12 @@ int hdg_lagrange_solve(hdg_lagrange* L, const hdg_solver* opts, double* u, hdg_s
     const int maxit = (opts && opts->maxit > 0) ? opts->maxit : 100000;
     cudaStream_t st = L->ctx->stream;
     const int n = L->ndofs;
-    const int nb = (int)std::min<int64_t>(nblk(n, LB), LMAX_BLOCKS);
-    L->d_x.alloc(n); L->d_r.alloc(n); L->d_z.alloc(n); L->d_p.alloc(n); L->d_p2.alloc(n); L->d_q.alloc(n);
-    L->d_dinv.alloc(n);
-    L->d_part.alloc((size_t)3 * nb);
-    HDG_CUDA(cudaMemsetAsync(L->d_sc.p + 1, 0, sizeof(double) * 7, st));
-    k_lag_cg_init<<<nb, LB, 0, st>>>(n, L->d_colptr.p, L->d_rowval.p, L->d_val.p, L->d_b.p, L->d_x.p, L->d_r.p,
-                                     L->d_z.p, L->d_p.p, L->d_dinv.p, L->d_part.p, nb);
-    L->ctx->launches++;
-    constexpr int CHUNK = 32;
     double sc[8];
-    int it = 0;
-    for (;;) {
-      for (int k = 0; k < CHUNK; ++k, ++it) {
-        double* pold = (it & 1) ? L->d_p2.p : L->d_p.p;
-        double* pnew = (it & 1) ? L->d_p.p : L->d_p2.p;
-        k_lag_cg_a<<<nb, LB, 0, st>>>(n, L->d_colptr.p, L->d_rowval.p, L->d_val.p, L->d_z.p, pold, pnew, L->d_q.p,
-                                      L->d_part.p, L->d_sc.p, nb, it, maxit, tol * tol);
-        k_lag_cg_b<<<nb, LB, 0, st>>>(n, pnew, L->d_q.p, L->d_dinv.p, L->d_x.p, L->d_r.p, L->d_z.p, L->d_part.p,
-                                      L->d_sc.p, nb, it);
-      }
-      HDG_CUDA(cudaGetLastError());
-      L->ctx->launches += 2 * CHUNK;
-      HDG_CUDA(cudaMemcpyAsync(sc, L->d_sc.p, sizeof(sc), cudaMemcpyDeviceToHost, st));
-      HDG_CUDA(cudaStreamSynchronize(st));
-      if (sc[4] != 0.0) break;
+    if (L->res.kind != CgResident::NONE) {
+      if (lag_solve_resident(L, tol, maxit, sc) == CG_LOST)
+        throw HdgError{HDG_ERR_CUDA, "a barrier of the resident CG iteration gave up"};
+    } else {
+      lag_solve_launched(L, tol, maxit, sc);
     }
     const int status = (int)sc[4];
     if (stats) {
