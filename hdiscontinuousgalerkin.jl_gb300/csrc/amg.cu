@@ -1058,12 +1058,75 @@ __global__ void k_amg_dp0(int nf, const int8_t* __restrict__ kdiag, const float*
     }
 }
 
-// Level-0 value storage of the cycle: FP32 or FP16, read as FP32.
-template <typename VT> __device__ __forceinline__ VT to_vt(float v);
-template <> __device__ __forceinline__ float to_vt<float>(float v) { return v; }
-template <> __device__ __forceinline__ __half to_vt<__half>(float v) { return __float2half_rn(v); }
-__device__ __forceinline__ float ldv(const float* p) { return *p; }
-__device__ __forceinline__ float ldv(const __half* p) { return __half2float(*p); }
+// Level-0 values of the cycle, D^-1 A0, read as FP32.
+//  FP16 (default): the 5 nt^2 values of a face in the order [row i][slot k][column j], padded to chunks of eight and laid
+//  out chunk by chunk over the faces, so that a thread reads its face in 16-byte loads that are contiguous over a warp
+//  (16 loads at nt = 5; one 2-byte load per value, as in the row-contiguous layout, kept the sweeps at half the
+//  bandwidth: see k_amg_face_cheb).
+//  FP32 (HDG_AMG_LEVEL0_FP32=1): the trace matrix's own layout.
+template <int NT> struct Chunks {
+  static constexpr int E = 5 * NT * NT, N = (E + 7) / 8;
+};
+inline int64_t chunk_values(int nt, int64_t nf) { return ((5 * nt * nt + 7) / 8) * 8 * nf; }
+// value (i, k, j) of face f
+template <int NT> __device__ __forceinline__ float ld0(const float* __restrict__ val, int64_t nf, int f, int i, int k, int j) {
+  return val[(k * NT + j) * nf * NT + (int64_t)f * NT + i];
+}
+template <int NT> __device__ __forceinline__ float ld0(const __half* __restrict__ val, int64_t nf, int f, int i, int k, int j) {
+  const int e = (i * 5 + k) * NT + j;
+  return __half2float(val[((int64_t)(e >> 3) * nf + f) * 8 + (e & 7)]);
+}
+// A face's NT values of a level-0 vector (whole allocations: NT = 2 and 4 give 8- and 16-byte aligned faces).
+template <int NT> __device__ __forceinline__ void load_face(const float* __restrict__ v, int64_t f, float* o) {
+  if constexpr (NT == 4) {
+    const float4 t = *reinterpret_cast<const float4*>(v + 4 * f);
+    o[0] = t.x;
+    o[1] = t.y;
+    o[2] = t.z;
+    o[3] = t.w;
+  } else if constexpr (NT == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(v + 2 * f);
+    o[0] = t.x;
+    o[1] = t.y;
+  } else {
+#pragma unroll
+    for (int i = 0; i < NT; ++i) o[i] = v[f * NT + i];
+  }
+}
+template <int NT> __device__ __forceinline__ void store_face(float* __restrict__ v, int64_t f, const float* o) {
+  if constexpr (NT == 4) {
+    *reinterpret_cast<float4*>(v + 4 * f) = make_float4(o[0], o[1], o[2], o[3]);
+  } else if constexpr (NT == 2) {
+    *reinterpret_cast<float2*>(v + 2 * f) = make_float2(o[0], o[1]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NT; ++i) v[f * NT + i] = o[i];
+  }
+}
+// t_i -= sum_kj value (i, k, j) x_kj, each row's terms in the order (k, j); x holds the five slots' neighbour values
+template <int NT>
+__device__ __forceinline__ void face_subtract(const float* __restrict__ val, int64_t nf, int f, const float (&x)[5 * NT],
+                                              float (&t)[NT]) {
+#pragma unroll
+  for (int kj = 0; kj < 5 * NT; ++kj)
+#pragma unroll
+    for (int i = 0; i < NT; ++i) t[i] -= val[kj * nf * NT + (int64_t)f * NT + i] * x[kj];
+}
+template <int NT>
+__device__ __forceinline__ void face_subtract(const __half* __restrict__ val, int64_t nf, int f, const float (&x)[5 * NT],
+                                              float (&t)[NT]) {
+  using C = Chunks<NT>;
+  uint4 c[C::N];
+  const uint4* from = reinterpret_cast<const uint4*>(val) + f;
+#pragma unroll
+  for (int n = 0; n < C::N; ++n) c[n] = __ldg(from + n * nf);
+#pragma unroll
+  for (int e = 0; e < C::E; ++e) {
+    const unsigned w = (e & 7) < 2 ? c[e >> 3].x : ((e & 7) < 4 ? c[e >> 3].y : ((e & 7) < 6 ? c[e >> 3].z : c[e >> 3].w));
+    const float v = __half2float(__ushort_as_half((unsigned short)((e & 1) ? w >> 16 : w & 0xffffu)));
+    t[e / (5 * NT)] -= v * x[e % (5 * NT)];
+  }
+}
 
 // A0 -> D^-1 A0, block row by block row, into `out` (FP32, which may be `val` itself: each face
 // reads and rewrites only its own rows, or FP16).  Runs after every set-up product that needs A0
@@ -1076,18 +1139,39 @@ __global__ void k_amg_scale0(int nf, const float* __restrict__ dinv, const float
   if (f >= nf) return;
   const int64_t nd = (int64_t)nf * NT;
   float di[NT][NT];
+#pragma unroll
   for (int i = 0; i < NT; ++i)
+#pragma unroll
     for (int l = 0; l < NT; ++l) di[i][l] = dinv[((int64_t)f * NT + i) * NT + l];
+  __half h[sizeof(VT) == 2 ? Chunks<NT>::N * 8 : 1];
+  if constexpr (sizeof(VT) == 2) {
+#pragma unroll
+    for (int e = Chunks<NT>::E; e < Chunks<NT>::N * 8; ++e) h[e] = __float2half_rn(0.f);
+  }
+#pragma unroll
   for (int k = 0; k < 5; ++k)
+#pragma unroll
     for (int j = 0; j < NT; ++j) {
       float col[NT];
+#pragma unroll
       for (int l = 0; l < NT; ++l) col[l] = val[(k * NT + j) * nd + (int64_t)f * NT + l];
+#pragma unroll
       for (int i = 0; i < NT; ++i) {
         float s = 0.f;
+#pragma unroll
         for (int l = 0; l < NT; ++l) s += di[i][l] * col[l];
-        out[(k * NT + j) * nd + (int64_t)f * NT + i] = to_vt<VT>(s);
+        if constexpr (sizeof(VT) == 2) h[(i * 5 + k) * NT + j] = __float2half_rn(s);
+        else out[(k * NT + j) * nd + (int64_t)f * NT + i] = s;
       }
     }
+  if constexpr (sizeof(VT) == 2) {
+    uint4* to = reinterpret_cast<uint4*>(out) + f;
+#pragma unroll
+    for (int n = 0; n < Chunks<NT>::N; ++n) {
+      auto two = [&](int e) { return (unsigned)__half_as_ushort(h[e]) | ((unsigned)__half_as_ushort(h[e + 1]) << 16); };
+      to[(int64_t)n * nf] = make_uint4(two(8 * n), two(8 * n + 2), two(8 * n + 4), two(8 * n + 6));
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1113,32 +1197,28 @@ __global__ void k_amg_face_cheb(int nf, const int32_t* __restrict__ bcol5, const
                                 float* __restrict__ d, int step, float ratio, const int32_t* __restrict__ st) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf || !amg_live(st, face_prob[f])) return;
-  const int64_t nd = (int64_t)nf * NT;
   // t = D^-1 (b - A x) = bt - (D^-1 A) x: val holds the block rows of A scaled by D^-1, and
   // the first step (x = 0) forms bt = D^-1 b for the rest of the cycle
   float t[NT];
   if (!xin) {
     float bv[NT];
-    for (int l = 0; l < NT; ++l) bv[l] = b[(int64_t)f * NT + l];
+    load_face<NT>(b, f, bv);
+#pragma unroll
     for (int i = 0; i < NT; ++i) {
       float s = 0.f;
+#pragma unroll
       for (int l = 0; l < NT; ++l) s += dinv[((int64_t)f * NT + i) * NT + l] * bv[l];
       t[i] = s;
-      bt[(int64_t)f * NT + i] = s;
     }
+    store_face<NT>(bt, f, t);
   } else {
-    for (int i = 0; i < NT; ++i) t[i] = bt[(int64_t)f * NT + i];
+    load_face<NT>(bt, f, t);
     // padding slots (faces with fewer than four neighbours) repeat the face with zero values,
     // so every slot is summed without a test and all loads can be issued up front
+    float xv[5 * NT];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const int g = bcol5[k * nf + f];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const float xv = xin[(int64_t)g * NT + j];
-        for (int i = 0; i < NT; ++i) t[i] -= ldv(&val[(k * NT + j) * nd + (int64_t)f * NT + i]) * xv;
-      }
-    }
+    for (int k = 0; k < 5; ++k) load_face<NT>(xin, bcol5[k * nf + f], xv + k * NT);
+    face_subtract<NT>(val, nf, f, xv, t);
   }
   const float hi = fmaxf(lam[face_prob[f]], 1e-30f), lo = hi / ratio;
   const float theta = 0.5f * (hi + lo), delta = 0.5f * (hi - lo), sigma = theta / delta;
@@ -1148,12 +1228,18 @@ __global__ void k_amg_face_cheb(int nf, const int32_t* __restrict__ bcol5, const
     if (u < step) rp = rc;
   }
   const float cd = (step == 0) ? 0.f : rc * rp, cr = (step == 0) ? 1.f / theta : 2.f * rc / delta;
+  float dv[NT], xo[NT];
+#pragma unroll
+  for (int i = 0; i < NT; ++i) dv[i] = xo[i] = 0.f;
+  if (step != 0) load_face<NT>(d, f, dv);
+  if (xin) load_face<NT>(xin, f, xo);
+#pragma unroll
   for (int i = 0; i < NT; ++i) {
-    const int64_t row = (int64_t)f * NT + i;
-    const float dn = cr * t[i] + (step == 0 ? 0.f : cd * d[row]);
-    d[row] = dn;
-    xout[row] = (xin ? xin[row] : 0.f) + dn;
+    dv[i] = cr * t[i] + (step == 0 ? 0.f : cd * dv[i]);
+    xo[i] += dv[i];
   }
+  store_face<NT>(d, f, dv);
+  store_face<NT>(xout, f, xo);
 }
 
 template <int NT, typename VT>
@@ -1185,7 +1271,7 @@ __global__ void k_amg_row_cheb(int nf, const int32_t* __restrict__ bcol5, const 
     for (int k = 0; k < 5; ++k) {
       const int g = bcol5[k * nf + f];
 #pragma unroll
-      for (int j = 0; j < NT; ++j) t -= ldv(&val[(k * NT + j) * nd + row]) * xin[(int64_t)g * NT + j];
+      for (int j = 0; j < NT; ++j) t -= ld0<NT>(val, nf, f, i, k, j) * xin[(int64_t)g * NT + j];
     }
   }
   const float hi = fmaxf(lam[face_prob[f]], 1e-30f), lo = hi / ratio;
@@ -1209,7 +1295,7 @@ __global__ void k_amg_face_residual(int nf, const int32_t* __restrict__ bcol5, c
   const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t nd = (int64_t)nf * NT;
   if (row >= nd) return;
-  const int f = (int)(row / NT);
+  const int f = (int)(row / NT), i = (int)(row - (int64_t)f * NT);
   if (!amg_live(st, face_prob[f])) return;
   float s = b[row];
   // padding slots repeat the face with zero values: no test needed
@@ -1217,7 +1303,7 @@ __global__ void k_amg_face_residual(int nf, const int32_t* __restrict__ bcol5, c
   for (int k = 0; k < 5; ++k) {
     const int g = bcol5[k * nf + f];
 #pragma unroll
-    for (int j = 0; j < NT; ++j) s -= ldv(&val[(k * NT + j) * nd + row]) * x[(int64_t)g * NT + j];
+    for (int j = 0; j < NT; ++j) s -= ld0<NT>(val, nf, f, i, k, j) * x[(int64_t)g * NT + j];
   }
   r[row] = s;
 }
@@ -1231,22 +1317,13 @@ __global__ void k_amg_face_residual_f(int nf, const int32_t* __restrict__ bcol5,
                                       const int32_t* __restrict__ st) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf || !amg_live(st, face_prob[f])) return;
-  const int64_t nd = (int64_t)nf * NT;
   float s[NT];
+  load_face<NT>(b, f, s);
+  float xv[5 * NT];
 #pragma unroll
-  for (int i = 0; i < NT; ++i) s[i] = b[(int64_t)f * NT + i];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    const int g = bcol5[k * nf + f];
-#pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      const float xv = x[(int64_t)g * NT + j];
-#pragma unroll
-      for (int i = 0; i < NT; ++i) s[i] -= ldv(&val[(k * NT + j) * nd + (int64_t)f * NT + i]) * xv;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < NT; ++i) r[(int64_t)f * NT + i] = s[i];
+  for (int k = 0; k < 5; ++k) load_face<NT>(x, bcol5[k * nf + f], xv + k * NT);
+  face_subtract<NT>(val, nf, f, xv, s);
+  store_face<NT>(r, f, s);
 }
 
 // b1 = P0' r0 = (D P0)' r~0 and the first l1-Jacobi sweep of level 1: x1 = b1 / dl1
@@ -1640,7 +1717,7 @@ template <int NT> void numeric_nt(hdg_system* s, const float* val0, cudaStream_t
   if (amg_level0_fp32()) {
     k_amg_scale0<NT, float><<<nblk(nf), 256, 0, st>>>(nf, H->dinv0.p, val0, const_cast<float*>(val0));
   } else {
-    H->val0h.alloc((size_t)hdg_system::SLOTS * NT * NT * nf);
+    H->val0h.alloc((size_t)chunk_values(NT, nf));
     k_amg_scale0<NT, __half><<<nblk(nf), 256, 0, st>>>(nf, H->dinv0.p, val0, H->val0h.p);
   }
   s->ctx->launches += 6;
@@ -1823,8 +1900,8 @@ void amg_setup_numeric(hdg_system* s, cudaStream_t st) {
 double amg_cycle_bytes(const hdg_system* s) {
   const AmgHierarchy* H = s->amg;
   const double nf = H->nf, nt = H->nt, n0 = nf * nt, n1 = H->lev.empty() ? 0.0 : H->lev[0].n;
-  const double vb = H->val0h.p ? 2.0 : 4.0;             // FP16 or FP32 level-0 values
-  const double mat0 = 5.0 * vb * nt * nt * nf + 20.0 * nf;  // values + block columns
+  // values (FP16 in chunks of eight, or FP32) + block columns
+  const double mat0 = (H->val0h.p ? 2.0 * (double)chunk_values(H->nt, H->nf) : 20.0 * nt * nt * nf) + 20.0 * nf;
   const double dinv = 4.0 * nt * nt * nf;
   const int k = amg_cheb_degree();
   double b = 16.0 * n0 + dinv;                             // first sweep: b, D^-1 -> bt, x, d
