@@ -324,6 +324,123 @@ int hdg_space_destroy(hdg_space* s) {
   return HDG_OK;
 }
 
+// ---------------------------------------------------------------- fields in fixed point
+// hdg_device.cuh: eval_part.  Rewrites the parameters of one field at prm (its FieldSpec's, in place) for coordinates
+// X = x 2^s and returns the fixed-point kind, or leaves them (a Gaussian's width prepared as in fprep) and returns
+// the plain one where a value does not fit the form.
+static int prepare_fixed(const FieldSpec& f, int s, double* prm) {
+  auto word = [](uint64_t v) {
+    double d;
+    std::memcpy(&d, &v, 8);
+    return d;
+  };
+  auto ceil_log2 = [](double v) {  // smallest e with v <= 2^e
+    int e;
+    const double m = std::frexp(v, &e);
+    return m == 0.5 ? e - 1 : e;
+  };
+  const std::vector<double>& p = f.prm;
+  const int K = (f.kind == HDG_FIELD_BUMPS || f.kind == HDG_FIELD_FOURIER || f.kind == HDG_FIELD_EXP_FOURIER) ? (int)p[0] : 0;
+  if (f.kind == HDG_FIELD_BUMPS) {
+    bool fits = true;
+    std::vector<uint64_t> w(4 * (size_t)K);
+    for (int k = 0; k < K && fits; ++k) {
+      const double* b = &p[1 + 4 * k];
+      fits = std::isfinite(b[0]) && std::isfinite(b[1]) && std::isfinite(b[2]) && b[2] != 0.0;
+      if (!fits) break;
+      // |dx| 2^s scaled to r sqrt(log2 e / 2) / sigma in units of 2^-59: a factor below 2^64 and a shift
+      const long double c = 0.84932180028801904272L / std::fabs((long double)b[2]);
+      int e;
+      const long double m = std::frexp(c, &e);  // c = m 2^e, m in [1/2, 1)
+      const int up = e + 59 - s;                // G = |dx| m 2^up
+      const int sh = std::max(0, up);
+      fits = sh <= 62 && up > -200;
+      if (!fits) break;
+      const long double q = std::ldexp(m, 64 + up - sh);  // at most 2^64 - 2^10
+      uint64_t sg = (uint64_t)q;
+      sg = (sg & ~63ull) | (uint64_t)sh;
+      w[4 * k] = (uint64_t)std::llrint(std::ldexp(b[0], s));
+      w[4 * k + 1] = (uint64_t)std::llrint(std::ldexp(b[1], s));
+      w[4 * k + 2] = sg;
+      std::memcpy(&w[4 * k + 3], &b[3], 8);
+    }
+    if (fits) {
+      prm[0] = word((uint64_t)K);
+      for (int k = 0; k < 4 * K; ++k) prm[1 + k] = word(w[k]);
+      return 100;
+    }
+    for (int k = 0; k < K; ++k) prm[1 + 4 * k + 2] = -1.0 / (2.0 * p[1 + 4 * k + 2] * p[1 + 4 * k + 2]);
+    return f.kind;
+  }
+  if (f.kind == HDG_FIELD_FOURIER || f.kind == HDG_FIELD_EXP_FOURIER) {
+    double kmax = 0.0, asum = 0.0;
+    bool fits = true;
+    for (int k = 0; k < K; ++k) {
+      const double* b = &p[2 + 4 * k];
+      fits = fits && std::isfinite(b[0]) && std::isfinite(b[1]) && std::isfinite(b[2]) && std::isfinite(b[3]);
+      kmax = std::max(kmax, std::max(std::fabs(b[0]), std::fabs(b[1])));
+      asum += std::fabs(b[3]);
+    }
+    if (!fits || !(asum < 1e300)) return f.kind;
+    const int u = kmax > 0.0 ? std::min(80, 60 - ceil_log2(kmax)) : 60;
+    const int w = asum > 0.0 ? 62 - ceil_log2(asum) : 0;
+    const int sh = s + u - 64;
+    if (sh < 0 || sh > 120 || w < -900 || w > 900) return f.kind;
+    prm[0] = word((uint64_t)(uint32_t)K | ((uint64_t)sh << 32) | ((uint64_t)(uint16_t)(int16_t)w << 48));
+    for (int k = 0; k < K; ++k) {
+      const double* b = &p[2 + 4 * k];
+      long double t = (long double)b[2] / 6.28318530717958647692528676655900577L;
+      t -= std::floor(t);
+      prm[2 + 4 * k] = word((uint64_t)std::llrint(std::ldexp(b[0], u)));
+      prm[2 + 4 * k + 1] = word((uint64_t)std::llrint(std::ldexp(b[1], u)));
+      prm[2 + 4 * k + 2] = word(t < 1.0L ? (uint64_t)(t * 18446744073709551616.0L) : 0ull);
+      prm[2 + 4 * k + 3] = word((uint64_t)std::llrint(std::ldexp(b[3], w)));
+    }
+    return f.kind == HDG_FIELD_FOURIER ? 101 : 102;
+  }
+  return f.kind;
+}
+
+extern "C++" void ensure_fixed_fields(hdg_system* s) {
+  const double xy = s->space->mesh->xy_max;
+  if (s->fix_max >= 0.0 && xy <= s->fix_max) return;
+  double top = xy;  // coordinates and the bumps' centres
+  for (auto* v : {&s->fsp, &s->ksp})
+    for (const FieldSpec& f : *v)
+      if (f.kind == HDG_FIELD_BUMPS)
+        for (int k = 0; k < (int)f.prm[0]; ++k)
+          for (int c = 0; c < 2; ++c)
+            if (std::isfinite(f.prm[1 + 4 * k + c])) top = std::max(top, std::fabs(f.prm[1 + 4 * k + c]));
+  top = std::min(std::max(top, 1e-6), 1e15);
+  int e;
+  std::frexp(top, &e);  // top < 2^e
+  const int sc = 61 - e;
+  s->fix_scale = std::ldexp(1.0, sc);
+  cudaStream_t st = s->ctx->stream;
+  auto make = [&](const std::vector<FieldSpec>& v, DevBuf<int32_t>* dk, DevBuf<int32_t>* doff, DevBuf<double>* dp) {
+    std::vector<int32_t> kind(v.size()), off(v.size());
+    std::vector<double> prm;
+    for (size_t P = 0; P < v.size(); ++P) {
+      const size_t at = prm.size();
+      off[P] = (int32_t)at;
+      prm.insert(prm.end(), v[P].prm.begin(), v[P].prm.end());
+      kind[P] = std::isfinite(xy) && xy <= 1e15 ? prepare_fixed(v[P], sc, prm.data() + at) : v[P].kind;
+      if (kind[P] == HDG_FIELD_BUMPS && !(std::isfinite(xy) && xy <= 1e15))
+        for (int k = 0; k < (int)v[P].prm[0]; ++k) {
+          double& sw = prm[at + 1 + 4 * k + 2];
+          sw = -1.0 / (2.0 * sw * sw);
+        }
+    }
+    dk->upload(kind.data(), kind.size(), st);
+    doff->upload(off.data(), off.size(), st);
+    dp->upload(prm.data(), prm.size(), st);
+    HDG_CUDA(cudaStreamSynchronize(st));  // the host vectors go out of scope
+  };
+  make(s->fsp, &s->d_fkfix, &s->d_fofix, &s->d_ffix);
+  make(s->ksp, &s->d_kkfix, &s->d_kofix, &s->d_kfix);
+  s->fix_max = std::ldexp(1.0, e);
+}
+
 // ---------------------------------------------------------------- assembly
 // Per-problem coefficients: f[P], kappa[P] (fields, or NULL), tau[P]; kappa_cell over all cells.
 static void set_coefficients_many(hdg_system* s, const double* taus, const hdg_field* const* f,
@@ -354,20 +471,17 @@ static void set_coefficients_many(hdg_system* s, const double* taus, const hdg_f
   s->d_fprm.upload(fp.data(), fp.size(), st);
   // the element kernels evaluate a Gaussian bump as a exp(|x - c|^2 k) with k = -1/(2 s^2) formed
   // here once, instead of dividing by 2 s^2 at every quadrature point
-  auto prepared = [&](std::vector<double> prm, const std::vector<int32_t>& kind, const std::vector<int32_t>& off) {
-    for (int P = 0; P < np; ++P)
-      if (kind[P] == HDG_FIELD_BUMPS) {
-        const int K = (int)prm[off[P]];
-        for (int b = 0; b < K; ++b) {
-          double& sw = prm[off[P] + 1 + 4 * b + 2];
-          sw = -1.0 / (2.0 * sw * sw);
-        }
+  std::vector<double> fpp(fp);
+  for (int P = 0; P < np; ++P)
+    if (fk[P] == HDG_FIELD_BUMPS) {
+      const int K = (int)fpp[fo[P]];
+      for (int b = 0; b < K; ++b) {
+        double& sw = fpp[fo[P] + 1 + 4 * b + 2];
+        sw = -1.0 / (2.0 * sw * sw);
       }
-    return prm;
-  };
-  const std::vector<double> fpp = prepared(fp, fk, fo), kpp = prepared(kp, kk, ko);
+    }
   s->d_fprep.upload(fpp.data(), fpp.size(), st);
-  s->d_kprep.upload(kpp.data(), kpp.size(), st);
+  s->fix_max = -1.0;  // the fixed-point form is of the old fields
   s->d_kkind.upload(kk.data(), np, st);
   s->d_koff.upload(ko.data(), np, st);
   s->d_kprm.upload(kp.data(), kp.size(), st);
@@ -379,6 +493,7 @@ static void set_coefficients_many(hdg_system* s, const double* taus, const hdg_f
       if (!(kappa_cell[c] > 0.0)) throw HdgError{HDG_ERR_ARG, "kappa must be positive"};
     s->d_kappa.upload(kappa_cell, (size_t)s->nc, st);
   }
+  ensure_fixed_fields(s);
   HDG_CUDA(cudaStreamSynchronize(st));  // the host staging vectors go out of scope
 }
 

@@ -27,6 +27,7 @@ struct ElemArgs {
   const double* ref;
   int ref_len, nq;
   int nc;
+  double fix_scale;  // coordinates to fixed point (CoefDev::ffix)
   CoefDev co;      // per-problem source, coefficient and tau (one problem unless batched)
   int kappa_mode;  // 0: kappa = 1, 1: per-cell array, 2: per-problem field
   const double* kcell;
@@ -267,9 +268,10 @@ __global__ void __launch_bounds__(EWARPS * 32) k_element_condense(ElemArgs a) {
 // p = 4, 2 of 13, 3 of 10, 4 of 7 at p = 3, 2, 1.  The lane keeps its column, and the column of S of the same number, in
 // registers; a row of S is broadcast through shared memory when it is final.  The pairs of columns are taken
 // cyclically (a lane its own column against the one d further on, d = 0..(m+1)/2), the source's terms are spread over
-// (point, part) pairs, and the entries of S over all lanes.  Measured on 65522 cells with eight bumps as the source, one
-// cell per warp before / here: p = 4 4.31 / 2.27 ms, p = 3 2.30 / 1.05, p = 2 (then by the pivoted elimination of the
-// 18 x 18 system) 2.70 / 0.59, p = 1 1.16 / 0.22.
+// (point, part) pairs and evaluated on the integer pipe (eval_part), and the entries of S spread over all lanes.  Measured
+// on 65522 cells with eight bumps as the source, one cell per warp before / this layout with FP64 exponentials / here:
+// p = 4 4.31 / 2.27 / 1.61 ms, p = 3 2.30 / 1.05 / 0.84, p = 2 (before: the pivoted elimination of the 18 x 18 system)
+// 2.70 / 0.59 / 0.45, p = 1 1.16 / 0.22 / 0.15.
 // v[f] for a face index f known only at run time, without indexing a local array (which would
 // place the array in local memory)
 __device__ __forceinline__ double sel3(int f, double v0, double v1, double v2) {
@@ -397,12 +399,14 @@ __global__ void __launch_bounds__(256) k_element_schur(ElemArgs a) {
       const int pr = __shfl_sync(0xffffffffu, prob, src);
       const double xi = tQ[2 * q], eta = tQ[2 * q + 1];
       double v = 0.0;
-      if (pt < CPW * nq)
-        v = eval_source_part(a.co.fkind[pr], a.co.fprep + a.co.foff[pr], fma(A01, eta, fma(A00, xi, X)),
-                             fma(A11, eta, fma(A10, xi, Yv)), part, PARTS);
+      if (pt < CPW * nq) {
+        const double xq = fma(A01, eta, fma(A00, xi, X)), yq = fma(A11, eta, fma(A10, xi, Yv));
+        v = eval_part(a.co.fkfix[pr], a.co.ffix + a.co.fofix[pr], xq, yq, __double2ll_rn(xq * a.fix_scale),
+                      __double2ll_rn(yq * a.fix_scale), part, PARTS);
+      }
 #pragma unroll
       for (int o = PARTS / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (part == 0 && pt < CPW * nq) sq0[pt] = finish_parts(a.co.fkind[pr], v);
+      if (part == 0 && pt < CPW * nq) sq0[pt] = finish_parts(a.co.fkfix[pr], v);
     }
     __syncwarp();
     if (col < NW && on_lane) {
@@ -515,8 +519,8 @@ __global__ void __launch_bounds__(256) k_element_schur(ElemArgs a) {
 // One cell per warp at p = 2 and 3 (21 and 32 columns, a lane each), two at p = 1.  The fields' modes are spread over
 // (point, part) pairs: at p = 3 and 64 modes each for f and kappa, a lane per point kept 12 of 32 lanes busy for more than
 // half of the 43 us a cell took an SM.  A cell with kappa <= 0 (or not finite) at a point may have an indefinite Aw; it goes
-// on the list for the pivoted kernel.  Measured on 65522 cells with 64 modes each, pivoted elimination / here: p = 3
-// 18.6 / 8.2 ms, p = 2 13.6 / 4.6, p = 1 11.9 / 1.7.
+// on the list for the pivoted kernel.  Measured on 65522 cells with 64 modes each, pivoted elimination / this layout with
+// FP64 cosines / here: p = 3 18.6 / 8.2 / 4.4 ms, p = 2 13.6 / 4.6 / 2.6, p = 1 11.9 / 1.7 / 0.74.
 template <int P, int NZ> struct FieldDims {
   using D = Dims<P>;
   static constexpr int NW = D::NW, NT = D::NT, M = D::M, N = D::N;
@@ -640,8 +644,9 @@ __global__ void __launch_bounds__(256) k_element_field(ElemArgs a) {
       const double xq = fma(A01, eta, fma(A00, xi, X)), yq = fma(A11, eta, fma(A10, xi, Yv));
       double v = 0.0, w = 0.0;
       if (in) {
-        v = eval_source_part(a.co.fkind[po], a.co.fprep + a.co.foff[po], xq, yq, part, PARTS);
-        w = eval_source_part(a.co.kkind[po], a.co.kprep + a.co.koff[po], xq, yq, part, PARTS);
+        const long long xf = __double2ll_rn(xq * a.fix_scale), yf = __double2ll_rn(yq * a.fix_scale);
+        v = eval_part(a.co.fkfix[po], a.co.ffix + a.co.fofix[po], xq, yq, xf, yf, part, PARTS);
+        w = eval_part(a.co.kkfix[po], a.co.kfix + a.co.kofix[po], xq, yq, xf, yf, part, PARTS);
       }
 #pragma unroll
       for (int o = PARTS / 2; o > 0; o >>= 1) {
@@ -649,8 +654,8 @@ __global__ void __launch_bounds__(256) k_element_field(ElemArgs a) {
         w += __shfl_xor_sync(0xffffffffu, w, o);
       }
       if (part == 0 && in) {
-        sq0[pt] = finish_parts(a.co.fkind[po], v);
-        w = finish_parts(a.co.kkind[po], w);
+        sq0[pt] = finish_parts(a.co.fkfix[po], v);
+        w = finish_parts(a.co.kkfix[po], w);
         sk0[pt] = 1.0 / w;
         good = good && w > 0.0 && w < 1e300;
       }
@@ -1066,6 +1071,8 @@ ElemArgs element_args(hdg_system* s) {
   a.ref = sp->d_ref.p;
   a.nq = sp->t.nq;
   a.nc = m->nc;
+  ensure_fixed_fields(s);
+  a.fix_scale = s->fix_scale;
   a.co = s->coef_dev();
   a.kappa_mode = s->kappa_cells ? 1 : (s->kappa_field ? 2 : 0);
   a.he_tau = s->he_tau ? 1 : 0;

@@ -116,7 +116,11 @@ struct CoefDev {
   const double* tau;         // [nprob]
   // fprm with each Gaussian bump's width s replaced by -1/(2 s^2) (element kernels' source)
   const double* fprep;
-  const double* kprep;  // kprm likewise
+  // source and kappa as the Schur kernels read them: kinds and parameters with bumps and modes in fixed point
+  const int32_t *fkfix, *fofix;
+  const double* ffix;
+  const int32_t *kkfix, *kofix;
+  const double* kfix;
 };
 
 // ------------------------------------------------------------------ objects
@@ -181,6 +185,7 @@ struct hdg_mesh {
   double LL[2] = {0, 0}, UR[2] = {1, 1};
   // device copies
   DevBuf<double> d_xy;
+  double xy_max = 0.0;        // largest |coordinate| (upload_coordinates)
   DevBuf<int32_t> d_cells, d_cfaces;
   DevBuf<uint8_t> d_orient;   // bit f = face_orientation(cell, f)
   DevBuf<int32_t> d_fcell;    // [nf][2] cells of a face (second -1 on the boundary)
@@ -269,7 +274,8 @@ struct hdg_system {
   std::vector<int32_t> h_seg_prob, h_seg_row0, h_seg_row1, h_prob_blk0, h_prob_nblk;  // host copies
   CoefDev coef_dev() const {
     return CoefDev{space->mesh->d_cell_prob.p, d_fkind.p, d_foff.p, d_fprm.p, d_kkind.p, d_koff.p, d_kprm.p,
-                   d_tau.p, d_fprep.p, d_kprep.p};
+                   d_tau.p, d_fprep.p, d_fkfix.p, d_fofix.p, d_ffix.p, d_kkfix.p, d_kofix.p,
+                   d_kfix.p};
   }
   // per-cell condensed blocks: AB = [Ate | bte] (m x (m+1)), KB = [K_e | b_e] (n x (m+1)), or,
   // after the Schur element path (kb_u_only), only its u rows [X_u | b_u] (nw x (m+1)), with the rows of the two
@@ -279,7 +285,10 @@ struct hdg_system {
   DevBuf<float> d_ABf, d_KBf;
   DevBuf<double> d_kappa;  // per-cell kappa (optional)
   DevBuf<double> d_fprm, d_kprm;
-  DevBuf<double> d_fprep, d_kprep;  // d_fprm, d_kprm prepared for the element kernels (CoefDev::fprep)
+  DevBuf<double> d_fprep;  // d_fprm prepared for the pivoted element kernel (CoefDev::fprep)
+  DevBuf<double> d_ffix, d_kfix;     // fields in fixed point (CoefDev::ffix), made for coordinates up to fix_max
+  DevBuf<int32_t> d_fkfix, d_fofix, d_kkfix, d_kofix;
+  double fix_max = 0.0, fix_scale = 1.0;
   FieldSpec f, kappa;
   bool kappa_field = false, kappa_cells = false;
   // Trace matrix.  Host: block rows sorted by face id (h_browptr/h_bcol, the export pattern).
@@ -357,6 +366,9 @@ constexpr int HDG_CG_ST = 4;
 
 // ------------------------------------------------------------------ kernel launchers
 void launch_element_condense(hdg_system* s, cudaStream_t st);
+// The fields' fixed-point form for the mesh's present coordinates (made anew when they have grown; uploads on the
+// context's stream).
+void ensure_fixed_fields(hdg_system* s);
 void launch_gather(hdg_system* s, cudaStream_t st);
 void launch_apply_dirichlet(hdg_system* s, const std::vector<int32_t>& dofs0, const std::vector<double>& vals,
                             cudaStream_t st);  // scatter + apply

@@ -244,4 +244,8 @@ void hdg_mesh::upload() {
   HDG_CUDA(cudaStreamSynchronize(s));
 }
 
-void hdg_mesh::upload_coordinates() { d_xy.upload(xy.data(), xy.size(), ctx->stream); }
+void hdg_mesh::upload_coordinates() {
+  xy_max = 0.0;
+  for (double v : xy) xy_max = std::max(xy_max, std::fabs(v));
+  d_xy.upload(xy.data(), xy.size(), ctx->stream);
+}

@@ -89,3 +89,19 @@ def test_field_blocks_match_full_elimination(H, monkeypatch, n, p, qd, kind):
     if p != 1:  # one cell per warp there: exactly the cells with a negative value are left to it
         for x, y in zip(got, want):
             assert np.array_equal(x[far], y[far])
+
+
+# phases that are exact multiples of an eighth, a quarter and a half turn, a phase beyond one turn, a zero amplitude
+@pytest.mark.parametrize("n", [2, 4, 10])
+@pytest.mark.parametrize("p,qd", [(1, 2), (2, 3), (4, 9)])
+@pytest.mark.parametrize("f", ["unit", "quarter", "wrapped", "flat", "far"])
+def test_fixed_point_fields_at_special_phases(H, monkeypatch, n, p, qd, f):
+    mesh = H.rectangle_mesh(H.TriangleCell, (n, n), (-1.0, -1.0), (1.0, 1.0))
+    f = {"unit": H.Field.sinsin(2 * np.pi ** 2, 1.0, 1.0),
+         "quarter": H.Field.fourier(0.5, [[1.0, 0.0, np.pi / 2, 1.0], [0.0, 4.0, -np.pi, 2.0], [0.5, 0.5, 0.0, 1.0]]),
+         "wrapped": H.Field.fourier(0.0, [[1.0, -2.0, 25.0, 1.0], [3.0, 1.0, -40.0, 0.5]]),
+         "flat": H.Field.fourier(1.5, [[0.0, 0.0, 0.3, 0.0]]),
+         "far": H.Field.bumps([[0.25, 0.25], [40.0, -3.0]], [0.01, 5.0], [1.0, 1e3])}[f]
+    got = blocks(H, mesh, p, qd, f)
+    monkeypatch.setenv("HDG_ELEMENT_FULL_LU", "1")
+    check(got, blocks(H, mesh, p, qd, f))
