@@ -1,5 +1,9 @@
 // C ABI of libhdg (include/hdg.h): argument checking, object lifetimes, error reporting.
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
+#include <cerrno>
 #include <cmath>
 #include <cstring>
 #include <functional>
@@ -401,6 +405,19 @@ static int prepare_fixed(const FieldSpec& f, int s, double* prm) {
   return f.kind;
 }
 
+extern "C++" void populate_pages(void* p, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+  if (!p || bytes == 0) return;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = (uintptr_t)p & ~(page - 1);
+  const int err = errno;
+  madvise((void*)a, (uintptr_t)p + bytes - a, MADV_POPULATE_WRITE);
+  errno = err;
+#else
+  (void)p;
+  (void)bytes;
+#endif
+}
+
 extern "C++" void ensure_fixed_fields(hdg_system* s) {
   const double xy = s->space->mesh->xy_max;
   if (s->fix_max >= 0.0 && xy <= s->fix_max) return;
@@ -649,53 +666,7 @@ int hdg_system_get_csc(const hdg_system* s, int base, int64_t* colptr, int64_t* 
   if (!s || (base != 0 && base != 1)) return HDG_ERR_ARG;
   return guard(s->ctx, [&]() -> int {
     set_device(s->ctx);
-    cudaStream_t st = s->ctx->stream;
-    const int nt = s->nt, nf = s->nf;
-    std::vector<double> val;
-    if (nzval) {
-      val.resize((size_t)hdg_system::SLOTS * nt * s->ndofs);
-      s->d_val.download(val.data(), val.size(), st);
-    }
-    const size_t nd = (size_t)s->ndofs;
-    // value of K[f nt + i, g nt + j] where g sits in slot k of block row f
-    auto kval = [&](int f, int k, int i, int j) { return val[(size_t)(k * nt + j) * nd + (size_t)f * nt + i]; };
-    std::vector<double> b;
-    if (rhs) {
-      b.resize(s->ndofs);
-      s->d_b.download(b.data(), b.size(), st);
-    }
-    std::vector<uint8_t> pres;
-    if (s->applied) {
-      pres.resize(s->ndofs);
-      s->d_pres.download(pres.data(), pres.size(), st);
-    }
-    HDG_CUDA(cudaStreamSynchronize(st));
-    auto sign = [&](int row) { return (s->applied && !pres[row]) ? -1.0 : 1.0; };
-    // the block pattern is symmetric: column g*nt+j of K holds K[f*nt+i, g*nt+j] for the
-    // blocks (f,g) with f in block row g's neighbour list, rows ascending
-    int64_t pos = 0;
-    if (colptr) colptr[0] = base;
-    for (int g = 0; g < nf; ++g) {
-      const int k0 = s->h_browptr[g], k1 = s->h_browptr[g + 1];
-      for (int j = 0; j < nt; ++j) {
-        for (int k = k0; k < k1; ++k) {
-          const int f = s->h_bcol[k];
-          // slot of block (f, g) in block row f
-          int kp = -1;
-          for (int q = s->h_browptr[f]; q < s->h_browptr[f + 1]; ++q)
-            if (s->h_bcol[q] == g) { kp = q - s->h_browptr[f]; break; }
-          for (int i = 0; i < nt; ++i) {
-            const int row = f * nt + i;
-            if (rowval) rowval[pos] = row + base;
-            if (nzval) nzval[pos] = sign(row) * kval(f, kp, i, j);
-            ++pos;
-          }
-        }
-        if (colptr) colptr[g * nt + j + 1] = pos + base;
-      }
-    }
-    if (rhs)
-      for (int r = 0; r < s->ndofs; ++r) rhs[r] = sign(r) * b[r];
+    run_export_csc(s, base, colptr, rowval, nzval, rhs, s->ctx->stream);
     return HDG_OK;
   });
 }
@@ -974,6 +945,9 @@ int hdg_recover_into(hdg_system* s, double* q, double* u, double* uhat_cell, int
     if (u) du.alloc((size_t)s->nc * s->nw);
     if (uhat_cell) dx.alloc((size_t)s->nc * s->m);
     if (q || u || uhat_cell) launch_recover_split(s, dq.p, du.p, dx.p, by_function != 0, st);
+    populate_pages(q, dq.n * sizeof(double));
+    populate_pages(u, du.n * sizeof(double));
+    populate_pages(uhat_cell, dx.n * sizeof(double));
     if (q) dq.download(q, dq.n, st);
     if (u) du.download(u, du.n, st);
     if (uhat_cell) dx.download(uhat_cell, dx.n, st);

@@ -85,6 +85,12 @@ template <class T> struct DevBuf {
   }
 };
 
+// Asks for the pages of a host array before the device copies into it, while the kernel that fills the copy's source is
+// still running.  The device can fault pages in by itself, but slowly: into 36 MB of a fresh mapping 1.3 to 2.3 ms
+// beyond the copy, into numpy's fresh arrays (advised for huge pages) 6 to 30 ms, asked for first 1.1 ms; where they are
+// there already some microseconds.  Contents are kept; where the kernel declines, the device faults them in after all.
+void populate_pages(void* p, size_t bytes);
+
 // ------------------------------------------------------------------ fields
 struct FieldSpec {
   int kind = HDG_FIELD_CONST;
@@ -411,6 +417,8 @@ void launch_recover(hdg_system* s, cudaStream_t st);
 // The recovered q (ncells x nv) and u (ncells x nw) and the cells' trace values (ncells x 3 x nt, or ncells x nt x 3
 // by_function) as arrays of their own on the device; a NULL one is left out.
 void launch_recover_split(hdg_system* s, double* q, double* u, double* uhat_cell, bool by_function, cudaStream_t st);
+void run_export_csc(const hdg_system* s, int base, int64_t* colptr, int64_t* rowval, double* nzval, double* rhs,
+                    cudaStream_t st);
 // The full [K_e | b_e] (ncells x n x (m+1), device) from the stored u rows (kb_u_only systems).
 void launch_expand_ke(hdg_system* s, double* out, cudaStream_t st);
 double run_errornorm(hdg_system* s, const FieldSpec& uex, cudaStream_t st);
