@@ -34,6 +34,7 @@
 // Everything in the hierarchy and the cycle is FP32: the preconditioner only has to be a fixed
 // SPD approximation.  All sums run in a fixed order, so the cycle is deterministic.
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -55,19 +56,20 @@ constexpr int AMG_MAX_COARSE = 96;  // per problem, dense inverse on the coarses
 constexpr int AMG_MAX_LEVELS = 12;
 constexpr int AMG_CINV_MAX = 150;   // largest dense coarsest block: (2 m^2 + m) floats of shared memory
 constexpr int PW = 5;               // level-0 prolongator row width (a face and its 4 neighbours)
-constexpr int AMG_TAIL_THREADS = 512;  // threads of a k_amg_tail CTA (one CTA per problem)
+constexpr int AMG_TAIL_THREADS = 512;      // of a k_amg_tail CTA
+constexpr int AMG_TAIL_SMEM = 216 * 1024;  // dynamic shared memory that the k_amg_tail CTAs of an SM may take
 
 // Lanes per row of a coarse level with n rows (see the coarse-level kernels).
 inline int amg_group(int n) { return n >= 16384 ? 4 : (n >= 2048 ? 8 : 32); }
 
-constexpr int AMG_TAIL_MAXROWS = 4096;  // largest problem level the tail kernel may take
+constexpr int AMG_TAIL_ROUNDS = 16;  // most rounds of a k_amg_tail CTA's threads over its rows of one level
 constexpr int AMG_ROW_SWEEP_FACES = 100000;  // untuned default: a thread per row below this many faces
 
-// The coarse levels below some level T can be cycled by one k_amg_tail launch (one CTA per
+// The coarse levels below some level T can be cycled by one k_amg_tail launch (a cluster of CTAs per
 // problem) instead of a launch per kernel per level; both give the same bits, and the V-cycle
-// autotuner (amg_tune) picks T by timing.  HDG_AMG_TAIL_ROWS=k forces T = the first level whose
-// largest problem has at most k rows (0: no tail) and leaves T out of the tuning; -1 (unset):
-// tuned.
+// autotuner (amg_tune) picks T by timing.  HDG_AMG_TAIL_ROWS=k forces T = the first level that
+// fits the cluster's shared memory and whose largest problem has at most k rows (0: no tail) and
+// leaves T out of the tuning; -1 (unset): tuned.
 int amg_tail_rows() {
   static const int v = [] {
     const char* e = std::getenv("HDG_AMG_TAIL_ROWS");
@@ -268,6 +270,7 @@ struct AmgLevel {  // a scalar level l >= 1 (rows = aggregates of level l-1)
   DevBuf<int32_t> agg;                // aggregate of each row
   DevBuf<float> tent;                 // tentative weight of each row
   DevBuf<int32_t> pptr, pcol;         // P (CSR, sorted columns)
+  std::vector<int32_t> h_pptr, h_rptr, h_prow0;  // host copies of pptr, rptr and prow0
   DevBuf<float> pval;
   DevBuf<int32_t> apptr, apcol;       // A P pattern
   DevBuf<float> apval;
@@ -276,12 +279,12 @@ struct AmgLevel {  // a scalar level l >= 1 (rows = aggregates of level l-1)
   int maxrows = 0;                    // rows of the largest problem
 };
 
-// One level as the tail kernel (k_amg_tail) reads it.
+// One level as the tail kernels (k_amg_tail_image, k_amg_tail) read it.
 struct TailLevel {
   int g;                                      // lanes per row (amg_group of the level's rows)
   const int32_t *ptr, *col, *prow0;
   const float *val, *dl1inv;
-  float *b, *x, *t, *r;
+  float *b, *x;
   const int32_t *pptr, *pcol, *rptr, *rent, *rrow;  // transfer to the next level
   const float* pval;
 };
@@ -313,8 +316,13 @@ struct AmgHierarchy {
   DevBuf<float> cinv;
   int cmax = 0;
   int tail_from = -1;        // first level (index into lev) cycled by k_amg_tail; -1: none
-  std::vector<int> tail_cands; // levels the tail may start at (problems' rows <= AMG_TAIL_MAXROWS)
-  DevBuf<TailLevel> tail_tab;  // every level's arrays for k_amg_tail
+  std::vector<int> tail_cands;  // levels the tail may start at, and each one's shared memory per CTA
+  std::vector<size_t> tail_smem;
+  int tail_ctas = 1;            // CTAs of a problem's cluster
+  DevBuf<TailLevel> tail_tab;   // every level's arrays for k_amg_tail
+  DevBuf<unsigned char> tail_head;
+  DevBuf<uint32_t> tail_image;  // what each CTA keeps of the matrices (k_amg_tail_image), tail_words words each
+  size_t tail_words = 0;
   bool row_sweep = false;    // level-0 smoother, residual and prolongation: a thread per row (else per face)
   bool tuned = false;        // the V-cycle autotuner has run (or its choice was taken from its cache)
   bool built = false;
@@ -350,6 +358,10 @@ double amg_theta() {
 
 // ------------------------------------------------------------------------------------------
 // Symbolic setup
+namespace {
+void tail_sizes(hdg_system* s, int tail_rows);
+}
+
 void amg_setup_symbolic(hdg_system* s, const std::vector<char>& dirichlet_face) {
   const bool verbose = std::getenv("HDG_AMG_VERBOSE") != nullptr;
   auto clk = [] { return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count(); };
@@ -621,6 +633,8 @@ void amg_setup_symbolic(hdg_system* s, const std::vector<char>& dirichlet_face) 
     F.rptr.upload(rptr.data(), rptr.size(), st);
     upload_min1(F.rent, rent, st);
     upload_min1(F.rrow, rrow, st);
+    F.h_pptr = std::move(pptr);
+    F.h_rptr = std::move(rptr);
     std::vector<int32_t> qptr, qadj;
     quotient(n, gptr, gadj, agg, na, &qptr, &qadj);
     gptr.swap(qptr);
@@ -655,18 +669,15 @@ void amg_setup_symbolic(hdg_system* s, const std::vector<char>& dirichlet_face) 
       r0[P + 1] += r0[P];
     }
     L.prow0.upload(r0.data(), r0.size(), st);
+    L.h_prow0 = std::move(r0);
   }
   H->tail_from = -1;
   H->tail_cands.clear();
   H->tuned = false;
   H->row_sweep = nf < AMG_ROW_SWEEP_FACES;
   const int tail_rows = amg_tail_rows();
-  if (grouped)
-    for (int l = 1; l + 1 < (int)H->lev.size(); ++l) {
-      if (tail_rows < 0 && H->lev[l].maxrows <= AMG_TAIL_MAXROWS) H->tail_cands.push_back(l);
-      if (tail_rows > 0 && H->tail_from < 0 && H->lev[l].maxrows <= tail_rows) H->tail_from = l;
-    }
-  if (H->tail_from >= 0) H->tail_cands.assign(1, H->tail_from);
+  H->tail_smem.clear();
+  if (grouped && tail_rows != 0) tail_sizes(s, tail_rows);
   // coarsest: per-problem dense blocks
   const AmgLevel& C = H->lev.back();
   H->h_crow0.assign(s->nprob + 1, 0);
@@ -688,8 +699,8 @@ void amg_setup_symbolic(hdg_system* s, const std::vector<char>& dirichlet_face) 
     std::vector<TailLevel> tab(H->lev.size());
     for (size_t l = 0; l < H->lev.size(); ++l) {
       const AmgLevel& L = H->lev[l];
-      tab[l] = TailLevel{amg_group(L.n), L.ptr.p, L.col.p, L.prow0.p, L.val.p, L.dl1inv.p, L.b.p, L.x.p, L.t.p,
-                         L.r.p, L.pptr.p, L.pcol.p, L.rptr.p, L.rent.p, L.rrow.p, L.pval.p};
+      tab[l] = TailLevel{amg_group(L.n), L.ptr.p, L.col.p, L.prow0.p, L.val.p, L.dl1inv.p, L.b.p, L.x.p,
+                         L.pptr.p, L.pcol.p, L.rptr.p, L.rent.p, L.rrow.p, L.pval.p};
     }
     H->tail_tab.upload(tab.data(), tab.size(), st);
   }
@@ -1471,6 +1482,13 @@ __global__ void k_amg_prolong(int n, const int32_t* __restrict__ pptr, const int
   if (lane == 0 && on) x[i] += s;
 }
 
+// A row of the coarsest inverse times b, a warp per row: at(j) = b_j
+template <typename AT> __device__ __forceinline__ float coarse_row(const float* __restrict__ A, int m, AT at) {
+  float s = 0.f;
+  for (int j = threadIdx.x & 31; j < m; j += 32) s += A[j] * at(j);
+  return group_sum_f<32>(s);
+}
+
 // coarsest: x = A^-1 b per problem (one CTA per problem)
 __global__ void k_amg_coarse_solve(const int32_t* __restrict__ crow0, const int32_t* __restrict__ coff,
                                    const float* __restrict__ cinv, const float* __restrict__ b, float* __restrict__ x,
@@ -1478,149 +1496,378 @@ __global__ void k_amg_coarse_solve(const int32_t* __restrict__ crow0, const int3
   const int P = blockIdx.x;
   if (!amg_live(st, P)) return;
   const int r0 = crow0[P], m = crow0[P + 1] - r0;
-  const float* A = cinv + coff[P];
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    float s = 0.f;
-    for (int j = 0; j < m; ++j) s += A[i * m + j] * b[r0 + j];
-    x[r0 + i] = s;
+  for (int i = threadIdx.x >> 5; i < m; i += blockDim.x >> 5) {
+    const float s = coarse_row(cinv + coff[P] + i * m, m, [&](int j) { return b[r0 + j]; });
+    if ((threadIdx.x & 31) == 0) x[r0 + i] = s;
   }
 }
 
-// ---- the coarse levels below a row limit, one CTA per problem ----------------------------
+// ---- the coarse levels that fit in shared memory, a cluster of CTAs per problem -----------
 // k_amg_tail runs the part of the V-cycle from level T down to the coarsest and back up to level
-// T for one problem per CTA, with a CTA barrier between the phases instead of a kernel boundary:
-// (nu - 1) sweeps, residual and restriction (with the next level's first sweep) on each level
-// going down, the dense coarsest solve, then prolongation and nu sweeps on each level going up.
-// Each row is computed exactly as the per-level kernels compute it (the same G lanes per row,
-// taken from the level's size, the same per-lane order and shuffle tree), and the iterates move
-// through the same buffers, so the cycle's result is bit-identical to theirs.
+// T, with a cluster barrier between the phases instead of a kernel boundary: (nu - 1) sweeps,
+// residual and restriction (with the next level's first sweep) on each level going down, the dense
+// coarsest solve, then prolongation and nu sweeps on each level going up.
+//
+// Each phase is a handful of loads per lane, so what bounds it is latency: a launch per phase is 1.5 us in a captured
+// graph.  Here the rows of a problem's levels are dealt out to the CTAs of a cluster, rpc consecutive ones to each, and
+// everything they need is in shared memory: the rows of A, P and P' (an image made once per set-up by k_amg_tail_image
+// and read at the start of each launch) and the whole of the vectors.  A phase ends with each CTA storing its rows'
+// values into the other CTAs' vectors, 16 bytes a lane, so that every gather is local: gathered from the other CTAs
+// four bytes at a time, a sweep over 4200 rows of 29 entries took 2 us.
+//
+// Each row is computed exactly as the per-level kernels compute it (the same G lanes per row, taken from the level's
+// size, the same per-lane order and shuffle tree), so the cycle's result is bit-identical to theirs.
+struct TailShare {  // one level's share of a CTA: rows ra .. ra + nown - 1 of the problem's r0 .. r0 + rows - 1
+  int r0, rows, rpc, ra, nown, g;
+  // offsets in words of shared memory: the vectors x and y, at the same ones in every CTA; the own rows' b and dl1inv; row
+  // starts and entries of A, P and (of the next level's rows) P'
+  int x, y, b;
+  int d, ptr, pptr, rptr, ent, pent, rent;
+  int unused;
+};
+struct TailHead {
+  int vec, words, unused[2];  // ends of the vectors (where the image begins) and of the image
+  TailShare S[AMG_MAX_LEVELS];
+};
+static_assert(sizeof(TailHead) % 16 == 0, "read in 16-byte words");
+
 struct TailArgs {
-  int T, nl, nu;
+  int T, nl, nu, ctas;
   const TailLevel* L;  // device copy of the level table (nl entries), built with the hierarchy
-  const int32_t *crow0, *coff;
+  const int32_t* coff;
   const float* cinv;
   const int32_t* st;
+  const float* b;      // level T's right-hand side and first sweep; the result goes to x
+  float* x;
+  TailHead* head;      // of each CTA
+  uint32_t* image;     // words of them for each CTA
+  size_t words;
 };
 
-__device__ __forceinline__ float group_sum_rt(float v, int G) {
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
+__device__ __host__ inline int tail_align(int w) { return (w + 3) & ~3; }
+// Rows of a level to a CTA: a multiple of four, so that each CTA's part of a vector is 16-byte aligned.
+__device__ __host__ inline int tail_rpc(int rows, int ctas) { return tail_align((rows + ctas - 1) / ctas); }
+
+// The heads and images of the CTAs of k_amg_tail: their rows of A, P and P' on the tail's levels.  An entry is the byte
+// offset of its column's x in shared memory and the value.
+__global__ void __launch_bounds__(256) k_amg_tail_image(TailArgs a) {
+  __shared__ TailHead h;
+  const int P = blockIdx.x / a.ctas, rank = blockIdx.x % a.ctas, t = threadIdx.x, nt = blockDim.x, last = a.nl - 1;
+  for (int l = a.T + t; l <= last; l += nt) {
+    const TailLevel L = a.L[l];
+    TailShare s = {};
+    s.g = L.g;
+    s.r0 = L.prow0[P];
+    s.rows = L.prow0[P + 1] - s.r0;
+    s.rpc = tail_rpc(s.rows, a.ctas);
+    s.ra = s.r0 + min(rank * s.rpc, s.rows);
+    s.nown = min(s.r0 + s.rows - s.ra, s.rpc);
+    h.S[l] = s;
+  }
+  __syncthreads();
+  if (t == 0) {
+    int w = 0;
+    for (int l = a.T; l <= last; ++l) {
+      TailShare& s = h.S[l];
+      s.x = w;
+      s.y = s.x + s.rpc * a.ctas;
+      s.b = s.y + s.rpc * a.ctas;
+      w = s.b + s.rpc;
+    }
+    h.vec = w;
+    for (int l = a.T; l < last; ++l) {
+      TailShare& s = h.S[l];
+      s.d = w;
+      s.ptr = s.d + s.rpc;
+      s.pptr = s.ptr + s.nown + 1;
+      s.rptr = s.pptr + s.nown + 1;
+      w = s.rptr + h.S[l + 1].nown + 1;
+    }
+    w = tail_align(w);
+    for (int l = a.T; l < last; ++l) {
+      TailShare& s = h.S[l];
+      const TailShare& c = h.S[l + 1];
+      const TailLevel L = a.L[l];
+      s.ent = w;
+      s.pent = s.ent + 2 * (L.ptr[s.ra + s.nown] - L.ptr[s.ra]);
+      s.rent = s.pent + 2 * (L.pptr[s.ra + s.nown] - L.pptr[s.ra]);
+      w = s.rent + 2 * (L.rptr[c.ra + c.nown] - L.rptr[c.ra]);
+    }
+    h.words = w;
+    a.head[blockIdx.x] = h;
+  }
+  __syncthreads();
+  uint32_t* const w = a.image + blockIdx.x * a.words;
+  const int vec = h.vec;
+  auto where = [](const TailShare& s, int row) { return 4u * (uint32_t)(s.x + row - s.r0); };
+  for (int l = a.T; l < last; ++l) {
+    const TailLevel L = a.L[l];
+    const TailShare s = h.S[l], c = h.S[l + 1];
+    const int e0 = L.ptr[s.ra], p0 = L.pptr[s.ra], q0 = L.rptr[c.ra];
+    for (int i = t; i < s.nown; i += nt) w[s.d - vec + i] = __float_as_uint(L.dl1inv[s.ra + i]);
+    for (int i = t; i <= s.nown; i += nt) {
+      w[s.ptr - vec + i] = L.ptr[s.ra + i] - e0;
+      w[s.pptr - vec + i] = L.pptr[s.ra + i] - p0;
+    }
+    for (int i = t; i <= c.nown; i += nt) w[s.rptr - vec + i] = L.rptr[c.ra + i] - q0;
+    for (int e = t; e < (s.pent - s.ent) / 2; e += nt) {
+      w[s.ent - vec + 2 * e] = where(s, L.col[e0 + e]);
+      w[s.ent - vec + 2 * e + 1] = __float_as_uint(L.val[e0 + e]);
+    }
+    for (int e = t; e < (s.rent - s.pent) / 2; e += nt) {
+      w[s.pent - vec + 2 * e] = where(c, L.pcol[p0 + e]);
+      w[s.pent - vec + 2 * e + 1] = __float_as_uint(L.pval[p0 + e]);
+    }
+    for (int e = t; e < L.rptr[c.ra + c.nown] - q0; e += nt) {
+      w[s.rent - vec + 2 * e] = where(s, L.rrow[q0 + e]);
+      w[s.rent - vec + 2 * e + 1] = __float_as_uint(L.pval[L.rent[q0 + e]]);
+    }
+  }
 }
 
-// Rows [r0, r1) in groups of G lanes: FN(row, lane, active) returns the lane's partial sum (0 when
-// inactive); every lane of a warp runs the same number of rounds, so the shuffles name all lanes.
-template <typename FN, typename OUT>
-__device__ __forceinline__ void tail_rows(int r0, int r1, int G, FN part, OUT out) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rpw = 32 / G;
-  const int nw = AMG_TAIL_THREADS / 32;
-  for (int base = r0 + warp * rpw; base < r1; base += nw * rpw) {
-    const int i = base + lane / G, gl = lane % G;
-    const bool on = i < r1;
-    float v = on ? part(i, gl) : 0.f;
-    v = group_sum_rt(v, G);
-    if (on && gl == 0) out(i, v);
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, uint4 v) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ void tail_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The rows 0 .. n - 1 of a CTA in groups of G lanes: the sum over a row's entries of value times the word at the entry's
+// offset in x, then out(row, sum) in the group's first lane; every lane of a warp runs the same number of rounds, so the
+// shuffles name all lanes.
+template <int G, typename OUT>
+__device__ __forceinline__ void tail_rows_g(int n, const uint32_t* ptr, const uint2* ent, const uint32_t* x, OUT out) {
+  const int lane = threadIdx.x & 31, gl = lane % G;
+  for (int base = (threadIdx.x >> 5) * (32 / G); base < n; base += (blockDim.x >> 5) * (32 / G)) {
+    const int i = base + lane / G;
+    float s = 0.f;
+    if (i < n) {
+      const int e1 = ptr[i + 1];
+#pragma unroll 4
+      for (int e = ptr[i] + gl; e < e1; e += G) {
+        const uint2 v = ent[e];
+        s += __uint_as_float(v.y) * *reinterpret_cast<const float*>(reinterpret_cast<const char*>(x) + v.x);
+      }
+    }
+    s = group_sum_f<G>(s);
+    if (i < n && gl == 0) out(i, s);
   }
+}
+template <typename OUT>
+__device__ __forceinline__ void tail_rows(int G, int n, const uint32_t* ptr, const uint2* ent, const uint32_t* x, OUT out) {
+  if (G == 4) tail_rows_g<4>(n, ptr, ent, x, out);
+  else if (G == 8) tail_rows_g<8>(n, ptr, ent, x, out);
+  else tail_rows_g<32>(n, ptr, ent, x, out);
 }
 
 __global__ void __launch_bounds__(AMG_TAIL_THREADS) k_amg_tail(TailArgs a) {
-  const int P = blockIdx.x;
-  if (!amg_live(a.st, P)) return;
-  float* iter[AMG_MAX_LEVELS];
+  extern __shared__ __align__(16) uint32_t tail_sm[];
+  __shared__ __align__(16) TailHead h;
+  const int P = blockIdx.x / a.ctas, rank = blockIdx.x % a.ctas, t = threadIdx.x;
+  if (!amg_live(a.st, P)) return;  // the whole cluster
+  const uint32_t base = (uint32_t)__cvta_generic_to_shared(tail_sm);
+  for (int i = t; i < (int)(sizeof(TailHead) / 16); i += blockDim.x)
+    reinterpret_cast<uint4*>(&h)[i] = reinterpret_cast<const uint4*>(a.head + blockIdx.x)[i];
+  __syncthreads();
+  const TailShare* const S = h.S;
   const int nu = a.nu, last = a.nl - 1;
-  // down
+  uint32_t* const sm = tail_sm;
+  float* const smf = reinterpret_cast<float*>(tail_sm);
+  {  // the image, and level T's first sweep and right-hand side
+    const TailShare s = S[a.T];
+    const uint4* im = reinterpret_cast<const uint4*>(a.image + blockIdx.x * a.words);
+    const int words = h.words;
+#pragma unroll 4
+    for (int i = h.vec + 4 * t; i < words; i += 4 * blockDim.x) *reinterpret_cast<uint4*>(sm + i) = im[(i - h.vec) >> 2];
+    for (int i = t; i < s.rows; i += blockDim.x) smf[s.x + i] = a.x[s.r0 + i];
+    for (int i = t; i < s.nown; i += blockDim.x) smf[s.b + i] = a.b[s.ra + i];
+  }
+  // the coarsest inverse's row of each warp (its rows beyond are read when they are needed)
+  constexpr int CW = (AMG_CINV_MAX + 31) / 32;
+  float av[CW];
+  const TailShare z = S[last];
+  const float* const A = a.cinv + a.coff[P] + (z.ra - z.r0) * z.rows;
+#pragma unroll
+  for (int k = 0; k < CW; ++k) {
+    const int j = (t & 31) + 32 * k, i = t >> 5;
+    av[k] = (i < z.nown && j < z.rows) ? A[i * z.rows + j] : 0.f;
+  }
+  tail_sync();  // every CTA of the cluster runs: its shared memory may be written
+  // The own rows of vector v to the other CTAs, the whole cluster past this phase: a warp, or several, to each CTA
+  auto publish = [&](const TailShare& s, int v) {
+    __syncthreads();
+    const int at = v + rank * s.rpc, n4 = (s.nown + 3) >> 2, warps = blockDim.x >> 5;
+    const int shares = max(1, warps / a.ctas);  // warps to a CTA, or the CTAs dealt out to the warps
+    for (int u = t >> 5; u < a.ctas * shares; u += warps) {
+      const int to = u % a.ctas;
+      if (to == rank) continue;
+      const uint32_t dst = cluster_addr(base + 4u * at, to);
+      for (int i = u / a.ctas * 32 + (t & 31); i < n4; i += 32 * shares)
+        cluster_store(dst + 16u * i, *reinterpret_cast<const uint4*>(sm + at + 4 * i));
+    }
+    tail_sync();
+  };
+  // a level's product with the rows of A, P or P' (its row starts and entries) with vector v of the level of s
+  auto rows = [&](int g, int n, int ptr, int ent, const TailShare& s, int v, auto out) {
+    tail_rows(g, n, sm + ptr, reinterpret_cast<const uint2*>(sm + ent), sm + (v - s.x), out);
+  };
+  auto sweep = [&](const TailShare& s, int in, int out) {
+    const int own = rank * s.rpc;
+    rows(s.g, s.nown, s.ptr, s.ent, s, in, [&](int i, float v) {
+      smf[out + own + i] = smf[in + own + i] + (smf[s.b + i] - v) * smf[s.d + i];
+    });
+    publish(s, out);
+  };
+  // down; the iterate starts in x, the residual is left in the other vector
   for (int l = a.T; l < last; ++l) {
-    const TailLevel L = a.L[l];
-    const TailLevel C = a.L[l + 1];
-    const int r0 = L.prow0[P], r1 = L.prow0[P + 1];
-    float* cur = L.x;
-    float* oth = L.t;
+    const TailShare s = S[l], c = S[l + 1];
+    int cur = s.x, oth = s.y;
     for (int sw = 1; sw < nu; ++sw) {
-      const float* xin = cur;
-      float* xout = oth;
-      tail_rows(r0, r1, L.g,
-                [&](int i, int gl) {
-                  float s = 0.f;
-                  for (int e = L.ptr[i] + gl; e < L.ptr[i + 1]; e += L.g) s += L.val[e] * xin[L.col[e]];
-                  return s;
-                },
-                [&](int i, float s) { xout[i] = xin[i] + (L.b[i] - s) * L.dl1inv[i]; });
-      __syncthreads();
-      float* tmp = cur;
+      sweep(s, cur, oth);
+      const int tmp = cur;
       cur = oth;
       oth = tmp;
     }
-    iter[l] = cur;
-    {
-      const float* x = cur;
-      tail_rows(r0, r1, L.g,
-                [&](int i, int gl) {
-                  float s = 0.f;
-                  for (int e = L.ptr[i] + gl; e < L.ptr[i + 1]; e += L.g) s += L.val[e] * x[L.col[e]];
-                  return s;
-                },
-                [&](int i, float s) { L.r[i] = L.b[i] - s; });
-    }
-    __syncthreads();
-    const bool coarsest = (l + 1 == last);
-    tail_rows(C.prow0[P], C.prow0[P + 1], C.g,
-              [&](int J, int gl) {
-                float s = 0.f;
-                for (int k = L.rptr[J] + gl; k < L.rptr[J + 1]; k += C.g) s += L.pval[L.rent[k]] * L.r[L.rrow[k]];
-                return s;
-              },
-              [&](int J, float s) {
-                C.b[J] = s;
-                if (!coarsest) C.x[J] = s * C.dl1inv[J];
-              });
-    __syncthreads();
+    rows(s.g, s.nown, s.ptr, s.ent, s, cur, [&](int i, float v) { smf[oth + rank * s.rpc + i] = smf[s.b + i] - v; });
+    publish(s, oth);
+    // the coarsest right-hand side is gathered too: it goes to y
+    rows(c.g, c.nown, s.rptr, s.rent, s, oth, [&](int J, float v) {
+      if (l + 1 < last) {
+        smf[c.b + J] = v;
+        smf[c.x + rank * c.rpc + J] = v * smf[c.d + J];
+      } else {
+        smf[c.y + rank * c.rpc + J] = v;
+      }
+    });
+    publish(c, l + 1 < last ? c.x : c.y);
   }
-  // coarsest: x = A^-1 b
-  {
-    const TailLevel C = a.L[last];
-    const int r0 = a.crow0[P], m = a.crow0[P + 1] - r0;
-    const float* A = a.cinv + a.coff[P];
-    for (int i = threadIdx.x; i < m; i += blockDim.x) {
-      float s = 0.f;
-      for (int j = 0; j < m; ++j) s += A[i * m + j] * C.b[r0 + j];
-      C.x[r0 + i] = s;
+  // coarsest: x = A^-1 b, in coarse_row's order
+  for (int i = t >> 5; i < z.nown; i += blockDim.x >> 5) {
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < CW; ++k) {
+      const int j = (t & 31) + 32 * k;
+      if (j < z.rows) v += (i == t >> 5 ? av[k] : A[i * z.rows + j]) * smf[z.y + j];
     }
+    v = group_sum_f<32>(v);
+    if ((t & 31) == 0) smf[z.x + rank * z.rpc + i] = v;
   }
-  __syncthreads();
-  // up
-  const float* fin = a.L[last].x;
+  publish(z, z.x);
+  // up; the first sweep reads the vector that the way down ended in
+  int fine = z.x;  // the coarser level's result
   for (int l = last - 1; l >= a.T; --l) {
-    const TailLevel L = a.L[l];
-    const int r0 = L.prow0[P], r1 = L.prow0[P + 1];
-    float* x = iter[l];
-    float* y = L.r;
-    {
-      const float* xc = fin;
-      tail_rows(r0, r1, L.g,
-                [&](int i, int gl) {
-                  float s = 0.f;
-                  for (int e = L.pptr[i] + gl; e < L.pptr[i + 1]; e += L.g) s += L.pval[e] * xc[L.pcol[e]];
-                  return s;
-                },
-                [&](int i, float s) { x[i] += s; });
-    }
-    __syncthreads();
+    const TailShare s = S[l], c = S[l + 1];
+    int cur = (nu & 1) ? s.x : s.y, oth = (nu & 1) ? s.y : s.x;
+    rows(s.g, s.nown, s.pptr, s.pent, c, fine, [&](int i, float v) { smf[cur + rank * s.rpc + i] += v; });
+    publish(s, cur);
     for (int sw = 0; sw < nu; ++sw) {
-      const float* xin = x;
-      float* xout = y;
-      tail_rows(r0, r1, L.g,
-                [&](int i, int gl) {
-                  float s = 0.f;
-                  for (int e = L.ptr[i] + gl; e < L.ptr[i + 1]; e += L.g) s += L.val[e] * xin[L.col[e]];
-                  return s;
-                },
-                [&](int i, float s) { xout[i] = xin[i] + (L.b[i] - s) * L.dl1inv[i]; });
-      __syncthreads();
-      float* tmp = x;
-      x = y;
-      y = tmp;
+      sweep(s, cur, oth);  // the last one too ends with the barrier: no CTA leaves while another writes to it
+      const int tmp = cur;
+      cur = oth;
+      oth = tmp;
     }
-    fin = x;
+    fine = cur;
   }
+  const TailShare s = S[a.T];
+  for (int i = t; i < s.nown; i += blockDim.x) a.x[s.ra + i] = smf[fine + rank * s.rpc + i];
+}
+
+int amg_coarse_sweeps(const hdg_system* s);
+TailArgs tail_args(hdg_system* s, const int32_t* cst) {
+  AmgHierarchy* H = s->amg;
+  AmgLevel& L = H->lev[H->tail_from];
+  return TailArgs{H->tail_from, (int)H->lev.size(), amg_coarse_sweeps(s), H->tail_ctas, H->tail_tab.p, H->coff.p, H->cinv.p,
+                  cst, L.b.p, L.x.p, reinterpret_cast<TailHead*>(H->tail_head.p), H->tail_image.p, H->tail_words};
+}
+
+// Clusters of k_amg_tail of 16, 8, 4, 2 CTAs that the device holds at once, a CTA to an SM.
+const int* tail_clusters(int device) {
+  static std::mutex mu;
+  static std::map<int, std::array<int, 4>> known;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = known.find(device);
+  if (it != known.end()) return it->second.data();
+  HDG_CUDA(cudaFuncSetAttribute(k_amg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, AMG_TAIL_SMEM));
+  HDG_CUDA(cudaFuncSetAttribute(k_amg_tail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  std::array<int, 4> n;
+  for (int k = 0; k < 4; ++k) {
+    const int ctas = 16 >> k;
+    cudaLaunchConfig_t cf = {};
+    cf.gridDim = dim3((unsigned)ctas);
+    cf.blockDim = dim3(AMG_TAIL_THREADS);
+    cf.dynamicSmemBytes = AMG_TAIL_SMEM;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cf.attrs = &at;
+    cf.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n[k], k_amg_tail, &cf) != cudaSuccess) {
+      cudaGetLastError();
+      n[k] = 0;
+    }
+  }
+  return known.emplace(device, n).first->second.data();
+}
+
+// The cluster's size, the levels that the tail may start at (the shared memory of every CTA holds its share and the
+// threads pass over its rows in a few rounds), and the image's buffers.  One V-cycle, us, by launches / clusters of 16, 8,
+// 4: one problem of 32787 rows on the first coarse level 117 / 112 / 117 / 128; 16 problems 112 / 114 / 103 / 109; 19 problems
+// 129 / 135 / 123 / 128.  The device holds 8 or 9 of 16 CTAs, 16 to 18 of 8, and so on: the largest of which at most half wait.
+void tail_sizes(hdg_system* s, int tail_rows) {
+  AmgHierarchy* H = s->amg;
+  const int np = s->nprob, nl = (int)H->lev.size(), last = nl - 1;
+  if (nl < 2 || np < 1) return;
+  const int* most = tail_clusters(s->ctx->device);
+  int C = 1, share = 2;  // CTAs to an SM
+  for (int k = 0; k < 4 && C == 1; ++k)
+    if (2 * np <= 3 * most[k]) {
+      C = 16 >> k;
+      share = (np + most[k] - 1) / most[k];
+    }
+  H->tail_ctas = C;
+  std::vector<int> vec((size_t)np * C, 0), mid(vec), ent(vec);  // words of each CTA, of the levels from l on
+  std::vector<int> rpc_c(np);
+  H->tail_words = 0;
+  for (int l = last; l >= 0; --l) {
+    const AmgLevel& L = H->lev[l];
+    int need = 0, image = 0, rounds = 0;
+    for (int P = 0; P < np; ++P) {
+      const int r0 = L.h_prow0[P], rows = L.h_prow0[P + 1] - r0, rpc = tail_rpc(rows, C);
+      rounds = std::max(rounds, (int)(((int64_t)rpc * amg_group(L.n) + AMG_TAIL_THREADS - 1) / AMG_TAIL_THREADS));
+      for (int k = 0; k < C; ++k) {
+        const int64_t q = (int64_t)P * C + k;
+        vec[q] += (2 * C + 1) * rpc;
+        if (l < last) {
+          const AmgLevel& N = H->lev[l + 1];
+          const int ra = r0 + std::min(k * rpc, rows), own = std::min(r0 + rows - ra, rpc);
+          const int c0 = N.h_prow0[P], nc = N.h_prow0[P + 1] - c0, cpc = tail_rpc(nc, C);
+          const int ca = c0 + std::min(k * cpc, nc), cn = std::min(c0 + nc - ca, cpc);
+          mid[q] += rpc + 2 * (own + 1) + cn + 1;
+          ent[q] += 2 * (L.h_ptr[ra + own] - L.h_ptr[ra] + L.h_pptr[ra + own] - L.h_pptr[ra] + L.h_rptr[ca + cn] - L.h_rptr[ca]);
+        }
+        const int im = tail_align(tail_align(mid[q]) + ent[q]);
+        image = std::max(image, im);
+        need = std::max(need, vec[q] + im);
+      }
+    }
+    if (need * 4 > AMG_TAIL_SMEM / share || rounds > AMG_TAIL_ROUNDS) break;
+    if (l == last) continue;
+    if (tail_rows > 0 && (l < 1 || L.maxrows > tail_rows)) break;
+    H->tail_cands.insert(H->tail_cands.begin(), l);
+    H->tail_smem.insert(H->tail_smem.begin(), (size_t)need * 4);
+    H->tail_words = (size_t)image;
+  }
+  if (H->tail_cands.empty()) return;
+  H->tail_from = H->tail_cands.front();
+  H->tail_image.alloc(H->tail_words * np * C);
+  H->tail_head.alloc(sizeof(TailHead) * np * C);
 }
 
 inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)std::max<int64_t>(1, (n + t - 1) / t); }
@@ -1748,6 +1995,32 @@ template <int NT> void numeric_nt(hdg_system* s, const float* val0, cudaStream_t
   HDG_CUDA(cudaGetLastError());
 }
 
+// The image for the tail that starts at H->tail_from, from the current values.
+void make_tail_image(hdg_system* s, cudaStream_t st) {
+  AmgHierarchy* H = s->amg;
+  if (H->tail_from < 0) return;
+  k_amg_tail_image<<<(unsigned)(s->nprob * H->tail_ctas), 256, 0, st>>>(tail_args(s, nullptr));
+  HDG_CUDA(cudaGetLastError());
+  s->ctx->launches++;
+}
+
+void launch_tail(hdg_system* s, const int32_t* cst, cudaStream_t st) {
+  AmgHierarchy* H = s->amg;
+  const size_t k = std::find(H->tail_cands.begin(), H->tail_cands.end(), H->tail_from) - H->tail_cands.begin();
+  cudaLaunchConfig_t cf = {};
+  cf.gridDim = dim3((unsigned)(s->nprob * H->tail_ctas));
+  cf.blockDim = dim3(AMG_TAIL_THREADS);
+  cf.dynamicSmemBytes = H->tail_smem[k];
+  cf.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)H->tail_ctas;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cf.attrs = &at;
+  cf.numAttrs = 1;
+  HDG_CUDA(cudaLaunchKernelEx(&cf, k_amg_tail, tail_args(s, cst)));
+}
+
 // One level-0 Chebyshev step, a thread per row or a thread per face (H->row_sweep, tuned; both
 // give the same bits).  Measured before the tuner: 49 k faces (p = 4): rows 15 -> 10 us per
 // sweep; 197 k faces (p = 2) and the batch's bins (0.4-0.7 M faces): faces faster.
@@ -1828,17 +2101,12 @@ void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const i
   }
   int up_from = nl - 2;
   if (T < nl) {
-    const TailArgs ta{T, nl, nu, H->tail_tab.p, H->crow0.p, H->coff.p, H->cinv.p, cst};
-    k_amg_tail<<<s->nprob, AMG_TAIL_THREADS, 0, st>>>(ta);
-    // where the tail leaves level T's result: the iterate after nu - 1 sweeps from x (alternating
-    // with t), then nu sweeps from it alternating with r
-    AmgLevel& L = H->lev[T];
-    float* it = ((nu - 1) % 2 == 0) ? L.x.p : L.t.p;
-    fin[T] = (nu % 2 == 0) ? it : L.r.p;
+    launch_tail(s, cst, st);
+    fin[T] = H->lev[T].x.p;
     up_from = T - 1;
   } else {
     AmgLevel& C = H->lev.back();
-    if (H->cmax > 0) k_amg_coarse_solve<<<s->nprob, 128, 0, st>>>(H->crow0.p, H->coff.p, H->cinv.p, C.b.p, C.x.p, cst);
+    if (H->cmax > 0) k_amg_coarse_solve<<<s->nprob, 512, 0, st>>>(H->crow0.p, H->coff.p, H->cinv.p, C.b.p, C.x.p, cst);
     fin[nl - 1] = C.x.p;
   }
   // coarse levels up: prolongate the coarser level's result into this level's iterate, then nu
@@ -1890,6 +2158,7 @@ void amg_setup_numeric(hdg_system* s, cudaStream_t st) {
     case 5: numeric_nt<5>(s, v0, st); break;
   }
   if (!s->amg->tuned) amg_tune(s, st);
+  make_tail_image(s, st);
 }
 
 // Algorithmic bytes of one V-cycle: every array a cycle kernel reads or writes, once (gathered
@@ -1977,7 +2246,7 @@ void amg_apply(hdg_system* s, const float* r, float* z, const int32_t* cg_state,
 // ---- V-cycle autotuner ---------------------------------------------------------------------
 // The launch shapes of the cycle that do not change its result are picked by timing, once per
 // hierarchy: the level-0 smoother with a thread per face or per row, and the level T from which
-// one k_amg_tail launch (a CTA per problem) replaces the per-level launches (or none).  Every
+// one k_amg_tail launch (a cluster per problem) replaces the per-level launches (or none).  Every
 // candidate computes the same bits, so the choice changes only the time.  Each candidate's cycle
 // is captured twice into a CUDA graph, as the CG chunks run it (timing un-graphed launches would
 // charge the host's launch overhead to the many-launch candidates), and the graph runs once
@@ -2025,12 +2294,12 @@ void amg_tune(hdg_system* s, cudaStream_t st) {
       if (tune_tail) {
         const int t = it->second.tail;
         const bool ok = t < 0 || std::find(H->tail_cands.begin(), H->tail_cands.end(), t) != H->tail_cands.end();
-        H->tail_from = ok ? t : -1;
+        H->tail_from = ok ? t : H->tail_cands.front();
       }
       return;
     }
   }
-  if (!s->amg_tune_time) return;  // the defaults: sweep by face count, no tail
+  if (!s->amg_tune_time) return;  // the defaults: sweep by face count, the longest tail that fits
   const int64_t n0 = (int64_t)H->nf * s->nt;
   DevBuf<float> rin, zout;
   rin.alloc((size_t)n0);
@@ -2056,6 +2325,7 @@ void amg_tune(hdg_system* s, cudaStream_t st) {
     for (int tl : tails) {
       H->row_sweep = (rw == 1);
       H->tail_from = tl;
+      make_tail_image(s, st);
       cudaGraph_t g;
       cudaGraphExec_t ge;
       HDG_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
