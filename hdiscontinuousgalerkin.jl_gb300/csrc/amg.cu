@@ -308,7 +308,7 @@ struct AmgHierarchy {
   DevBuf<__half> val0h;      // D^-1 A0 in FP16, read by the cycle's level-0 sweeps (default storage)
   DevBuf<float> x0, r0, d0;  // level-0 cycle vectors (iterate, scaled residual, Chebyshev correction)
   DevBuf<float> bt0;         // D^-1 b of the current cycle
-  DevBuf<float> dpval0;      // [nf*nt][PW] D P0 (restriction of the scaled residual)
+  DevBuf<float> rval0;       // [entries of P0'][nt] D P0 (restriction of the scaled residual), in the order of rent0
   std::vector<AmgLevel> lev; // lev[0] is level 1
   // coarsest (last level): per-problem dense inverses
   std::vector<int32_t> h_crow0;  // [nprob+1] first coarsest row of each problem
@@ -552,7 +552,7 @@ void amg_setup_symbolic(hdg_system* s, const std::vector<char>& dirichlet_face) 
   H->r0.alloc((size_t)nf * nt);
   H->d0.alloc((size_t)nf * nt);
   H->bt0.alloc((size_t)nf * nt);
-  H->dpval0.alloc((size_t)nf * nt * PW);
+  H->rval0.alloc(std::max<size_t>(rent0.size() * nt, 1));
   H->lev.clear();
   H->lev.push_back(std::move(L1));
   tph[5] = clk();
@@ -1052,21 +1052,18 @@ __global__ void k_amg_coarse_inv(const int32_t* __restrict__ crow0, const int32_
   }
 }
 
-// D P0 (D the face-block diagonal of A0), for the restriction of the scaled residual.
+// D P0 (D the face-block diagonal of A0), for the restriction of the scaled residual: the nt values of each entry of P0'.
 template <int NT>
-__global__ void k_amg_dp0(int nf, const int8_t* __restrict__ kdiag, const float* __restrict__ val,
-                          const float* __restrict__ pval0, float* __restrict__ dpval0) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nf) return;
+__global__ void k_amg_dp0(int64_t n, int nf, const int8_t* __restrict__ kdiag, const float* __restrict__ val,
+                          const int32_t* __restrict__ rent0, const float* __restrict__ pval0, float* __restrict__ rval0) {
+  const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (m >= n) return;
+  const int e = rent0[m / NT], f = e / PW, c = e - f * PW, i = (int)(m % NT), kd = kdiag[f];
   const int64_t nd = (int64_t)nf * NT;
-  const int kd = kdiag[f];
-  for (int i = 0; i < NT; ++i)
-    for (int c = 0; c < PW; ++c) {
-      float s = 0.f;
-      for (int l = 0; l < NT; ++l)
-        s += val[(kd * NT + l) * nd + (int64_t)f * NT + i] * pval0[((int64_t)f * NT + l) * PW + c];
-      dpval0[((int64_t)f * NT + i) * PW + c] = s;
-    }
+  float s = 0.f;
+  for (int l = 0; l < NT; ++l)
+    s += val[(kd * NT + l) * nd + (int64_t)f * NT + i] * pval0[((int64_t)f * NT + l) * PW + c];
+  rval0[m] = s;
 }
 
 // Level-0 values of the cycle, D^-1 A0, read as FP32.
@@ -1337,21 +1334,43 @@ __global__ void k_amg_face_residual_f(int nf, const int32_t* __restrict__ bcol5,
   store_face<NT>(r, f, s);
 }
 
-// b1 = P0' r0 = (D P0)' r~0 and the first l1-Jacobi sweep of level 1: x1 = b1 / dl1
-template <int NT>
+// Row and lane of a thread.  Warps whose first row is past the end leave at once (uniformly);
+// in the last warp every lane stays until the shuffle, which names all 32 lanes.
+#define AMG_GROUP_ROW(ROW, LANE, N)                                                   \
+  const int64_t t_ = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;                 \
+  if ((t_ - (threadIdx.x & 31)) / G >= (N)) return;                                   \
+  const int ROW = (int)(t_ / G), LANE = (int)(t_ % G)
+
+template <int G> __device__ __forceinline__ float group_sum_f(float v) {
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// b1 = P0' r0 = (D P0)' r~0 and the first l1-Jacobi sweep of level 1: x1 = b1 / dl1.  What bounds it is the memory: G lanes
+// share a row, and its values lie in the order in which they read them.  (A thread per row over values stored by face
+// touched five times the bytes.)  One V-cycle before / with G = 4, 8, 16: 787456 faces of p = 3 387 / 373, 375, 386 us, 98645
+// of p = 4 113.7 / 111.3, 111.2, 111.9.
+template <int NT, int G>
 __global__ void k_amg_restrict0(int na, const int32_t* __restrict__ rptr0, const int32_t* __restrict__ rent0,
-                                const float* __restrict__ pval0, const float* __restrict__ r0,
+                                const float* __restrict__ rval0, const float* __restrict__ r0,
                                 const float* __restrict__ dl1inv, float* __restrict__ b1, float* __restrict__ x1,
                                 const int32_t* __restrict__ prob1, const int32_t* __restrict__ st) {
-  const int J = blockIdx.x * blockDim.x + threadIdx.x;
-  if (J >= na || !amg_live(st, prob1[J])) return;
+  AMG_GROUP_ROW(J, lane, na);
+  const bool on = J < na && amg_live(st, prob1[J]);
   float s = 0.f;
-  for (int t = rptr0[J]; t < rptr0[J + 1]; ++t) {
-    const int f = rent0[t] / PW, c = rent0[t] - f * PW;
-    for (int i = 0; i < NT; ++i) s += pval0[((int64_t)f * NT + i) * PW + c] * r0[(int64_t)f * NT + i];
+  if (on) {
+    const int t0 = rptr0[J], n = (rptr0[J + 1] - t0) * NT;
+    const int32_t* ent = rent0 + t0;
+    const float* v = rval0 + (int64_t)t0 * NT;
+#pragma unroll 4
+    for (int q = lane; q < n; q += G) s += v[q] * r0[(int64_t)(ent[q / NT] / PW) * NT + q % NT];
   }
-  b1[J] = s;
-  x1[J] = s * dl1inv[J];
+  s = group_sum_f<G>(s);
+  if (lane == 0 && on) {
+    b1[J] = s;
+    x1[J] = s * dl1inv[J];
+  }
 }
 
 // x0 += P0 x1
@@ -1406,19 +1425,6 @@ __global__ void k_amg_prolong0_f(int nf, const int32_t* __restrict__ pcol0, cons
 // and use whole warps, which shortens each row's chain of dependent loads; large levels (the
 // first coarse levels of a batch hold 10^5 rows and more) are bandwidth-bound and use 4 lanes,
 // which keeps most lanes busy on rows of 10-20 entries.
-// Row and lane of a thread.  Warps whose first row is past the end leave at once (uniformly);
-// in the last warp every lane stays until the shuffle, which names all 32 lanes.
-#define AMG_GROUP_ROW(ROW, LANE, N)                                                   \
-  const int64_t t_ = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;                 \
-  if ((t_ - (threadIdx.x & 31)) / G >= (N)) return;                                   \
-  const int ROW = (int)(t_ / G), LANE = (int)(t_ % G)
-
-template <int G> __device__ __forceinline__ float group_sum_f(float v) {
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // x_out = x_in + (b - A x_in) / dl1
 template <int G>
 __global__ void k_amg_l1_sweep(int n, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
@@ -1960,7 +1966,8 @@ template <int NT> void numeric_nt(hdg_system* s, const float* val0, cudaStream_t
   AmgLevel& L1 = H->lev[0];
   k_amg_rap0<NT><<<nblk((int64_t)L1.n * 32), 256, 0, st>>>(L1.n, H->wap, H->rptr0.p, H->rent0.p, H->pval0.p, H->apcol0.p,
                                              H->apval0.p, L1.ptr.p, L1.col.p, L1.val.p);
-  k_amg_dp0<NT><<<nblk(nf), 256, 0, st>>>(nf, s->d_kdiag.p, val0, H->pval0.p, H->dpval0.p);
+  const int64_t nr = (int64_t)H->rent0.n * NT;
+  k_amg_dp0<NT><<<nblk(nr), 256, 0, st>>>(nr, nf, s->d_kdiag.p, val0, H->rent0.p, H->pval0.p, H->rval0.p);
   if (amg_level0_fp32()) {
     k_amg_scale0<NT, float><<<nblk(nf), 256, 0, st>>>(nf, H->dinv0.p, val0, const_cast<float*>(val0));
   } else {
@@ -2068,8 +2075,8 @@ void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const i
     k_amg_face_residual_f<NT, VT><<<nblk(nf), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->bt0.p, z0, H->r0.p,
                                                             H->face_prob.p, cst);
   AmgLevel& L1 = H->lev[0];
-  k_amg_restrict0<NT><<<nblk(L1.n), 256, 0, st>>>(L1.n, H->rptr0.p, H->rent0.p, H->dpval0.p, H->r0.p, L1.dl1inv.p,
-                                                  L1.b.p, L1.x.p, L1.prob.p, cst);
+  k_amg_restrict0<NT, 4><<<nblk((int64_t)L1.n * 4), 256, 0, st>>>(L1.n, H->rptr0.p, H->rent0.p, H->rval0.p, H->r0.p,
+                                                                 L1.dl1inv.p, L1.b.p, L1.x.p, L1.prob.p, cst);
   // coarse levels down: x holds the first l1-Jacobi sweep (done by the restriction); the other
   // nu - 1 sweeps alternate between x and t; the iterate then stays where it is until the way up
   const int nu = amg_coarse_sweeps(s);
