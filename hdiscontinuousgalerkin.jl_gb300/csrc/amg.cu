@@ -1191,6 +1191,8 @@ __global__ void k_amg_scale0(int nf, const float* __restrict__ dinv, const float
 __device__ __forceinline__ bool amg_live(const int32_t* __restrict__ st, int P) {
   return !st || st[HDG_CG_ST * P] == 0 || st[HDG_CG_ST * P + 3] != 0;
 }
+// A row's problem; a single one has no list (a link less in the chain of loads).
+__device__ __forceinline__ int prob_at(const int32_t* __restrict__ prob, int i) { return prob ? prob[i] : 0; }
 
 
 // Level-0 smoother: step `step` of the Chebyshev iteration (Saad, Iterative Methods, 12.3) for
@@ -1204,7 +1206,7 @@ __global__ void k_amg_face_cheb(int nf, const int32_t* __restrict__ bcol5, const
                                 float* __restrict__ bt, const float* __restrict__ xin, float* __restrict__ xout,
                                 float* __restrict__ d, int step, float ratio, const int32_t* __restrict__ st) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nf || !amg_live(st, face_prob[f])) return;
+  if (f >= nf || !amg_live(st, prob_at(face_prob, f))) return;
   // t = D^-1 (b - A x) = bt - (D^-1 A) x: val holds the block rows of A scaled by D^-1, and
   // the first step (x = 0) forms bt = D^-1 b for the rest of the cycle
   float t[NT];
@@ -1228,7 +1230,7 @@ __global__ void k_amg_face_cheb(int nf, const int32_t* __restrict__ bcol5, const
     for (int k = 0; k < 5; ++k) load_face<NT>(xin, bcol5[k * nf + f], xv + k * NT);
     face_subtract<NT>(val, nf, f, xv, t);
   }
-  const float hi = fmaxf(lam[face_prob[f]], 1e-30f), lo = hi / ratio;
+  const float hi = fmaxf(lam[prob_at(face_prob, f)], 1e-30f), lo = hi / ratio;
   const float theta = 0.5f * (hi + lo), delta = 0.5f * (hi - lo), sigma = theta / delta;
   float rp = 1.f / sigma, rc = rp;  // rho_{step-1}, rho_step
   for (int u = 1; u <= step; ++u) {
@@ -1264,7 +1266,7 @@ __global__ void k_amg_row_cheb(int nf, const int32_t* __restrict__ bcol5, const 
   const int64_t nd = (int64_t)nf * NT;
   if (row >= nd) return;
   const int f = (int)(row / NT), i = (int)(row - (int64_t)f * NT);
-  if (!amg_live(st, face_prob[f])) return;
+  if (!amg_live(st, prob_at(face_prob, f))) return;
   // t = D^-1 (b - A x) = bt - (D^-1 A) x: the first step (x = 0) forms bt = D^-1 b for the rest
   // of the cycle
   float t;
@@ -1282,7 +1284,7 @@ __global__ void k_amg_row_cheb(int nf, const int32_t* __restrict__ bcol5, const 
       for (int j = 0; j < NT; ++j) t -= ld0<NT>(val, nf, f, i, k, j) * xin[(int64_t)g * NT + j];
     }
   }
-  const float hi = fmaxf(lam[face_prob[f]], 1e-30f), lo = hi / ratio;
+  const float hi = fmaxf(lam[prob_at(face_prob, f)], 1e-30f), lo = hi / ratio;
   const float theta = 0.5f * (hi + lo), delta = 0.5f * (hi - lo), sigma = theta / delta;
   float rp = 1.f / sigma, rc = rp;  // rho_{step-1}, rho_step
   for (int u = 1; u <= step; ++u) {
@@ -1304,7 +1306,7 @@ __global__ void k_amg_face_residual(int nf, const int32_t* __restrict__ bcol5, c
   const int64_t nd = (int64_t)nf * NT;
   if (row >= nd) return;
   const int f = (int)(row / NT), i = (int)(row - (int64_t)f * NT);
-  if (!amg_live(st, face_prob[f])) return;
+  if (!amg_live(st, prob_at(face_prob, f))) return;
   float s = b[row];
   // padding slots repeat the face with zero values: no test needed
 #pragma unroll
@@ -1324,7 +1326,7 @@ __global__ void k_amg_face_residual_f(int nf, const int32_t* __restrict__ bcol5,
                                       float* __restrict__ r, const int32_t* __restrict__ face_prob,
                                       const int32_t* __restrict__ st) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nf || !amg_live(st, face_prob[f])) return;
+  if (f >= nf || !amg_live(st, prob_at(face_prob, f))) return;
   float s[NT];
   load_face<NT>(b, f, s);
   float xv[5 * NT];
@@ -1357,7 +1359,7 @@ __global__ void k_amg_restrict0(int na, const int32_t* __restrict__ rptr0, const
                                 const float* __restrict__ dl1inv, float* __restrict__ b1, float* __restrict__ x1,
                                 const int32_t* __restrict__ prob1, const int32_t* __restrict__ st) {
   AMG_GROUP_ROW(J, lane, na);
-  const bool on = J < na && amg_live(st, prob1[J]);
+  const bool on = J < na && amg_live(st, prob_at(prob1, J));
   float s = 0.f;
   if (on) {
     const int t0 = rptr0[J], n = (rptr0[J + 1] - t0) * NT;
@@ -1381,7 +1383,7 @@ __global__ void k_amg_prolong0(int nf, const int32_t* __restrict__ pcol0, const 
   const int64_t row = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (row >= (int64_t)nf * NT) return;
   const int f = (int)(row / NT);
-  if (!amg_live(st, face_prob[f])) return;
+  if (!amg_live(st, prob_at(face_prob, f))) return;
   float s = 0.f;
   for (int c = 0; c < PW; ++c) {
     const int J = pcol0[f * PW + c];
@@ -1398,7 +1400,7 @@ __global__ void k_amg_prolong0_f(int nf, const int32_t* __restrict__ pcol0, cons
                                  const float* __restrict__ x1, float* __restrict__ x0,
                                  const int32_t* __restrict__ face_prob, const int32_t* __restrict__ st) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= nf || !amg_live(st, face_prob[f])) return;
+  if (f >= nf || !amg_live(st, prob_at(face_prob, f))) return;
   float xv[PW];
   int nc = 0;
 #pragma unroll
@@ -1425,6 +1427,55 @@ __global__ void k_amg_prolong0_f(int nf, const int32_t* __restrict__ pcol0, cons
 // and use whole warps, which shortens each row's chain of dependent loads; large levels (the
 // first coarse levels of a batch hold 10^5 rows and more) are bandwidth-bound and use 4 lanes,
 // which keeps most lanes busy on rows of 10-20 entries.
+// What bounds these kernels is the chain of dependent loads: a row's ends and whether its problem runs, its columns, the
+// gathered values.  So the loads of a link are issued together, four entries of a lane at a time, and what the row's end
+// needs is loaded ahead.  One V-cycle, us, entry by entry / four at a time: 98645 faces of p = 4 111 / 105, 197120 of p = 2
+// 70 / 66, 787456 of p = 3 373 / 348, 16 problems 101 / 100, 14 of p = 3 178 / 172.
+
+// A lane's part of a row: entries e0 + lane, + G, ..., added in that order; ent(e, v, at): an entry's value and where its
+// column's value is.
+template <int G, typename ENT> __device__ __forceinline__ float row_part(int e0, int e1, int lane, ENT ent) {
+  constexpr int U = 4;
+  float s = 0.f;
+  int e = e0 + lane;
+  for (; e + (U - 1) * G < e1; e += U * G) {
+    float v[U], xv[U];
+    const float* at[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) ent(e + u * G, v[u], at[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) xv[u] = *at[u];
+#pragma unroll
+    for (int u = 0; u < U; ++u) s += v[u] * xv[u];
+  }
+  if (e < e1) {  // the rest, three at most
+    float v[U - 1], xv[U - 1];
+    const float* at[U - 1];
+#pragma unroll
+    for (int u = 0; u < U - 1; ++u) {
+      at[u] = nullptr;
+      if (e + u * G < e1) ent(e + u * G, v[u], at[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U - 1; ++u)
+      if (at[u]) xv[u] = *at[u];
+#pragma unroll
+    for (int u = 0; u < U - 1; ++u)
+      if (at[u]) s += v[u] * xv[u];
+  }
+  return s;
+}
+// The row's ends, and whether its problem runs (prob NULL: the only one).
+#define AMG_ROW_ENDS(I, N, PTR, PROB)                          \
+  int e0_ = 0, e1_ = 0, P_ = 0;                                \
+  if (I < (N)) {                                               \
+    e0_ = PTR[I];                                              \
+    e1_ = PTR[I + 1];                                          \
+    P_ = prob_at(PROB, I);                                     \
+  }                                                            \
+  const bool on = I < (N) && amg_live(st, P_);                 \
+  if (!on) e1_ = e0_
+
 // x_out = x_in + (b - A x_in) / dl1
 template <int G>
 __global__ void k_amg_l1_sweep(int n, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
@@ -1432,12 +1483,16 @@ __global__ void k_amg_l1_sweep(int n, const int32_t* __restrict__ ptr, const int
                                const float* __restrict__ b, const float* __restrict__ xin, float* __restrict__ xout,
                                const int32_t* __restrict__ prob, const int32_t* __restrict__ st) {
   AMG_GROUP_ROW(i, lane, n);
-  const bool on = i < n && amg_live(st, prob[i]);
-  float s = 0.f;
-  if (on)
-    for (int e = ptr[i] + lane; e < ptr[i + 1]; e += G) s += val[e] * xin[col[e]];
+  AMG_ROW_ENDS(i, n, ptr, prob);
+  float bi = 0.f, di = 0.f, xi = 0.f;
+  if (lane == 0 && on) {
+    bi = b[i];
+    di = dl1inv[i];
+    xi = xin[i];
+  }
+  float s = row_part<G>(e0_, e1_, lane, [&](int e, float& v, const float*& at) { v = val[e]; at = xin + col[e]; });
   s = group_sum_f<G>(s);
-  if (lane == 0 && on) xout[i] = xin[i] + (b[i] - s) * dl1inv[i];
+  if (lane == 0 && on) xout[i] = xi + (bi - s) * di;
 }
 
 // r = b - A x
@@ -1447,12 +1502,11 @@ __global__ void k_amg_residual(int n, const int32_t* __restrict__ ptr, const int
                                float* __restrict__ r, const int32_t* __restrict__ prob,
                                const int32_t* __restrict__ st) {
   AMG_GROUP_ROW(i, lane, n);
-  const bool on = i < n && amg_live(st, prob[i]);
-  float s = 0.f;
-  if (on)
-    for (int e = ptr[i] + lane; e < ptr[i + 1]; e += G) s += val[e] * x[col[e]];
+  AMG_ROW_ENDS(i, n, ptr, prob);
+  const float bi = (lane == 0 && on) ? b[i] : 0.f;
+  float s = row_part<G>(e0_, e1_, lane, [&](int e, float& v, const float*& at) { v = val[e]; at = x + col[e]; });
   s = group_sum_f<G>(s);
-  if (lane == 0 && on) r[i] = b[i] - s;
+  if (lane == 0 && on) r[i] = bi - s;
 }
 
 // b_c = P' r and x_c = b_c / dl1_c (first sweep of the coarse level; dl1 NULL on the coarsest)
@@ -1463,14 +1517,13 @@ __global__ void k_amg_restrict(int nc, const int32_t* __restrict__ rptr, const i
                                float* __restrict__ xc, const int32_t* __restrict__ probc,
                                const int32_t* __restrict__ st) {
   AMG_GROUP_ROW(J, lane, nc);
-  const bool on = J < nc && amg_live(st, probc[J]);
-  float s = 0.f;
-  if (on)
-    for (int k = rptr[J] + lane; k < rptr[J + 1]; k += G) s += pval[rent[k]] * r[rrow[k]];
+  AMG_ROW_ENDS(J, nc, rptr, probc);
+  const float dj = (lane == 0 && on && dl1inv) ? dl1inv[J] : 0.f;
+  float s = row_part<G>(e0_, e1_, lane, [&](int k, float& v, const float*& at) { v = pval[rent[k]]; at = r + rrow[k]; });
   s = group_sum_f<G>(s);
   if (lane == 0 && on) {
     bc[J] = s;
-    if (dl1inv) xc[J] = s * dl1inv[J];
+    if (dl1inv) xc[J] = s * dj;
   }
 }
 
@@ -1480,12 +1533,11 @@ __global__ void k_amg_prolong(int n, const int32_t* __restrict__ pptr, const int
                               const float* __restrict__ pval, const float* __restrict__ xc, float* __restrict__ x,
                               const int32_t* __restrict__ prob, const int32_t* __restrict__ st) {
   AMG_GROUP_ROW(i, lane, n);
-  const bool on = i < n && amg_live(st, prob[i]);
-  float s = 0.f;
-  if (on)
-    for (int e = pptr[i] + lane; e < pptr[i + 1]; e += G) s += pval[e] * xc[pcol[e]];
+  AMG_ROW_ENDS(i, n, pptr, prob);
+  const float xi = (lane == 0 && on) ? x[i] : 0.f;
+  float s = row_part<G>(e0_, e1_, lane, [&](int e, float& v, const float*& at) { v = pval[e]; at = xc + pcol[e]; });
   s = group_sum_f<G>(s);
-  if (lane == 0 && on) x[i] += s;
+  if (lane == 0 && on) x[i] = xi + s;
 }
 
 // A row of the coarsest inverse times b, a warp per row: at(j) = b_j
@@ -2036,6 +2088,7 @@ void cheb_sweep(hdg_system* s, const VT* val0, const float* b0, const float* in,
                 const int32_t* cst, cudaStream_t st) {
   AmgHierarchy* H = s->amg;
   const int nf = H->nf;
+  const int32_t* fprob = s->nprob > 1 ? H->face_prob.p : nullptr;
   EventPair* ep = nullptr;
   if (s->prof_cheb0) {  // a sampled chunk: each sweep timed on its own
     ep = new EventPair();
@@ -2043,10 +2096,10 @@ void cheb_sweep(hdg_system* s, const VT* val0, const float* b0, const float* in,
   }
   if (H->row_sweep)
     k_amg_row_cheb<NT, VT><<<nblk((int64_t)nf * NT), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->dinv0.p, H->lam0.p,
-                                                              H->face_prob.p, b0, H->bt0.p, in, out, H->d0.p, step,
+                                                              fprob, b0, H->bt0.p, in, out, H->d0.p, step,
                                                               amg_cheb_ratio(s), cst);
   else
-    k_amg_face_cheb<NT, VT><<<nblk(nf), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->dinv0.p, H->lam0.p, H->face_prob.p, b0,
+    k_amg_face_cheb<NT, VT><<<nblk(nf), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->dinv0.p, H->lam0.p, fprob, b0,
                                                   H->bt0.p, in, out, H->d0.p, step, amg_cheb_ratio(s), cst);
   if (ep) {
     ep->stop(st);
@@ -2058,6 +2111,7 @@ template <int NT, typename VT>
 void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const int32_t* cst, cudaStream_t st) {
   AmgHierarchy* H = s->amg;
   const int nf = H->nf;
+  const int32_t* fprob = s->nprob > 1 ? H->face_prob.p : nullptr;
   const int64_t n0 = (int64_t)nf * NT;
   const int nl = (int)H->lev.size();
   // level 0 pre-smoothing: Chebyshev of degree k from x = 0; the steps alternate between x0
@@ -2070,13 +2124,14 @@ void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const i
   }
   if (H->row_sweep)
     k_amg_face_residual<NT, VT><<<nblk(n0), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->bt0.p, z0, H->r0.p,
-                                                          H->face_prob.p, cst);
+                                                          fprob, cst);
   else
     k_amg_face_residual_f<NT, VT><<<nblk(nf), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->bt0.p, z0, H->r0.p,
-                                                            H->face_prob.p, cst);
+                                                            fprob, cst);
   AmgLevel& L1 = H->lev[0];
+  auto prob_of = [&](const AmgLevel& L) { return s->nprob > 1 ? L.prob.p : nullptr; };
   k_amg_restrict0<NT, 4><<<nblk((int64_t)L1.n * 4), 256, 0, st>>>(L1.n, H->rptr0.p, H->rent0.p, H->rval0.p, H->r0.p,
-                                                                 L1.dl1inv.p, L1.b.p, L1.x.p, L1.prob.p, cst);
+                                                                 L1.dl1inv.p, L1.b.p, L1.x.p, prob_of(L1), cst);
   // coarse levels down: x holds the first l1-Jacobi sweep (done by the restriction); the other
   // nu - 1 sweeps alternate between x and t; the iterate then stays where it is until the way up
   const int nu = amg_coarse_sweeps(s);
@@ -2092,7 +2147,7 @@ void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const i
     for (int sw = 1; sw < nu; ++sw) {
       EventPair* ep = (s->prof_cheb0 && l == 0) ? new EventPair() : nullptr;  // sampled chunk: time level 1
       if (ep) ep->start(st);
-      AMG_LAUNCH_G(k_amg_l1_sweep, L.n, st, L.n, L.ptr.p, L.col.p, L.val.p, L.dl1inv.p, L.b.p, cur, oth, L.prob.p,
+      AMG_LAUNCH_G(k_amg_l1_sweep, L.n, st, L.n, L.ptr.p, L.col.p, L.val.p, L.dl1inv.p, L.b.p, cur, oth, prob_of(L),
                    cst);
       if (ep) {
         ep->stop(st);
@@ -2101,10 +2156,10 @@ void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const i
       std::swap(cur, oth);
     }
     iter[l] = cur;
-    AMG_LAUNCH_G(k_amg_residual, L.n, st, L.n, L.ptr.p, L.col.p, L.val.p, L.b.p, cur, L.r.p, L.prob.p, cst);
+    AMG_LAUNCH_G(k_amg_residual, L.n, st, L.n, L.ptr.p, L.col.p, L.val.p, L.b.p, cur, L.r.p, prob_of(L), cst);
     const bool coarsest = (l + 2 == nl);
     AMG_LAUNCH_G(k_amg_restrict, C.n, st, C.n, L.rptr.p, L.rent.p, L.rrow.p, L.pval.p, L.r.p,
-                 coarsest ? nullptr : C.dl1inv.p, C.b.p, C.x.p, C.prob.p, cst);
+                 coarsest ? nullptr : C.dl1inv.p, C.b.p, C.x.p, prob_of(C), cst);
   }
   int up_from = nl - 2;
   if (T < nl) {
@@ -2122,11 +2177,11 @@ void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const i
     AmgLevel& L = H->lev[l];
     float* a = iter[l];
     float* b = L.r.p;
-    AMG_LAUNCH_G(k_amg_prolong, L.n, st, L.n, L.pptr.p, L.pcol.p, L.pval.p, fin[l + 1], a, L.prob.p, cst);
+    AMG_LAUNCH_G(k_amg_prolong, L.n, st, L.n, L.pptr.p, L.pcol.p, L.pval.p, fin[l + 1], a, prob_of(L), cst);
     for (int sw = 0; sw < nu; ++sw) {
       EventPair* ep = (s->prof_cheb0 && l == 0) ? new EventPair() : nullptr;
       if (ep) ep->start(st);
-      AMG_LAUNCH_G(k_amg_l1_sweep, L.n, st, L.n, L.ptr.p, L.col.p, L.val.p, L.dl1inv.p, L.b.p, a, b, L.prob.p, cst);
+      AMG_LAUNCH_G(k_amg_l1_sweep, L.n, st, L.n, L.ptr.p, L.col.p, L.val.p, L.dl1inv.p, L.b.p, a, b, prob_of(L), cst);
       if (ep) {
         ep->stop(st);
         s->ev_l1.push_back(ep);
@@ -2138,9 +2193,9 @@ void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const i
   // level 0 up: prolongate, then the same Chebyshev polynomial from the corrected iterate (z0,
   // x0, z0, ...); for odd k the result lands in x0 and is copied to z0
   if (H->row_sweep)
-    k_amg_prolong0<NT><<<nblk(n0), 256, 0, st>>>(nf, H->pcol0.p, H->pval0.p, fin[0], z0, H->face_prob.p, cst);
+    k_amg_prolong0<NT><<<nblk(n0), 256, 0, st>>>(nf, H->pcol0.p, H->pval0.p, fin[0], z0, fprob, cst);
   else
-    k_amg_prolong0_f<NT><<<nblk(nf), 256, 0, st>>>(nf, H->pcol0.p, H->pval0.p, fin[0], z0, H->face_prob.p, cst);
+    k_amg_prolong0_f<NT><<<nblk(nf), 256, 0, st>>>(nf, H->pcol0.p, H->pval0.p, fin[0], z0, fprob, cst);
   for (int t = 0; t < k; ++t) {
     const float* in = (t % 2 == 0) ? z0 : H->x0.p;
     float* out = (t % 2 == 0) ? H->x0.p : z0;

@@ -380,17 +380,32 @@ template <int NT> __global__ void __launch_bounds__(CG_BLOCK, 4) k_cg_b_mg(CgArg
 // z = z32 (FP64), r.z and beta.  mode 0: a regular iteration of the running problems (beta =
 // rz / rz_old); mode 1: a (re)start of the running problems (init) or of the problems whose
 // refine flag is set (restart), beta = 0.
-template <int NT> __global__ void __launch_bounds__(CG_BLOCK) k_cg_c(CgArgs<double> a, const float* z32, int mode,
+template <int NT> __global__ void __launch_bounds__(CG_BLOCK, 4) k_cg_c(CgArgs<double> a, const float* z32, int mode,
                                                                       int restart) {
   const int P = a.g.seg_prob[blockIdx.x];
   const int status = a.st[ST * P];
   const int flag = a.st[ST * P + 3];
   if (restart ? (flag == 0) : (status != 0)) return;
   double rz = 0.0;
-  for (int row = a.g.seg_row0[blockIdx.x] + threadIdx.x; row < a.g.seg_row1[blockIdx.x]; row += CG_BLOCK) {
-    const double zv = (double)z32[row];
-    a.z[row] = zv;
-    rz = fma(a.r[row], zv, rz);
+  const int r0 = a.g.seg_row0[blockIdx.x], r1 = a.g.seg_row1[blockIdx.x];
+  constexpr int ROWS = 4;
+  for (int base = r0 + threadIdx.x; base < r1; base += ROWS * CG_BLOCK) {
+    float zv[ROWS];
+    double rv[ROWS];
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+      const int row = min(base + u * CG_BLOCK, r1 - 1);
+      zv[u] = z32[row];
+      rv[u] = a.r[row];
+    }
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+      const int row = base + u * CG_BLOCK;
+      if (row < r1) {
+        a.z[row] = (double)zv[u];
+        rz = fma(rv[u], (double)zv[u], rz);
+      }
+    }
   }
   double s0;
   if (seg_finish1<CG_BLOCK>(a.g, P, 2, rz, &s0) && threadIdx.x == 0) {
