@@ -857,23 +857,31 @@ __global__ void k_amg_ap0(int nf, int wap, const int32_t* __restrict__ bcol5, co
   const int f = (int)(r / NT);
   float acc[32];
   for (int q = 0; q < wap && q < 32; ++q) acc[q] = 0.f;
-  int seen[5];
-  int ns = 0;
+  int g[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) g[k] = bcol5[k * nf + f];
+#pragma unroll
   for (int k = 0; k < 5; ++k) {
-    const int g = bcol5[k * nf + f];
     bool dup = false;
-    for (int t = 0; t < ns; ++t) dup |= (seen[t] == g);
+    for (int t = 0; t < k; ++t) dup |= (g[t] == g[k]);
     if (dup) continue;
-    seen[ns++] = g;
+    // the products of the block with the columns of P0, each added to its place once
+    float v[PW];
+    int q[PW];
+#pragma unroll
+    for (int c = 0; c < PW; ++c) {
+      q[c] = pcol0[g[k] * PW + c] < 0 ? -1 : apmap0[((int64_t)f * 5 + k) * PW + c];
+      v[c] = 0.f;
+    }
+#pragma unroll
     for (int j = 0; j < NT; ++j) {
       const float a = val[(k * NT + j) * nd + r];
-      if (a == 0.f) continue;
-      for (int c = 0; c < PW; ++c) {
-        if (pcol0[g * PW + c] < 0) break;
-        const int q = apmap0[((int64_t)f * 5 + k) * PW + c];
-        if (q >= 0 && q < wap) acc[q] += a * pval0[((int64_t)g * NT + j) * PW + c];
-      }
+#pragma unroll
+      for (int c = 0; c < PW; ++c) v[c] += a * pval0[((int64_t)g[k] * NT + j) * PW + c];
     }
+#pragma unroll
+    for (int c = 0; c < PW; ++c)
+      if (q[c] >= 0 && q[c] < wap) acc[q[c]] += v[c];
   }
   for (int q = 0; q < wap; ++q) apval0[r * wap + q] = acc[q];
 }
@@ -895,10 +903,13 @@ __device__ __forceinline__ void add_at(const int32_t* __restrict__ col, float* _
   if (e < b && col[e] == key) val[e] += v;
 }
 
-// A1 = P0' (A0 P0), one warp per coarse row.  For each of the row's P0' entries (face f, mode c)
-// and each of the face's rows i in turn, the lanes take the entries of the A0 P0 row: their
-// columns are distinct, so no two lanes add to the same coarse entry at once, and every entry
-// receives its terms in the order (t, i) whatever the launch.
+// The triple products, one warp per row of the result.  The terms of an entry are added in the order of the fine rows
+// whatever the launch: the fine rows take turns, the lanes take a turn's entries, whose columns are distinct.  What bounds
+// them is each turn's chain of loads (the fine row, its ends, its entries, the search in the result's columns, the sum so
+// far), so the loads of four turns are issued together.  Before / now: A1 of 98645 faces of p = 4 225 / 63 us, of 787456 of
+// p = 3 1010 / 307; the whole numeric set-up 1.25 / 0.76 and 2.9 / 1.95 ms.
+
+// A1 = P0' (A0 P0): a turn is an entry of the row of P0' (face f, mode c), the face's rows summed in the turn.
 template <int NT>
 __global__ void k_amg_rap0(int na, int wap, const int32_t* __restrict__ rptr0, const int32_t* __restrict__ rent0,
                            const float* __restrict__ pval0, const int32_t* __restrict__ apcol0,
@@ -907,22 +918,32 @@ __global__ void k_amg_rap0(int na, int wap, const int32_t* __restrict__ rptr0, c
   const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int J = (int)(gt >> 5), lane = threadIdx.x & 31;
   if (J >= na) return;  // whole warps
-  const int a0 = ptr1[J], a1 = ptr1[J + 1];
+  const int a0 = ptr1[J], a1 = ptr1[J + 1], t1 = rptr0[J + 1];
   for (int e = a0 + lane; e < a1; e += 32) val1[e] = 0.f;
   __syncwarp();
-  for (int t = rptr0[J]; t < rptr0[J + 1]; ++t) {
-    const int f = rent0[t] / PW, c = rent0[t] - f * PW;
-    for (int i = 0; i < NT; ++i) {
-      const float p = pval0[((int64_t)f * NT + i) * PW + c];
-      if (p == 0.f) continue;
-      const float* apr = apval0 + ((int64_t)f * NT + i) * wap;
-      for (int q = lane; q < wap; q += 32) {
-        const int K = apcol0[(int64_t)f * wap + q];
-        if (K >= 0) add_at(col1, val1, a0, a1, K, p * apr[q]);
+  constexpr int U = 4;
+  for (int t0 = rptr0[J]; t0 < t1; t0 += U)
+    for (int q = lane; q - lane < wap; q += 32) {
+      int K[U];
+      float v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        K[u] = -1;
+        v[u] = 0.f;
+        if (t0 + u < t1 && q < wap) {
+          const int e = rent0[t0 + u], f = e / PW, c = e - f * PW;
+          K[u] = apcol0[(int64_t)f * wap + q];
+#pragma unroll
+          for (int i = 0; i < NT; ++i)
+            v[u] += pval0[((int64_t)f * NT + i) * PW + c] * apval0[((int64_t)f * NT + i) * wap + q];
+        }
       }
-      __syncwarp();
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (K[u] >= 0) add_at(col1, val1, a0, a1, K[u], v[u]);
+        __syncwarp();
+      }
     }
-  }
 }
 
 // 1 / l1 row sums of a CSR level
@@ -945,16 +966,62 @@ __global__ void k_amg_p(int n, const int32_t* __restrict__ ptr, const int32_t* _
   const int p0 = pptr[i], p1 = pptr[i + 1];
   for (int e = p0; e < p1; ++e) pval[e] = 0.f;
   const float w = (4.f / 3.f) * dl1inv[i];
-  for (int e = ptr[i]; e < ptr[i + 1]; ++e) {
-    const int k = col[e];
-    add_at(pcol, pval, p0, p1, agg[k], -w * val[e] * tent[k]);
+  constexpr int U = 4;
+  const int e1 = ptr[i + 1];
+  for (int e = ptr[i]; e < e1; e += U) {
+    int J[U];
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = col[min(e + u, e1 - 1)];
+      J[u] = agg[k];
+      v[u] = -w * val[min(e + u, e1 - 1)] * tent[k];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (e + u < e1) add_at(pcol, pval, p0, p1, J[u], v[u]);
   }
   add_at(pcol, pval, p0, p1, agg[i], tent[i]);
 }
 
-// A P on a CSR level, one warp per row: for each entry (i, k) of A's row in turn, the lanes take
-// the entries of P's row k, whose columns are distinct (so no two lanes add to the same entry at
-// once, and each entry receives its terms in the order of A's row).
+// The turns of one row of a product: turn t adds coef(t) times the entries of row src(t) of (sptr, scol, sval) to the result's
+// row, whose sorted columns are col[a0 .. a1).
+template <typename SRC>
+__device__ __forceinline__ void add_rows(int t0, int t1, SRC src, const int32_t* __restrict__ sptr,
+                                         const int32_t* __restrict__ scol, const float* __restrict__ sval, int a0, int a1,
+                                         const int32_t* __restrict__ col, float* __restrict__ val) {
+  const int lane = threadIdx.x & 31;
+  constexpr int U = 4;
+  for (; t0 < t1; t0 += U) {
+    int b0[U], b1[U], K[U];
+    float p[U], v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      b0[u] = b1[u] = 0;
+      K[u] = -1;
+      p[u] = v[u] = 0.f;
+      if (t0 + u < t1) {
+        const int i = src(t0 + u, p[u]);
+        b0[u] = sptr[i];
+        b1[u] = sptr[i + 1];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (b0[u] + lane < b1[u]) {
+        K[u] = scol[b0[u] + lane];
+        v[u] = sval[b0[u] + lane];
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (K[u] >= 0) add_at(col, val, a0, a1, K[u], p[u] * v[u]);
+      for (int q = b0[u] + lane + 32; q < b1[u]; q += 32) add_at(col, val, a0, a1, scol[q], p[u] * sval[q]);
+      __syncwarp();
+    }
+  }
+}
+
+// A P on a CSR level: a turn is an entry (i, k) of A's row, with P's row k.
 __global__ void k_amg_ap(int n, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
                          const float* __restrict__ val, const int32_t* __restrict__ pptr,
                          const int32_t* __restrict__ pcol, const float* __restrict__ pval,
@@ -966,16 +1033,10 @@ __global__ void k_amg_ap(int n, const int32_t* __restrict__ ptr, const int32_t* 
   const int a0 = apptr[i], a1 = apptr[i + 1];
   for (int e = a0 + lane; e < a1; e += 32) apval[e] = 0.f;
   __syncwarp();
-  for (int e = ptr[i]; e < ptr[i + 1]; ++e) {
-    const int k = col[e];
-    const float a = val[e];
-    for (int t = pptr[k] + lane; t < pptr[k + 1]; t += 32) add_at(apcol, apval, a0, a1, pcol[t], a * pval[t]);
-    __syncwarp();
-  }
+  add_rows(ptr[i], ptr[i + 1], [&](int e, float& p) { p = val[e]; return col[e]; }, pptr, pcol, pval, a0, a1, apcol, apval);
 }
 
-// A_{l+1} = P' (A P), one warp per coarse row: for each of the row's P' entries (fine row i) in
-// turn, the lanes take the entries of the A P row i (distinct columns), as in k_amg_rap0.
+// A_{l+1} = P' (A P): a turn is an entry of the row of P' (fine row i), with the row i of A P.
 __global__ void k_amg_rap(int nc, const int32_t* __restrict__ rptr, const int32_t* __restrict__ rent,
                           const int32_t* __restrict__ rrow, const float* __restrict__ pval,
                           const int32_t* __restrict__ apptr, const int32_t* __restrict__ apcol,
@@ -987,16 +1048,14 @@ __global__ void k_amg_rap(int nc, const int32_t* __restrict__ rptr, const int32_
   const int a0 = cptr[J], a1 = cptr[J + 1];
   for (int e = a0 + lane; e < a1; e += 32) cval[e] = 0.f;
   __syncwarp();
-  for (int t = rptr[J]; t < rptr[J + 1]; ++t) {
-    const float p = pval[rent[t]];
-    const int i = rrow[t];
-    for (int q = apptr[i] + lane; q < apptr[i + 1]; q += 32) add_at(ccol, cval, a0, a1, apcol[q], p * apval[q]);
-    __syncwarp();
-  }
+  add_rows(rptr[J], rptr[J + 1], [&](int t, float& p) { p = pval[rent[t]]; return rrow[t]; }, apptr, apcol, apval, a0, a1, ccol,
+           cval);
 }
 
 // Dense inverse of each problem's coarsest matrix (Gauss-Jordan with partial pivoting in shared
-// memory, one CTA per problem).  Sizes are at most AMG_CINV_MAX (the symbolic setup checks).
+// memory, one CTA per problem).  Sizes are at most AMG_CINV_MAX (the symbolic setup checks).  A column is three barriers: a
+// warp finds the pivot, the rows are exchanged and scaled, a warp per row subtracts.  Before (one thread looked for the
+// pivot, 256 threads divided for their places) / now: 68 rows 324 / 97 us.
 __global__ void k_amg_coarse_inv(const int32_t* __restrict__ crow0, const int32_t* __restrict__ coff,
                                  const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
                                  const float* __restrict__ val, float* __restrict__ cinv) {
@@ -1008,6 +1067,8 @@ __global__ void k_amg_coarse_inv(const int32_t* __restrict__ crow0, const int32_
   float* a = sm;          // m x 2m augmented matrix
   float* mult = sm + m * w;  // m multipliers of the current column
   __shared__ int piv;
+  __shared__ float pinv;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   for (int t = threadIdx.x; t < m * w; t += blockDim.x) a[t] = 0.f;
   __syncthreads();
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
@@ -1019,30 +1080,48 @@ __global__ void k_amg_coarse_inv(const int32_t* __restrict__ crow0, const int32_
   }
   __syncthreads();
   for (int c = 0; c < m; ++c) {
-    if (threadIdx.x == 0) {
+    if (warp == 0) {  // the first of the largest entries from the diagonal on, and the multipliers
+      float best = -1.f;
       int p = c;
-      for (int i = c + 1; i < m; ++i)
-        if (fabsf(a[i * w + c]) > fabsf(a[p * w + c])) p = i;
-      piv = p;
+      for (int i = lane; i < m; i += 32) {
+        const float v = a[i * w + c];
+        mult[i] = v;
+        if (i >= c && fabsf(v) > best) {
+          best = fabsf(v);
+          p = i;
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float b = __shfl_xor_sync(0xffffffffu, best, o);
+        const int q = __shfl_xor_sync(0xffffffffu, p, o);
+        if (b > best || (b == best && q < p)) {
+          best = b;
+          p = q;
+        }
+      }
+      __syncwarp();
+      if (lane == 0) {
+        const float d = mult[p];
+        pinv = d != 0.f ? 1.f / d : 0.f;
+        piv = p;
+        mult[p] = mult[c];  // the rows change places
+        mult[c] = 0.f;
+      }
     }
     __syncthreads();
     const int pr = piv;
-    if (pr != c)
-      for (int j = threadIdx.x; j < w; j += blockDim.x) {
-        const float t = a[c * w + j];
-        a[c * w + j] = a[pr * w + j];
-        a[pr * w + j] = t;
-      }
+    for (int j = threadIdx.x; j < w; j += blockDim.x) {
+      const float t = a[pr * w + j];
+      if (pr != c) a[pr * w + j] = a[c * w + j];
+      a[c * w + j] = t * pinv;
+    }
     __syncthreads();
-    const float d = a[c * w + c];
-    const float inv = d != 0.f ? 1.f / d : 0.f;
-    __syncthreads();
-    for (int j = threadIdx.x; j < w; j += blockDim.x) a[c * w + j] *= inv;
-    for (int i = threadIdx.x; i < m; i += blockDim.x) mult[i] = (i == c) ? 0.f : a[i * w + c];
-    __syncthreads();
-    for (int t = threadIdx.x; t < m * w; t += blockDim.x) {
-      const int i = t / w, j = t - i * w;
-      if (i != c) a[t] -= mult[i] * a[c * w + j];
+    // columns before c are done (zero in row c)
+    for (int i = warp; i < m; i += warps) {
+      if (i == c) continue;
+      const float f = mult[i];
+      for (int j = c + lane; j < w; j += 32) a[i * w + j] -= f * a[c * w + j];
     }
     __syncthreads();
   }
@@ -2049,7 +2128,7 @@ template <int NT> void numeric_nt(hdg_system* s, const float* val0, cudaStream_t
     attr = true;
   }
   if (H->cmax > 0)
-    k_amg_coarse_inv<<<s->nprob, 256, smem, st>>>(H->crow0.p, H->coff.p, C.ptr.p, C.col.p, C.val.p, H->cinv.p);
+    k_amg_coarse_inv<<<s->nprob, 1024, smem, st>>>(H->crow0.p, H->coff.p, C.ptr.p, C.col.p, C.val.p, H->cinv.p);
   s->ctx->launches++;
   HDG_CUDA(cudaGetLastError());
 }
