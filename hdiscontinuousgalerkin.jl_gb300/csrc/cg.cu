@@ -128,7 +128,39 @@ template <int NT, typename T> __global__ void __launch_bounds__(CG_BLOCK) k_cg_i
   }
 }
 
-// FP64 product kernel with the q recurrence (p, q in place)
+// The rows base, base + CG_BLOCK, ... (ROWS of them, in flight together) of k_cg_a
+template <int NT, typename T, int ROWS>
+__device__ __forceinline__ void cg_a_rows(const CgArgs<T>& a, int base, int r1, double beta, double& pq) {
+  double w[ROWS];
+#pragma unroll
+  for (int u = 0; u < ROWS; ++u) {
+    const int row = min(base + u * CG_BLOCK, r1 - 1);
+    w[u] = row_dot<NT>(a.bcol5, a.nf, a.val, row, a.z);
+  }
+  T qo[ROWS], po[ROWS], zo[ROWS];
+#pragma unroll
+  for (int u = 0; u < ROWS; ++u) {
+    const int row = min(base + u * CG_BLOCK, r1 - 1);
+    qo[u] = a.q[row];
+    po[u] = a.p[row];
+    zo[u] = a.z[row];
+  }
+#pragma unroll
+  for (int u = 0; u < ROWS; ++u) {
+    const int row = base + u * CG_BLOCK;
+    if (row < r1) {
+      const T qn = (T)(w[u] + beta * (double)qo[u]);
+      const T pn = zo[u] + (T)beta * po[u];
+      a.q[row] = qn;
+      a.p[row] = pn;
+      pq += (double)pn * (double)qn;
+    }
+  }
+}
+
+// FP64 product kernel with the q recurrence (p, q in place).  The FP64 pipe bounds it, and a warp with no row left in
+// the last of its four takes it as long as any other: so a warp does only as many as it has (segments of 811 rows, 493 k
+// rows of p = 4: an iteration 180.5 us with four always, 177.3 now).
 template <int NT, typename T> __global__ void __launch_bounds__(CG_BLOCK, cg_min_blocks<T>()) k_cg_a(CgArgs<T> a) {
   const int P = a.g.seg_prob[blockIdx.x];
   // status and beta are loaded together (one round trip); beta is formed once by the reducing
@@ -136,37 +168,15 @@ template <int NT, typename T> __global__ void __launch_bounds__(CG_BLOCK, cg_min
   const int status = a.st[ST * P];
   const double beta = a.sc[SC * P + 7];
   if (status != 0) return;
-  const T bt = (T)beta;
   double pq = 0.0;
   const int r0 = a.g.seg_row0[blockIdx.x], r1 = a.g.seg_row1[blockIdx.x];
-  // four rows per thread in flight together (independent gathers and accumulation chains)
-  constexpr int ROWS = 4;
-  for (int base = r0 + threadIdx.x; base < r1; base += ROWS * CG_BLOCK) {
-    double w[ROWS];
-#pragma unroll
-    for (int u = 0; u < ROWS; ++u) {
-      const int row = min(base + u * CG_BLOCK, r1 - 1);
-      w[u] = row_dot<NT>(a.bcol5, a.nf, a.val, row, a.z);
-    }
-    T qo[ROWS], po[ROWS], zo[ROWS];
-#pragma unroll
-    for (int u = 0; u < ROWS; ++u) {
-      const int row = min(base + u * CG_BLOCK, r1 - 1);
-      qo[u] = a.q[row];
-      po[u] = a.p[row];
-      zo[u] = a.z[row];
-    }
-#pragma unroll
-    for (int u = 0; u < ROWS; ++u) {
-      const int row = base + u * CG_BLOCK;
-      if (row < r1) {
-        const T qn = (T)(w[u] + beta * (double)qo[u]);
-        const T pn = zo[u] + bt * po[u];
-        a.q[row] = qn;
-        a.p[row] = pn;
-        pq += (double)pn * (double)qn;
-      }
-    }
+  const int lane = threadIdx.x & 31;
+  for (int base = r0 + threadIdx.x; base - lane < r1; base += 4 * CG_BLOCK) {
+    const int left = r1 - (base - lane);  // of the warp
+    if (left > 3 * CG_BLOCK) cg_a_rows<NT, T, 4>(a, base, r1, beta, pq);
+    else if (left > 2 * CG_BLOCK) cg_a_rows<NT, T, 3>(a, base, r1, beta, pq);
+    else if (left > CG_BLOCK) cg_a_rows<NT, T, 2>(a, base, r1, beta, pq);
+    else cg_a_rows<NT, T, 1>(a, base, r1, beta, pq);
   }
   double s0;
   if (seg_finish1<CG_BLOCK>(a.g, P, 0, pq, &s0) && threadIdx.x == 0) {
