@@ -56,6 +56,7 @@ constexpr int AMG_MAX_COARSE = 96;  // per problem, dense inverse on the coarses
 constexpr int AMG_MAX_LEVELS = 12;
 constexpr int AMG_CINV_MAX = 150;   // largest dense coarsest block: (2 m^2 + m) floats of shared memory
 constexpr int PW = 5;               // level-0 prolongator row width (a face and its 4 neighbours)
+constexpr size_t AMG_STREAM_BYTES = size_t(64) << 20;  // half the L2
 constexpr int AMG_TAIL_THREADS = 512;      // of a k_amg_tail CTA
 constexpr int AMG_TAIL_SMEM = 216 * 1024;  // dynamic shared memory that the k_amg_tail CTAs of an SM may take
 
@@ -1191,7 +1192,8 @@ template <int NT> __device__ __forceinline__ void store_face(float* __restrict__
   }
 }
 // t_i -= sum_kj value (i, k, j) x_kj, each row's terms in the order (k, j); x holds the five slots' neighbour values
-template <int NT>
+// STREAM: the values are loaded as data to be replaced first.
+template <int NT, bool STREAM>
 __device__ __forceinline__ void face_subtract(const float* __restrict__ val, int64_t nf, int f, const float (&x)[5 * NT],
                                               float (&t)[NT]) {
 #pragma unroll
@@ -1199,14 +1201,14 @@ __device__ __forceinline__ void face_subtract(const float* __restrict__ val, int
 #pragma unroll
     for (int i = 0; i < NT; ++i) t[i] -= val[kj * nf * NT + (int64_t)f * NT + i] * x[kj];
 }
-template <int NT>
+template <int NT, bool STREAM>
 __device__ __forceinline__ void face_subtract(const __half* __restrict__ val, int64_t nf, int f, const float (&x)[5 * NT],
                                               float (&t)[NT]) {
   using C = Chunks<NT>;
   uint4 c[C::N];
   const uint4* from = reinterpret_cast<const uint4*>(val) + f;
 #pragma unroll
-  for (int n = 0; n < C::N; ++n) c[n] = __ldg(from + n * nf);
+  for (int n = 0; n < C::N; ++n) c[n] = STREAM ? __ldcs(from + n * nf) : __ldg(from + n * nf);
 #pragma unroll
   for (int e = 0; e < C::E; ++e) {
     const unsigned w = (e & 7) < 2 ? c[e >> 3].x : ((e & 7) < 4 ? c[e >> 3].y : ((e & 7) < 6 ? c[e >> 3].z : c[e >> 3].w));
@@ -1278,7 +1280,7 @@ __device__ __forceinline__ int prob_at(const int32_t* __restrict__ prob, int i) 
 // D^-1 A0 on [lambda / ratio, lambda], D the face-block diagonal and lambda the problem's
 // Gershgorin bound.  xin == NULL stands for x = 0 (no product); d holds the previous step's
 // correction and is updated in place (each face reads and writes only its own rows of d).
-template <int NT, typename VT>
+template <int NT, typename VT, bool STREAM>
 __global__ void k_amg_face_cheb(int nf, const int32_t* __restrict__ bcol5, const VT* __restrict__ val,
                                 const float* __restrict__ dinv, const float* __restrict__ lam,
                                 const int32_t* __restrict__ face_prob, const float* __restrict__ b,
@@ -1307,7 +1309,7 @@ __global__ void k_amg_face_cheb(int nf, const int32_t* __restrict__ bcol5, const
     float xv[5 * NT];
 #pragma unroll
     for (int k = 0; k < 5; ++k) load_face<NT>(xin, bcol5[k * nf + f], xv + k * NT);
-    face_subtract<NT>(val, nf, f, xv, t);
+    face_subtract<NT, STREAM>(val, nf, f, xv, t);
   }
   const float hi = fmaxf(lam[prob_at(face_prob, f)], 1e-30f), lo = hi / ratio;
   const float theta = 0.5f * (hi + lo), delta = 0.5f * (hi - lo), sigma = theta / delta;
@@ -1399,7 +1401,7 @@ __global__ void k_amg_face_residual(int nf, const int32_t* __restrict__ bcol5, c
 
 // The same residual with a thread per face (its nt rows): the face's block columns and neighbour
 // values are read once instead of nt times; each row's operations are those of the row kernel.
-template <int NT, typename VT>
+template <int NT, typename VT, bool STREAM>
 __global__ void k_amg_face_residual_f(int nf, const int32_t* __restrict__ bcol5, const VT* __restrict__ val,
                                       const float* __restrict__ b, const float* __restrict__ x,
                                       float* __restrict__ r, const int32_t* __restrict__ face_prob,
@@ -1411,7 +1413,7 @@ __global__ void k_amg_face_residual_f(int nf, const int32_t* __restrict__ bcol5,
   float xv[5 * NT];
 #pragma unroll
   for (int k = 0; k < 5; ++k) load_face<NT>(x, bcol5[k * nf + f], xv + k * NT);
-  face_subtract<NT>(val, nf, f, xv, s);
+  face_subtract<NT, STREAM>(val, nf, f, xv, s);
   store_face<NT>(r, f, s);
 }
 
@@ -2159,6 +2161,11 @@ void launch_tail(hdg_system* s, const int32_t* cst, cudaStream_t st) {
   HDG_CUDA(cudaLaunchKernelEx(&cf, k_amg_tail, tail_args(s, cst)));
 }
 
+// Whether the level-0 values are loaded as data to be replaced first: above half the L2 they do not stay there from sweep
+// to sweep anyway, and the vectors do then.  An iteration kept / streamed, us: p = 3 30 MB 243 / 257, 47 MB 297 / 306, 59 MB
+// 364 / 369, 73 MB 445 / 436, 89 MB 486 / 473, 120 MB 591 / 573; p = 4 61 MB 334 / 337, 75 MB 369 / 367.
+bool stream0(const AmgHierarchy* H) { return 2 * H->val0h.n > AMG_STREAM_BYTES; }
+
 // One level-0 Chebyshev step, a thread per row or a thread per face (H->row_sweep, tuned; both
 // give the same bits).  Measured before the tuner: 49 k faces (p = 4): rows 15 -> 10 us per
 // sweep; 197 k faces (p = 2) and the batch's bins (0.4-0.7 M faces): faces faster.
@@ -2178,8 +2185,8 @@ void cheb_sweep(hdg_system* s, const VT* val0, const float* b0, const float* in,
                                                               fprob, b0, H->bt0.p, in, out, H->d0.p, step,
                                                               amg_cheb_ratio(s), cst);
   else
-    k_amg_face_cheb<NT, VT><<<nblk(nf), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->dinv0.p, H->lam0.p, fprob, b0,
-                                                  H->bt0.p, in, out, H->d0.p, step, amg_cheb_ratio(s), cst);
+    (stream0(H) ? k_amg_face_cheb<NT, VT, true> : k_amg_face_cheb<NT, VT, false>)<<<nblk(nf), 256, 0, st>>>(
+        nf, s->d_bcol5.p, val0, H->dinv0.p, H->lam0.p, fprob, b0, H->bt0.p, in, out, H->d0.p, step, amg_cheb_ratio(s), cst);
   if (ep) {
     ep->stop(st);
     s->ev_cheb0.push_back(ep);
@@ -2205,8 +2212,8 @@ void apply_nt(hdg_system* s, const VT* val0, const float* b0, float* z0, const i
     k_amg_face_residual<NT, VT><<<nblk(n0), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->bt0.p, z0, H->r0.p,
                                                           fprob, cst);
   else
-    k_amg_face_residual_f<NT, VT><<<nblk(nf), 256, 0, st>>>(nf, s->d_bcol5.p, val0, H->bt0.p, z0, H->r0.p,
-                                                            fprob, cst);
+    (stream0(H) ? k_amg_face_residual_f<NT, VT, true> : k_amg_face_residual_f<NT, VT, false>)<<<nblk(nf), 256, 0, st>>>(
+        nf, s->d_bcol5.p, val0, H->bt0.p, z0, H->r0.p, fprob, cst);
   AmgLevel& L1 = H->lev[0];
   auto prob_of = [&](const AmgLevel& L) { return s->nprob > 1 ? L.prob.p : nullptr; };
   k_amg_restrict0<NT, 4><<<nblk((int64_t)L1.n * 4), 256, 0, st>>>(L1.n, H->rptr0.p, H->rent0.p, H->rval0.p, H->r0.p,

@@ -75,7 +75,9 @@ void destroy_cg(CgState* c) { delete c; }
 
 namespace {
 
-// (A v)_row over the block-ELL layout: 5 block slots, values slot-major and row-contiguous.
+// (A v)_row over the block-ELL layout: 5 block slots, values slot-major and row-contiguous.  The values, read once an
+// iteration, are loaded as data to be replaced first: what the rest of the iteration reads again stays in L2 (multigrid
+// iterations of 493 k rows of p = 4 and 591 k of p = 2: 177 -> 169 and 129 -> 121.5 us).
 template <int NT, typename T, typename V>
 __device__ __forceinline__ double row_dot(const int32_t* __restrict__ bcol5, int nf, const T* __restrict__ val, int row,
                                           const V* __restrict__ v) {
@@ -88,7 +90,7 @@ __device__ __forceinline__ double row_dot(const int32_t* __restrict__ bcol5, int
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
 #pragma unroll
-    for (int j = 0; j < NT; ++j) acc += __ldg(val + (k * NT + j) * ndofs + row) * (T)__ldg(v + g[k] * NT + j);
+    for (int j = 0; j < NT; ++j) acc += __ldcs(val + (k * NT + j) * ndofs + row) * (T)__ldg(v + g[k] * NT + j);
   }
   return (double)acc;
 }
