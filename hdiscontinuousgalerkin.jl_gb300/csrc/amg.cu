@@ -1650,9 +1650,10 @@ __global__ void k_amg_coarse_solve(const int32_t* __restrict__ crow0, const int3
 // Each phase is a handful of loads per lane, so what bounds it is latency: a launch per phase is 1.5 us in a captured
 // graph.  Here the rows of a problem's levels are dealt out to the CTAs of a cluster, rpc consecutive ones to each, and
 // everything they need is in shared memory: the rows of A, P and P' (an image made once per set-up by k_amg_tail_image
-// and read at the start of each launch) and the whole of the vectors.  A phase ends with each CTA storing its rows'
-// values into the other CTAs' vectors, 16 bytes a lane, so that every gather is local: gathered from the other CTAs
-// four bytes at a time, a sweep over 4200 rows of 29 entries took 2 us.
+// and read at the start of each launch) and the whole of the vectors.  A row's new value is stored into every CTA's vector as
+// soon as it is formed, four rows to a store, so that every gather is local: gathered from the other CTAs four bytes at a
+// time, a sweep over 4200 rows of 29 entries took 2 us.  (Copied to the others after a barrier of the CTA, one V-cycle of 15
+// and of 16 problems took 115 and 99 us instead of 111 and 97.)
 //
 // Each row is computed exactly as the per-level kernels compute it (the same G lanes per row, taken from the level's
 // size, the same per-lane order and shuffle tree), so the cycle's result is bit-identical to theirs.
@@ -1773,15 +1774,20 @@ __device__ __forceinline__ void cluster_store(uint32_t addr, uint4 v) {
   asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                : "memory");
 }
+__device__ __forceinline__ void cluster_store(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
 __device__ __forceinline__ void tail_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // The rows 0 .. n - 1 of a CTA in groups of G lanes: the sum over a row's entries of value times the word at the entry's
-// offset in x, then out(row, sum) in the group's first lane; every lane of a warp runs the same number of rounds, so the
-// shuffles name all lanes.
+// offset in x, made the row's new value by out(row, sum) in each lane of the group, and stored to every CTA: dst, of this
+// lane, is the place of row 0 in CTA lane % 16 (0: none).  Four rows make a store of 16 bytes; every lane of a warp runs
+// the same number of rounds, so the shuffles name all lanes.
 template <int G, typename OUT>
-__device__ __forceinline__ void tail_rows_g(int n, const uint32_t* ptr, const uint2* ent, const uint32_t* x, OUT out) {
+__device__ __forceinline__ void tail_rows_g(int n, const uint32_t* ptr, const uint2* ent, const uint32_t* x, uint32_t dst,
+                                            OUT out) {
   const int lane = threadIdx.x & 31, gl = lane % G;
   for (int base = (threadIdx.x >> 5) * (32 / G); base < n; base += (blockDim.x >> 5) * (32 / G)) {
     const int i = base + lane / G;
@@ -1795,14 +1801,28 @@ __device__ __forceinline__ void tail_rows_g(int n, const uint32_t* ptr, const ui
       }
     }
     s = group_sum_f<G>(s);
-    if (i < n && gl == 0) out(i, s);
+    const float v = i < n ? out(i, s) : 0.f;
+    if (G == 32) {
+      __syncwarp();  // a row's old value may be read by every lane
+      if (dst && lane < 16) cluster_store(dst + 4u * base, v);
+    } else {  // lanes 0 .. 15 the first four rows of the round, lanes 16 .. 31 (G = 4) the next four
+      const int h = G == 4 ? lane & 16 : 0;
+      uint4 w;
+      w.x = __float_as_uint(__shfl_sync(0xffffffffu, v, h));
+      w.y = __float_as_uint(__shfl_sync(0xffffffffu, v, h + G));
+      w.z = __float_as_uint(__shfl_sync(0xffffffffu, v, h + 2 * G));
+      w.w = __float_as_uint(__shfl_sync(0xffffffffu, v, h + 3 * G));
+      const int row = base + (h ? 4 : 0);
+      if (dst && (G == 4 || lane < 16) && row < n) cluster_store(dst + 4u * row, w);
+    }
   }
 }
 template <typename OUT>
-__device__ __forceinline__ void tail_rows(int G, int n, const uint32_t* ptr, const uint2* ent, const uint32_t* x, OUT out) {
-  if (G == 4) tail_rows_g<4>(n, ptr, ent, x, out);
-  else if (G == 8) tail_rows_g<8>(n, ptr, ent, x, out);
-  else tail_rows_g<32>(n, ptr, ent, x, out);
+__device__ __forceinline__ void tail_rows(int G, int n, const uint32_t* ptr, const uint2* ent, const uint32_t* x, uint32_t dst,
+                                          OUT out) {
+  if (G == 4) tail_rows_g<4>(n, ptr, ent, x, dst, out);
+  else if (G == 8) tail_rows_g<8>(n, ptr, ent, x, dst, out);
+  else tail_rows_g<32>(n, ptr, ent, x, dst, out);
 }
 
 __global__ void __launch_bounds__(AMG_TAIL_THREADS) k_amg_tail(TailArgs a) {
@@ -1838,30 +1858,21 @@ __global__ void __launch_bounds__(AMG_TAIL_THREADS) k_amg_tail(TailArgs a) {
     av[k] = (i < z.nown && j < z.rows) ? A[i * z.rows + j] : 0.f;
   }
   tail_sync();  // every CTA of the cluster runs: its shared memory may be written
-  // The own rows of vector v to the other CTAs, the whole cluster past this phase: a warp, or several, to each CTA
-  auto publish = [&](const TailShare& s, int v) {
-    __syncthreads();
-    const int at = v + rank * s.rpc, n4 = (s.nown + 3) >> 2, warps = blockDim.x >> 5;
-    const int shares = max(1, warps / a.ctas);  // warps to a CTA, or the CTAs dealt out to the warps
-    for (int u = t >> 5; u < a.ctas * shares; u += warps) {
-      const int to = u % a.ctas;
-      if (to == rank) continue;
-      const uint32_t dst = cluster_addr(base + 4u * at, to);
-      for (int i = u / a.ctas * 32 + (t & 31); i < n4; i += 32 * shares)
-        cluster_store(dst + 16u * i, *reinterpret_cast<const uint4*>(sm + at + 4 * i));
-    }
-    tail_sync();
+  // where this lane stores the own rows of vector v: in CTA lane % 16 of the cluster
+  auto dest = [&](const TailShare& s, int v) {
+    const int to = t & 15;
+    return to < a.ctas ? cluster_addr(base + 4u * (v + rank * s.rpc), to) : 0u;
   };
-  // a level's product with the rows of A, P or P' (its row starts and entries) with vector v of the level of s
-  auto rows = [&](int g, int n, int ptr, int ent, const TailShare& s, int v, auto out) {
-    tail_rows(g, n, sm + ptr, reinterpret_cast<const uint2*>(sm + ent), sm + (v - s.x), out);
+  // A phase: the product of the rows of A, P or P' with vector v of the level of s, made the new values of the own rows of
+  // vector to of the level of d, in every CTA; the whole cluster past it
+  auto phase = [&](int g, int n, int ptr, int ent, const TailShare& s, int v, const TailShare& d, int to, auto out) {
+    tail_rows(g, n, sm + ptr, reinterpret_cast<const uint2*>(sm + ent), sm + (v - s.x), dest(d, to), out);
+    tail_sync();
   };
   auto sweep = [&](const TailShare& s, int in, int out) {
     const int own = rank * s.rpc;
-    rows(s.g, s.nown, s.ptr, s.ent, s, in, [&](int i, float v) {
-      smf[out + own + i] = smf[in + own + i] + (smf[s.b + i] - v) * smf[s.d + i];
-    });
-    publish(s, out);
+    phase(s.g, s.nown, s.ptr, s.ent, s, in, s, out,
+          [&](int i, float v) { return smf[in + own + i] + (smf[s.b + i] - v) * smf[s.d + i]; });
   };
   // down; the iterate starts in x, the residual is left in the other vector
   for (int l = a.T; l < last; ++l) {
@@ -1873,20 +1884,18 @@ __global__ void __launch_bounds__(AMG_TAIL_THREADS) k_amg_tail(TailArgs a) {
       cur = oth;
       oth = tmp;
     }
-    rows(s.g, s.nown, s.ptr, s.ent, s, cur, [&](int i, float v) { smf[oth + rank * s.rpc + i] = smf[s.b + i] - v; });
-    publish(s, oth);
+    phase(s.g, s.nown, s.ptr, s.ent, s, cur, s, oth, [&](int i, float v) { return smf[s.b + i] - v; });
     // the coarsest right-hand side is gathered too: it goes to y
-    rows(c.g, c.nown, s.rptr, s.rent, s, oth, [&](int J, float v) {
-      if (l + 1 < last) {
-        smf[c.b + J] = v;
-        smf[c.x + rank * c.rpc + J] = v * smf[c.d + J];
-      } else {
-        smf[c.y + rank * c.rpc + J] = v;
-      }
-    });
-    publish(c, l + 1 < last ? c.x : c.y);
+    if (l + 1 < last)
+      phase(c.g, c.nown, s.rptr, s.rent, s, oth, c, c.x, [&](int J, float v) {
+        smf[c.b + J] = v;  // the same from each lane of the group
+        return v * smf[c.d + J];
+      });
+    else
+      phase(c.g, c.nown, s.rptr, s.rent, s, oth, c, c.y, [&](int J, float v) { return v; });
   }
   // coarsest: x = A^-1 b, in coarse_row's order
+  const uint32_t zdst = dest(z, z.x);
   for (int i = t >> 5; i < z.nown; i += blockDim.x >> 5) {
     float v = 0.f;
 #pragma unroll
@@ -1895,16 +1904,16 @@ __global__ void __launch_bounds__(AMG_TAIL_THREADS) k_amg_tail(TailArgs a) {
       if (j < z.rows) v += (i == t >> 5 ? av[k] : A[i * z.rows + j]) * smf[z.y + j];
     }
     v = group_sum_f<32>(v);
-    if ((t & 31) == 0) smf[z.x + rank * z.rpc + i] = v;
+    if (zdst && (t & 31) < 16) cluster_store(zdst + 4u * i, v);
   }
-  publish(z, z.x);
+  tail_sync();
   // up; the first sweep reads the vector that the way down ended in
   int fine = z.x;  // the coarser level's result
   for (int l = last - 1; l >= a.T; --l) {
     const TailShare s = S[l], c = S[l + 1];
     int cur = (nu & 1) ? s.x : s.y, oth = (nu & 1) ? s.y : s.x;
-    rows(s.g, s.nown, s.pptr, s.pent, c, fine, [&](int i, float v) { smf[cur + rank * s.rpc + i] += v; });
-    publish(s, cur);
+    phase(s.g, s.nown, s.pptr, s.pent, c, fine, s, cur,
+          [&](int i, float v) { return smf[cur + rank * s.rpc + i] + v; });
     for (int sw = 0; sw < nu; ++sw) {
       sweep(s, cur, oth);  // the last one too ends with the barrier: no CTA leaves while another writes to it
       const int tmp = cur;
