@@ -188,40 +188,60 @@ void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w) {
 // reference edges of the triangle (src/shapes.jl:19-23): 1: (1,0)->(0,1), 2: (0,1)->(0,0), 3: (0,0)->(1,0)
 const double EDGE[3][4] = {{1, 0, 0, 1}, {0, 1, 0, 0}, {0, 0, 1, 0}};
 
-// Eigenvalues and eigenvectors (columns) of a small symmetric matrix, cyclic Jacobi rotations in long double.
-void symmetric_eigen(int n, const double* m, std::vector<long double>* lam, std::vector<long double>* vec) {
-  std::vector<long double> a(m, m + (size_t)n * n);
-  vec->assign((size_t)n * n, 0.0L);
-  for (int i = 0; i < n; ++i) (*vec)[(size_t)i * n + i] = 1.0L;
-  for (int sweep = 0; sweep < 60; ++sweep) {
-    long double off = 0.0L, all = 0.0L;
+// Cyclic Jacobi rotations of the symmetric a (n x n) until its off-diagonal entries are below tol of its norm or the
+// sweeps are done; the columns of vec turn along.
+template <typename R> void jacobi_sweeps(int n, R tol, int sweeps, std::vector<R>& a, std::vector<R>& vec) {
+  for (int sweep = 0; sweep < sweeps; ++sweep) {
+    R off = 0, all = 0;
     for (int i = 0; i < n; ++i)
       for (int j = 0; j < n; ++j) (i == j ? all : off) += a[(size_t)i * n + j] * a[(size_t)i * n + j];
-    if (off <= 1e-40L * all) break;
+    if (off <= tol * tol * all) break;
     for (int p = 0; p < n; ++p)
       for (int q = p + 1; q < n; ++q) {
-        const long double apq = a[(size_t)p * n + q];
-        if (apq == 0.0L) continue;
-        const long double th = (a[(size_t)q * n + q] - a[(size_t)p * n + p]) / (2.0L * apq);
-        const long double t = (th >= 0 ? 1.0L : -1.0L) / (std::fabs(th) + std::sqrt(th * th + 1.0L));
-        const long double c = 1.0L / std::sqrt(t * t + 1.0L), s = t * c;
+        const R apq = a[(size_t)p * n + q];
+        if (apq * apq <= R(1e-4) * tol * tol * all) continue;
+        const R th = (a[(size_t)q * n + q] - a[(size_t)p * n + p]) / (2 * apq);
+        const R t = (th >= 0 ? 1 : -1) / (std::fabs(th) + std::sqrt(th * th + 1));
+        const R c = 1 / std::sqrt(t * t + 1), s = t * c;
         for (int k = 0; k < n; ++k) {
-          const long double x = a[(size_t)k * n + p], y = a[(size_t)k * n + q];
+          const R x = a[(size_t)k * n + p], y = a[(size_t)k * n + q];
           a[(size_t)k * n + p] = c * x - s * y;
           a[(size_t)k * n + q] = s * x + c * y;
         }
         for (int k = 0; k < n; ++k) {
-          const long double x = a[(size_t)p * n + k], y = a[(size_t)q * n + k];
+          const R x = a[(size_t)p * n + k], y = a[(size_t)q * n + k];
           a[(size_t)p * n + k] = c * x - s * y;
           a[(size_t)q * n + k] = s * x + c * y;
         }
         for (int k = 0; k < n; ++k) {
-          const long double x = (*vec)[(size_t)k * n + p], y = (*vec)[(size_t)k * n + q];
-          (*vec)[(size_t)k * n + p] = c * x - s * y;
-          (*vec)[(size_t)k * n + q] = s * x + c * y;
+          const R x = vec[(size_t)k * n + p], y = vec[(size_t)k * n + q];
+          vec[(size_t)k * n + p] = c * x - s * y;
+          vec[(size_t)k * n + q] = s * x + c * y;
         }
       }
   }
+}
+
+// Eigenvalues and eigenvectors (columns) of a small symmetric matrix in long double: rotations in double first (long
+// double is software where it has 128 bits: all sweeps in it took 2 ms), their product made orthogonal to long double, and
+// what the matrix still has off its diagonal in that basis rotated away.
+void symmetric_eigen(int n, const double* m, std::vector<long double>* lam, std::vector<long double>* vec) {
+  std::vector<double> ad(m, m + (size_t)n * n), vd((size_t)n * n, 0.0);
+  for (int i = 0; i < n; ++i) vd[(size_t)i * n + i] = 1.0;
+  jacobi_sweeps<double>(n, 1e-15, 30, ad, vd);
+  auto mul = [n](const std::vector<long double>& x, bool xt, const std::vector<long double>& y) {
+    std::vector<long double> r((size_t)n * n, 0.0L);
+    for (int i = 0; i < n; ++i)
+      for (int j = 0; j < n; ++j)
+        for (int k = 0; k < n; ++k) r[(size_t)i * n + j] += x[xt ? (size_t)k * n + i : (size_t)i * n + k] * y[(size_t)k * n + j];
+    return r;
+  };
+  std::vector<long double> v(vd.begin(), vd.end()), g = mul(v, true, v);  // V (3 I - V'V) / 2
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j < n; ++j) g[(size_t)i * n + j] = 0.5L * ((i == j ? 3.0L : 0.0L) - g[(size_t)i * n + j]);
+  *vec = mul(v, false, g);
+  std::vector<long double> a = mul(*vec, true, mul(std::vector<long double>(m, m + (size_t)n * n), false, *vec));
+  jacobi_sweeps<long double>(n, 1e-18L, 30, a, *vec);
   lam->resize(n);
   for (int i = 0; i < n; ++i) (*lam)[i] = a[(size_t)i * n + i];
 }
