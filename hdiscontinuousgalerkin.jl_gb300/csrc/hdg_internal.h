@@ -216,7 +216,8 @@ struct RefTables {
   // packed device tables (see tables.cpp: ref_layout)
   std::vector<double> packed;
 };
-bool build_ref_tables(int p, int qd, RefTables* t);
+// condensation: with the products that the Schur element kernels read (a nodal system needs none of them).
+bool build_ref_tables(int p, int qd, RefTables* t, bool condensation = true);
 
 // Nodal (continuous Lagrange) basis of order k on the reference triangle, at the volume points of
 // QuadratureRule{2}(qd): nodes in the order of get_nodal_points (vertices, edge points, interior

@@ -282,7 +282,7 @@ RefLayout ref_layout(int nw, int nt, int nq) {
 
 // QuadratureRule{2}(DefaultQuad(), qd) dispatch of src/quadrature.jl:17-26: Strang for qd <= 6,
 // Grundmann–Möller of index (qd-1)/2 for odd qd > 6, otherwise not available.
-bool build_ref_tables(int p, int qd, RefTables* t) {
+bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
   if (p < 1 || p > HDG_MAX_P) return false;
   t->p = p;
   t->qd = qd;
@@ -392,7 +392,7 @@ bool build_ref_tables(int p, int qd, RefTables* t) {
   // with the pseudo-inverse M^+ and one unknown a per component, which the element kernel carries as two more rows of
   // S, [S Z; Z' 0] with Z = [D_l' z] (the rows z' (Be u - Ee u_hat) = 0 of the local system).  Other rank-deficient
   // rules keep the full LU.
-  {
+  if (condensation) {
     std::vector<long double> a((size_t)nw * 2 * nw, 0.0L);
     for (int i = 0; i < nw; ++i) {
       for (int j = 0; j < nw; ++j) a[(size_t)i * 2 * nw + j] = P[L.M + i * nw + j];
@@ -554,7 +554,7 @@ bool build_ref_tables(int p, int qd, RefTables* t) {
 bool build_lagrange_tables(int order, int qd, LagrangeTables* t) {
   if (order < 1 || order > HDG_MAX_P) return false;
   RefTables r;
-  if (!build_ref_tables(order, qd, &r)) return false;  // the rule and the Dubiner tables
+  if (!build_ref_tables(order, qd, &r, false)) return false;  // the rule and the Dubiner tables
   const int k = order, nl = (k + 1) * (k + 2) / 2, nq = r.nq;
   std::vector<double> px, py;
   const double V0[3][2] = {{0, 0}, {1, 0}, {0, 1}};
