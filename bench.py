@@ -169,7 +169,7 @@ def element_cost(p, schur):
     nw, nt = (p + 1) * (p + 2) // 2, p + 1
     n, m = 3 * nw, 3 * nt
     rc = nw + m + 1
-    rows = nw if schur else n
+    rows = nw + (2 if p == 2 else 0) if schur else n  # p = 2: and the null function's coefficients of q
     nbytes = 69 + 8 * (m * (m + 1) + rows * (m + 1))
     if schur:
         chol = sum((rc - k - 1) + sum(rc - i for i in range(k + 1, nw)) for k in range(nw))
@@ -257,11 +257,11 @@ def c4_rooflines(H, B, tims, pc, hbm, peak_kind):
     el = []
     tot_b = tot_f = tot_nom = tot_ms = 0.0
     for bn, t in zip(B.bins, tims):
-        schur = bn.p != 2
+        schur = True
         nb, fl, nom = element_cost(bn.p, schur)
         cells = bn.mesh.ncells
         ms = t["element_ms"]
-        el.append({"p": bn.p, "path": "cholesky-schur" if schur else "full LU", "cells": cells, "ms": ms,
+        el.append({"p": bn.p, "path": "cholesky-schur", "cells": cells, "ms": ms,
                    "elements_per_s": cells / (ms / 1e3) if ms else None,
                    "gbs": cells * nb / (ms / 1e3) / 1e9 if ms else None,
                    "fp64_tflops": cells * fl / (ms / 1e3) / 1e12 if ms else None})
@@ -270,7 +270,7 @@ def c4_rooflines(H, B, tims, pc, hbm, peak_kind):
         tot_nom += cells * nom
         tot_ms += ms
     ach = tot_b / (tot_ms / 1e3) / 1e9 if tot_ms else None
-    rl_el = {"kernel": "k_element_chol (p=1,3,4) + k_element_condense (p=2), all bins", "bound": "fp64 pipe",
+    rl_el = {"kernel": "k_element_schur, all bins", "bound": "fp64 pipe",
              "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm if ach else None,
              "fp64_tflops": tot_f / (tot_ms / 1e3) / 1e12 if tot_ms else None,
              "fp64_peak_tflops": FP64_TFLOPS_MEASURED,

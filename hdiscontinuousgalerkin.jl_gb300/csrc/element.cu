@@ -1,7 +1,8 @@
 // Element assembly + static condensation (the body of doassemble,
-// examples/poisson2D_HDG.jl:77-174), one warp per cell.
+// examples/poisson2D_HDG.jl:77-174): k_element_schur and, with kappa a field, k_element_field, several
+// cells to a warp; k_element_condense, a warp per cell, for cells whose reduced system is not positive.
 //
-// Per cell the warp
+// Per cell k_element_condense
 //   1. gathers the three vertices and forms J, det J, adj(J) = det J * J^-1, the weighted
 //      outward normals wn_f (|wn_f| = |e_f|) and the orientation bits (src/mesh.jl:51-54);
 //   2. writes the augmented local system [Me | EF | Bte] of size n x (n+m+1) into shared memory,
