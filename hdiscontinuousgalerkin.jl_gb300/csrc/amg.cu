@@ -302,6 +302,7 @@ struct AmgHierarchy {
   DevBuf<int8_t> apmap0;     // [nf][5 slots][PW]: position of pcol0[g_k][c] in apcol0[f]
   DevBuf<float> apval0;      // [nf*nt][wap]
   DevBuf<int32_t> rptr0, rent0;  // P0': per coarse row J the (face*PW + c) entries with pcol0 == J
+  int64_t nrent0 = 0;            // entries of P0' (rent0 holds one element where there is none: every face prescribed)
   DevBuf<float> dinv0;       // [nf][nt][nt]
   DevBuf<float> lam0;        // [nprob] Gershgorin bound of D^-1 A0
   DevBuf<int32_t> face_prob; // [nf]
@@ -546,6 +547,7 @@ void amg_setup_symbolic(hdg_system* s, const std::vector<char>& dirichlet_face) 
   H->apval0.alloc((size_t)nf * nt * wap);
   H->rptr0.upload(rptr0.data(), rptr0.size(), st);
   upload_min1(H->rent0, rent0, st);
+  H->nrent0 = (int64_t)rent0.size();
   H->dinv0.alloc((size_t)nf * nt * nt);
   H->lam0.alloc(std::max(s->nprob, 1));
   H->face_prob.upload(fprob.data(), fprob.size(), st);
@@ -2115,8 +2117,8 @@ template <int NT> void numeric_nt(hdg_system* s, const float* val0, cudaStream_t
   AmgLevel& L1 = H->lev[0];
   k_amg_rap0<NT><<<nblk((int64_t)L1.n * 32), 256, 0, st>>>(L1.n, H->wap, H->rptr0.p, H->rent0.p, H->pval0.p, H->apcol0.p,
                                              H->apval0.p, L1.ptr.p, L1.col.p, L1.val.p);
-  const int64_t nr = (int64_t)H->rent0.n * NT;
-  k_amg_dp0<NT><<<nblk(nr), 256, 0, st>>>(nr, nf, s->d_kdiag.p, val0, H->rent0.p, H->pval0.p, H->rval0.p);
+  const int64_t nr = H->nrent0 * NT;
+  if (nr > 0) k_amg_dp0<NT><<<nblk(nr), 256, 0, st>>>(nr, nf, s->d_kdiag.p, val0, H->rent0.p, H->pval0.p, H->rval0.p);
   if (amg_level0_fp32()) {
     k_amg_scale0<NT, float><<<nblk(nf), 256, 0, st>>>(nf, H->dinv0.p, val0, const_cast<float*>(val0));
   } else {
