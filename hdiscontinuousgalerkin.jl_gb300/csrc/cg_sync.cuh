@@ -117,6 +117,7 @@ __device__ __forceinline__ bool all_sum(ResShared& sh, unsigned* count, double* 
           }
         } while (seen < want);
       }
+      __syncwarp();  // orders the other lanes' loads of the partials after lane 0's acquire (a shuffle does not)
       ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
       // all partials are loaded before the first is added (one L2 latency)
       constexpr int PER = MAX_GRID / 32;
