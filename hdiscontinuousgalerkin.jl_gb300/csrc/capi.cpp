@@ -329,10 +329,41 @@ int hdg_space_destroy(hdg_space* s) {
 }
 
 // ---------------------------------------------------------------- fields in fixed point
-// hdg_device.cuh: eval_part.  Rewrites the parameters of one field at prm (its FieldSpec's, in place) for coordinates
-// X = x 2^s and returns the fixed-point kind, or leaves them (a Gaussian's width prepared as in fprep) and returns
-// the plain one where a value does not fit the form.
-static int prepare_fixed(const FieldSpec& f, int s, double* prm) {
+// hdg_device.cuh: eval_part.  A problem's coordinates are below 2^e in magnitude, its fixed-point numbers are X = x 2^s.
+// FP64 holds a coordinate to 2^-53 of its own magnitude, the fixed point every one to 2^-s; a field takes the fixed form
+// only where the latter costs it nothing against the former, and no other problem of the system has a say in it.
+
+static int coordinate_exponent(double xy_max) {  // smallest e with xy_max < 2^e
+  int e;
+  std::frexp(xy_max, &e);
+  return e;
+}
+
+// A bump that adds nothing anywhere below 2^e: of amplitude 0, or so far off that its exponential is 0 in FP64
+// (exp(-x) from x = 745.2 on, 38.7 widths).
+static bool bump_is_off(const double* b, int e) {
+  const double edge = std::ldexp(1.0, e), dx = std::max(std::fabs(b[0]) - edge, 0.0), dy = std::max(std::fabs(b[1]) - edge, 0.0);
+  return b[3] == 0.0 || std::hypot(dx, dy) > 38.7 * std::fabs(b[2]);
+}
+static bool bumps_finite(const std::vector<double>& p) {
+  return std::all_of(p.begin() + 1, p.begin() + 1 + 4 * (int)p[0], [](double v) { return std::isfinite(v); });
+}
+
+// The exponent of one problem's fixed point: above its coordinates and the centres of the bumps that matter to it.
+static int fixed_exponent(int e, const FieldSpec& f) {
+  if (f.kind != HDG_FIELD_BUMPS || !bumps_finite(f.prm)) return e;
+  int top = e;
+  for (int k = 0; k < (int)f.prm[0]; ++k) {
+    const double* b = &f.prm[1 + 4 * k];
+    if (!bump_is_off(b, e)) top = std::max(top, coordinate_exponent(std::max(std::fabs(b[0]), std::fabs(b[1]))));
+  }
+  return top;
+}
+
+// Rewrites the parameters of one field at prm (its FieldSpec's, in place) for coordinates X = x 2^s, |x| < 2^e, and
+// returns the fixed-point kind, or leaves them (a Gaussian's width prepared as in fprep) and returns the plain one where
+// a value does not fit the form or the form would lose digits to FP64.
+static int prepare_fixed(const FieldSpec& f, int s, int e, bool usable, double* prm) {
   auto word = [](uint64_t v) {
     double d;
     std::memcpy(&d, &v, 8);
@@ -346,47 +377,55 @@ static int prepare_fixed(const FieldSpec& f, int s, double* prm) {
   const std::vector<double>& p = f.prm;
   const int K = (f.kind == HDG_FIELD_BUMPS || f.kind == HDG_FIELD_FOURIER || f.kind == HDG_FIELD_EXP_FOURIER) ? (int)p[0] : 0;
   if (f.kind == HDG_FIELD_BUMPS) {
-    bool fits = true;
-    std::vector<uint64_t> w(4 * (size_t)K);
+    bool fits = usable && bumps_finite(p);
+    std::vector<uint64_t> w;
+    w.reserve(4 * (size_t)K);
     for (int k = 0; k < K && fits; ++k) {
       const double* b = &p[1 + 4 * k];
-      fits = std::isfinite(b[0]) && std::isfinite(b[1]) && std::isfinite(b[2]) && b[2] != 0.0;
+      if (b[2] != 0.0 && bump_is_off(b, e)) continue;
+      // A bump is wide against the grid, or lies where FP64's own spacing of the coordinates is no finer: 2^-s at most
+      // 2^-54 of the larger.
+      const double size = std::max(std::max(std::fabs(b[0]), std::fabs(b[1])), std::fabs(b[2]));
+      fits = b[2] != 0.0 && size >= std::ldexp(1.0, 54 - s);
       if (!fits) break;
       // |dx| 2^s scaled to r sqrt(log2 e / 2) / sigma in units of 2^-59: a factor below 2^64 and a shift
       const long double c = 0.84932180028801904272L / std::fabs((long double)b[2]);
-      int e;
-      const long double m = std::frexp(c, &e);  // c = m 2^e, m in [1/2, 1)
-      const int up = e + 59 - s;                // G = |dx| m 2^up
+      int ec;
+      const long double m = std::frexp(c, &ec);  // c = m 2^ec, m in [1/2, 1)
+      const int up = ec + 59 - s;                // G = |dx| m 2^up
       const int sh = std::max(0, up);
       fits = sh <= 62 && up > -200;
       if (!fits) break;
       const long double q = std::ldexp(m, 64 + up - sh);  // at most 2^64 - 2^10
-      uint64_t sg = (uint64_t)q;
-      sg = (sg & ~63ull) | (uint64_t)sh;
-      w[4 * k] = (uint64_t)std::llrint(std::ldexp(b[0], s));
-      w[4 * k + 1] = (uint64_t)std::llrint(std::ldexp(b[1], s));
-      w[4 * k + 2] = sg;
-      std::memcpy(&w[4 * k + 3], &b[3], 8);
+      w.push_back((uint64_t)std::llrint(std::ldexp(b[0], s)));
+      w.push_back((uint64_t)std::llrint(std::ldexp(b[1], s)));
+      w.push_back(((uint64_t)q & ~63ull) | (uint64_t)sh);
+      uint64_t amplitude;
+      std::memcpy(&amplitude, &b[3], 8);
+      w.push_back(amplitude);
     }
     if (fits) {
-      prm[0] = word((uint64_t)K);
-      for (int k = 0; k < 4 * K; ++k) prm[1 + k] = word(w[k]);
+      prm[0] = word((uint64_t)(w.size() / 4));
+      for (size_t k = 0; k < w.size(); ++k) prm[1 + k] = word(w[k]);
       return 100;
     }
     for (int k = 0; k < K; ++k) prm[1 + 4 * k + 2] = -1.0 / (2.0 * p[1 + 4 * k + 2] * p[1 + 4 * k + 2]);
     return f.kind;
   }
   if (f.kind == HDG_FIELD_FOURIER || f.kind == HDG_FIELD_EXP_FOURIER) {
-    double kmax = 0.0, asum = 0.0;
-    bool fits = true;
+    double kmax = 0.0, ksum = 0.0, asum = 0.0;
+    bool fits = usable;
     for (int k = 0; k < K; ++k) {
       const double* b = &p[2 + 4 * k];
       fits = fits && std::isfinite(b[0]) && std::isfinite(b[1]) && std::isfinite(b[2]) && std::isfinite(b[3]);
       kmax = std::max(kmax, std::max(std::fabs(b[0]), std::fabs(b[1])));
+      ksum = std::max(ksum, std::fabs(b[0]) + std::fabs(b[1]));
       asum += std::fabs(b[3]);
     }
-    if (!fits || !(asum < 1e300)) return f.kind;
-    const int u = kmax > 0.0 ? std::min(80, 60 - ceil_log2(kmax)) : 60;
+    // the grid moves a phase by pi 2^-s (|kx| + |ky|) at most: no more than FP64's rounding of a phase of one turn, 2^-51
+    if (!fits || !(asum < 1e300) || !(ksum <= std::ldexp(1.0 / 3.141592653589793, s - 51))) return f.kind;
+    // wave numbers to 2^-60 of the largest, or to where the shift ends: 2^-123 of a turn over the domain
+    const int u = std::min(kmax > 0.0 ? 60 - ceil_log2(kmax) : 60, 184 - s);
     const int w = asum > 0.0 ? 62 - ceil_log2(asum) : 0;
     const int sh = s + u - 64;
     if (sh < 0 || sh > 120 || w < -900 || w > 900) return f.kind;
@@ -419,20 +458,22 @@ extern "C++" void populate_pages(void* p, size_t bytes) {
 }
 
 extern "C++" void ensure_fixed_fields(hdg_system* s) {
-  const double xy = s->space->mesh->xy_max;
-  if (s->fix_max >= 0.0 && xy <= s->fix_max) return;
-  double top = xy;  // coordinates and the bumps' centres
-  for (auto* v : {&s->fsp, &s->ksp})
-    for (const FieldSpec& f : *v)
-      if (f.kind == HDG_FIELD_BUMPS)
-        for (int k = 0; k < (int)f.prm[0]; ++k)
-          for (int c = 0; c < 2; ++c)
-            if (std::isfinite(f.prm[1 + 4 * k + c])) top = std::max(top, std::fabs(f.prm[1 + 4 * k + c]));
-  top = std::min(std::max(top, 1e-6), 1e15);
-  int e;
-  std::frexp(top, &e);  // top < 2^e
-  const int sc = 61 - e;
-  s->fix_scale = std::ldexp(1.0, sc);
+  const std::vector<double>& xy = s->space->mesh->prob_xy_max;
+  const int np = s->nprob;
+  // magnitudes beyond which a product of the evaluation could leave FP64's range: the plain form
+  constexpr int E_MIN = -400, E_MAX = 400;
+  std::vector<int> ex(np);
+  for (int P = 0; P < np; ++P) ex[P] = xy[P] > 0.0 && std::isfinite(xy[P]) ? coordinate_exponent(xy[P]) : E_MAX + 1;
+  if (ex == s->fix_exp) return;
+  std::vector<int> sc(np);
+  std::vector<char> usable(np);
+  std::vector<double> scale(np);
+  for (int P = 0; P < np; ++P) {
+    const int top = std::max(fixed_exponent(ex[P], s->fsp[P]), fixed_exponent(ex[P], s->ksp[P]));
+    usable[P] = top >= E_MIN && top <= E_MAX;
+    sc[P] = usable[P] ? 61 - top : 0;
+    scale[P] = std::ldexp(1.0, sc[P]);
+  }
   cudaStream_t st = s->ctx->stream;
   auto make = [&](const std::vector<FieldSpec>& v, DevBuf<int32_t>* dk, DevBuf<int32_t>* doff, DevBuf<double>* dp) {
     std::vector<int32_t> kind(v.size()), off(v.size());
@@ -441,21 +482,17 @@ extern "C++" void ensure_fixed_fields(hdg_system* s) {
       const size_t at = prm.size();
       off[P] = (int32_t)at;
       prm.insert(prm.end(), v[P].prm.begin(), v[P].prm.end());
-      kind[P] = std::isfinite(xy) && xy <= 1e15 ? prepare_fixed(v[P], sc, prm.data() + at) : v[P].kind;
-      if (kind[P] == HDG_FIELD_BUMPS && !(std::isfinite(xy) && xy <= 1e15))
-        for (int k = 0; k < (int)v[P].prm[0]; ++k) {
-          double& sw = prm[at + 1 + 4 * k + 2];
-          sw = -1.0 / (2.0 * sw * sw);
-        }
+      kind[P] = prepare_fixed(v[P], sc[P], ex[P], usable[P], prm.data() + at);
     }
     dk->upload(kind.data(), kind.size(), st);
     doff->upload(off.data(), off.size(), st);
     dp->upload(prm.data(), prm.size(), st);
     HDG_CUDA(cudaStreamSynchronize(st));  // the host vectors go out of scope
   };
+  s->d_fix_scale.upload(scale.data(), scale.size(), st);
   make(s->fsp, &s->d_fkfix, &s->d_fofix, &s->d_ffix);
   make(s->ksp, &s->d_kkfix, &s->d_kofix, &s->d_kfix);
-  s->fix_max = std::ldexp(1.0, e);
+  s->fix_exp = ex;
 }
 
 // ---------------------------------------------------------------- assembly
@@ -498,7 +535,7 @@ static void set_coefficients_many(hdg_system* s, const double* taus, const hdg_f
       }
     }
   s->d_fprep.upload(fpp.data(), fpp.size(), st);
-  s->fix_max = -1.0;  // the fixed-point form is of the old fields
+  s->fix_exp.clear();  // the fixed-point form is of the old fields
   s->d_kkind.upload(kk.data(), np, st);
   s->d_koff.upload(ko.data(), np, st);
   s->d_kprm.upload(kp.data(), kp.size(), st);

@@ -28,7 +28,6 @@ struct ElemArgs {
   const double* ref;
   int ref_len, nq;
   int nc;
-  double fix_scale;  // coordinates to fixed point (CoefDev::ffix)
   CoefDev co;      // per-problem source, coefficient and tau (one problem unless batched)
   int kappa_mode;  // 0: kappa = 1, 1: per-cell array, 2: per-problem field
   const double* kcell;
@@ -402,8 +401,9 @@ __global__ void __launch_bounds__(256) k_element_schur(ElemArgs a) {
       double v = 0.0;
       if (pt < CPW * nq) {
         const double xq = fma(A01, eta, fma(A00, xi, X)), yq = fma(A11, eta, fma(A10, xi, Yv));
-        v = eval_part(a.co.fkfix[pr], a.co.ffix + a.co.fofix[pr], xq, yq, __double2ll_rn(xq * a.fix_scale),
-                      __double2ll_rn(yq * a.fix_scale), part, PARTS);
+        const double sc = a.co.fix_scale[pr];
+        v = eval_part(a.co.fkfix[pr], a.co.ffix + a.co.fofix[pr], xq, yq, __double2ll_rn(xq * sc),
+                      __double2ll_rn(yq * sc), part, PARTS);
       }
 #pragma unroll
       for (int o = PARTS / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -645,7 +645,8 @@ __global__ void __launch_bounds__(256) k_element_field(ElemArgs a) {
       const double xq = fma(A01, eta, fma(A00, xi, X)), yq = fma(A11, eta, fma(A10, xi, Yv));
       double v = 0.0, w = 0.0;
       if (in) {
-        const long long xf = __double2ll_rn(xq * a.fix_scale), yf = __double2ll_rn(yq * a.fix_scale);
+        const double sc = a.co.fix_scale[po];
+        const long long xf = __double2ll_rn(xq * sc), yf = __double2ll_rn(yq * sc);
         v = eval_part(a.co.fkfix[po], a.co.ffix + a.co.fofix[po], xq, yq, xf, yf, part, PARTS);
         w = eval_part(a.co.kkfix[po], a.co.kfix + a.co.kofix[po], xq, yq, xf, yf, part, PARTS);
       }
@@ -1073,7 +1074,6 @@ ElemArgs element_args(hdg_system* s) {
   a.nq = sp->t.nq;
   a.nc = m->nc;
   ensure_fixed_fields(s);
-  a.fix_scale = s->fix_scale;
   a.co = s->coef_dev();
   a.kappa_mode = s->kappa_cells ? 1 : (s->kappa_field ? 2 : 0);
   a.he_tau = s->he_tau ? 1 : 0;

@@ -62,7 +62,7 @@ __device__ __forceinline__ double eval_source_prepared(int kind, const double* _
 // exp or a cos is some 16 to 19 FP64 instructions: the element kernels spent most of their time on the modes
 // of a field.  A sum of Gaussian bumps or Fourier modes is therefore evaluated in 64-bit fixed point, with
 // its parameters laid out by the host (capi.cpp: prepare_fixed):
-//   coordinates  X = x 2^s with |X| <= 2^61, s the same for the whole system
+//   coordinates  X = x 2^s with |X| <= 2^61, s of the problem (its coordinates and the centres of its bumps)
 //   a mode       the phase k.x + phi / 2 pi in turns, modulo one, as a 64-bit fraction: reducing the argument is
 //                the wrap-around; cos by folding to a quarter turn and a polynomial in its square
 //   a bump       the exponent of two (r sqrt(log2 e / 2) / sigma)^2 with 54 fraction bits; 2^-f by a polynomial, the
@@ -71,8 +71,9 @@ __device__ __forceinline__ double eval_source_prepared(int kind, const double* _
 // and the exponent to some 2^-52, where FP64 loses 2^-53 of the argument itself (of 90 radians in the workloads): the
 // sums are closer to the exact ones than before: largest error over the sum of |terms| at 2e5 points, FP64 / here: 64 modes
 // up to |k| = 10 1.5e-15 / 1.1e-16, their exponential 1.7e-14 / 1.2e-15, eight bumps 5.4e-15 / 4.7e-16 (rms 1.3e-16 /
-// 1.2e-16).  A product of sines stays in FP64: it is small without being a difference, at the sides of a domain, and keeps
-// its relative accuracy there.
+// 1.2e-16).  That is of a unit square; where the grid 2^-s costs a field digits against FP64 (a narrow bump near the
+// origin of a large domain, hundreds of turns over it) the field stays in FP64, as a product of sines does: it is small
+// without being a difference, at the sides of a domain, and keeps its relative accuracy there.
 enum { FIX_BUMPS = 100, FIX_FOURIER = 101, FIX_EXP_FOURIER = 102 };
 
 // cos(2 pi t / 2^64) in units of 2^-62
@@ -100,7 +101,7 @@ __device__ __forceinline__ long long cos_turns(unsigned long long t) {
 // 2^-e, e in units of 2^-54
 __device__ __forceinline__ double exp2_minus(unsigned long long e) {
   const unsigned n = (unsigned)(e >> 54);
-  if (n > 1000u) return 0.0;
+  if (n > 1020u) return 0.0;  // below the smallest normal number
   const unsigned long long f = e << 10;
   const unsigned fh = (unsigned)(f >> 32);
   unsigned long long q = 62120492029ull - __umulhi(2906043853u, fh);

@@ -127,6 +127,7 @@ struct CoefDev {
   const double* ffix;
   const int32_t *kkfix, *kofix;
   const double* kfix;
+  const double* fix_scale;   // [nprob] coordinates to fixed point
 };
 
 // ------------------------------------------------------------------ objects
@@ -191,7 +192,7 @@ struct hdg_mesh {
   double LL[2] = {0, 0}, UR[2] = {1, 1};
   // device copies
   DevBuf<double> d_xy;
-  double xy_max = 0.0;        // largest |coordinate| (upload_coordinates)
+  std::vector<double> prob_xy_max;  // largest |coordinate| of each problem, infinite if one is no number (upload_coordinates)
   DevBuf<int32_t> d_cells, d_cfaces;
   DevBuf<uint8_t> d_orient;   // bit f = face_orientation(cell, f)
   DevBuf<int32_t> d_fcell;    // [nf][2] cells of a face (second -1 on the boundary)
@@ -282,7 +283,7 @@ struct hdg_system {
   CoefDev coef_dev() const {
     return CoefDev{space->mesh->d_cell_prob.p, d_fkind.p, d_foff.p, d_fprm.p, d_kkind.p, d_koff.p, d_kprm.p,
                    d_tau.p, d_fprep.p, d_fkfix.p, d_fofix.p, d_ffix.p, d_kkfix.p, d_kofix.p,
-                   d_kfix.p};
+                   d_kfix.p, d_fix_scale.p};
   }
   // per-cell condensed blocks: AB = [Ate | bte] (m x (m+1)), KB = [K_e | b_e] (n x (m+1)), or,
   // after the Schur element path (kb_u_only), only its u rows [X_u | b_u] (nw x (m+1)), with the rows of the two
@@ -293,9 +294,9 @@ struct hdg_system {
   DevBuf<double> d_kappa;  // per-cell kappa (optional)
   DevBuf<double> d_fprm, d_kprm;
   DevBuf<double> d_fprep;  // d_fprm prepared for the pivoted element kernel (CoefDev::fprep)
-  DevBuf<double> d_ffix, d_kfix;     // fields in fixed point (CoefDev::ffix), made for coordinates up to fix_max
+  DevBuf<double> d_ffix, d_kfix, d_fix_scale;  // fields in fixed point (CoefDev::ffix), made for the mesh's coordinates
   DevBuf<int32_t> d_fkfix, d_fofix, d_kkfix, d_kofix;
-  double fix_max = 0.0, fix_scale = 1.0;
+  std::vector<int> fix_exp;  // ... below 2^fix_exp[P] in problem P (coordinate_exponent); empty: not made yet
   FieldSpec f, kappa;
   bool kappa_field = false, kappa_cells = false;
   // Trace matrix.  Host: block rows sorted by face id (h_browptr/h_bcol, the export pattern).
@@ -373,8 +374,8 @@ constexpr int HDG_CG_ST = 4;
 
 // ------------------------------------------------------------------ kernel launchers
 void launch_element_condense(hdg_system* s, cudaStream_t st);
-// The fields' fixed-point form for the mesh's present coordinates (made anew when they have grown; uploads on the
-// context's stream).
+// The fields' fixed-point form for the mesh's present coordinates (made anew when their magnitude has changed; uploads
+// on the context's stream).
 void ensure_fixed_fields(hdg_system* s);
 void launch_gather(hdg_system* s, cudaStream_t st);
 void launch_apply_dirichlet(hdg_system* s, const std::vector<int32_t>& dofs0, const std::vector<double>& vals,

@@ -245,7 +245,11 @@ void hdg_mesh::upload() {
 }
 
 void hdg_mesh::upload_coordinates() {
-  xy_max = 0.0;
-  for (double v : xy) xy_max = std::max(xy_max, std::fabs(v));
+  prob_xy_max.assign(nprob, 0.0);
+  for (int P = 0; P < nprob; ++P)
+    for (size_t k = 2 * (size_t)prob_node0[P]; k < 2 * (size_t)prob_node0[P + 1]; ++k) {
+      const double v = std::fabs(xy[k]);
+      if (!(v <= prob_xy_max[P])) prob_xy_max[P] = v < INFINITY ? v : INFINITY;  // a NaN as an infinity
+    }
   d_xy.upload(xy.data(), xy.size(), ctx->stream);
 }
