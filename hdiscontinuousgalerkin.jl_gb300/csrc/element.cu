@@ -38,6 +38,7 @@ struct ElemArgs {
   int schur;  // 1: the Schur path (invertible reference mass, kappa constant per cell), 2: with one null function,
               // 3: kappa a field, 4: with one null function
   int he_tau; // 1: He carries tau
+  int unit;   // the rows of Ate have a sum that is known (RefTables::unit)
   RefLayout L;  // offsets of the packed reference tables (tables.cpp: ref_layout)
 };
 
@@ -259,7 +260,12 @@ __global__ void __launch_bounds__(EWARPS * 32) k_element_condense(ElemArgs a) {
 //   bte_{fi}    = -(R~' D^-1 R~)_{fi,be}
 // (the same Ate = [Ee;Fe]' Me^-1 [-Ee;Fe] - He and bte = -[Ee;Fe]' Me^-1 [0;be] that the full
 // elimination of examples/poisson2D_HDG.jl:155-174 forms, reordered), symmetric by construction, so
-// every pair of columns is formed once.  The u rows of [K_e | b_e], X_u = U^-1 D^-1 R~ (and a_c), are stored;
+// every pair of columns is formed once.  A constant trace is the trace of a constant u with q = 0, so every row of Ate sums
+// over the constants of the three faces to (tau - 1) |e_f| int mu_i (0 where He carries tau).  As differences of products the entries
+// miss that by some roundings, the same ones in cells of one shape, and 1/h^2 of them goes into the solution: so the
+// entries between a face's functions and its own constant are taken from the row's sum instead.  Error of u_hat against
+// extended precision, pivoted elimination / without / with: 64^2 squares of p = 2 1.3e-12 / 1.1e-12 / 3.7e-13, distorted
+// with kappa within a decade, 32^2 of p = 3 6.4e-14 / 7.2e-13 / 2.6e-14, 24^2 of p = 4 9.0e-14 / 1.6e-12 / 1.0e-14.  The u rows of [K_e | b_e], X_u = U^-1 D^-1 R~ (and a_c), are stored;
 // the q rows follow linearly from them, q = kf (adl0 M^-1 D0 u + adl1 M^-1 D1 u - sum_f wn_f M^-1
 // F_f u_hat_f) + z a, and are formed at recovery (k_recover_u) or when the blocks are exported (k_expand_ke).
 //
@@ -292,7 +298,7 @@ template <int P, int NZ> struct SchurDims {
   __host__ __device__ static constexpr int tables(int nq) {  // doubles staged per CTA
     return 6 * TRI + 18 * NW * NT + NT * NT + NW * nq + 2 * nq + 36 * NT * NT + NZ * (2 * NW + 6 * NT);
   }
-  __host__ __device__ static constexpr int per_warp(int nq) { return CPW * (W + Y + GEO + NW + nq); }
+  __host__ __device__ static constexpr int per_warp(int nq) { return CPW * (W + Y + GEO + NW + nq + 3 * M); }
 };
 
 template <int P, int NZ>
@@ -346,6 +352,7 @@ __global__ void __launch_bounds__(256) k_element_schur(ElemArgs a) {
   double* be0 = geo0 + CPW * GEO;
   double* be = be0 + cl * NW;
   double* sq0 = be0 + CPW * NW;
+  double* us = sq0 + CPW * nq + cl * 3 * M;              // Ate of each row and the constant of each other face
   const int f = col < M ? col / NT : 0, fj = col < M ? col - f * NT : 0;
   const int nwarps = blockDim.x >> 5;
   __syncthreads();
@@ -492,10 +499,19 @@ __global__ void __launch_bounds__(256) k_element_schur(ElemArgs a) {
           const int lo = min(f, g), hi = max(f, g);
           double v = dot - geo[6 + lo + hi + (lo > 0 ? 1 : 0)] * tP[((fo * 6 + go) * NT + fj) * NT + gj];
           if (f == g) v -= he * Hh[gj];
+          if (f != g && gj == 0) us[col * 3 + g] = v;
+          if (f != g && fj == 0) us[o * 3 + f] = v;
+          if (a.unit && f == g && (fj == 0 || gj == 0)) continue;  // from the row's sum below
           AB[col * COLS + o] = v;
           if (d) AB[o * COLS + col] = v;
         }
       }
+    }
+    __syncwarp();
+    if (a.unit && mine && col < M) {
+      const double v = (a.he_tau ? 0.0 : tau - 1.0) * el * Hh[0] - (us[col * 3 + (f + 1) % 3] + us[col * 3 + (f + 2) % 3]);
+      AB[col * COLS + f * NT] = v;
+      if (fj) AB[f * NT * COLS + col] = v;
     }
     // ---- X_u = U^-1 Y in the lane's registers; a row goes out as m+1 consecutive values -----------
     double* KB = a.KB + (size_t)e * NA * COLS + col;
@@ -539,7 +555,7 @@ template <int P, int NZ> struct FieldDims {
            NZ * (3 * NW + 6 * NT);
   }
   __host__ __device__ static constexpr int per_warp(int nq) {
-    return CPW * (YA + WA + PR + W + Y + GEO + NW + 2 * nq);
+    return CPW * (YA + WA + PR + W + Y + GEO + NW + 2 * nq + 3 * M);
   }
 };
 
@@ -598,6 +614,7 @@ __global__ void __launch_bounds__(256) k_element_field(ElemArgs a) {
   double* be = geo0 + CPW * GEO + cl * NW;
   double* sq0 = geo0 + CPW * (GEO + NW);                    // f at the points, then kappa^-1
   double* sk0 = sq0 + CPW * nq;
+  double* us = sk0 + CPW * nq + cl * 3 * M;                 // as in k_element_schur
   // second elimination: the first COLS lanes of a cell, a right-hand side each
   const bool on2 = on1 && c1 < COLS;
   const int col = min(c1, COLS - 1);
@@ -803,10 +820,19 @@ __global__ void __launch_bounds__(256) k_element_field(ElemArgs a) {
           const double gx = sel3(g, wx0, -J11, J10), gy = sel3(g, wy0, J01, -J00);
           double v = dot - (wx * gx + wy * gy) * pr[pair_at(2 * NW + col, 2 * NW + o)];
           if (f == g) v -= he * Hh[gj];
+          if (f != g && gj == 0) us[col * 3 + g] = v;
+          if (f != g && fj == 0) us[o * 3 + f] = v;
+          if (a.unit && f == g && (fj == 0 || gj == 0)) continue;
           AB[col * COLS + o] = v;
           if (d) AB[o * COLS + col] = v;
         }
       }
+    }
+    __syncwarp();
+    if (a.unit && mine && on2 && col < M) {
+      const double v = (a.he_tau ? 0.0 : tau - 1.0) * el * Hh[0] - (us[col * 3 + (f + 1) % 3] + us[col * 3 + (f + 2) % 3]);
+      AB[col * COLS + f * NT] = v;
+      if (fj) AB[f * NT * COLS + col] = v;
     }
     // ---- X_u (and a_c), kept for the q rows in the place of Y -----------------------------------------
     double* KB = a.KB + (size_t)e * N * COLS;
@@ -1077,6 +1103,7 @@ ElemArgs element_args(hdg_system* s) {
   a.co = s->coef_dev();
   a.kappa_mode = s->kappa_cells ? 1 : (s->kappa_field ? 2 : 0);
   a.he_tau = s->he_tau ? 1 : 0;
+  a.unit = sp->t.unit ? 1 : 0;
   a.kcell = s->d_kappa.p;
   a.AB = s->d_AB.p;
   a.KB = s->d_KB.p;

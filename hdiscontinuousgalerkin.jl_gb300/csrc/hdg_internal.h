@@ -213,6 +213,7 @@ struct RefTables {
   std::vector<double> Nv;          // [nw][3] basis at the reference vertices (0,0), (1,0), (0,1)
   bool schur = false;              // the Schur tables are valid (see tables.cpp)
   bool positive = false;           // every volume weight is positive
+  bool unit = false;               // the rules integrate what makes a constant trace that of a constant u with q = 0
   int nullity = 0;                 // dimension of the reference mass matrix's null space (0 or 1 with schur)
   // packed device tables (see tables.cpp: ref_layout)
   std::vector<double> packed;

@@ -419,6 +419,26 @@ bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
     }
     t->schur = ok && minpiv > 1e-10L * maxpiv;
     t->positive = std::all_of(t->qw.begin(), t->qw.end(), [](double w) { return w > 0.0; });
+    // Be 1 = Ee 1 and Ce 1 = Fe 1 on the reference triangle (outward normals times edge lengths (1,1), (-1,0), (0,-1)); the
+    // first function of either basis is the constant
+    {
+      static const double WN[3][2] = {{1, 1}, {-1, 0}, {0, -1}};
+      const double u1 = 1.0 / t->N[0], t1 = 1.0 / t->T[0];
+      double off = 0.0, top = 0.0;
+      for (int a = 0; a < nw; ++a) {
+        for (int l = 0; l < 2; ++l) {
+          double s = P[(l ? L.D1 : L.D0) + a * nw] * u1;
+          top = std::max(top, std::fabs(s));
+          for (int f = 0; f < 3; ++f) s -= WN[f][l] * P[L.F + ((f * 2 + 1) * nw + a) * nt] * t1;
+          off = std::max(off, std::fabs(s));
+        }
+        for (int fo = 0; fo < 6; ++fo) {
+          const double s = P[L.C + (fo / 2 * nw + a) * nw] * u1 - P[L.F + (fo * nw + a) * nt] * t1;
+          off = std::max(off, std::fabs(s));
+        }
+      }
+      t->unit = off <= 1e-12 * std::max(top, 1.0);
+    }
     std::vector<long double> inv((size_t)nw * nw, 0.0L), range((size_t)nw * nw, 0.0L);  // range: V, nr columns
     int nr = nw;
     for (int i = 0; i < nw; ++i) range[(size_t)i * nw + i] = 1.0L;
