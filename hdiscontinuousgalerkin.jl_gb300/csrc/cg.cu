@@ -516,11 +516,11 @@ template <int NT> struct SolverNT : CgSolver {
   CgResident res;   // one problem with Jacobi whose state fits on the chip: chunks are single launches
   CgArgs<double> a64;
   CgArgs<float> a32;
-  // Segment compaction: once most problems have finished, the launch grid is rebuilt from the
-  // segments of the problems still running, so the tail of a batch does not pay for blocks that
-  // would only return.  The full tables are restored when the solve ends.
-  std::vector<int32_t> full_prob, full_r0, full_r1, full_b0, full_nb;
-  int nseg_full = 0;
+  // Segment compaction: once most rows belong to problems that have finished, the rows of the others are cut anew, so
+  // the tail of a batch neither pays for blocks that would only return nor leaves the GPU to a few long ones.  The full
+  // table is restored when the solve ends.
+  SegTable* tab = nullptr;
+  int64_t rows_cut = 0;  // rows that the table covers
   // Byte accounting of sampled chunks: iteration counts at the launch of the sampled chunk; and of
   // every chunk: iteration counts at the previous read-back.
   std::vector<int32_t> sample_it0, it_prev;
@@ -538,23 +538,22 @@ template <int NT> struct SolverNT : CgSolver {
   void set_stream(cudaStream_t stream) override { st = stream; }
 
   SegArgs seg() const {
-    return SegArgs{s->d_seg_prob.p, s->d_seg_row0.p, s->d_seg_row1.p, s->d_prob_blk0.p, s->d_prob_nblk.p,
-                   s->d_part.p, s->d_cnt.p};
+    return SegArgs{tab->d_prob.p, tab->d_row0.p, tab->d_row1.p, tab->d_blk0.p, tab->d_nblk.p, s->d_part.p, s->d_cnt.p};
   }
 
   template <typename T> void launch_pair(const CgArgs<T>& a, cudaStream_t stream, int it) {
     if constexpr (sizeof(T) == sizeof(double)) {
-      k_cg_a<NT, T><<<s->nseg, CG_BLOCK, 0, stream>>>(a);
+      k_cg_a<NT, T><<<tab->nseg, CG_BLOCK, 0, stream>>>(a);
       if (mg) {
-        k_cg_b_mg<NT><<<s->nseg, CG_BLOCK, 0, stream>>>(a, c->r32.p);
+        k_cg_b_mg<NT><<<tab->nseg, CG_BLOCK, 0, stream>>>(a, c->r32.p);
         amg_apply(s, c->r32.p, c->z32.p, c->st.p, stream);
-        k_cg_c<NT><<<s->nseg, CG_BLOCK, 0, stream>>>(a, c->z32.p, 0, 0);
+        k_cg_c<NT><<<tab->nseg, CG_BLOCK, 0, stream>>>(a, c->z32.p, 0, 0);
       } else {
-        k_cg_b<NT, T><<<s->nseg, CG_BLOCK, 0, stream>>>(a, 0);
+        k_cg_b<NT, T><<<tab->nseg, CG_BLOCK, 0, stream>>>(a, 0);
       }
     } else {
-      k_cg_a_fresh<NT, T><<<s->nseg, CG_BLOCK, 0, stream>>>(a, it & 1);
-      k_cg_b<NT, T><<<s->nseg, CG_BLOCK, 0, stream>>>(a, (it & 1) ^ 1);
+      k_cg_a_fresh<NT, T><<<tab->nseg, CG_BLOCK, 0, stream>>>(a, it & 1);
+      k_cg_b<NT, T><<<tab->nseg, CG_BLOCK, 0, stream>>>(a, (it & 1) ^ 1);
     }
   }
 
@@ -596,12 +595,8 @@ template <int NT> struct SolverNT : CgSolver {
     }
     s->ensure_reduction_buffers();
     s->d_x.alloc(nrow);
-    nseg_full = s->nseg;  // full tables (a solve restores them when it ends)
-    full_prob = s->h_seg_prob;
-    full_r0 = s->h_seg_row0;
-    full_r1 = s->h_seg_row1;
-    full_b0 = s->h_prob_blk0;
-    full_nb = s->h_prob_nblk;
+    tab = &segments_of(s, mixed);
+    rows_cut = nrow;
     for (auto* e : s->ev_cg_a) delete e;
     for (auto* e : s->ev_cg_b) delete e;
     s->ev_cg_a.clear();
@@ -645,9 +640,9 @@ template <int NT> struct SolverNT : CgSolver {
       amg_setup_numeric(s, st);
       a64 = CgArgs<double>{seg(), s->d_bcol5.p, s->nf, s->d_val.p, s->d_b.p, c->dinv.p, s->d_x.p, c->r.p, c->z.p,
                            c->p.p, c->q.p, c->p.p, c->sc.p, c->st.p, nullptr, nullptr};
-      k_cg_init_mg<NT><<<s->nseg, CG_BLOCK, 0, st>>>(a64, c->r32.p);
+      k_cg_init_mg<NT><<<tab->nseg, CG_BLOCK, 0, st>>>(a64, c->r32.p);
       amg_apply(s, c->r32.p, c->z32.p, c->st.p, st);
-      k_cg_c<NT><<<s->nseg, CG_BLOCK, 0, st>>>(a64, c->z32.p, 1, 0);
+      k_cg_c<NT><<<tab->nseg, CG_BLOCK, 0, st>>>(a64, c->z32.p, 1, 0);
       // the graph holds the hierarchy's buffers: rebuilt after a Jacobi solve or a new setup
       if (c->graph64 && (!c->graph_mg || c->graph_amg_gen != s->amg_gen)) {
         cudaGraphExecDestroy(c->graph64);
@@ -661,7 +656,7 @@ template <int NT> struct SolverNT : CgSolver {
       k_dinv<NT, double><<<(nrow + 255) / 256, 256, 0, st>>>(nrow, s->d_kdiag.p, s->d_val.p, c->dinv.p);
       a64 = CgArgs<double>{seg(), s->d_bcol5.p, s->nf, s->d_val.p, s->d_b.p, c->dinv.p, s->d_x.p, c->r.p, c->z.p,
                            c->p.p, c->q.p, c->p.p, c->sc.p, c->st.p, nullptr, nullptr};
-      k_cg_init<NT, double><<<s->nseg, CG_BLOCK, 0, st>>>(a64);
+      k_cg_init<NT, double><<<tab->nseg, CG_BLOCK, 0, st>>>(a64);
       if (c->graph_mg && c->graph64) { cudaGraphExecDestroy(c->graph64); c->graph64 = nullptr; }
       c->graph_mg = false;
       if (res.kind == CgResident::NONE) build_graph<double>(a64, &c->graph64, &c->chunk64);
@@ -675,7 +670,7 @@ template <int NT> struct SolverNT : CgSolver {
       k_dinv<NT, float><<<(nrow + 255) / 256, 256, 0, st>>>(nrow, s->d_kdiag.p, s->d_val.p, c->dinvf.p);
       a32 = CgArgs<float>{seg(), s->d_bcol5.p, s->nf, s->d_valf.p, s->d_b.p, c->dinvf.p, s->d_x.p, c->rf.p, c->zf.p,
                           c->pf.p, c->qf.p, c->pf2.p, c->sc.p, c->st.p, c->xh.p, c->xl.p};
-      k_cg_init<NT, float><<<s->nseg, CG_BLOCK, 0, st>>>(a32);
+      k_cg_init<NT, float><<<tab->nseg, CG_BLOCK, 0, st>>>(a32);
       if (res.kind == CgResident::NONE) build_graph<float>(a32, &c->graph32, &c->chunk32);
       s->ctx->launches++;
     }
@@ -707,22 +702,22 @@ template <int NT> struct SolverNT : CgSolver {
         EventPair* ea = new EventPair();
         EventPair* eb = new EventPair();
         ea->start(st);
-        if constexpr (sizeof(T) == sizeof(double)) k_cg_a<NT, T><<<s->nseg, CG_BLOCK, 0, st>>>(a);
-        else k_cg_a_fresh<NT, T><<<s->nseg, CG_BLOCK, 0, st>>>(a, it & 1);
+        if constexpr (sizeof(T) == sizeof(double)) k_cg_a<NT, T><<<tab->nseg, CG_BLOCK, 0, st>>>(a);
+        else k_cg_a_fresh<NT, T><<<tab->nseg, CG_BLOCK, 0, st>>>(a, it & 1);
         ea->stop(st);
         eb->start(st);
         if constexpr (sizeof(T) == sizeof(double)) {
           if (mg) {  // the update, the V-cycle and the r.z kernel are timed together
-            k_cg_b_mg<NT><<<s->nseg, CG_BLOCK, 0, st>>>(a, c->r32.p);
+            k_cg_b_mg<NT><<<tab->nseg, CG_BLOCK, 0, st>>>(a, c->r32.p);
             s->prof_cheb0 = true;  // and each level-0 smoother sweep on its own
             amg_apply(s, c->r32.p, c->z32.p, c->st.p, st);
             s->prof_cheb0 = false;
-            k_cg_c<NT><<<s->nseg, CG_BLOCK, 0, st>>>(a, c->z32.p, 0, 0);
+            k_cg_c<NT><<<tab->nseg, CG_BLOCK, 0, st>>>(a, c->z32.p, 0, 0);
           } else {
-            k_cg_b<NT, T><<<s->nseg, CG_BLOCK, 0, st>>>(a, 0);
+            k_cg_b<NT, T><<<tab->nseg, CG_BLOCK, 0, st>>>(a, 0);
           }
         } else {
-          k_cg_b<NT, T><<<s->nseg, CG_BLOCK, 0, st>>>(a, (it & 1) ^ 1);
+          k_cg_b<NT, T><<<tab->nseg, CG_BLOCK, 0, st>>>(a, (it & 1) ^ 1);
         }
         eb->stop(st);
         s->ev_cg_a.push_back(ea);
@@ -757,14 +752,14 @@ template <int NT> struct SolverNT : CgSolver {
   void residual(bool replace, bool sync = true) {
     HDG_CUDA(cudaMemcpyAsync(c->st.p, c->h_st, sizeof(int32_t) * ST * nprob, cudaMemcpyHostToDevice, st));
     if (mixed) x_to_double();
-    if (mixed) k_cg_residual<NT, float><<<s->nseg, CG_BLOCK, 0, st>>>(a32, s->d_val.p, replace ? 1 : 0, nullptr);
-    else k_cg_residual<NT, double><<<s->nseg, CG_BLOCK, 0, st>>>(a64, s->d_val.p, replace ? 1 : 0,
+    if (mixed) k_cg_residual<NT, float><<<tab->nseg, CG_BLOCK, 0, st>>>(a32, s->d_val.p, replace ? 1 : 0, nullptr);
+    else k_cg_residual<NT, double><<<tab->nseg, CG_BLOCK, 0, st>>>(a64, s->d_val.p, replace ? 1 : 0,
                                                                  mg ? c->r32.p : nullptr);
     HDG_CUDA(cudaGetLastError());
     s->ctx->launches++;
     if (mg && replace) {  // z for the replaced residuals, and a restart (beta = 0) of those problems
       amg_apply(s, c->r32.p, c->z32.p, c->st.p, st);
-      k_cg_c<NT><<<s->nseg, CG_BLOCK, 0, st>>>(a64, c->z32.p, 1, 1);
+      k_cg_c<NT><<<tab->nseg, CG_BLOCK, 0, st>>>(a64, c->z32.p, 1, 1);
       HDG_CUDA(cudaGetLastError());
       s->ctx->launches++;
     }
@@ -772,37 +767,27 @@ template <int NT> struct SolverNT : CgSolver {
     if (sync) HDG_CUDA(cudaStreamSynchronize(st));
   }
 
-  // Rebuilds the segment tables from the running problems (all = restore the full tables).
+  // Replaces the table's contents by a cut of the running problems' rows (all: restores the full one).
   void set_segments(bool all) {
-    std::vector<int32_t> sp, r0, r1, b0(full_b0), nb(full_nb);
-    for (int P = 0; P < nprob; ++P) {
-      if (!all && c->h_st[ST * P] != 0) continue;
-      b0[P] = (int32_t)sp.size();
-      for (int k = full_b0[P]; k < full_b0[P] + full_nb[P]; ++k) {
-        sp.push_back(full_prob[k]);
-        r0.push_back(full_r0[k]);
-        r1.push_back(full_r1[k]);
-      }
-    }
-    if (sp.empty()) return;
-    const int n = (int)sp.size();
-    HDG_CUDA(cudaMemcpyAsync(s->d_seg_prob.p, sp.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    HDG_CUDA(cudaMemcpyAsync(s->d_seg_row0.p, r0.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    HDG_CUDA(cudaMemcpyAsync(s->d_seg_row1.p, r1.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    HDG_CUDA(cudaMemcpyAsync(s->d_prob_blk0.p, b0.data(), nprob * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-    HDG_CUDA(cudaStreamSynchronize(st));  // host staging vectors go out of scope
-    if (n != s->nseg) {
-      s->nseg = n;
+    std::vector<char> on(nprob, 1);
+    if (!all)
+      for (int P = 0; P < nprob; ++P) on[P] = c->h_st[ST * P] == 0;
+    const int before = tab->nseg;
+    put_segments(s, all ? tab->full : cut_segments(s, on.data(), mixed), tab, st);
+    if (tab->nseg != before) {
       if (mixed) { c->chunk32 = 0; build_graph<float>(a32, &c->graph32, &c->chunk32); }
       else { c->chunk64 = 0; build_graph<double>(a64, &c->graph64, &c->chunk64); }
     }
   }
 
   void maybe_compact() {
-    int active = 0;
+    int64_t active = 0;
     for (int P = 0; P < nprob; ++P)
-      if (c->h_st[ST * P] == 0) active += full_nb[P];
-    if (active > 0 && s->nseg >= 16 && 2 * active <= s->nseg) set_segments(false);
+      if (c->h_st[ST * P] == 0) active += s->h_prob_row0[P + 1] - s->h_prob_row0[P];
+    if (active > 0 && tab->nseg >= 16 && 2 * active <= rows_cut) {
+      rows_cut = active;
+      set_segments(false);
+    }
   }
 
   // Algorithmic bytes per row of the two iteration kernels: the matrix row (5 blocks of NT values),
@@ -915,7 +900,7 @@ template <int NT> struct SolverNT : CgSolver {
   }
 
   void finish_enqueue() override {
-    if (s->nseg != nseg_full) set_segments(true);  // restore the full tables (other kernels use them)
+    if (rows_cut != nrow) set_segments(true);  // restore the full table (other kernels use it)
     if (mixed) x_to_double();
     if (!mixed) {  // report the true FP64 residual of every problem
       for (int P = 0; P < nprob; ++P) c->h_st[ST * P + 3] = 1;

@@ -253,6 +253,17 @@ struct hdg_space {
 struct CgState;       // cg.cu
 struct AmgHierarchy;  // amg.cu
 
+// The rows of a system's problems cut into segments: problem and row range of each, first segment and number of them
+// of each problem.
+struct SegCut {
+  std::vector<int32_t> prob, row0, row1, blk0, nblk;
+};
+struct SegTable {
+  int nseg = 0;
+  SegCut full;  // host copy of the cut of all problems
+  DevBuf<int32_t> d_prob, d_row0, d_row1, d_blk0, d_nblk;
+};
+
 struct hdg_system {
   hdg_space* space = nullptr;
   hdg_ctx* ctx = nullptr;
@@ -278,9 +289,11 @@ struct hdg_system {
   }
   // Segments: the CUDA blocks of the row-parallel kernels (CG, meandiag, residual); each block
   // covers a row range inside one problem, so per-problem reductions need no cross-problem sums.
-  int nseg = 0;
-  DevBuf<int32_t> d_seg_prob, d_seg_row0, d_seg_row1, d_prob_blk0, d_prob_nblk;
-  std::vector<int32_t> h_seg_prob, h_seg_row0, h_seg_row1, h_prob_blk0, h_prob_nblk;  // host copies
+  // seg32: of the FP32 iteration where its wave of blocks is another (made by its first solve), else unused.
+  SegTable seg, seg32;
+  bool seg32_known = false;
+  size_t seg_room = 0;  // segments that any cut of any of the problems may take
+  int num_sm = 152;
   CoefDev coef_dev() const {
     return CoefDev{space->mesh->d_cell_prob.p, d_fkind.p, d_foff.p, d_fprm.p, d_kkind.p, d_koff.p, d_kprm.p,
                    d_tau.p, d_fprep.p, d_fkfix.p, d_fofix.p, d_ffix.p, d_kkfix.p, d_kofix.p,
@@ -361,7 +374,7 @@ struct hdg_system {
   ~hdg_system();
   // partials: 2 per segment; tickets: 4 per problem (CG product, CG update, residual, meandiag)
   void ensure_reduction_buffers() {
-    const size_t np = 2 * (size_t)std::max(nseg, 1024), nc = 4 * (size_t)nprob;
+    const size_t np = 2 * std::max<size_t>(seg_room, 1024), nc = 4 * (size_t)nprob;
     if (d_part.n < np) d_part.alloc(np);
     if (d_cnt.n < nc) {
       d_cnt.alloc(nc);
@@ -398,6 +411,12 @@ int run_refine(hdg_system* s, const hdg_solver& o, int steps, double ctol, std::
 int run_solve_many(const std::vector<hdg_system*>& sys, const hdg_solver& o,
                    std::vector<std::vector<hdg_stats>>* stats);
 void build_segments(hdg_system* s);
+// The segments of an iteration: the system's, or those of the FP32 iteration.
+SegTable& segments_of(hdg_system* s, bool fp32);
+// The cut of the problems that on[P] names (NULL: all), and a cut's copy into a table (host arrays are read before the
+// return).
+SegCut cut_segments(const hdg_system* s, const char* on, bool fp32);
+void put_segments(hdg_system* s, const SegCut& c, SegTable* t, cudaStream_t st);
 
 // The CG of one system, driven chunk by chunk by a host loop (run_solve_many, the serving engine).
 struct CgSolver {

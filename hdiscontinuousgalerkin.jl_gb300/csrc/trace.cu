@@ -75,74 +75,115 @@ void build_block_structure(hdg_system* s) {
   HDG_CUDA(cudaStreamSynchronize(st));
 }
 
-// Segments of the row-parallel kernels: every problem's trace rows are cut into ranges of at most
-// SEG_ROWS rows, one CUDA block each, so a block never spans two problems.
+// Segments of the row-parallel kernels: every problem's trace rows are cut into ranges, one CUDA block each, so a block never
+// spans two problems.
+// A range has about 1024 rows (four per thread in the CG kernels).  Once the segments can fill the GPU, their number is
+// rounded up to a multiple of the SM count (the extra segments go to the largest problems), so that every SM gets the
+// same number of equal blocks.
+// Far beyond one wave of resident blocks (4 to an SM in the FP64 iteration and all of multigrid, 6 in the FP32 one), a wave of
+// longer ranges, as equal as the problems allow: a block spends 3 us on its reduction whatever its rows.  An iteration,
+// us, segments of 1024 rows / 608 segments / 912: multigrid, 3.15 M rows of p = 3 473 / 436 / 460, 1.44 M of p = 2 332 / 318 /
+// 333; FP64 Jacobi, 3.15 M rows 220 / 178 / 224; FP32 Jacobi 133 / 143 / 120.
+SegCut cut_segments(const hdg_system* s, const char* on, bool fp32) {
+  constexpr int64_t SEG_ROWS = 1024;
+  const int np = s->nprob, sms = s->num_sm;
+  auto rows_of = [&](int P) { return (int64_t)std::max(s->h_prob_row0[P + 1] - s->h_prob_row0[P], 1); };
+  std::vector<int> of;
+  int64_t longest = 1;
+  for (int P = 0; P < np; ++P)
+    if (!on || on[P]) {
+      of.push_back(P);
+      longest = std::max(longest, rows_of(P));
+    }
+  auto count = [&](int64_t len) {
+    int64_t n = 0;
+    for (int P : of) n += (rows_of(P) + len - 1) / len;
+    return n;
+  };
+  int64_t len = SEG_ROWS, total = count(len);
+  const int64_t wave = (int64_t)(fp32 ? 6 : 4) * sms;
+  if (total > 8 * sms && (int64_t)of.size() <= wave) {  // the shortest ranges of which a wave holds all
+    int64_t lo = len;
+    for (len = longest; lo < len;) {
+      const int64_t mid = (lo + len) / 2;
+      if (count(mid) <= wave) len = mid;
+      else lo = mid + 1;
+    }
+    total = count(len);
+  }
+  std::vector<int64_t> nseg(np, 0);
+  for (int P : of) nseg[P] = (rows_of(P) + len - 1) / len;
+  if (total >= sms) {
+    int64_t extra = (sms - total % sms) % sms;
+    std::vector<int> order(of);
+    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return rows_of(x) > rows_of(y); });
+    for (size_t k = 0; extra > 0; k = (k + 1) % order.size(), --extra) ++nseg[order[k]];
+  }
+  SegCut c;
+  c.blk0.assign(np, 0);
+  c.nblk.assign(np, 0);
+  for (int P : of) {
+    const int64_t a = s->h_prob_row0[P], e = s->h_prob_row0[P + 1], n = std::min(nseg[P], rows_of(P));
+    const int64_t per = (rows_of(P) + n - 1) / n;
+    c.blk0[P] = (int32_t)c.prob.size();
+    c.nblk[P] = (int32_t)n;
+    for (int64_t k = 0; k < n; ++k) {
+      c.prob.push_back(P);
+      c.row0.push_back((int32_t)std::min(e, a + k * per));
+      c.row1.push_back((int32_t)std::min(e, a + (k + 1) * per));
+    }
+  }
+  return c;
+}
+
+void put_segments(hdg_system* s, const SegCut& c, SegTable* t, cudaStream_t st) {
+  const size_t n = c.prob.size(), np = (size_t)s->nprob;
+  for (auto* b : {&t->d_prob, &t->d_row0, &t->d_row1}) b->alloc(s->seg_room);  // captured graphs hold the addresses
+  for (auto* b : {&t->d_blk0, &t->d_nblk}) b->alloc(np);
+  auto put = [&](DevBuf<int32_t>& to, const std::vector<int32_t>& v, size_t k) {
+    HDG_CUDA(cudaMemcpyAsync(to.p, v.data(), k * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  };
+  put(t->d_prob, c.prob, n);
+  put(t->d_row0, c.row0, n);
+  put(t->d_row1, c.row1, n);
+  put(t->d_blk0, c.blk0, np);
+  put(t->d_nblk, c.nblk, np);
+  HDG_CUDA(cudaStreamSynchronize(st));
+  t->nseg = (int)n;
+}
+
+SegTable& segments_of(hdg_system* s, bool fp32) {
+  if (fp32 && !s->seg32_known) {
+    s->seg32_known = true;
+    SegCut c = cut_segments(s, nullptr, true);
+    if (c.prob.size() != s->seg.full.prob.size()) {
+      put_segments(s, c, &s->seg32, s->ctx->stream);
+      s->seg32.full = std::move(c);
+    }
+  }
+  return fp32 && s->seg32.nseg > 0 ? s->seg32 : s->seg;
+}
+
 void build_segments(hdg_system* s) {
-  // About 1024 rows per segment (four per thread in the CG kernels).  Once the segments can fill
-  // the GPU, their number is rounded up to a multiple of the SM count (the extra segments go to
-  // the largest problems), so that every SM gets the same number of equal blocks.
-  constexpr int SEG_ROWS = 1024, NUM_SM = 152;
   const hdg_mesh* m = s->space->mesh;
   s->nprob = m->nprob;
+  HDG_CUDA(cudaDeviceGetAttribute(&s->num_sm, cudaDevAttrMultiProcessorCount, s->ctx->device));
   s->h_prob_row0.assign(s->nprob + 1, 0);
-  std::vector<int32_t> sp, r0, r1, b0(s->nprob), nb(s->nprob), rowp((size_t)s->ndofs);
-  std::vector<int> nseg(s->nprob);
-  int64_t total = 0;
+  std::vector<int32_t> rowp((size_t)s->ndofs);
+  size_t all = 0;
   for (int P = 0; P < s->nprob; ++P) {
     s->h_prob_row0[P] = m->prob_face0[P] * s->nt;
     s->h_prob_row0[P + 1] = m->prob_face0[P + 1] * s->nt;
-    const int rows = std::max(s->h_prob_row0[P + 1] - s->h_prob_row0[P], 1);
-    nseg[P] = (rows + SEG_ROWS - 1) / SEG_ROWS;
-    total += nseg[P];
+    all += std::max(s->h_prob_row0[P + 1] - s->h_prob_row0[P], 1) / 1024 + 1;
+    for (int r = s->h_prob_row0[P]; r < s->h_prob_row0[P + 1]; ++r) rowp[r] = P;
   }
-  // Far beyond one wave of resident blocks (4 to an SM in the FP64 iteration, 6 in the FP32 one), a wave of longer
-  // segments: a block spends 3 us on its reduction whatever its rows.  An iteration, us, segments of 1024 rows / 608
-  // segments / 912: multigrid, 3.15 M rows of p = 3 473 / 436 / 460, 1.44 M of p = 2 332 / 318 / 333; FP64 Jacobi, 3.15 M rows
-  // 220 / 178 / 224; FP32 Jacobi 133 / 143 / 120.
-  if (total > 8 * NUM_SM) {
-    const int64_t wave = (s->precision == HDG_PREC_MIXED ? 6 : 4) * NUM_SM;
-    total = 0;
-    for (int P = 0; P < s->nprob; ++P) {
-      const int64_t rows = s->h_prob_row0[P + 1] - s->h_prob_row0[P];
-      nseg[P] = (int)std::max<int64_t>(1, rows * wave / s->ndofs);
-      total += nseg[P];
-    }
-  }
-  if (total >= NUM_SM) {
-    int64_t extra = (NUM_SM - total % NUM_SM) % NUM_SM;
-    std::vector<int> order(s->nprob);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
-      return s->h_prob_row0[x + 1] - s->h_prob_row0[x] > s->h_prob_row0[y + 1] - s->h_prob_row0[y];
-    });
-    for (size_t k = 0; extra > 0; k = (k + 1) % order.size(), --extra) ++nseg[order[k]];
-  }
-  for (int P = 0; P < s->nprob; ++P) {
-    const int a = s->h_prob_row0[P], e = s->h_prob_row0[P + 1];
-    const int rows = std::max(e - a, 1);
-    const int n = std::min(nseg[P], rows);
-    const int per = (rows + n - 1) / n;
-    b0[P] = (int32_t)sp.size();
-    nb[P] = n;
-    for (int k = 0; k < n; ++k) {
-      sp.push_back(P);
-      r0.push_back(std::min(e, a + k * per));
-      r1.push_back(std::min(e, a + (k + 1) * per));
-    }
-    for (int r = a; r < e; ++r) rowp[r] = P;
-  }
-  s->nseg = (int)sp.size();
-  s->h_seg_prob = sp;
-  s->h_seg_row0 = r0;
-  s->h_seg_row1 = r1;
-  s->h_prob_blk0 = b0;
-  s->h_prob_nblk = nb;
+  // segments of 1024 rows and the extra ones; beyond 8 to an SM only where a wave is too few for the problems
+  s->seg_room = all + s->num_sm;
+  if (s->nprob <= 4 * s->num_sm) s->seg_room = std::min(s->seg_room, (size_t)9 * s->num_sm);
+  SegCut c = cut_segments(s, nullptr, false);
+  put_segments(s, c, &s->seg, s->ctx->stream);
+  s->seg.full = std::move(c);
   cudaStream_t st = s->ctx->stream;
-  s->d_seg_prob.upload(sp.data(), sp.size(), st);
-  s->d_seg_row0.upload(r0.data(), r0.size(), st);
-  s->d_seg_row1.upload(r1.data(), r1.size(), st);
-  s->d_prob_blk0.upload(b0.data(), b0.size(), st);
-  s->d_prob_nblk.upload(nb.data(), nb.size(), st);
   s->d_row_prob.upload(rowp.data(), rowp.size(), st);
   s->ensure_reduction_buffers();
   HDG_CUDA(cudaStreamSynchronize(st));
@@ -365,9 +406,9 @@ void dirichlet_scatter(hdg_system* s, const std::vector<int32_t>& dofs0, const s
 template <int NT> void apply_t(hdg_system* s, cudaStream_t st) {
   hdg_mesh* m = s->space->mesh;
   const int nrow = m->nf * NT;
-  const SegArgs g{s->d_seg_prob.p, s->d_seg_row0.p, s->d_seg_row1.p, s->d_prob_blk0.p, s->d_prob_nblk.p, s->d_part.p,
-                  s->d_cnt.p};
-  k_meandiag<NT><<<s->nseg, 256, 0, st>>>(g, s->d_prob_row0.p, m->nf, s->d_kdiag.p, s->d_val.p, s->d_mdiag.p);
+  const SegTable& t = s->seg;
+  const SegArgs g{t.d_prob.p, t.d_row0.p, t.d_row1.p, t.d_blk0.p, t.d_nblk.p, s->d_part.p, s->d_cnt.p};
+  k_meandiag<NT><<<t.nseg, 256, 0, st>>>(g, s->d_prob_row0.p, m->nf, s->d_kdiag.p, s->d_val.p, s->d_mdiag.p);
   HDG_CUDA(cudaGetLastError());
   if (s->dir_lift) {
     k_lift<NT><<<(nrow + 255) / 256, 256, 0, st>>>(m->nf, s->d_bcol5.p, s->d_val.p, s->d_gv.p, s->d_b.p);
