@@ -75,10 +75,9 @@ void destroy_cg(CgState* c) { delete c; }
 
 namespace {
 
-// (A v)_row over the block-ELL layout: 5 block slots, values slot-major and row-contiguous.  The values, read once an
-// iteration, are loaded as data to be replaced first: what the rest of the iteration reads again stays in L2 (multigrid
-// iterations of 493 k rows of p = 4 and 591 k of p = 2: 177 -> 169 and 129 -> 121.5 us).
-template <int NT, typename T, typename V>
+// (A v)_row over the block-ELL layout: 5 block slots, values slot-major and row-contiguous.  STREAM: the values are loaded as
+// data to be replaced first (stream_matrix).
+template <int NT, bool STREAM, typename T, typename V>
 __device__ __forceinline__ double row_dot(const int32_t* __restrict__ bcol5, int nf, const T* __restrict__ val, int row,
                                           const V* __restrict__ v) {
   const int f = row / NT;
@@ -90,7 +89,10 @@ __device__ __forceinline__ double row_dot(const int32_t* __restrict__ bcol5, int
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
 #pragma unroll
-    for (int j = 0; j < NT; ++j) acc += __ldcs(val + (k * NT + j) * ndofs + row) * (T)__ldg(v + g[k] * NT + j);
+    for (int j = 0; j < NT; ++j) {
+      const T* at = val + (k * NT + j) * ndofs + row;
+      acc += (STREAM ? __ldcs(at) : __ldg(at)) * (T)__ldg(v + g[k] * NT + j);
+    }
   }
   return (double)acc;
 }
@@ -131,13 +133,13 @@ template <int NT, typename T> __global__ void __launch_bounds__(CG_BLOCK) k_cg_i
 }
 
 // The rows base, base + CG_BLOCK, ... (ROWS of them, in flight together) of k_cg_a
-template <int NT, typename T, int ROWS>
+template <int NT, typename T, bool STREAM, int ROWS>
 __device__ __forceinline__ void cg_a_rows(const CgArgs<T>& a, int base, int r1, double beta, double& pq) {
   double w[ROWS];
 #pragma unroll
   for (int u = 0; u < ROWS; ++u) {
     const int row = min(base + u * CG_BLOCK, r1 - 1);
-    w[u] = row_dot<NT>(a.bcol5, a.nf, a.val, row, a.z);
+    w[u] = row_dot<NT, STREAM>(a.bcol5, a.nf, a.val, row, a.z);
   }
   T qo[ROWS], po[ROWS], zo[ROWS];
 #pragma unroll
@@ -163,7 +165,8 @@ __device__ __forceinline__ void cg_a_rows(const CgArgs<T>& a, int base, int r1, 
 // FP64 product kernel with the q recurrence (p, q in place).  The FP64 pipe bounds it, and a warp with no row left in
 // the last of its four takes it as long as any other: so a warp does only as many as it has (segments of 811 rows, 493 k
 // rows of p = 4: an iteration 180.5 us with four always, 177.3 now).
-template <int NT, typename T> __global__ void __launch_bounds__(CG_BLOCK, cg_min_blocks<T>()) k_cg_a(CgArgs<T> a) {
+template <int NT, typename T, bool STREAM>
+__global__ void __launch_bounds__(CG_BLOCK, cg_min_blocks<T>()) k_cg_a(CgArgs<T> a) {
   const int P = a.g.seg_prob[blockIdx.x];
   // status and beta are loaded together (one round trip); beta is formed once by the reducing
   // block of the update kernel
@@ -175,10 +178,10 @@ template <int NT, typename T> __global__ void __launch_bounds__(CG_BLOCK, cg_min
   const int lane = threadIdx.x & 31;
   for (int base = r0 + threadIdx.x; base - lane < r1; base += 4 * CG_BLOCK) {
     const int left = r1 - (base - lane);  // of the warp
-    if (left > 3 * CG_BLOCK) cg_a_rows<NT, T, 4>(a, base, r1, beta, pq);
-    else if (left > 2 * CG_BLOCK) cg_a_rows<NT, T, 3>(a, base, r1, beta, pq);
-    else if (left > CG_BLOCK) cg_a_rows<NT, T, 2>(a, base, r1, beta, pq);
-    else cg_a_rows<NT, T, 1>(a, base, r1, beta, pq);
+    if (left > 3 * CG_BLOCK) cg_a_rows<NT, T, STREAM, 4>(a, base, r1, beta, pq);
+    else if (left > 2 * CG_BLOCK) cg_a_rows<NT, T, STREAM, 3>(a, base, r1, beta, pq);
+    else if (left > CG_BLOCK) cg_a_rows<NT, T, STREAM, 2>(a, base, r1, beta, pq);
+    else cg_a_rows<NT, T, STREAM, 1>(a, base, r1, beta, pq);
   }
   double s0;
   if (seg_finish1<CG_BLOCK>(a.g, P, 0, pq, &s0) && threadIdx.x == 0) {
@@ -450,7 +453,7 @@ __global__ void __launch_bounds__(CG_BLOCK) k_cg_residual(CgArgs<T> a, const dou
   const bool move_p = replace && a.p2 != a.p && a.sc[SC * P + 9] != 0.0;
   double rz = 0.0, rr = 0.0;
   for (int row = a.g.seg_row0[blockIdx.x] + threadIdx.x; row < a.g.seg_row1[blockIdx.x]; row += CG_BLOCK) {
-    const double rv = a.b[row] - row_dot<NT>(a.bcol5, a.nf, val64, row, a.x);
+    const double rv = a.b[row] - row_dot<NT, false>(a.bcol5, a.nf, val64, row, a.x);
     rr += rv * rv;
     if (replace && r32) {
       a.r[row] = (T)rv;
@@ -541,9 +544,24 @@ template <int NT> struct SolverNT : CgSolver {
     return SegArgs{tab->d_prob.p, tab->d_row0.p, tab->d_row1.p, tab->d_blk0.p, tab->d_nblk.p, s->d_part.p, s->d_cnt.p};
   }
 
+  // Whether the FP64 matrix, read once an iteration, is loaded as data to be replaced first, so that what the rest of the
+  // iteration reads again stays in L2: where it takes half of the L2 itself, a quarter beside a V-cycle's data.  Below that
+  // it is in L2 from one iteration to the next, also with other systems' beside it (four bins of 20 problems of 8^2 to
+  // 64^2 squares, Jacobi: kept 45.3 ms, streamed 50.8).  Solves, kept / streamed: Jacobi, p = 2 50 MB 170.2 / 170.8 ms, 60
+  // 227 / 235, 70 279 / 266, 85 436 / 396, p = 4 60 MB 79.1 / 83.6, 70 114.2 / 116.6, 85 131.2 / 125.0, 160 418 / 354;
+  // multigrid, p = 2 20 MB 10.46 / 10.63, 35 13.22 / 12.95, 50 15.3 / 14.4, 85 24.3 / 23.8, p = 4 20 MB 6.66 / 6.83, 35
+  // 8.11 / 8.17, 50 9.47 / 9.15, 85 12.15 / 11.51.
+  bool stream_matrix() const {
+    return sizeof(double) * hdg_system::SLOTS * NT * (size_t)nrow > (mg ? size_t(32) << 20 : size_t(64) << 20);
+  }
+  void product(const CgArgs<double>& a, cudaStream_t stream) {
+    if (stream_matrix()) k_cg_a<NT, double, true><<<tab->nseg, CG_BLOCK, 0, stream>>>(a);
+    else k_cg_a<NT, double, false><<<tab->nseg, CG_BLOCK, 0, stream>>>(a);
+  }
+
   template <typename T> void launch_pair(const CgArgs<T>& a, cudaStream_t stream, int it) {
     if constexpr (sizeof(T) == sizeof(double)) {
-      k_cg_a<NT, T><<<tab->nseg, CG_BLOCK, 0, stream>>>(a);
+      product(a, stream);
       if (mg) {
         k_cg_b_mg<NT><<<tab->nseg, CG_BLOCK, 0, stream>>>(a, c->r32.p);
         amg_apply(s, c->r32.p, c->z32.p, c->st.p, stream);
@@ -702,7 +720,7 @@ template <int NT> struct SolverNT : CgSolver {
         EventPair* ea = new EventPair();
         EventPair* eb = new EventPair();
         ea->start(st);
-        if constexpr (sizeof(T) == sizeof(double)) k_cg_a<NT, T><<<tab->nseg, CG_BLOCK, 0, st>>>(a);
+        if constexpr (sizeof(T) == sizeof(double)) product(a, st);
         else k_cg_a_fresh<NT, T><<<tab->nseg, CG_BLOCK, 0, st>>>(a, it & 1);
         ea->stop(st);
         eb->start(st);
