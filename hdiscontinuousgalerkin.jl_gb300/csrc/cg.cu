@@ -24,6 +24,7 @@
 // FP32 the product is recomputed every iteration (no q recurrence, whose rounding would
 // accumulate), with p alternating between two buffers.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <thread>
@@ -528,6 +529,7 @@ template <int NT> struct SolverNT : CgSolver {
   // every chunk: iteration counts at the previous read-back.
   std::vector<int32_t> sample_it0, it_prev;
   bool sample_pending = false;
+  bool chunk_resident = false;  // the last chunk was a launch of the resident iteration
 
   explicit SolverNT(hdg_system* s_) {
     s = s_;
@@ -539,6 +541,13 @@ template <int NT> struct SolverNT : CgSolver {
   }
 
   void set_stream(cudaStream_t stream) override { st = stream; }
+
+  double grid_weight(const hdg_solver& o) override {
+    if (nprob != 1 || o.preconditioner == HDG_PRECOND_AMG) return 0.0;
+    const CgResident pl = o.precision == HDG_PREC_MIXED ? cg_resident_plan<float>(NT, s->nf, s->ctx->device, true)
+                                                        : cg_resident_plan<double>(NT, s->nf, s->ctx->device, true);
+    return pl.kind == CgResident::GRID ? std::sqrt((double)s->nf) : 0.0;
+  }
 
   SegArgs seg() const {
     return SegArgs{tab->d_prob.p, tab->d_row0.p, tab->d_row1.p, tab->d_blk0.p, tab->d_nblk.p, s->d_part.p, s->d_cnt.p};
@@ -645,8 +654,8 @@ template <int NT> struct SolverNT : CgSolver {
     HDG_CUDA(cudaMemcpyAsync(c->st.p, c->h_st, sizeof(int32_t) * ST * nprob, cudaMemcpyHostToDevice, st));
     res = CgResident{};
     if (!mg && nprob == 1)
-      res = mixed ? cg_resident_plan<float>(NT, s->nf, s->ctx->device)
-                  : cg_resident_plan<double>(NT, s->nf, s->ctx->device);
+      res = mixed ? cg_resident_plan<float>(NT, s->nf, s->ctx->device, grid_allowed)
+                  : cg_resident_plan<double>(NT, s->nf, s->ctx->device, grid_allowed);
     if (res.kind != CgResident::NONE) {
       c->sync.alloc(CG_SYNC_BYTES);
       if (mixed) c->pairs.alloc(2 * (size_t)nrow);
@@ -699,8 +708,14 @@ template <int NT> struct SolverNT : CgSolver {
     c->outer.assign(nprob, 0);
   }
 
-  template <typename T> void chunk_t(const CgArgs<T>& a, cudaGraphExec_t graph, int rep) {
-    if (res.kind != CgResident::NONE) {
+  // The state between chunks is the same whichever form made them.  A grid beside other solves starves them, or waits for
+  // theirs: 12 flights of one request of 64^2 squares 226 ms by grids, 95 launched, three threads with a 64^2 solve each 99
+  // and 56.
+  template <typename T> void chunk_t(const CgArgs<T>& a, cudaGraphExec_t* graph, int* graph_chunk, int rep) {
+    const bool crowded = res.kind == CgResident::GRID && !res.forced && SolvesUnderWay::on(s->ctx->device) > own;
+    if (crowded) build_graph<T>(a, graph, graph_chunk);
+    chunk_resident = res.kind != CgResident::NONE && !crowded;
+    if (chunk_resident) {
       // one launch per chunk; a chunk's end costs a host round trip (about 20 us), so it is long
       EventPair* ep = s->ctx->profiling ? new EventPair() : nullptr;
       if (ep) ep->start(st);
@@ -743,14 +758,14 @@ template <int NT> struct SolverNT : CgSolver {
       }
       HDG_CUDA(cudaGetLastError());
     } else {
-      HDG_CUDA(cudaGraphLaunch(graph, st));
+      HDG_CUDA(cudaGraphLaunch(*graph, st));
     }
     s->ctx->launches += (int64_t)chunk * (mg ? 3 + amg_cycle_launches(s) : 2);
   }
 
   void launch_chunk(int rep) override {
-    if (mixed) chunk_t<float>(a32, c->graph32, rep);
-    else chunk_t<double>(a64, c->graph64, rep);
+    if (mixed) chunk_t<float>(a32, &c->graph32, &c->chunk32, rep);
+    else chunk_t<double>(a64, &c->graph64, &c->chunk64, rep);
   }
 
   void enqueue_status_copy() override {
@@ -824,7 +839,7 @@ template <int NT> struct SolverNT : CgSolver {
     double rows_all = 0.0;
     for (int P = 0; P < nprob; ++P) {
       const int32_t now = c->h_st[ST * P + 1];
-      if (!s->ev_res.empty()) s->prof_res_iters += now - it_prev[P];
+      if (chunk_resident && !s->ev_res.empty()) s->prof_res_iters += now - it_prev[P];
       rows_all += (double)(now - it_prev[P]) * (double)(s->h_prob_row0[P + 1] - s->h_prob_row0[P]);
       it_prev[P] = now;
     }
@@ -951,6 +966,33 @@ template <int NT> struct SolverNT : CgSolver {
 
 }  // namespace
 
+namespace {
+std::atomic<int> g_under_way[64];
+
+// Which of the systems solved together may take the whole chip, while no other solve is under way (SolverNT::chunk_t).  Their
+// grids run one after the other, at about half a launched iteration's time each, where launched iterations overlap: so all
+// may while the sum of their work is at most 1.5 times the largest, and none beyond that.  Grids / launched, ms, batches of
+// one problem a degree: 4 of 96^2 squares FP64 152 / 118, mixed 128 / 112, 4 of 64^2 77 / 55 and 72 / 61, 128^2 of p = 4 and 32^2 of
+// p = 3 106 / 137 and 78 / 127, 40^2 of p = 4, 128^2 of p = 1 and 24^2 of p = 2 50 / 52 and 44 / 61.
+void grid_turns(const std::vector<CgSolver*>& sv, const hdg_solver& o) {
+  double sum = 0.0, top = 0.0;
+  if (sv.size() > 1)
+    for (CgSolver* c : sv) {
+      const double w = c->grid_weight(o);
+      sum += w;
+      top = std::max(top, w);
+    }
+  for (CgSolver* c : sv) {
+    c->grid_allowed = sum <= 1.5 * top;
+    c->own = (int)sv.size();
+  }
+}
+}  // namespace
+
+SolvesUnderWay::SolvesUnderWay(int device_, int count_) : device(device_), count(count_) { g_under_way[device & 63] += count; }
+SolvesUnderWay::~SolvesUnderWay() { g_under_way[device & 63] -= count; }
+int SolvesUnderWay::on(int device) { return g_under_way[device & 63]; }
+
 CgSolver* make_cg_solver(hdg_system* s) {
   switch (s->nt) {
     case 2: return new SolverNT<2>(s);
@@ -976,6 +1018,8 @@ int run_batch_step(const std::vector<hdg_system*>& sys, const hdg_solver& o, int
   if (o.preconditioner == HDG_PRECOND_AMG)
     for (auto* s : sys)
       if (!s->amg) amg_setup_symbolic(s, s->h_dir_face);
+  SolvesUnderWay under_way(sys[0]->ctx->device, (int)sv.size());
+  grid_turns(sv, o);
   // Several systems (degree bins) run on streams of their own, forked from and joined back to
   // the context's stream: one system's assembly, reduction tails, chunk boundaries and recovery
   // overlap the other systems' iterations.

@@ -17,6 +17,8 @@
 //            hardware's (0.24 us at 16 CTAs), but only 16 SMs' FP64 pipes work on the rows;
 //   grid     a cooperative launch of one CTA per SM: partials go through L2 and the barrier is a counter (1.3 us at
 //            152 CTAs), which pays once the rows' arithmetic on 16 SMs costs more.
+// A grid has the chip to itself (others of the process wait for it: res_launch), so it is for a solve that is alone: grid_turns
+// in cg.cu.
 // A counter barrier gives up after SPIN_LIMIT polls (seconds) and reports CG_LOST instead of waiting for ever.
 //
 // What bounds it: the FP64 pipe issues a warp instruction per 16 clocks whatever its active lanes, with 64 clocks of
@@ -297,7 +299,7 @@ template <int NT, typename T, bool MAT> int max_clusters(int ctas, size_t smem) 
 // 30.8k rows 18.0 / 15.8 ms.
 template <typename T> constexpr int cluster_rows() { return sizeof(T) == sizeof(double) ? 11000 : 20000; }
 
-template <int NT, typename T> CgResident plan_nt(int nf, int device) {
+template <int NT, typename T> CgResident plan_nt(int nf, int device, bool grid_allowed) {
   CgResident pl;
   const int forced = res_forced_kind();
   if (forced == CgResident::NONE) return pl;
@@ -311,12 +313,13 @@ template <int NT, typename T> CgResident plan_nt(int nf, int device) {
       return CgResident{CgResident::CLUSTER, c, fpc, mat != 0, sm};
     }
   }
+  if (!grid_allowed && forced != CgResident::GRID) return pl;
   int sms = 0;
   if ((sms = res_grid_ctas(device)) == 0) return pl;
   const int fpc = (nf + sms - 1) / sms;
   for (int mat = 1; mat >= 0; --mat) {
     const size_t sm = res_smem<NT, T>(fpc, mat);
-    if (sm <= SMEM_MAX) return CgResident{CgResident::GRID, sms, fpc, mat != 0, sm};
+    if (sm <= SMEM_MAX) return CgResident{CgResident::GRID, sms, fpc, mat != 0, sm, forced == CgResident::GRID};
   }
   return pl;  // the vectors do not fit on the chip
 }
@@ -342,12 +345,12 @@ void launch_nt(const CgResident& pl, const CgArgs<T>& a, float2* pairs, void* sy
 
 }  // namespace
 
-template <typename T> CgResident cg_resident_plan(int nt, int nf, int device) {
+template <typename T> CgResident cg_resident_plan(int nt, int nf, int device, bool grid_allowed) {
   switch (nt) {
-    case 2: return plan_nt<2, T>(nf, device);
-    case 3: return plan_nt<3, T>(nf, device);
-    case 4: return plan_nt<4, T>(nf, device);
-    case 5: return plan_nt<5, T>(nf, device);
+    case 2: return plan_nt<2, T>(nf, device, grid_allowed);
+    case 3: return plan_nt<3, T>(nf, device, grid_allowed);
+    case 4: return plan_nt<4, T>(nf, device, grid_allowed);
+    case 5: return plan_nt<5, T>(nf, device, grid_allowed);
   }
   return CgResident{};
 }
@@ -363,8 +366,8 @@ void cg_resident_launch(const CgResident& pl, int nt, const CgArgs<T>& a, float2
   }
 }
 
-template CgResident cg_resident_plan<double>(int, int, int);
-template CgResident cg_resident_plan<float>(int, int, int);
+template CgResident cg_resident_plan<double>(int, int, int, bool);
+template CgResident cg_resident_plan<float>(int, int, int, bool);
 template void cg_resident_launch<double>(const CgResident&, int, const CgArgs<double>&, float2*, void*, int, int,
                                          cudaStream_t);
 template void cg_resident_launch<float>(const CgResident&, int, const CgArgs<float>&, float2*, void*, int, int,

@@ -32,12 +32,13 @@ struct CgResident {
   int ctas = 0, faces_per_cta = 0;
   bool mat_smem = false;  // the CTA's matrix rows are kept in shared memory
   size_t smem = 0;
+  bool forced = false;  // by HDG_CG_RESIDENT
 };
-// The plan of a system with one problem (NONE where its state does not fit), and one launch of at
-// most `iters` iterations of it.  `sync`: CG_SYNC_BYTES of device memory for the barriers; `pairs`: 2 x
+// The plan of a system with one problem (NONE where its state does not fit, or only a grid's would and that is not
+// allowed), and one launch of at most `iters` iterations of it.  `sync`: CG_SYNC_BYTES of device memory for the barriers; `pairs`: 2 x
 // rows (z, p) pairs of the FP32 iteration.
 constexpr size_t CG_SYNC_BYTES = 16384;
-template <typename T> CgResident cg_resident_plan(int nt, int nf, int device);
+template <typename T> CgResident cg_resident_plan(int nt, int nf, int device, bool grid_allowed);
 template <typename T>
 void cg_resident_launch(const CgResident& pl, int nt, const CgArgs<T>& a, float2* pairs, void* sync, int iters,
                         int device, cudaStream_t st);

@@ -418,9 +418,25 @@ SegTable& segments_of(hdg_system* s, bool fp32);
 SegCut cut_segments(const hdg_system* s, const char* on, bool fp32);
 void put_segments(hdg_system* s, const SegCut& c, SegTable* t, cudaStream_t st);
 
+// Counts the solves under way on a device in this process: while it lives, `count` more.
+struct SolvesUnderWay {
+  int device, count;
+  SolvesUnderWay(int device, int count);
+  ~SolvesUnderWay();
+  SolvesUnderWay(const SolvesUnderWay&) = delete;
+  SolvesUnderWay& operator=(const SolvesUnderWay&) = delete;
+  static int on(int device);
+};
+
 // The CG of one system, driven chunk by chunk by a host loop (run_solve_many, the serving engine).
 struct CgSolver {
   virtual ~CgSolver() {}
+  // prepare() may choose the form that takes the whole chip (CgResident::GRID), whose chunks then take it while no more
+  // than `own` solves are under way on the device; and what the form would weigh: the square root of the system's faces, as
+  // its iterations go, or 0 where it would not be chosen anyway
+  bool grid_allowed = true;
+  int own = 1;
+  virtual double grid_weight(const hdg_solver& o) = 0;
   virtual void prepare(const hdg_solver& o) = 0;      // allocate, initialise, capture the chunk graph
   virtual void launch_chunk(int rep) = 0;             // enqueue one chunk of iterations
   virtual void enqueue_status_copy() = 0;             // enqueue the per-problem status read-back

@@ -618,7 +618,7 @@ void lag_plan(hdg_lagrange* L) {
         L->d_sync.alloc(CG_SYNC_BYTES);
         HDG_CUDA(cudaStreamSynchronize(st));
         L->slots = slots;
-        L->res = CgResident{kind, ctas, 0, mat, smem};
+        L->res = CgResident{kind, ctas, 0, mat, smem, forced == kind};
         return;
       }
     }
@@ -901,7 +901,10 @@ int hdg_lagrange_solve(hdg_lagrange* L, const hdg_solver* opts, double* u, hdg_s
     cudaStream_t st = L->ctx->stream;
     const int n = L->ndofs;
     double sc[8];
-    if (L->res.kind != CgResident::NONE) {
+    // a grid would have the chip to itself: beside other solves the launched iteration (SolverNT::chunk_t in cg.cu)
+    SolvesUnderWay under_way(L->ctx->device, 1);
+    const bool alone = SolvesUnderWay::on(L->ctx->device) == 1 || L->res.forced;
+    if (L->res.kind == CgResident::CLUSTER || (L->res.kind == CgResident::GRID && alone)) {
       if (lag_solve_resident(L, tol, maxit, sc) == CG_LOST)
         throw HdgError{HDG_ERR_CUDA, "a barrier of the resident CG iteration gave up"};
     } else {

@@ -74,6 +74,7 @@ struct Flight {
   int rep = 0;
   size_t bytes = 0;
   cudaEvent_t ready = nullptr;  // recorded after each chunk's status read-back
+  std::unique_ptr<SolvesUnderWay> under_way;
   double t[5] = {0, 0, 0, 0, 0};  // build time: concat, space, assemble, apply, prepare
   ~Flight() {
     if (ready) cudaEventDestroy(ready);
@@ -103,6 +104,7 @@ struct ResidentSys {
   int rep = 0;
   size_t bytes = 0;
   std::vector<Request> reqs;  // the request being served (one)
+  std::unique_ptr<SolvesUnderWay> under_way;
   double* h_x = nullptr;      // page-locked destinations of the solution downloads
   double* h_qu = nullptr;
   explicit ResidentSys(int device) {
@@ -254,6 +256,7 @@ Flight* launch_flight(hdg_engine* e, std::vector<Request>&& reqs, int slot) {
   t0 = now_s();
   fl->t[3] += t0 - t1;
   g_alloc_stream = c->stream;
+  fl->under_way.reset(new SolvesUnderWay(c->device, 1));
   fl->cg = make_cg_solver(fl->sys);
   fl->cg->prepare(e->solver);
   HDG_CUDA(cudaEventCreateWithFlags(&fl->ready, cudaEventDisableTiming));
@@ -289,6 +292,7 @@ void build_resident(hdg_engine* e, ResidentSys* rs, std::vector<Request>&& reqs)
   g_alloc_stream = c->stream;
   HDG_CUDA(cudaMallocHost(&rs->h_x, sizeof(double) * rs->sys->ndofs));
   HDG_CUDA(cudaMallocHost(&rs->h_qu, sizeof(double) * (size_t)rs->sys->nc * rs->sys->n));
+  rs->under_way.reset(new SolvesUnderWay(c->device, 1));
   rs->cg = make_cg_solver(rs->sys);
   rs->cg->prepare(e->solver);
   rs->reqs = std::move(reqs);
@@ -309,6 +313,7 @@ void start_resident(hdg_engine* e, ResidentSys* rs, Request&& r) {
   assemble_async(s, st);
   launch_dirichlet_apply(s, st);
   s->applied = true;
+  if (!rs->under_way) rs->under_way.reset(new SolvesUnderWay(rs->ctx.device, 1));
   rs->cg->prepare(e->solver);
   rs->reqs.clear();
   rs->reqs.push_back(std::move(r));
@@ -684,6 +689,7 @@ int hdg_engine_step(hdg_engine* e, int* n_inflight, int* n_pending) {
             }
             HDG_CUDA(cudaEventRecord(rs->ready, rs->ctx.stream));
             rs->completing = true;
+            rs->under_way.reset();
             e->t_complete += now_s() - tc;
             ++i;
             continue;
