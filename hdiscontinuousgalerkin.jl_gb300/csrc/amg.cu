@@ -49,6 +49,7 @@
 #include <cuda_fp16.h>
 
 #include "hdg_device.cuh"
+#include "once_per_device.h"
 
 namespace {
 
@@ -2142,11 +2143,10 @@ template <int NT> void numeric_nt(hdg_system* s, const float* val0, cudaStream_t
   }
   const AmgLevel& C = H->lev.back();
   const size_t smem = sizeof(float) * ((size_t)H->cmax * 2 * H->cmax + H->cmax);
-  static bool attr = false;
-  if (!attr) {
+  static OncePerDevice once;
+  once(s->ctx->device, [] {
     HDG_CUDA(cudaFuncSetAttribute(k_amg_coarse_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attr = true;
-  }
+  });
   if (H->cmax > 0)
     k_amg_coarse_inv<<<s->nprob, 1024, smem, st>>>(H->crow0.p, H->coff.p, C.ptr.p, C.col.p, C.val.p, H->cinv.p);
   s->ctx->launches++;

@@ -32,6 +32,7 @@
 
 #include "cg_resident.cuh"
 #include "cg_sync.cuh"
+#include "once_per_device.h"
 
 namespace {
 
@@ -279,17 +280,17 @@ template <int NT, typename T> size_t res_smem(int fpc, bool mat) {
   return sizeof(T) * (size_t)fpc * NT * (vec + (mat ? 5 * NT : 0)) + sizeof(int32_t) * 5 * (size_t)fpc;
 }
 
-template <int NT, typename T, bool GRID, bool MAT> void set_attributes() {
-  static std::once_flag once;
-  std::call_once(once, [] {
+template <int NT, typename T, bool GRID, bool MAT> void set_attributes(int device) {
+  static OncePerDevice once;
+  once(device, [] {
     auto* k = k_cg_resident<NT, T, GRID, MAT>;
     HDG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
     if (!GRID) HDG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   });
 }
 
-template <int NT, typename T, bool MAT> int max_clusters(int ctas, size_t smem) {
-  set_attributes<NT, T, false, MAT>();
+template <int NT, typename T, bool MAT> int max_clusters(int ctas, size_t smem, int device) {
+  set_attributes<NT, T, false, MAT>(device);
   return res_max_clusters(k_cg_resident<NT, T, false, MAT>, ctas, smem);
 }
 
@@ -309,7 +310,7 @@ template <int NT, typename T> CgResident plan_nt(int nf, int device, bool grid_a
     for (int mat = 1; mat >= 0; --mat) {
       const size_t sm = res_smem<NT, T>(fpc, mat);
       if (sm > SMEM_MAX) continue;
-      if ((mat ? max_clusters<NT, T, true>(c, sm) : max_clusters<NT, T, false>(c, sm)) < 1) continue;
+      if ((mat ? max_clusters<NT, T, true>(c, sm, device) : max_clusters<NT, T, false>(c, sm, device)) < 1) continue;
       return CgResident{CgResident::CLUSTER, c, fpc, mat != 0, sm};
     }
   }
@@ -326,7 +327,7 @@ template <int NT, typename T> CgResident plan_nt(int nf, int device, bool grid_a
 
 template <int NT, typename T, bool GRID, bool MAT>
 void launch_one(const CgResident& pl, ResArgs<T> q, int device, cudaStream_t st) {
-  set_attributes<NT, T, GRID, MAT>();
+  set_attributes<NT, T, GRID, MAT>(device);
   if (GRID) HDG_CUDA(cudaMemsetAsync(q.count, 0, sizeof(unsigned), st));
   res_launch<GRID>(k_cg_resident<NT, T, GRID, MAT>, pl.ctas, pl.smem, q, device, st);
 }
