@@ -457,7 +457,7 @@ extern "C++" void populate_pages(void* p, size_t bytes) {
 #endif
 }
 
-extern "C++" void ensure_fixed_fields(hdg_system* s) {
+extern "C++" void ensure_fixed_fields(hdg_system* s, bool wait) {
   const std::vector<double>& xy = s->space->mesh->prob_xy_max;
   const int np = s->nprob;
   // magnitudes beyond which a product of the evaluation could leave FP64's range: the plain form
@@ -474,24 +474,24 @@ extern "C++" void ensure_fixed_fields(hdg_system* s) {
     sc[P] = usable[P] ? 61 - top : 0;
     scale[P] = std::ldexp(1.0, sc[P]);
   }
-  cudaStream_t st = s->ctx->stream;
-  auto make = [&](const std::vector<FieldSpec>& v, DevBuf<int32_t>* dk, DevBuf<int32_t>* doff, DevBuf<double>* dp) {
-    std::vector<int32_t> kind(v.size()), off(v.size());
-    std::vector<double> prm;
-    for (size_t P = 0; P < v.size(); ++P) {
-      const size_t at = prm.size();
-      off[P] = (int32_t)at;
-      prm.insert(prm.end(), v[P].prm.begin(), v[P].prm.end());
-      kind[P] = prepare_fixed(v[P], sc[P], ex[P], usable[P], prm.data() + at);
+  std::vector<double> all(scale);
+  std::vector<int32_t> ints;
+  for (auto* v : {&s->fsp, &s->ksp}) {
+    std::vector<int32_t> off(np);
+    for (int P = 0; P < np; ++P) {
+      const FieldSpec& f = (*v)[P];
+      const size_t at = all.size();
+      off[P] = (int32_t)(at - np);
+      all.insert(all.end(), f.prm.begin(), f.prm.end());
+      ints.push_back(prepare_fixed(f, sc[P], ex[P], usable[P], all.data() + at));
     }
-    dk->upload(kind.data(), kind.size(), st);
-    doff->upload(off.data(), off.size(), st);
-    dp->upload(prm.data(), prm.size(), st);
-    HDG_CUDA(cudaStreamSynchronize(st));  // the host vectors go out of scope
-  };
-  s->d_fix_scale.upload(scale.data(), scale.size(), st);
-  make(s->fsp, &s->d_fkfix, &s->d_fofix, &s->d_ffix);
-  make(s->ksp, &s->d_kkfix, &s->d_kofix, &s->d_kfix);
+    ints.insert(ints.end(), off.begin(), off.end());
+  }
+  s->fix_ints = all.size();
+  all.resize(all.size() + (ints.size() + 1) / 2);
+  std::memcpy(&all[s->fix_ints], ints.data(), ints.size() * sizeof(int32_t));
+  s->d_fix.upload(all.data(), all.size(), s->ctx->stream);
+  if (wait) HDG_CUDA(cudaStreamSynchronize(s->ctx->stream));
   s->fix_exp = ex;
 }
 
@@ -547,7 +547,7 @@ static void set_coefficients_many(hdg_system* s, const double* taus, const hdg_f
       if (!(kappa_cell[c] > 0.0)) throw HdgError{HDG_ERR_ARG, "kappa must be positive"};
     s->d_kappa.upload(kappa_cell, (size_t)s->nc, st);
   }
-  ensure_fixed_fields(s);
+  ensure_fixed_fields(s, false);
   HDG_CUDA(cudaStreamSynchronize(st));  // the host staging vectors go out of scope
 }
 

@@ -806,7 +806,10 @@ template <int NT> struct SolverNT : CgSolver {
     if (!all)
       for (int P = 0; P < nprob; ++P) on[P] = c->h_st[ST * P] == 0;
     const int before = tab->nseg;
-    put_segments(s, all ? tab->full : cut_segments(s, on.data(), mixed), tab, st);
+    SegCut cut;
+    if (!all) cut = cut_segments(s, on.data(), mixed);
+    put_segments(s, all ? tab->full : cut, tab, st);
+    HDG_CUDA(cudaStreamSynchronize(st));
     if (tab->nseg != before) {
       if (mixed) { c->chunk32 = 0; build_graph<float>(a32, &c->graph32, &c->chunk32); }
       else { c->chunk64 = 0; build_graph<double>(a64, &c->graph64, &c->chunk64); }

@@ -1099,7 +1099,7 @@ ElemArgs element_args(hdg_system* s) {
   a.ref = sp->d_ref.p;
   a.nq = sp->t.nq;
   a.nc = m->nc;
-  ensure_fixed_fields(s);
+  ensure_fixed_fields(s, true);
   a.co = s->coef_dev();
   a.kappa_mode = s->kappa_cells ? 1 : (s->kappa_field ? 2 : 0);
   a.he_tau = s->he_tau ? 1 : 0;

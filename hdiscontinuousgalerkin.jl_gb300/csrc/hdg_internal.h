@@ -296,8 +296,8 @@ struct hdg_system {
   int num_sm = 152;
   CoefDev coef_dev() const {
     return CoefDev{space->mesh->d_cell_prob.p, d_fkind.p, d_foff.p, d_fprm.p, d_kkind.p, d_koff.p, d_kprm.p,
-                   d_tau.p, d_fprep.p, d_fkfix.p, d_fofix.p, d_ffix.p, d_kkfix.p, d_kofix.p,
-                   d_kfix.p, d_fix_scale.p};
+                   d_tau.p, d_fprep.p, fix_int(0), fix_int(1), d_fix.p + nprob, fix_int(2), fix_int(3),
+                   d_fix.p + nprob, d_fix.p};
   }
   // per-cell condensed blocks: AB = [Ate | bte] (m x (m+1)), KB = [K_e | b_e] (n x (m+1)), or,
   // after the Schur element path (kb_u_only), only its u rows [X_u | b_u] (nw x (m+1)), with the rows of the two
@@ -308,9 +308,13 @@ struct hdg_system {
   DevBuf<double> d_kappa;  // per-cell kappa (optional)
   DevBuf<double> d_fprm, d_kprm;
   DevBuf<double> d_fprep;  // d_fprm prepared for the pivoted element kernel (CoefDev::fprep)
-  DevBuf<double> d_ffix, d_kfix, d_fix_scale;  // fields in fixed point (CoefDev::ffix), made for the mesh's coordinates
-  DevBuf<int32_t> d_fkfix, d_fofix, d_kkfix, d_kofix;
-  std::vector<int> fix_exp;  // ... below 2^fix_exp[P] in problem P (coordinate_exponent); empty: not made yet
+  // fields in fixed point (CoefDev::ffix), made for the mesh's coordinates below 2^fix_exp[P] in problem P
+  // (coordinate_exponent; empty: not made yet): scales, parameters of source and kappa, and as integers the kinds and
+  // offsets of either
+  DevBuf<double> d_fix;
+  size_t fix_ints = 0;  // where the integers begin
+  std::vector<int> fix_exp;
+  const int32_t* fix_int(int k) const { return reinterpret_cast<const int32_t*>(d_fix.p + fix_ints) + (size_t)k * nprob; }
   FieldSpec f, kappa;
   bool kappa_field = false, kappa_cells = false;
   // Trace matrix.  Host: block rows sorted by face id (h_browptr/h_bcol, the export pattern).
@@ -388,9 +392,9 @@ constexpr int HDG_CG_ST = 4;
 
 // ------------------------------------------------------------------ kernel launchers
 void launch_element_condense(hdg_system* s, cudaStream_t st);
-// The fields' fixed-point form for the mesh's present coordinates (made anew when their magnitude has changed; uploads
-// on the context's stream).
-void ensure_fixed_fields(hdg_system* s);
+// The fields' fixed-point form for the mesh's present coordinates (made anew when their magnitude has changed; uploaded
+// on the context's stream, and waited for there unless the caller does).
+void ensure_fixed_fields(hdg_system* s, bool wait);
 void launch_gather(hdg_system* s, cudaStream_t st);
 void launch_apply_dirichlet(hdg_system* s, const std::vector<int32_t>& dofs0, const std::vector<double>& vals,
                             cudaStream_t st);  // scatter + apply
@@ -413,8 +417,8 @@ int run_solve_many(const std::vector<hdg_system*>& sys, const hdg_solver& o,
 void build_segments(hdg_system* s);
 // The segments of an iteration: the system's, or those of the FP32 iteration.
 SegTable& segments_of(hdg_system* s, bool fp32);
-// The cut of the problems that on[P] names (NULL: all), and a cut's copy into a table (host arrays are read before the
-// return).
+// The cut of the problems that on[P] names (NULL: all), and a cut's copy into a table (the caller keeps c until it has
+// waited for the stream).
 SegCut cut_segments(const hdg_system* s, const char* on, bool fp32);
 void put_segments(hdg_system* s, const SegCut& c, SegTable* t, cudaStream_t st);
 

@@ -539,6 +539,31 @@ template <bool GRID, bool MAT> __global__ void __launch_bounds__(RB, 1) k_lag_re
   if (threadIdx.x == 0 && (blockIdx.x == 0 || status == CG_LOST)) a.sc[4] = status;
 }
 
+// The entries of a slot's row (column and place in the CSC values) in its slice, and its diagonal's place, a thread a slot.
+// Slots and entries without a row or value read a column that is there, times zero.
+__global__ void k_lag_layout(int64_t n, const int32_t* __restrict__ srow, const int64_t* __restrict__ sptr,
+                             const int32_t* __restrict__ colptr, const int32_t* __restrict__ rowval,
+                             int32_t* __restrict__ scol, int32_t* __restrict__ ssrc, int32_t* __restrict__ sdiag) {
+  const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (g >= n) return;
+  const int i = srow[g];
+  int64_t k = sptr[g / 32] + g % 32;
+  const int64_t end = sptr[g / 32 + 1];
+  int diag = -1;
+  if (i >= 0)
+    for (int e = colptr[i]; e < colptr[i + 1]; ++e, k += 32) {
+      const int c = rowval[e];
+      scol[k] = c;
+      ssrc[k] = e;
+      if (c == i) diag = e;
+    }
+  for (; k < end; k += 32) {
+    scol[k] = max(i, 0);
+    ssrc[k] = -1;
+  }
+  sdiag[g] = diag;
+}
+
 __global__ void k_lag_slices(int64_t n, const int32_t* __restrict__ src, const double* __restrict__ val,
                              double* __restrict__ out) {
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
@@ -570,20 +595,23 @@ void lag_plan(hdg_lagrange* L) {
     if (ctas > 0) {
       const int per = (n + ctas - 1) / ctas, slots = (per + 31) / 32 * 32;
       // rows of every CTA by length (longest first, rows of one length in order), slices as long as their longest row
-      std::vector<int32_t> srow((size_t)ctas * slots, -1), order;
+      std::vector<int32_t> srow((size_t)ctas * slots, -1), at;
       std::vector<int64_t> sptr(1, 0);
       int64_t most = 0;
       auto len = [&](int i) { return L->h_colptr[i + 1] - L->h_colptr[i]; };
+      int longest = 0;
+      for (int i = 0; i < n; ++i) longest = std::max(longest, len(i));
       for (int c = 0; c < ctas; ++c) {
         const int r0 = std::min(n, c * per), r1 = std::min(n, r0 + per);
-        order.resize(r1 - r0);
-        for (int i = r0; i < r1; ++i) order[i - r0] = i;
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return len(x) > len(y); });
-        std::copy(order.begin(), order.end(), srow.begin() + (size_t)c * slots);
-        const int64_t at = sptr.back();
+        int32_t* to = srow.data() + (size_t)c * slots;
+        at.assign(longest + 2, 0);  // at[longest - length + 1]: rows of that length, then the place of its first
+        for (int i = r0; i < r1; ++i) ++at[longest - len(i) + 1];
+        for (int l = 0; l <= longest; ++l) at[l + 1] += at[l];
+        for (int i = r0; i < r1; ++i) to[at[longest - len(i)]++] = i;
+        const int64_t first = sptr.back();
         for (int s = 0; s < slots; s += 32)
-          sptr.push_back(sptr.back() + 32 * (int64_t)(s < r1 - r0 ? len(order[s]) : 0));
-        most = std::max(most, sptr.back() - at);
+          sptr.push_back(sptr.back() + 32 * (int64_t)(s < r1 - r0 ? len(to[s]) : 0));
+        most = std::max(most, sptr.back() - first);
       }
       const bool small = lag_smem(slots, 0) <= SMEM_MAX, mat = lag_smem(slots, most) <= SMEM_MAX;
       const size_t smem = lag_smem(slots, mat ? most : 0);
@@ -595,26 +623,18 @@ void lag_plan(hdg_lagrange* L) {
                     : res_max_clusters(k_lag_resident<false, false>, ctas, smem)) >= 1;
       }
       if (fits) {
-        std::vector<int32_t> scol((size_t)sptr.back(), 0), ssrc((size_t)sptr.back(), -1), sdiag(srow.size(), -1);
-        for (size_t g = 0; g < srow.size(); ++g) {
-          const int64_t base = sptr[g / 32] + (int64_t)(g % 32), end = sptr[g / 32 + 1];
-          const int i = srow[g];
-          int64_t k = base;
-          if (i >= 0)
-            for (int e = L->h_colptr[i]; e < L->h_colptr[i + 1]; ++e, k += 32) {
-              scol[k] = L->h_rowval[e];
-              ssrc[k] = e;
-              if (L->h_rowval[e] == i) sdiag[g] = e;
-            }
-          for (; k < end; k += 32) scol[k] = i >= 0 ? i : 0;  // padding: zero times a value that is there
-        }
         cudaStream_t st = L->ctx->stream;
+        const size_t entries = (size_t)sptr.back();
         L->d_srow.upload(srow.data(), srow.size(), st);
-        L->d_sdiag.upload(sdiag.data(), sdiag.size(), st);
         L->d_sptr.upload(sptr.data(), sptr.size(), st);
-        L->d_scol.upload(scol.data(), scol.size(), st);
-        L->d_ssrc.upload(ssrc.data(), ssrc.size(), st);
-        L->d_sval.alloc(scol.size());
+        L->d_sdiag.alloc(srow.size());
+        L->d_scol.alloc(entries);
+        L->d_ssrc.alloc(entries);
+        L->d_sval.alloc(entries);
+        k_lag_layout<<<nblk((int64_t)srow.size()), 256, 0, st>>>((int64_t)srow.size(), L->d_srow.p, L->d_sptr.p, L->d_colptr.p,
+                                                                 L->d_rowval.p, L->d_scol.p, L->d_ssrc.p, L->d_sdiag.p);
+        HDG_CUDA(cudaGetLastError());
+        L->ctx->launches++;
         L->d_sync.alloc(CG_SYNC_BYTES);
         HDG_CUDA(cudaStreamSynchronize(st));
         L->slots = slots;

@@ -188,6 +188,56 @@ void gauss_legendre(int n, std::vector<double>& x, std::vector<double>& w) {
 // reference edges of the triangle (src/shapes.jl:19-23): 1: (1,0)->(0,1), 2: (0,1)->(0,0), 3: (0,0)->(1,0)
 const double EDGE[3][4] = {{1, 0, 0, 1}, {0, 1, 0, 0}, {0, 0, 1, 0}};
 
+// A number as an unevaluated sum of two doubles, good to some 104 bits (Dekker 1971; Knuth's two-sum, the product's error by
+// a fused multiply-add): the tables' products are rounded once, to double.  (long double is software where it has 128
+// bits, 40 ns an operation: the tables of p = 4 took 2.4 ms.)
+struct Wide {
+  double hi = 0.0, lo = 0.0;
+  Wide() = default;
+  Wide(double v) : hi(v) {}
+  Wide(double h, double l) : hi(h + l), lo(l - (hi - h)) {}  // |h| >= |l|
+  explicit operator double() const { return hi; }
+  friend Wide operator+(const Wide& a, const Wide& b) {
+    const double s = a.hi + b.hi, v = s - a.hi, e = (a.hi - (s - v)) + (b.hi - v);
+    const double t = a.lo + b.lo, w = t - a.lo, f = (a.lo - (t - w)) + (b.lo - w);
+    const Wide r(s, e + t);
+    return Wide(r.hi, r.lo + f);
+  }
+  friend Wide operator-(const Wide& a) {
+    Wide r;
+    r.hi = -a.hi;
+    r.lo = -a.lo;
+    return r;
+  }
+  friend Wide operator-(const Wide& a, const Wide& b) { return a + -b; }
+  friend Wide operator*(const Wide& a, const Wide& b) {
+    const double p = a.hi * b.hi;
+    return Wide(p, std::fma(a.hi, b.hi, -p) + (a.hi * b.lo + a.lo * b.hi));
+  }
+  friend Wide operator/(const Wide& a, const Wide& b) {
+    const double q = a.hi / b.hi;
+    const Wide r = a - b * q;
+    const double q1 = r.hi / b.hi;
+    return Wide(q, q1) + (r - b * q1).hi / b.hi;
+  }
+  Wide& operator+=(const Wide& o) { return *this = *this + o; }
+  Wide& operator-=(const Wide& o) { return *this = *this - o; }
+  Wide& operator/=(const Wide& o) { return *this = *this / o; }
+  friend bool operator<(const Wide& a, const Wide& b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
+  friend bool operator>(const Wide& a, const Wide& b) { return b < a; }
+  friend bool operator<=(const Wide& a, const Wide& b) { return !(b < a); }
+  friend bool operator>=(const Wide& a, const Wide& b) { return !(a < b); }
+  friend bool operator==(const Wide& a, const Wide& b) { return a.hi == b.hi && a.lo == b.lo; }
+};
+Wide mag(const Wide& a) { return a.hi < 0.0 ? -a : a; }
+double mag(double a) { return std::fabs(a); }
+double root(double a) { return std::sqrt(a); }
+Wide root(const Wide& a) {  // one Newton step on the double's
+  if (!(a.hi > 0.0)) return Wide(std::sqrt(a.hi));
+  const double x = std::sqrt(a.hi);
+  return Wide(x, (a - Wide(x) * Wide(x)).hi / (2.0 * x));
+}
+
 // Cyclic Jacobi rotations of the symmetric a (n x n) until its off-diagonal entries are below tol of its norm or the
 // sweeps are done; the columns of vec turn along.
 template <typename R> void jacobi_sweeps(int n, R tol, int sweeps, std::vector<R>& a, std::vector<R>& vec) {
@@ -201,8 +251,8 @@ template <typename R> void jacobi_sweeps(int n, R tol, int sweeps, std::vector<R
         const R apq = a[(size_t)p * n + q];
         if (apq * apq <= R(1e-4) * tol * tol * all) continue;
         const R th = (a[(size_t)q * n + q] - a[(size_t)p * n + p]) / (2 * apq);
-        const R t = (th >= 0 ? 1 : -1) / (std::fabs(th) + std::sqrt(th * th + 1));
-        const R c = 1 / std::sqrt(t * t + 1), s = t * c;
+        const R t = (th >= 0 ? 1 : -1) / (mag(th) + root(th * th + 1));
+        const R c = 1 / root(t * t + 1), s = t * c;
         for (int k = 0; k < n; ++k) {
           const R x = a[(size_t)k * n + p], y = a[(size_t)k * n + q];
           a[(size_t)k * n + p] = c * x - s * y;
@@ -222,26 +272,26 @@ template <typename R> void jacobi_sweeps(int n, R tol, int sweeps, std::vector<R
   }
 }
 
-// Eigenvalues and eigenvectors (columns) of a small symmetric matrix in long double: rotations in double first (long
-// double is software where it has 128 bits: all sweeps in it took 2 ms), their product made orthogonal to long double, and
+// Eigenvalues and eigenvectors (columns) of a small symmetric matrix in Wide: rotations in double first, their product made
+// orthogonal to Wide, and
 // what the matrix still has off its diagonal in that basis rotated away.
-void symmetric_eigen(int n, const double* m, std::vector<long double>* lam, std::vector<long double>* vec) {
+void symmetric_eigen(int n, const double* m, std::vector<Wide>* lam, std::vector<Wide>* vec) {
   std::vector<double> ad(m, m + (size_t)n * n), vd((size_t)n * n, 0.0);
   for (int i = 0; i < n; ++i) vd[(size_t)i * n + i] = 1.0;
   jacobi_sweeps<double>(n, 1e-15, 30, ad, vd);
-  auto mul = [n](const std::vector<long double>& x, bool xt, const std::vector<long double>& y) {
-    std::vector<long double> r((size_t)n * n, 0.0L);
+  auto mul = [n](const std::vector<Wide>& x, bool xt, const std::vector<Wide>& y) {
+    std::vector<Wide> r((size_t)n * n, 0.0);
     for (int i = 0; i < n; ++i)
       for (int j = 0; j < n; ++j)
         for (int k = 0; k < n; ++k) r[(size_t)i * n + j] += x[xt ? (size_t)k * n + i : (size_t)i * n + k] * y[(size_t)k * n + j];
     return r;
   };
-  std::vector<long double> v(vd.begin(), vd.end()), g = mul(v, true, v);  // V (3 I - V'V) / 2
+  std::vector<Wide> v(vd.begin(), vd.end()), g = mul(v, true, v);  // V (3 I - V'V) / 2
   for (int i = 0; i < n; ++i)
-    for (int j = 0; j < n; ++j) g[(size_t)i * n + j] = 0.5L * ((i == j ? 3.0L : 0.0L) - g[(size_t)i * n + j]);
+    for (int j = 0; j < n; ++j) g[(size_t)i * n + j] = 0.5 * ((i == j ? 3.0 : 0.0) - g[(size_t)i * n + j]);
   *vec = mul(v, false, g);
-  std::vector<long double> a = mul(*vec, true, mul(std::vector<long double>(m, m + (size_t)n * n), false, *vec));
-  jacobi_sweeps<long double>(n, 1e-18L, 30, a, *vec);
+  std::vector<Wide> a = mul(*vec, true, mul(std::vector<Wide>(m, m + (size_t)n * n), false, *vec));
+  jacobi_sweeps<Wide>(n, 1e-18, 30, a, *vec);
   lam->resize(n);
   for (int i = 0; i < n; ++i) (*lam)[i] = a[(size_t)i * n + i];
 }
@@ -393,31 +443,31 @@ bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
   // S, [S Z; Z' 0] with Z = [D_l' z] (the rows z' (Be u - Ee u_hat) = 0 of the local system).  Other rank-deficient
   // rules keep the full LU.
   if (condensation) {
-    std::vector<long double> a((size_t)nw * 2 * nw, 0.0L);
+    std::vector<Wide> a((size_t)nw * 2 * nw, 0.0);
     for (int i = 0; i < nw; ++i) {
       for (int j = 0; j < nw; ++j) a[(size_t)i * 2 * nw + j] = P[L.M + i * nw + j];
-      a[(size_t)i * 2 * nw + nw + i] = 1.0L;
+      a[(size_t)i * 2 * nw + nw + i] = 1.0;
     }
-    long double maxpiv = 0.0L, minpiv = 1e300L;
+    Wide maxpiv = 0.0, minpiv = 1e300;
     bool ok = true;
     for (int c = 0; c < nw && ok; ++c) {
       int piv = c;
       for (int i = c + 1; i < nw; ++i)
-        if (std::fabs(a[(size_t)i * 2 * nw + c]) > std::fabs(a[(size_t)piv * 2 * nw + c])) piv = i;
+        if (mag(a[(size_t)i * 2 * nw + c]) > mag(a[(size_t)piv * 2 * nw + c])) piv = i;
       if (piv != c)
         for (int j = 0; j < 2 * nw; ++j) std::swap(a[(size_t)c * 2 * nw + j], a[(size_t)piv * 2 * nw + j]);
-      const long double d = a[(size_t)c * 2 * nw + c];
-      maxpiv = std::max(maxpiv, std::fabs(d));
-      minpiv = std::min(minpiv, std::fabs(d));
-      if (d == 0.0L) { ok = false; break; }
+      const Wide d = a[(size_t)c * 2 * nw + c];
+      maxpiv = std::max(maxpiv, mag(d));
+      minpiv = std::min(minpiv, mag(d));
+      if (d == 0.0) { ok = false; break; }
       for (int j = 0; j < 2 * nw; ++j) a[(size_t)c * 2 * nw + j] /= d;
       for (int i = 0; i < nw; ++i) {
         if (i == c) continue;
-        const long double m = a[(size_t)i * 2 * nw + c];
+        const Wide m = a[(size_t)i * 2 * nw + c];
         for (int j = 0; j < 2 * nw; ++j) a[(size_t)i * 2 * nw + j] -= m * a[(size_t)c * 2 * nw + j];
       }
     }
-    t->schur = ok && minpiv > 1e-10L * maxpiv;
+    t->schur = ok && minpiv > 1e-10 * maxpiv;
     t->positive = std::all_of(t->qw.begin(), t->qw.end(), [](double w) { return w > 0.0; });
     // Be 1 = Ee 1 and Ce 1 = Fe 1 on the reference triangle (outward normals times edge lengths (1,1), (-1,0), (0,-1)); the
     // first function of either basis is the constant
@@ -439,27 +489,27 @@ bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
       }
       t->unit = off <= 1e-12 * std::max(top, 1.0);
     }
-    std::vector<long double> inv((size_t)nw * nw, 0.0L), range((size_t)nw * nw, 0.0L);  // range: V, nr columns
+    std::vector<Wide> inv((size_t)nw * nw, 0.0), range((size_t)nw * nw, 0.0);  // range: V, nr columns
     int nr = nw;
-    for (int i = 0; i < nw; ++i) range[(size_t)i * nw + i] = 1.0L;
+    for (int i = 0; i < nw; ++i) range[(size_t)i * nw + i] = 1.0;
     if (t->schur) {
       for (int i = 0; i < nw; ++i)
         for (int j = 0; j < nw; ++j) inv[(size_t)i * nw + j] = a[(size_t)i * 2 * nw + nw + j];
     } else if (p == 2) {
-      std::vector<long double> lam, vec;
+      std::vector<Wide> lam, vec;
       symmetric_eigen(nw, &P[L.M], &lam, &vec);
       int nul = 0, iz = 0;
-      long double top = 0.0L, low = 1e300L;
-      for (long double v : lam) top = std::max(top, std::fabs(v));
+      Wide top = 0.0, low = 1e300;
+      for (Wide v : lam) top = std::max(top, mag(v));
       for (int k = 0; k < nw; ++k) {
-        if (std::fabs(lam[k]) <= 1e-12L * top) {
+        if (mag(lam[k]) <= 1e-12 * top) {
           ++nul;
           iz = k;
         } else {
           low = std::min(low, lam[k]);
         }
       }
-      if (nul == 1 && low > 1e-6L * top) {
+      if (nul == 1 && low > 1e-6 * top) {
         t->schur = true;
         t->nullity = 1;
         nr = 0;
@@ -476,13 +526,13 @@ bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
         for (int i = 0; i < nw; ++i) P[L.ZV + i] = (double)vec[(size_t)i * nw + iz];
         for (int l = 0; l < 2; ++l)
           for (int j = 0; j < nw; ++j) {
-            long double s = 0;
+            Wide s = 0;
             for (int i = 0; i < nw; ++i) s += vec[(size_t)i * nw + iz] * P[(l ? L.D1 : L.D0) + i * nw + j];
             P[L.ZD + l * nw + j] = (double)s;
           }
         for (int fo = 0; fo < 6; ++fo)
           for (int j = 0; j < nt; ++j) {
-            long double s = 0;
+            Wide s = 0;
             for (int i = 0; i < nw; ++i) s += vec[(size_t)i * nw + iz] * P[L.F + (fo * nw + i) * nt + j];
             P[L.ZF + fo * nt + j] = (double)s;
           }
@@ -493,7 +543,7 @@ bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
       for (int i = 0; i < nw; ++i)
         for (int k = 0; k < nr; ++k) P[L.RV + i * nr + k] = (double)V(i, k);
       for (int q = 0; q < nq; ++q) {
-        std::vector<long double> v(nr, 0.0L);
+        std::vector<Wide> v(nr, 0.0);
         for (int k = 0; k < nr; ++k)
           for (int i = 0; i < nw; ++i) v[k] += V(i, k) * t->N[(size_t)i * nq + q];
         for (int j = 0; j < nr; ++j)
@@ -502,25 +552,25 @@ bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
       for (int l = 0; l < 2; ++l)
         for (int k = 0; k < nr; ++k)
           for (int j = 0; j < nw; ++j) {
-            long double s = 0;
+            Wide s = 0;
             for (int i = 0; i < nw; ++i) s += V(i, k) * P[(l ? L.D1 : L.D0) + i * nw + j];
             P[L.RD + (l * nr + k) * nw + j] = (double)s;
           }
       for (int fo = 0; fo < 6; ++fo)
         for (int k = 0; k < nr; ++k)
           for (int j = 0; j < nt; ++j) {
-            long double s = 0;
+            Wide s = 0;
             for (int i = 0; i < nw; ++i) s += V(i, k) * P[L.F + (fo * nw + i) * nt + j];
             P[L.RF + (fo * nr + k) * nt + j] = (double)s;
           }
       auto Mi = [&](int i, int j) { return inv[(size_t)i * nw + j]; };
       const double* D[2] = {&P[L.D0], &P[L.D1]};
-      std::vector<long double> MD[2];
+      std::vector<Wide> MD[2];
       for (int l = 0; l < 2; ++l) {
-        MD[l].assign((size_t)nw * nw, 0.0L);
+        MD[l].assign((size_t)nw * nw, 0.0);
         for (int i = 0; i < nw; ++i)
           for (int j = 0; j < nw; ++j) {
-            long double s = 0;
+            Wide s = 0;
             for (int k = 0; k < nw; ++k) s += Mi(i, k) * D[l][k * nw + j];
             MD[l][(size_t)i * nw + j] = s;
             P[(l ? L.SMD1 : L.SMD0) + i * nw + j] = (double)s;
@@ -531,15 +581,15 @@ bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
       for (int q = 0; q < 3; ++q)
         for (int i = 0; i < nw; ++i)
           for (int j = 0; j < nw; ++j) {
-            long double s = 0;  // (D_l' M^-1 D_m)[i][j] = sum_k D_l[k][i] (M^-1 D_m)[k][j]
-            for (int k = 0; k < nw; ++k) s += (long double)D[QL[q][0]][k * nw + i] * MD[QL[q][1]][(size_t)k * nw + j];
+            Wide s = 0;  // (D_l' M^-1 D_m)[i][j] = sum_k D_l[k][i] (M^-1 D_m)[k][j]
+            for (int k = 0; k < nw; ++k) s += (Wide)D[QL[q][0]][k * nw + i] * MD[QL[q][1]][(size_t)k * nw + j];
             P[QO[q] + i * nw + j] = (double)s;
           }
       for (int fo = 0; fo < 6; ++fo) {
-        std::vector<long double> MF((size_t)nw * nt, 0.0L);
+        std::vector<Wide> MF((size_t)nw * nt, 0.0);
         for (int i = 0; i < nw; ++i)
           for (int j = 0; j < nt; ++j) {
-            long double s = 0;
+            Wide s = 0;
             for (int k = 0; k < nw; ++k) s += Mi(i, k) * P[L.F + (fo * nw + k) * nt + j];
             MF[(size_t)i * nt + j] = s;
             P[L.SMF + (fo * nw + i) * nt + j] = (double)s;
@@ -547,16 +597,16 @@ bool build_ref_tables(int p, int qd, RefTables* t, bool condensation) {
         for (int l = 0; l < 2; ++l)
           for (int i = 0; i < nw; ++i)
             for (int j = 0; j < nt; ++j) {
-              long double s = 0;
-              for (int k = 0; k < nw; ++k) s += (long double)D[l][k * nw + i] * MF[(size_t)k * nt + j];
+              Wide s = 0;
+              for (int k = 0; k < nw; ++k) s += (Wide)D[l][k * nw + i] * MF[(size_t)k * nt + j];
               P[L.SDMF + ((l * 6 + fo) * nw + i) * nt + j] = (double)s;
             }
         // PFF_{go,fo} = F_{go}' M^-1 F_{fo} (nt x nt), the face-face term of the condensed operator
         for (int go = 0; go < 6; ++go)
           for (int i = 0; i < nt; ++i)
             for (int j = 0; j < nt; ++j) {
-              long double s = 0;
-              for (int k = 0; k < nw; ++k) s += (long double)P[L.F + (go * nw + k) * nt + i] * MF[(size_t)k * nt + j];
+              Wide s = 0;
+              for (int k = 0; k < nw; ++k) s += (Wide)P[L.F + (go * nw + k) * nt + i] * MF[(size_t)k * nt + j];
               P[L.PFF + ((go * 6 + fo) * nt + i) * nt + j] = (double)s;
             }
       }

@@ -148,7 +148,6 @@ void put_segments(hdg_system* s, const SegCut& c, SegTable* t, cudaStream_t st) 
   put(t->d_row1, c.row1, n);
   put(t->d_blk0, c.blk0, np);
   put(t->d_nblk, c.nblk, np);
-  HDG_CUDA(cudaStreamSynchronize(st));
   t->nseg = (int)n;
 }
 
@@ -158,6 +157,7 @@ SegTable& segments_of(hdg_system* s, bool fp32) {
     SegCut c = cut_segments(s, nullptr, true);
     if (c.prob.size() != s->seg.full.prob.size()) {
       put_segments(s, c, &s->seg32, s->ctx->stream);
+      HDG_CUDA(cudaStreamSynchronize(s->ctx->stream));  // the solve's stream may be another
       s->seg32.full = std::move(c);
     }
   }
