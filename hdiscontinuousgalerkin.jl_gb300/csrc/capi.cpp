@@ -976,19 +976,29 @@ int hdg_recover_into(hdg_system* s, double* q, double* u, double* uhat_cell, int
     if (s->ctx->profiling) s->ev_recover.stop(st);
     s->have_recovery = true;
     // the three arrays are laid out on the device and copied straight to the caller's: through a host staging vector,
-    // a host loop per cell and a second copy, 2*512^2 cells of p = 3 took 36 ms
-    DevBuf<double> dq, du, dx;
-    if (q) dq.alloc((size_t)s->nc * 2 * s->nw);
-    if (u) du.alloc((size_t)s->nc * s->nw);
-    if (uhat_cell) dx.alloc((size_t)s->nc * s->m);
-    if (q || u || uhat_cell) launch_recover_split(s, dq.p, du.p, dx.p, by_function != 0, st);
-    populate_pages(q, dq.n * sizeof(double));
-    populate_pages(u, du.n * sizeof(double));
-    populate_pages(uhat_cell, dx.n * sizeof(double));
-    if (q) dq.download(q, dq.n, st);
-    if (u) du.download(u, du.n, st);
-    if (uhat_cell) dx.download(uhat_cell, dx.n, st);
-    if (q || u || uhat_cell) HDG_CUDA(cudaStreamSynchronize(st));
+    // a host loop per cell and a second copy, 2*512^2 cells of p = 3 took 36 ms.  In pieces of 32 MB, whatever the system.
+    if (q || u || uhat_cell) {
+      const size_t per_cell = sizeof(double) * ((q ? 2 * s->nw : 0) + (u ? s->nw : 0) + (uhat_cell ? s->m : 0));
+      const int piece = (int)std::min<size_t>(s->nc, std::max<size_t>(1, (size_t(32) << 20) / per_cell));
+      DevBuf<double> dq, du, dx;
+      struct Part {
+        double* to;
+        DevBuf<double>* from;
+        int width;
+      };
+      const Part parts[3] = {{q, &dq, 2 * s->nw}, {u, &du, s->nw}, {uhat_cell, &dx, s->m}};
+      for (const Part& p : parts)
+        if (p.to) p.from->alloc((size_t)piece * p.width);
+      for (int c0 = 0; c0 < s->nc; c0 += piece) {
+        const int c1 = std::min(s->nc, c0 + piece);
+        launch_recover_split(s, c0, c1, dq.p, du.p, dx.p, by_function != 0, st);
+        for (const Part& p : parts)
+          if (p.to) populate_pages(p.to + (size_t)c0 * p.width, sizeof(double) * (size_t)(c1 - c0) * p.width);
+        for (const Part& p : parts)
+          if (p.to) p.from->download(p.to + (size_t)c0 * p.width, (size_t)(c1 - c0) * p.width, st);
+      }
+      HDG_CUDA(cudaStreamSynchronize(st));
+    }
     return HDG_OK;
   });
 }

@@ -456,9 +456,10 @@ struct CgSolver {
 CgSolver* make_cg_solver(hdg_system* s);
 void mesh_concat(hdg_mesh* out, const std::vector<const hdg_mesh*>& parts);
 void launch_recover(hdg_system* s, cudaStream_t st);
-// The recovered q (ncells x nv) and u (ncells x nw) and the cells' trace values (ncells x 3 x nt, or ncells x nt x 3
-// by_function) as arrays of their own on the device; a NULL one is left out.
-void launch_recover_split(hdg_system* s, double* q, double* u, double* uhat_cell, bool by_function, cudaStream_t st);
+// The recovered q (cells x nv) and u (cells x nw) and the trace values (cells x 3 x nt, or cells x nt x 3 by_function) of the
+// cells c0 .. c1 - 1 as arrays of their own on the device; a NULL one is left out.
+void launch_recover_split(hdg_system* s, int c0, int c1, double* q, double* u, double* uhat_cell, bool by_function,
+                          cudaStream_t st);
 void run_export_csc(const hdg_system* s, int base, int64_t* colptr, int64_t* rowval, double* nzval, double* rhs,
                     cudaStream_t st);
 // The full [K_e | b_e] (ncells x n x (m+1), device) from the stored u rows (kb_u_only systems).

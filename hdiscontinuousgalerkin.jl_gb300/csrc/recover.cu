@@ -100,8 +100,8 @@ __global__ void k_recover_u(const int nc, const int32_t* __restrict__ cells, con
   }
 }
 
-// q, u and the cells' trace values out of [q; u] and u_hat, a thread per value (grid-stride); bound by HBM, and small
-// beside the copies to the host that follow.
+// q, u and the trace values of nc cells out of [q; u] and u_hat, a thread per value (grid-stride); bound by HBM, and small
+// beside the copies to the host that follow.  cfaces and qu begin at the first of the cells.
 __global__ void k_recover_split(const int64_t nc, const int nw, const int nt, const int32_t* __restrict__ cfaces,
                                 const double* __restrict__ qu, const double* __restrict__ x, double* __restrict__ q,
                                 double* __restrict__ u, double* __restrict__ uc, const bool by_function) {
@@ -293,10 +293,12 @@ void launch_recover(hdg_system* s, cudaStream_t st) {
   }
 }
 
-void launch_recover_split(hdg_system* s, double* q, double* u, double* uhat_cell, bool by_function, cudaStream_t st) {
-  const int64_t tot = (int64_t)s->nc * s->n;
+void launch_recover_split(hdg_system* s, int c0, int c1, double* q, double* u, double* uhat_cell, bool by_function,
+                          cudaStream_t st) {
+  const int64_t tot = (int64_t)(c1 - c0) * s->n;
   k_recover_split<<<(unsigned)std::min<int64_t>((tot + 255) / 256, 152 * 16), 256, 0, st>>>(
-      s->nc, s->nw, s->nt, s->space->mesh->d_cfaces.p, s->d_qu.p, s->d_x.p, q, u, uhat_cell, by_function);
+      c1 - c0, s->nw, s->nt, s->space->mesh->d_cfaces.p + 3 * (int64_t)c0, s->d_qu.p + (int64_t)c0 * s->n, s->d_x.p, q, u,
+      uhat_cell, by_function);
   HDG_CUDA(cudaGetLastError());
   s->ctx->launches++;
 }
