@@ -2,8 +2,8 @@
 //
 // With two kernels per iteration (cg.cu) a small system pays for launches, reduction tails and
 // re-read vectors, not for arithmetic.  Measured per iteration, two kernels / here (whole solves): 14.9 / 6.1 us at 6272
-// rows (p = 1, FP64), 22 / 10 us at 142k rows (p = 4, FP32), 43 / 32.5 us at 591k rows (p = 2, FP64; 27 us of it are the
-// FP64 pipe's, 23 FMAs a row).  Here every CTA owns a contiguous range of faces for the whole launch.  Its rows of x, r, p, q,
+// rows (p = 1, FP64), 22 / 10 us at 142k rows (p = 4, FP32), 43 / 32.5 us at 591k rows (p = 2, FP64; 22.7 us of it are the
+// FP64 pipe's 23 instructions a row).  Here every CTA owns a contiguous range of faces for the whole launch.  Its rows of x, r, p, q,
 // D^-1 and z stay in shared memory (and its matrix rows too, where they fit), only z travels through L2 (the
 // columns of a row belong to other CTAs), and an iteration is two phases with a reduction over all CTAs after
 // each:
